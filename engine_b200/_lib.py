@@ -104,6 +104,7 @@ SIGNATURES = {
     "hq_config_get": (_I64, [_I32]),
     "hq_convert": (_I32, [_P, _I32, _P, _I32, _I64, _P]),
     "hq_convert_status": (_I32, [_P, _I32, _P, _I32, _I64, _P, _P]),
+    "hq_gather_rows_f16": (_I32, [_P, _I32, _I64, _P, _P, _I64, _I64, _P, _P, _P]),
     "hq_probe_tensor_peak": (_I32, [_I32, _I32, _I32, _P, C.POINTER(C.c_double), _P]),
     "hq_gated_act": (_I32, [_P, _P, _I32, _I64, _I32, C.POINTER(HqActArgs), _P, _P]),
 }

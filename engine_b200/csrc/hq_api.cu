@@ -71,6 +71,7 @@ void fill_grouped(GroupedParams& g, const hq_weight* w, const hq_weight* w_up) {
   g.format = w->format;
   g.n = (int)w->n;
   g.k = (int)w->k;
+  g.n_experts = w->n_experts;
   g.w = w->data;
   g.scales = w->scales;
   g.bias = w->bias;
@@ -195,9 +196,7 @@ int32_t hq_linear_forward_ws(const hq_weight* w, const void* x, int32_t x_dtype,
     g.y = y; g.y_dtype = y_dtype; g.y_stride = y_stride;
     g.act.act = HQ_ACT_NONE;
     g.status = status_dev;
-    g.tile_rows = m >= 512 ? 256 : 128;
-    g.weights_in_tmem = w->format != HQ_FMT_FP8_BLOCK && w->format != HQ_FMT_Q8_0;
-    return launch_grouped_gemm(g, (int)((m + g.tile_rows - 1) / g.tile_rows), (cudaStream_t)stream);
+    return launch_grouped_gemm(g, m, (cudaStream_t)stream);
   }
   GemvParams p{};
   fill_weight(p, w, nullptr);
@@ -247,9 +246,7 @@ int32_t hq_linear_glu_forward(const hq_weight* w_gate, const hq_weight* w_up, co
     g.y = y; g.y_dtype = y_dtype; g.y_stride = y_stride;
     g.act = *act;
     g.status = status_dev;
-    g.tile_rows = 128;
-    g.weights_in_tmem = w_gate->format != HQ_FMT_FP8_BLOCK;
-    return launch_grouped_gemm(g, (int)((m + 127) / 128), (cudaStream_t)stream);
+    return launch_grouped_gemm(g, m, (cudaStream_t)stream);
   }
   GemvParams p{};
   fill_weight(p, w_gate, w_up);
@@ -387,22 +384,12 @@ int32_t hq_moe_gather_forward(const hq_weight* w, const hq_weight* w_up, const h
     g.x = x; g.x_dtype = x_dtype; g.x_stride = w->k;
     g.y = out; g.y_dtype = out_dtype;
     g.y_stride = (has_act && w_up == nullptr) ? w->n / 2 : w->n;
-    // 256-token tiles when experts hold enough rows on average to fill them and a single bank leaves tensor
-    // memory for two accumulator buffers
-    const bool many_rows = n_tokens * top_k >= 192 * (int64_t)w->n_experts;
-    g.tile_rows = (w_up == nullptr && many_rows) ? 256 : 128;
-    // the variant that expands the weights into tensor memory (128-token tiles): MXFP4 always, Q4_K while the
-    // experts do not fill 256-token tiles; block-FP8 and Q8_0 expand into shared memory
-    g.weights_in_tmem = w->format == HQ_FMT_MXFP4 || (w->format == HQ_FMT_Q4_K && !many_rows);
-    if (w->format == HQ_FMT_MXFP4) g.tile_rows = 128;
-    g.tiles = ws + (g.tile_rows == 256 ? l.off_tiles256 : l.off_tiles128);
-    g.tile_count = ws + (g.tile_rows == 256 ? 3 : 1);
     g.expert_bounds = expert_bounds;
     g.x_rows = x_rows;
     g.y_rows = y_rows;
     if (has_act) g.act = *act; else g.act.act = HQ_ACT_NONE;
     g.status = status_dev;
-    return launch_grouped_gemm(g, (int)(g.tile_rows == 256 ? l.max_tiles256 : l.max_tiles128), (cudaStream_t)stream);
+    return launch_grouped_gemm(g, n_tokens * top_k, (cudaStream_t)stream);
   }
   GemvParams p{};
   fill_weight(p, w, w_up);
@@ -818,6 +805,18 @@ int32_t hq_convert(const void* src, int32_t src_dtype, void* dst, int32_t dst_dt
   return hq_convert_status(src, src_dtype, dst, dst_dtype, n_elems, nullptr, stream);
 }
 
+int32_t hq_gather_rows_f16(const void* x, int32_t x_dtype, int64_t x_stride, const int32_t* row_map,
+                           const int32_t* n_valid_dev, int64_t n_rows, int64_t k, void* out, int32_t* status_dev,
+                           void* stream) {
+  if (n_rows < 0 || k < 8 || k % 8 != 0 || k > (1 << 30) || x_stride < k) return HQ_ERR_SHAPE;
+  if (n_rows == 0) return HQ_OK;
+  if (x == nullptr || row_map == nullptr || out == nullptr) return HQ_ERR_NULL;
+  if (!valid_dtype(x_dtype)) return HQ_ERR_FORMAT;
+  if (!aligned16(x) || !aligned16(out) || (x_stride * dtype_size(x_dtype)) % 16 != 0) return HQ_ERR_ALIGN;
+  return launch_gather_rows_f16(x, x_dtype, x_stride, row_map, n_valid_dev, n_rows, k, out, status_dev,
+                                (cudaStream_t)stream);
+}
+
 int32_t hq_gated_act(const void* gate, const void* up, int32_t dtype, int64_t n_elems, int32_t interleaved,
                      const hq_act_args* act, void* out, void* stream) {
   if (n_elems < 0) return HQ_ERR_SHAPE;
@@ -838,7 +837,7 @@ int32_t hq_probe_tensor_peak(int32_t kind, int32_t n, int32_t iters, int32_t* st
 namespace {
 struct MoeLayerPlan {
   int64_t t, k, e, hidden, inter, rows;
-  bool interleaved, cast_x;
+  bool interleaved, gather_x;
   int64_t off_ids, off_w, off_bounds, off_sa, off_st, off_inv, off_dws, dws_bytes, off_x16, off_h, off_y, total;
 };
 int64_t up256(int64_t v) { return (v + 255) / 256 * 256; }
@@ -858,8 +857,8 @@ int32_t plan_moe_layer(const hq_moe_layer* l, int64_t n_tokens, int32_t x_dtype,
   if (l->down->k != p.inter || l->down->n != p.hidden) return HQ_ERR_SHAPE;
   if (l->act.act == HQ_ACT_NONE) return HQ_ERR_FORMAT;
   p.rows = p.t * p.k;
-  // the tensor-core kernel copies activations as f16: cast once per token here instead of per (token, slot) there
-  p.cast_x = x_dtype != HQ_DT_F16 && p.rows >= moe_tensor_min_rows(l->gate->format) * p.e &&
+  // the tensor-core kernel takes f16 rows and copies them fastest in expert order: one pass converts and permutes
+  p.gather_x = p.rows >= moe_tensor_min_rows(l->gate->format) * p.e &&
              tensor_path_ok(l->gate, l->up, HQ_DT_F16, l->gate->k);
   int64_t o = 0;
   p.off_ids = o;    o += up256(p.rows * 4);
@@ -870,7 +869,7 @@ int32_t plan_moe_layer(const hq_moe_layer* l, int64_t n_tokens, int32_t x_dtype,
   p.off_inv = o;    o += up256(p.rows * 4);
   p.dws_bytes = hq_moe_dispatch_workspace_bytes(p.t, (int32_t)p.k, (int32_t)p.e);
   p.off_dws = o;    o += up256(p.dws_bytes);
-  p.off_x16 = o;    o += p.cast_x ? up256(p.t * p.hidden * 2) : 0;
+  p.off_x16 = o;    o += p.gather_x ? up256(p.rows * p.hidden * 2) : 0;
   p.off_h = o;      o += up256(p.rows * p.inter * 2);
   p.off_y = o;      o += up256(p.rows * p.hidden * 4);
   p.total = o;
@@ -910,15 +909,16 @@ int32_t hq_moe_layer_forward(const hq_moe_layer* layer, const void* logits, int3
   rc = hq_moe_dispatch_build(ids, n_tokens, (int32_t)p.k, (int32_t)p.e, bounds, sa, st, inv, dws, p.dws_bytes, stream);
   if (rc != HQ_OK) return rc;
   const void* xin = x;
-  int32_t xin_dtype = x_dtype;
-  if (p.cast_x) {
-    rc = hq_convert_status(x, x_dtype, ws + p.off_x16, HQ_DT_F16, n_tokens * p.hidden, status_dev, stream);
+  int32_t xin_dtype = x_dtype, xin_layout = HQ_ROWS_PER_TOKEN;
+  if (p.gather_x) {
+    rc = hq_gather_rows_f16(x, x_dtype, p.hidden, st, bounds + p.e, p.rows, p.hidden, ws + p.off_x16, status_dev, stream);
     if (rc != HQ_OK) return rc;
     xin = ws + p.off_x16;
     xin_dtype = HQ_DT_F16;
+    xin_layout = HQ_ROWS_SORTED;
   }
   void* h = ws + p.off_h;
-  rc = hq_moe_gather_forward(layer->gate, layer->up, &layer->act, xin, xin_dtype, HQ_ROWS_PER_TOKEN, n_tokens,
+  rc = hq_moe_gather_forward(layer->gate, layer->up, &layer->act, xin, xin_dtype, xin_layout, n_tokens,
                              (int32_t)p.k, bounds, sa, st, dws, h, HQ_DT_F16, HQ_ROWS_SORTED, status_dev, stream);
   if (rc != HQ_OK) return rc;
   void* y = ws + p.off_y;

@@ -1,0 +1,8 @@
+// Instances of the dequantizing GEMM (hq_dq_gemm.cuh): Q5_0 Q4_1 Q5_1.
+#include "hq_dq_launch.cuh"
+
+namespace hq {
+template int32_t launch_dq<HQ_FMT_Q5_0>(const GroupedParams&, int64_t, cudaStream_t);
+template int32_t launch_dq<HQ_FMT_Q4_1>(const GroupedParams&, int64_t, cudaStream_t);
+template int32_t launch_dq<HQ_FMT_Q5_1>(const GroupedParams&, int64_t, cudaStream_t);
+}  // namespace hq

@@ -338,6 +338,80 @@ int32_t launch_convert(const void* src, int src_dtype, void* dst, int dst_dtype,
   return cudaGetLastError() == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
 }
 
+// a finite value beyond the f16 range is clamped to +-65504 (inf / NaN pass through)
+__device__ __forceinline__ uint4 f32x8_to_f16x8(float (&v)[8], bool& clamped) {
+  uint32_t w[4];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float a = fabsf(v[j]);
+    if (a > 65504.f && a <= 3.4028235e38f) {
+      v[j] = copysignf(65504.f, v[j]);
+      clamped = true;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) w[j] = pack_half2(v[2 * j], v[2 * j + 1]);
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ uint4 bf16x8_to_f16x8(uint4 r, bool& clamped) {
+  float v[8] = {__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xFFFF0000u), __uint_as_float(r.y << 16),
+                __uint_as_float(r.y & 0xFFFF0000u), __uint_as_float(r.z << 16), __uint_as_float(r.z & 0xFFFF0000u),
+                __uint_as_float(r.w << 16), __uint_as_float(r.w & 0xFFFF0000u)};
+  return f32x8_to_f16x8(v, clamped);
+}
+
+// Rows x[row_map[r]] as f16 in the order of the map (expert-sorted rows for the dequantizing GEMM, which then copies its
+// token tiles as whole boxes instead of gathering 16-byte pieces).  Rows at or past *n_valid are left unwritten.  Bytes:
+// rows * k * 2 written; the sources are re-read through L2, once per slot of a token.
+__global__ void __launch_bounds__(256) gather_rows_f16_kernel(const void* __restrict__ x, int dtype, int64_t x_stride,
+                                                              const int32_t* __restrict__ row_map,
+                                                              const int32_t* __restrict__ n_valid, int64_t n_rows, int k8,
+                                                              uint16_t* __restrict__ out, int32_t* __restrict__ status) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // a warp per row, four 8-element chunks of it in flight per lane
+  const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= n_rows || (n_valid != nullptr && row >= (int64_t)*n_valid)) return;
+  const int64_t src = (int64_t)row_map[row] * x_stride;
+  uint16_t* const dst = out + row * ((int64_t)k8 * 8);
+  bool clamped = false;
+  for (int c0 = threadIdx.x & 31; c0 < k8; c0 += 128) {
+    if (dtype != HQ_DT_F32) {
+      uint4 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (c0 + 32 * i < k8) v[i] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(x) + src) + c0 + 32 * i);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (c0 + 32 * i < k8) {
+          if (dtype == HQ_DT_BF16) v[i] = bf16x8_to_f16x8(v[i], clamped);
+          *(reinterpret_cast<uint4*>(dst) + c0 + 32 * i) = v[i];
+        }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (c0 + 32 * i < k8) {
+          float v[8];
+          load4_as_float(x, dtype, src + 8 * (c0 + 32 * i), *reinterpret_cast<float(*)[4]>(&v[0]));
+          load4_as_float(x, dtype, src + 8 * (c0 + 32 * i) + 4, *reinterpret_cast<float(*)[4]>(&v[4]));
+          *(reinterpret_cast<uint4*>(dst) + c0 + 32 * i) = f32x8_to_f16x8(v, clamped);
+        }
+    }
+  }
+  if (clamped) report_status(status, HQ_DEV_F16_RANGE, 901);
+}
+
+int32_t launch_gather_rows_f16(const void* x, int dtype, int64_t x_stride, const int32_t* row_map, const int32_t* n_valid,
+                               int64_t n_rows, int64_t k, void* out, int32_t* status, cudaStream_t stream) {
+  if (n_rows == 0) return HQ_OK;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((n_rows + 7) / 8));
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  return cudaLaunchKernelEx(&cfg, gather_rows_f16_kernel, x, dtype, x_stride, row_map, n_valid, n_rows, (int)(k / 8),
+                            (uint16_t*)out, status) == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
+}
+
 // ---- gated activations --------------------------------------------------------------
 __device__ __forceinline__ float gated_act(float g, float u, const hq_act_args& a) {
   if (a.act == HQ_ACT_GPTOSS) {

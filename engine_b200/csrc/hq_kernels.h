@@ -42,10 +42,11 @@ int32_t launch_gemv(const GemvParams& p, int grid_y, cudaStream_t stream);
 // scratch bytes the Q8_0 / Q4_K decode kernel wants for a dense [m, k] x [n, k] call (0 = none)
 int64_t gemv_int8_workspace_bytes(int format, int64_t n, int64_t k, int64_t m);
 
-// ---- grouped expert GEMM on tcgen05 (hq_grouped_gemm.cu) -----------------------------
+// ---- dequantizing GEMM on tcgen05, dense and expert-indexed (hq_dq_gemm.cuh) -----------------------------
 struct GroupedParams {
   int format;
-  int n, k, m;                 // m: dense rows (used when tiles == nullptr)
+  int n, k, m;                 // m: dense rows (used when expert_bounds == nullptr)
+  int n_experts;
   const void* w;
   const void* w_up;            // second (up) bank for a fused gated activation, or nullptr
   const void* scales;          // MXFP4: e8m0 bytes [E, N, K/32]
@@ -66,18 +67,17 @@ struct GroupedParams {
   void* y;
   int y_dtype;
   int64_t y_stride;
-  const int32_t* tiles;         // [n_tiles][2] = (expert, first sorted row), tiles of <= tile_rows rows
-  const int32_t* tile_count;    // device word holding n_tiles
-  int tile_rows;                // 128 or 256 tokens per tile
-  bool weights_in_tmem;         // 128-token tiles only: take the kernel that expands the weights into tensor memory
-  const int32_t* expert_bounds;
+  const int32_t* expert_bounds; // [E+1] sorted rows of every expert; token tiles are cut from it inside the kernel
   const int32_t* x_rows;        // sorted row -> activation row (nullptr = identity)
   const int32_t* y_rows;        // sorted row -> output row (nullptr = identity)
   hq_act_args act;
   int32_t* status;
 };
 bool grouped_gemm_supported(int format, int64_t n, int64_t k);
-int32_t launch_grouped_gemm(const GroupedParams& p, int max_tiles, cudaStream_t stream);
+// rows: dense rows, or the number of assignments of an expert-indexed call
+int32_t launch_grouped_gemm(const GroupedParams& p, int64_t rows, cudaStream_t stream);
+template <int FMT>
+int32_t launch_dq(const GroupedParams& p, int64_t rows, cudaStream_t stream);
 int32_t launch_fp8_scale_prepare(const float* scales, int64_t n_groups, int kb, float* tile_scale, float* rel_scale,
                                  cudaStream_t stream);
 
@@ -191,6 +191,8 @@ int32_t launch_fp8_gated_quant_rows(const void* gu, int dtype, int64_t n_rows, i
                                     uint8_t* codes, float* scales, cudaStream_t stream);
 int32_t launch_convert(const void* src, int src_dtype, void* dst, int dst_dtype, int64_t n, int32_t* status,
                        cudaStream_t stream);
+int32_t launch_gather_rows_f16(const void* x, int dtype, int64_t x_stride, const int32_t* row_map, const int32_t* n_valid,
+                               int64_t n_rows, int64_t k, void* out, int32_t* status, cudaStream_t stream);
 int32_t launch_gated_act(const void* gate, const void* up, int dtype, int64_t n, int interleaved,
                          const hq_act_args& act, void* out, cudaStream_t stream);
 

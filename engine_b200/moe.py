@@ -10,7 +10,7 @@ from dataclasses import dataclass
 import torch
 
 from . import _lib as L
-from .quant import (DispatchTables, QuantMethod, _ptr, _require_cuda, _stream, convert, dt_code,
+from .quant import (DispatchTables, QuantMethod, _ptr, _require_cuda, _stream, dt_code, gather_rows_f16,
                     moe_dispatch_build, mxfp8_quantize_rows, tensor_path_expected)
 
 
@@ -132,9 +132,11 @@ class MoEExperts:
         t, k = topk_ids.shape
         tables = tables or moe_dispatch_build(topk_ids, self.n_experts)
         first = self.gate_up if self.gate_up is not None else self.gate
-        if x.dtype != torch.float16 and tensor_path_expected(first, t * k, dense=False):
-            # one cast per token instead of one conversion per (token, slot) in the kernel
-            x = convert(x, torch.float16, first._status_buf(x.device))
+        layout = L.ROWS_PER_TOKEN
+        if tensor_path_expected(first, t * k, dense=False):
+            # f16 rows in expert order: the tensor-core kernel then copies its token tiles as whole boxes
+            x = gather_rows_f16(x, tables.sorted_token, tables.expert_bounds[self.n_experts:], first._status_buf(x.device))
+            layout = L.ROWS_SORTED
         inter = first.n // 2 if self.gate_up is not None else first.n
         h = torch.empty((t * k, inter), dtype=self.inter_dtype, device=x.device)
         w0 = first._weight_struct()
@@ -143,7 +145,7 @@ class MoEExperts:
         self._last_tables = tables
         ev0 = self._mark()
         L.check(L.lib().hq_moe_gather_forward(C.byref(w0), None if w1 is None else C.byref(w1), C.byref(self.act),
-                                              _ptr(x), dt_code(x.dtype), L.ROWS_PER_TOKEN, t, k,
+                                              _ptr(x), dt_code(x.dtype), layout, t, k,
                                               _ptr(tables.expert_bounds), _ptr(tables.sorted_assign),
                                               _ptr(tables.sorted_token), _ptr(tables.workspace), _ptr(h),
                                               dt_code(h.dtype), L.ROWS_SORTED, _ptr(status), _stream()),

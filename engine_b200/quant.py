@@ -85,6 +85,17 @@ def convert(x: torch.Tensor, dtype: torch.dtype, status: torch.Tensor | None = N
     return out
 
 
+def gather_rows_f16(x: torch.Tensor, row_map: torch.Tensor, n_valid: torch.Tensor | None,
+                    status: torch.Tensor | None) -> torch.Tensor:
+    """Rows x[row_map[r]] as f16 in the order of the map (hq_gather_rows_f16): expert-sorted rows for the tensor path."""
+    x = x.contiguous()
+    k = x.shape[-1]
+    out = torch.empty((row_map.numel(), k), dtype=torch.float16, device=x.device)
+    L.check(L.lib().hq_gather_rows_f16(_ptr(x), dt_code(x.dtype), k, _ptr(row_map), _ptr(n_valid), row_map.numel(), k,
+                                       _ptr(out), _ptr(status), _stream()), "hq_gather_rows_f16")
+    return out
+
+
 def tensor_path_expected(layer, n_rows_total: int, dense: bool) -> bool:
     """Mirror of the C-side rule that sends a call to the tensor-core grouped GEMM (prefill-sized row counts,
     K % 64 == 0; Q8_0 from four times the configured row thresholds, because its decode kernel streams at HBM
@@ -92,7 +103,7 @@ def tensor_path_expected(layer, n_rows_total: int, dense: bool) -> bool:
     operand tiles without a conversion pass."""
     if layer.k % 64:
         return False
-    if layer.format == L.FMT_FP8_BLOCK and (layer.n % 128 or layer.k % 128):
+    if layer.format == L.FMT_FP8_BLOCK and layer.k % 128:
         return False
     lib = L.lib()
     mult = 4 if layer.format == L.FMT_Q8_0 else 1
@@ -217,9 +228,11 @@ class QuantMethod:
         if a.shape[0] != t or a.shape[-1] != self.k:
             raise L.HqError("gather_forward: input / indices / weight shapes disagree")
         x = a.contiguous()
-        if x.dtype != torch.float16 and tensor_path_expected(self, t * k, dense=False):
-            x = convert(x, torch.float16, self._status_buf(a.device))
         tables = tables or moe_dispatch_build(indices, self.n_experts)
+        if tensor_path_expected(self, t * k, dense=False):
+            rows = tables.sorted_token if layout == L.ROWS_PER_TOKEN else tables.sorted_assign
+            x = gather_rows_f16(x, rows, tables.expert_bounds[self.n_experts:], self._status_buf(a.device))
+            layout = L.ROWS_SORTED
         out_dtype = out_dtype or a.dtype
         out = torch.empty((t, k, self.n), dtype=out_dtype, device=a.device)
         w = self._weight_struct()

@@ -499,6 +499,13 @@ int32_t hq_convert(const void* src, int32_t src_dtype, void* dst, int32_t dst_dt
 int32_t hq_convert_status(const void* src, int32_t src_dtype, void* dst, int32_t dst_dtype, int64_t n_elems,
                           int32_t* status_dev, void* stream);
 
+/* Rows x[row_map[r]] of a [*, k] matrix as f16, out [n_rows, k] (k a multiple of 8; x rows 16-byte aligned): token rows in
+ * expert order for hq_moe_gather_forward with HQ_ROWS_SORTED, in one pass with the conversion.  Rows at or past
+ * *n_valid_dev (may be NULL) are left unwritten; values beyond the f16 range as for hq_convert_status. */
+int32_t hq_gather_rows_f16(const void* x, int32_t x_dtype, int64_t x_stride, const int32_t* row_map,
+                           const int32_t* n_valid_dev, int64_t n_rows, int64_t k, void* out, int32_t* status_dev,
+                           void* stream);
+
 /* Measurement aid, no counterpart in the reference: every SM issues iters x 4 tcgen05.mma instructions back to back
  * (M = 128, N = n, operands resident in shared memory; kind 0 = f16 x f16, K = 16 per instruction; kind 1 = e4m3 x
  * e4m3 on kind::f8f6f4, K = 32).  *flops_host receives the floating-point operations of the launch; the caller

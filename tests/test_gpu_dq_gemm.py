@@ -1,0 +1,63 @@
+"""The dequantizing GEMM at the edges of its plans: token tiles of 16 .. 256 columns (one or two accumulator buffers, two
+or four 64-k steps per stage), K slices over clusters, K tails, and weight rows whose pitch is not a multiple of 16 bytes."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+from oracle import moe as M
+from tests import hq_testlib as T
+from tests.test_gpu_linear import TOL, run_case
+
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("m", [9, 16, 17, 64, 65, 128, 129, 192, 193, 256, 257, 521])
+@pytest.mark.parametrize("fmt,n,k", [("Q4_K", 200, 1280), ("FP8", 576, 640), ("MXFP4", 130, 320)])
+def test_token_tile_edges(fmt, n, k, m):
+    # MXFP4: K = 320 ends in a stage with one 64-k step; FP8: N = 576 ends in half a 128-row scale block, K = 640 in half
+    # a 256-k stage; few features: K is cut into slices
+    got, want = run_case(fmt, n, k, m, torch.float16, torch.float32, 700 + m, bias=True)
+    assert T.rel_l2(got, want) <= TOL[fmt]
+
+
+@pytest.mark.parametrize("k", [256, 768, 2048, 4096])
+@pytest.mark.parametrize("fmt", ["Q6_K", "Q3_K", "Q2_K"])
+def test_narrow_rows_copied_as_boxes_and_in_words(fmt, k):
+    # K = 2048 and 4096: row pitch a multiple of 16 bytes, blocks at every even offset of a 16-byte unit; else words
+    got, want = run_case(fmt, 300, k, 40, torch.bfloat16, torch.float32, 720)
+    assert T.rel_l2(got, want) <= TOL[fmt]
+
+
+@pytest.mark.parametrize("m", [20, 300])
+@pytest.mark.parametrize("fmt", ["Q4_K", "Q5_1", "FP8"])
+def test_gate_and_up_bank(fmt, m):
+    import engine_b200 as hq
+    rng = T.rng_for(7, m)
+    n, k = 320, 1024
+    (ga, gd), (ua, ud) = T.make_weight(fmt, rng, n, k), T.make_weight(fmt, rng, n, k)
+    x = T.to_dev(rng.standard_normal((m, k)).astype(np.float32), torch.float16, DEV)
+    gate, up = T.make_layer(fmt, ga, k, DEV), T.make_layer(fmt, ua, k, DEV)
+    got = hq.try_fused_quantized_gate_up(x, gate, up, out_dtype=torch.float32).cpu().numpy()
+    xf = x.float().cpu().numpy()
+    want = M.swiglu(M.dense_forward(xf, gd), M.dense_forward(xf, ud))
+    assert gate.device_status()[0] == 0
+    assert T.rel_l2(got, want) <= 2e-3
+
+
+@pytest.mark.parametrize("per_expert", [9, 40, 150, 300])
+def test_expert_rows_cut_into_equal_tiles(per_expert):
+    # skewed counts: experts without rows, with a few, and with more than one tile
+    import engine_b200 as hq
+    rng = T.rng_for(8, per_expert)
+    e, n, k, topk = 4, 192, 512, 2
+    arrays, deq = T.make_weight("Q4_K", rng, n, k, experts=e)
+    t = per_expert * e // topk
+    ids = np.stack([rng.choice(e - 1, size=topk, replace=False, p=[0.7, 0.25, 0.05]) for _ in range(t)]).astype(np.int32)
+    x = T.to_dev(rng.standard_normal((t, k)).astype(np.float32), torch.bfloat16, DEV)
+    layer = T.make_layer("Q4_K", arrays, k, DEV)
+    got = layer.gather_forward_raw(x, T.to_dev(ids, torch.int32, DEV), torch.float32).cpu().numpy()
+    want = np.einsum("tk,tsnk->tsn", x.float().cpu().numpy(), deq[ids])
+    assert layer.device_status()[0] == 0
+    assert T.rel_l2(got, want) <= 1e-3
