@@ -132,6 +132,24 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native host path (csrc/hq_torch.cpp): argument checks, allocation and library calls of one forward."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _hqtorch
+        except ImportError as exc:
+            raise HqError(f"engine_b200/_hqtorch.so cannot be loaded ({exc}): run "
+                          "`python -c 'import __graft_entry__ as g; g.build()'` (there is no fallback path)") from exc
+        _hqtorch.set_error(HqError)
+        _host = _hqtorch
+    return _host
+
+
 def check(rc: int, what: str) -> None:
     if rc != 0:
         raise HqError(f"{what}: {lib().hq_error_string(rc).decode()} ({rc})")

@@ -16,6 +16,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB_PATH = os.path.join(HERE, "libhanzoquant_b200.so")
+HOST_SRC = os.path.join(CSRC, "hq_torch.cpp")
+HOST_PATH = os.path.join(HERE, "_hqtorch.so")
 PUBLIC_HEADER = os.path.join(HERE, "..", "include", "hanzoquant_b200.h")
 
 NVCC_FLAGS = [
@@ -48,7 +50,14 @@ def needs_build() -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile every .cu under csrc/ and link them into one shared library; returns its path."""
+    """Compile every .cu under csrc/ and link them into one shared library, then the host path's extension module;
+    returns the library's path."""
+    path = build_library(force, verbose)
+    build_host(force)
+    return path
+
+
+def build_library(force: bool = False, verbose: bool = False) -> str:
     if not force and not needs_build():
         return LIB_PATH
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
@@ -75,6 +84,26 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if res.returncode != 0:
         raise RuntimeError("link failed:\n" + res.stdout + res.stderr)
     return LIB_PATH
+
+
+def build_host(force: bool = False) -> str:
+    """The Python layer's host path (csrc/hq_torch.cpp) as an extension module beside the library it calls."""
+    if not force and not _stale(HOST_PATH, [HOST_SRC, PUBLIC_HEADER]):
+        return HOST_PATH
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wno-deprecated-declarations",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", HOST_SRC, "-o", HOST_PATH,
+           *[f"-I{p}" for p in cpp_extension.include_paths("cuda") + [sysconfig.get_paths()["include"]]],
+           f"-L{libs}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python",
+           f"-L{HERE}", "-l:libhanzoquant_b200.so", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed on hq_torch.cpp:\n" + res.stdout + res.stderr)
+    return HOST_PATH
 
 
 if __name__ == "__main__":

@@ -32,36 +32,13 @@ class TopKOutput:
     indices: torch.Tensor   # int32 [T, k] (bit pattern of the reference's u32 ids)
 
 
-def _router_args(e: int, config: MoeRouterTopKConfig, bias, scale) -> "L.HqRouterArgs":
-    clip = config.logit_clip
-    return L.HqRouterArgs(e, config.top_k, config.score_function, config.selected_weight, int(config.renormalize),
-                          int(clip is not None), clip[0] if clip else 0.0, clip[1] if clip else 0.0,
-                          config.norm_min, config.output_scale, 0 if bias is None else bias.data_ptr(),
-                          0 if scale is None else scale.data_ptr())
-
-
 def moe_router_topk(logits: torch.Tensor, config: MoeRouterTopKConfig, selection_bias: torch.Tensor | None = None,
                     expert_scale: torch.Tensor | None = None, n_group: int = 1, topk_group: int = 1,
                     group_score: str = "top2_sum") -> TopKOutput:
     """`n_group` > 1 adds the DeepSeek group-limited selection (hanzo-engine/src/models/deepseek3.rs:623-690):
     group_score "top2_sum" = noaux_tc, "max" = group_limited_greedy."""
-    _require_cuda(logits, "logits")
-    t, e = logits.shape
-    logits = logits.contiguous()
-    ids = torch.empty((t, config.top_k), dtype=torch.int32, device=logits.device)
-    w = torch.empty((t, config.top_k), dtype=torch.float32, device=logits.device)
-    bias = None if selection_bias is None else selection_bias.to(torch.float32).contiguous()
-    scale = None if expert_scale is None else expert_scale.to(torch.float32).contiguous()
-    args = _router_args(e, config, bias, scale)
-    if n_group > 1:
-        mode = {"top2_sum": 0, "max": 1}[group_score]
-        L.check(L.lib().hq_router_topk_grouped(_ptr(logits), dt_code(logits.dtype), t, C.byref(args), n_group,
-                                               topk_group, mode, _ptr(ids), _ptr(w), _stream()),
-                "hq_router_topk_grouped")
-    else:
-        L.check(L.lib().hq_router_topk(_ptr(logits), dt_code(logits.dtype), t, C.byref(args), _ptr(ids), _ptr(w),
-                                       _stream()), "hq_router_topk")
-    return TopKOutput(w, ids)
+    mode = 0 if n_group <= 1 else {"top2_sum": 0, "max": 1}[group_score]
+    return TopKOutput(*L.host().router(logits, config, selection_bias, expert_scale, n_group, topk_group, mode))
 
 
 def moe_router_forward(xs: torch.Tensor, router_weight: torch.Tensor, config: MoeRouterTopKConfig,
@@ -113,6 +90,10 @@ class MoEExperts:
     `gate_up_proj` [E, 2I, H] whose rows interleave gate/up (gpt-oss).  The intermediate stays expert-sorted
     between the two projections; one dispatch build serves both."""
 
+    gemm_events = None      # see _mark
+    _last_tables = None
+    _dense_bounds = None
+
     def __init__(self, down_proj: QuantMethod, gate_proj: QuantMethod | None = None, up_proj: QuantMethod | None = None,
                  gate_up_proj: QuantMethod | None = None, act: int = L.ACT_SWIGLU, limit: float | None = None,
                  alpha: float = 1.702, inter_dtype: torch.dtype = torch.float16):
@@ -120,6 +101,7 @@ class MoEExperts:
             raise L.HqError("give either gate_proj+up_proj or gate_up_proj")
         self.gate, self.up, self.gate_up, self.down = gate_proj, up_proj, gate_up_proj, down_proj
         self.act = L.HqActArgs(act, int(limit is not None), 0.0 if limit is None else limit, alpha)
+        self._act_at = C.addressof(self.act)
         self.inter_dtype = inter_dtype
         self.n_experts = down_proj.n_experts
 
@@ -178,6 +160,10 @@ class MoEExperts:
         Slots whose id is outside [0, n_experts) are skipped."""
         if self.gate is None or self.gate.format != L.FMT_FP8_BLOCK:
             raise L.HqError("forward_fp8_act needs block-FP8 experts with separate gate and up banks")
+        if tables is None and fp8_rows is None and not _skip_reduce and self.gemm_events is None:
+            self._last_tables = None
+            g, u, d = self._handles()
+            return L.host().moe_fp8(g, u, d, self._act_at, xs, topk_weights, topk_ids, shared_out, out_dtype)
         t, k = topk_ids.shape
         if fp8_rows is None:
             _require_cuda(xs, "xs")
@@ -238,6 +224,11 @@ class MoEExperts:
         banks = [first, self.down] + ([self.up] if self.up is not None else [])
         if any(b.format != L.FMT_MXFP4 or not b.mx_supported() for b in banks):
             raise L.HqError("forward_mx_act needs MXFP4 experts with K % 64 == 0")
+        if self.gate_up is not None and tables is None and not _skip_reduce and self.gemm_events is None and \
+                first.n % 64 == 0:
+            self._last_tables = None
+            g, _, d = self._handles()
+            return L.host().moe_mx(g, d, self._act_at, xs, topk_weights, topk_ids, shared_out, out_dtype)
         _require_cuda(xs, "xs")
         lead = xs.shape[:-1]
         x = xs.reshape(-1, xs.shape[-1]).contiguous()
@@ -294,38 +285,26 @@ class MoEExperts:
         _require_cuda(xs, "xs")
         if self.gate is None or self.gate.format != L.FMT_FP8_BLOCK or self.n_experts != 1:
             raise L.HqError("forward_fp8_dense needs a one-expert block-FP8 bank with separate gate and up")
-        lead = xs.shape[:-1]
-        x = xs.reshape(-1, xs.shape[-1]).contiguous()
-        t, hidden = x.shape
-        dev = x.device
-        lib = L.lib()
-        status = self.gate._status_buf(dev)
-        bounds = getattr(self, "_dense_bounds", None)
+        t, dev = xs.numel() // xs.shape[-1], xs.device
+        bounds = self._dense_bounds
         if bounds is None or bounds[1] != t or bounds[0].device != dev:
             bounds = (torch.tensor([0, t], dtype=torch.int32, device=dev), t)
             self._dense_bounds = bounds
-        xq = torch.empty((t, hidden), dtype=torch.uint8, device=dev)
-        xsc = torch.empty((t, hidden // 128), dtype=torch.float32, device=dev)
-        L.check(lib.hq_fp8_quant_rows(_ptr(x), dt_code(x.dtype), hidden, None, t, hidden, _ptr(xq), _ptr(xsc),
-                                      _stream()), "hq_fp8_quant_rows")
-        inter = self.gate.n
-        hq_ = torch.empty((t, inter), dtype=torch.uint8, device=dev)
-        hs = torch.empty((t, inter // 128), dtype=torch.float32, device=dev)
-        wg, wu, wd = self.gate._weight_struct(), self.up._weight_struct(), self.down._weight_struct()
-        L.check(lib.hq_moe_fp8_gate_up_forward(C.byref(wg), C.byref(wu), C.byref(self.act), _ptr(xq), _ptr(xsc), t, 1,
-                                               _ptr(bounds[0]), _ptr(hq_), _ptr(hs), _ptr(status), _stream()),
-                "hq_moe_fp8_gate_up_forward(shared)")
-        out_dtype = out_dtype or xs.dtype
-        y = torch.empty((t, self.down.n), dtype=out_dtype, device=dev)
-        L.check(lib.hq_fp8_linear_forward(C.byref(wd), _ptr(hq_), _ptr(hs), t, _ptr(y), dt_code(out_dtype), self.down.n,
-                                          _ptr(status), _stream()), "hq_fp8_linear_forward(shared)")
-        return y.reshape(*lead, self.down.n)
+        g, u, d = self._handles()
+        return L.host().fp8_dense(g, u, d, self._act_at, xs, bounds[0], out_dtype)
+
+    def _handles(self):
+        """(gate or gate_up, up or None, down) for the native host path."""
+        first = self.gate_up if self.gate_up is not None else self.gate
+        up = self.up
+        return (first._h or first._handle(), None if up is None else up._h or up._handle(),
+                self.down._h or self.down._handle())
 
     def _mark(self, start=None):
         """Measurement hook: with `gemm_events` set to a list, every forward appends a (start, end) CUDA event
         pair around its two expert-GEMM launches.  While the stream is being captured into a CUDA graph the
         events are created as external event nodes, so they can be read after every replay of the graph."""
-        evs = getattr(self, "gemm_events", None)
+        evs = self.gemm_events
         if evs is None:
             return None
         if torch.cuda.is_current_stream_capturing():
@@ -341,35 +320,7 @@ class MoEExperts:
                       selection_bias: torch.Tensor | None = None, expert_scale: torch.Tensor | None = None,
                       shared_out: torch.Tensor | None = None, out_dtype: torch.dtype | None = None) -> torch.Tensor:
         """Router, dispatch, both projections and the weighted sum in one library call (hq_moe_layer_forward): the
-        same kernels as moe_router_topk + forward, launched back to back without host work in between.  The
-        scratch is kept by the object and grown when a call needs more."""
-        _require_cuda(xs, "xs")
-        lead = xs.shape[:-1]
-        x = xs.reshape(-1, xs.shape[-1]).contiguous()
-        t = x.shape[0]
-        logits = logits.reshape(t, -1).contiguous()
-        out_dtype = out_dtype or xs.dtype
-        bias = None if selection_bias is None else selection_bias.to(torch.float32).contiguous()
-        scale = None if expert_scale is None else expert_scale.to(torch.float32).contiguous()
-        first = self.gate_up if self.gate_up is not None else self.gate
-        w0, wd = first._weight_struct(), self.down._weight_struct()
-        w1 = self.up._weight_struct() if self.up is not None else None
-        layer = L.HqMoeLayer(C.pointer(w0), C.pointer(w1) if w1 is not None else None, C.pointer(wd), self.act,
-                             _router_args(self.n_experts, config, bias, scale))
-        lib = L.lib()
-        need = int(lib.hq_moe_layer_workspace_bytes(C.byref(layer), t, dt_code(x.dtype)))
-        if need == 0 and t > 0:
-            raise L.HqError("hq_moe_layer_workspace_bytes: the layer description is inconsistent")
-        ws = getattr(self, "_layer_ws", None)
-        if ws is None or ws.numel() < need or ws.device != x.device:
-            ws = torch.empty(max(need, 256), dtype=torch.uint8, device=x.device)
-            self._layer_ws = ws
-        out = torch.empty((t, self.down.n), dtype=out_dtype, device=x.device)
-        add = None
-        if shared_out is not None:
-            add = shared_out.reshape(t, -1)
-            add = add.to(out_dtype).contiguous() if add.dtype != out_dtype else add.contiguous()
-        L.check(lib.hq_moe_layer_forward(C.byref(layer), _ptr(logits), dt_code(logits.dtype), _ptr(x), dt_code(x.dtype),
-                                         t, _ptr(add), _ptr(out), dt_code(out_dtype), _ptr(ws), ws.numel(),
-                                         _ptr(first._status_buf(x.device)), _stream()), "hq_moe_layer_forward")
-        return out.reshape(*lead, self.down.n)
+        same kernels as moe_router_topk + forward, launched back to back without host work in between."""
+        g, u, d = self._handles()
+        return L.host().moe_layer(g, u, d, self._act_at, xs, logits, config, selection_bias, expert_scale, shared_out,
+                                  out_dtype)

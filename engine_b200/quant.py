@@ -119,12 +119,11 @@ class QuantMethod:
     n_experts: int
     n: int
     k: int
+    bias: torch.Tensor | None = None
 
     def __init__(self):
         self._status = None
-        self._ws = {}
-        self._ws_need = {}
-        self._w_cached = None
+        self._h = None
 
     # -- plumbing -------------------------------------------------------------------
     # QuantizedSerde (hanzo-quant/src/lib.rs:911-945): layer types the reference does not serialise say so
@@ -161,52 +160,25 @@ class QuantMethod:
 
     def forward(self, a: torch.Tensor) -> torch.Tensor:
         """y = a . W^T (+ b); leading dims are flattened to rows (lib.rs:1014-1021)."""
-        return self.forward_raw(a)
+        return L.host().linear(self._h or self._handle(), a, None)
 
     def forward_raw(self, a: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
-        _require_cuda(a, "a")
-        if self.n_experts != 1:
-            raise L.HqError("forward on an expert bank: use gather_forward")
-        if a.shape[-1] != self.k:
-            raise L.HqError(f"shape mismatch: input has {a.shape[-1]} features, weight expects {self.k}")
-        lead = a.shape[:-1]
-        x = a.reshape(-1, self.k)
-        if x.stride(-1) != 1:
-            x = x.contiguous()
-        m = x.shape[0]
-        out_dtype = out_dtype or a.dtype
-        if x.dtype != torch.float16 and tensor_path_expected(self, m, dense=True):
-            # the tensor-core kernel multiplies in f16 either way (values beyond +-65504 are clamped and flagged)
-            x = convert(x if x.is_contiguous() else x.contiguous(), torch.float16, self._status_buf(a.device))
-        y = torch.empty((m, self.n), dtype=out_dtype, device=a.device)
-        # the weight descriptor never changes after construction: built once (a decode call is a few microseconds
-        # of GPU time, so host work per call matters)
-        w = self._w_cached
-        if w is None:
-            w = self._w_cached = self._weight_struct()
-        stream = torch.cuda.current_stream(a.device).cuda_stream
-        ws, ws_bytes = self._linear_workspace(w, m, a.device, stream)
-        rc = L.lib().hq_linear_forward_ws(C.byref(w), x.data_ptr(), dt_code(x.dtype), x.stride(0) if m > 1 else self.k,
-                                          y.data_ptr(), dt_code(out_dtype), self.n, m, ws, ws_bytes,
-                                          self._status_buf(a.device).data_ptr(), stream)
-        if rc != 0:
-            L.check(rc, "hq_linear_forward_ws")
-        return y.reshape(*lead, self.n)
+        """forward with a choice of the output's dtype.  From the row count of the tensor path on, bf16 / f32 rows are
+        cast to f16 first (that kernel multiplies in f16 either way; values beyond +-65504 are clamped and flagged)."""
+        return L.host().linear(self._h or self._handle(), a, out_dtype)
 
-    def _linear_workspace(self, w, m: int, device, stream: int):
-        """Scratch for hq_linear_forward_ws, owned by the layer like the reference's Q8_1 activation buffer
-        (fast_mmvq.rs:107-148): zero-filled once, grown when a call asks for more, one per CUDA stream."""
-        need = self._ws_need.get(m)
-        if need is None:
-            need = self._ws_need[m] = int(L.lib().hq_linear_workspace_bytes(C.byref(w), m))
-        if need == 0:
-            return None, 0
-        key = (device.index, stream)
-        buf = self._ws.get(key)
-        if buf is None or buf.numel() < need:
-            buf = torch.zeros(need, dtype=torch.uint8, device=device)
-            self._ws[key] = buf
-        return buf.data_ptr(), buf.numel()
+    def _handle(self):
+        """The layer for the native host path: its weight descriptor (which never changes after construction), its
+        status words and its decode scratch (zero-filled once, grown when a call asks for more, one per CUDA stream;
+        the reference's Q8_1 activation buffer, fast_mmvq.rs:107-148)."""
+        w = self._weight_struct()
+        self._h = L.host().layer(C.addressof(w), self._status_buf(self._device()))
+        return self._h
+
+    @property
+    def _ws(self) -> dict:
+        """The layer's decode scratch tensors (one per stream it has run on)."""
+        return {} if self._h is None else dict(enumerate(L.host().scratch(self._h)))
 
     def gather_forward(self, a: torch.Tensor, indices: torch.Tensor) -> torch.Tensor:
         """Per-assignment projection out of the bank (lib.rs:1032-1040): a is [T, K], [T, 1, K] (one row per
@@ -481,55 +453,32 @@ def try_fused_quantized_gate_up(xs: torch.Tensor, gate: QuantMethod, up: QuantMe
                                 out_dtype: torch.dtype | None = None) -> torch.Tensor | None:
     """act(xs . Wgate^T) * (xs . Wup^T) in one launch (hanzo-quant/src/lib.rs:1116-1160).  Returns None where the
     reference's function would (biases, mismatched layers, expert banks), so callers keep their unfused route."""
-    if getattr(gate, "bias", None) is not None or getattr(up, "bias", None) is not None:
+    if gate.bias is not None or up.bias is not None:
         return None
     if gate.format != up.format or (gate.n, gate.k) != (up.n, up.k) or gate.n_experts != 1 or up.n_experts != 1:
         return None
     if xs.shape[-1] != gate.k or xs.dtype not in _DT:
         return None
     _require_cuda(xs, "xs")
-    lead = xs.shape[:-1]
-    x = xs.reshape(-1, gate.k)
-    if x.stride(-1) != 1:
-        x = x.contiguous()
-    m = x.shape[0]
-    if m == 0:
+    if xs.numel() == 0:
         return None
-    if x.dtype != torch.float16 and tensor_path_expected(gate, m, dense=True):
-        x = convert(x.contiguous(), torch.float16, gate._status_buf(xs.device))
-    out_dtype = out_dtype or xs.dtype
-    y = torch.empty((m, gate.n), dtype=out_dtype, device=xs.device)
     a = L.HqActArgs(act, int(limit is not None), 0.0 if limit is None else limit, alpha)
-    wg, wu = gate._weight_struct(), up._weight_struct()
-    L.check(L.lib().hq_linear_glu_forward(C.byref(wg), C.byref(wu), C.byref(a), _ptr(x), dt_code(x.dtype),
-                                          x.stride(0) if m > 1 else gate.k, _ptr(y), dt_code(out_dtype), gate.n, m,
-                                          _ptr(gate._status_buf(xs.device)), _stream()), "hq_linear_glu_forward")
-    return y.reshape(*lead, gate.n)
+    return L.host().glu(gate._h or gate._handle(), up._h or up._handle(), xs, C.addressof(a), out_dtype)
 
 
 def try_fused_quantized_qkv(xs: torch.Tensor, q: QuantMethod, k: QuantMethod, v: QuantMethod,
                             out_dtype: torch.dtype | None = None):
     """The three attention projections of one activation in one call (hanzo-quant/src/lib.rs:1162-1204)."""
-    layers = (q, k, v)
-    if any(getattr(l, "bias", None) is not None for l in layers) or any(l.n_experts != 1 for l in layers):
+    if not (q.format == k.format == v.format and q.n_experts == k.n_experts == v.n_experts == 1):
         return None
-    if len({l.format for l in layers}) != 1 or any(l.k != xs.shape[-1] for l in layers) or xs.dtype not in _DT:
+    if not (q.bias is None and k.bias is None and v.bias is None) or not q.k == k.k == v.k == xs.shape[-1]:
+        return None
+    if xs.dtype not in _DT:
         return None
     _require_cuda(xs, "xs")
-    lead = xs.shape[:-1]
-    x = xs.reshape(-1, q.k).contiguous()
-    m = x.shape[0]
-    if m == 0:
+    if xs.numel() == 0:
         return None
-    if x.dtype != torch.float16 and tensor_path_expected(q, m, dense=True):
-        x = convert(x, torch.float16, q._status_buf(xs.device))
-    out_dtype = out_dtype or xs.dtype
-    outs = [torch.empty((m, l.n), dtype=out_dtype, device=xs.device) for l in layers]
-    ws = [l._weight_struct() for l in layers]
-    L.check(L.lib().hq_linear_qkv_forward(C.byref(ws[0]), C.byref(ws[1]), C.byref(ws[2]), _ptr(x), dt_code(x.dtype),
-                                          q.k, _ptr(outs[0]), _ptr(outs[1]), _ptr(outs[2]), dt_code(out_dtype), m,
-                                          _ptr(q._status_buf(xs.device)), _stream()), "hq_linear_qkv_forward")
-    return tuple(o.reshape(*lead, o.shape[-1]) for o in outs)
+    return L.host().qkv(q._h or q._handle(), k._h or k._handle(), v._h or v._handle(), xs, out_dtype)
 
 
 MAX_GEMV_BATCH_SIZE = 8
