@@ -9,17 +9,20 @@
 //
 // One persistent CTA per SM, 28 or 32 warps:
 //   warp 0       issues tcgen05.mma (A = expanded weights in tensor memory, B = tokens in shared memory)
-//   warps 1-4    epilogue: tcgen05.ld, bias, gated activation, store
-//   warps 5-6    stream the f16 activation rows (gathered: token order -> expert order) into a ring of 64-k operand tiles
-//   next 2 or 4  stream the raw weight bytes of 256 k x 128 rows into a second ring (cp.async, completion on an mbarrier)
+//   warps 1-8    epilogue, two per lane quarter: tcgen05.ld, bias, gated activation, store
+//   warp 9       raw weight bytes of 256 k x 128 rows into a second ring, as boxes
+//   warps 10-11  the f16 activation rows into a ring of operand stages of two or four 64-k tiles: boxes when the rows are
+//                in order (warp 10; warp 11 then takes every second raw stage), else gathered with cp.async
+//   warps 12-15  (types whose rows are no multiple of 16 bytes apart only) raw bytes in 4-byte pieces with cp.async
 //   last 16      expand: four groups of four warps; group c owns the 64 weights 64c .. of every 256-k stage, so where
 //                its codes, scales and bits lie inside the block is a compile-time constant.  A thread owns one weight
 //                row: it picks the bytes out of shared memory (row pitch = an odd number of 16-byte units: no bank
 //                conflicts), expands 64 weights in registers and writes them to a ring of A stages in tensor memory
 //                (tcgen05.st), so the expanded weights never pass through shared memory.
-// What bounds it: shared-memory bandwidth for wide tiles (per 64 k the MMA reads tokens x 128 bytes, the same again is
-// written by the copies, plus the raw bytes twice), the expanding warps' issue slots for narrow ones (about 3.5
-// instructions per Q4_K weight, 200 of 186 cycles a 64-k stage takes at HBM speed).
+// What bounds it: narrow tiles, the expanding warps' issue slots (410-740 cycles per 128 x 64 weights) and, for FP8 and
+// MXFP4, HBM (65,536 x 4,096 at 16 rows: FP8 55 us, 4.9 TB/s); wide tiles, the MMA (14,336 x 4,096 Q4_K at 2,048 rows:
+// 212 us, 1.13 PFLOP/s).  The MMA, commit, arrival and copy instructions are issued by whole warps under an elected
+// predicate: from a branch for one lane a tcgen05.mma costs 75 cycles and a commit 125, whatever the width.
 //
 // Split K: a problem with fewer tiles than SMs gives each tile to a cluster of CTAs, one K slice each; the slices'
 // partial sums are exchanged through distributed shared memory (each CTA finishes a share of the tile's tokens) and
@@ -34,7 +37,8 @@
 
 namespace hq {
 
-constexpr uint32_t kDqSpin = 1u << 22;
+constexpr uint32_t kDqSpin = 1u << 16;       // polls of a wait, each suspended for up to kDqSuspendNs
+constexpr uint32_t kDqSuspendNs = 20000;
 constexpr int kDqMaxTokens = 256;
 constexpr int kDqExpandWarps = 16;
 constexpr int kDqTokenWarps = 2;
@@ -87,7 +91,8 @@ struct DqPlan {
   int nr;             // raw stages in shared memory
   int kslices;        // CTAs (cluster size) per tile
   int cpc;            // split K: most token columns a CTA of the cluster finishes
-  int x_tma;          // token rows lie in tile order: copied as boxes (box rows: x_box, and 16 for the rest)
+  int x_tma;          // token rows lie in tile order: copied as boxes
+  int x_stage;        // ... one box per stage (tn rows, every 64-k step); else boxes of x_box rows, and 16 for the rest
   int x_box;
   int raw_tma;        // raw rows copied as boxes (else in 4-byte pieces)
   int off_raw, off_recv, off_rows, off_pref, off_bar, smem;
@@ -223,7 +228,7 @@ struct DqRow {
       for (int j = 0; j < 8; ++j) w[j] = w[9 + j];
     } else if constexpr (FMT == HQ_FMT_FP8_BLOCK) {
       a.aux = sc;
-      const uint32_t at = addr + 16384 * (c >> 1);
+      const uint32_t at = addr + mis * (c >> 1);      // the second 128 columns of the rows lie behind the first
       const int ch = 4 * (c & 1) + 2 * i;
       a.q = dq_lds128(at + ((ch ^ sw) << 4));
       emit_fp8(a, o);
@@ -381,11 +386,11 @@ __device__ __forceinline__ bool dq_wait_cluster(uint64_t* bar, uint32_t parity, 
     asm volatile(
         "{\n"
         ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n"
         "selp.u32 %0, 1, 0, p;\n"
         "}\n"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(kDqSuspendNs)
         : "memory");
     if (ok) return true;
   }
@@ -426,7 +431,17 @@ __device__ __forceinline__ void dq_commit(uint64_t* bar) {
       : "memory");
 }
 
-// box copy by the elected lane of a whole warp
+// box copies by the elected lane of a whole warp
+__device__ __forceinline__ void dq_tma_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n"
+      "}\n" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      : "memory");
+}
 __device__ __forceinline__ void dq_tma_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "{\n"
@@ -435,6 +450,46 @@ __device__ __forceinline__ void dq_tma_2d(uint32_t dst, const CUtensorMap* map, 
       "@e cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
       "}\n" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
+      : "memory");
+}
+
+// Bounded wait whose polls suspend the warp for long: twenty-odd warps that poll at the default rate keep the barrier unit
+// busy enough to slow down the arrivals and copy instructions of the others.
+__device__ __forceinline__ bool dq_wait(uint64_t* bar, uint32_t parity, uint32_t spin_limit) {
+  for (uint32_t i = 0; i < spin_limit; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(kDqSuspendNs)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+// mbarrier arrivals by the elected lane of a whole warp, as a predicated instruction: a branch for one lane costs the
+// other roles' warps instruction fetches (and this one several hundred cycles when it misses)
+__device__ __forceinline__ void dq_arrive(uint64_t* bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e mbarrier.arrive.shared::cta.b64 _, [%0];\n"
+      "}\n" ::"r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void dq_arrive_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
+      "}\n" ::"r"(smem_u32(bar)),
+      "r"(bytes)
       : "memory");
 }
 
@@ -477,7 +532,10 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
   const int bank = two ? lane >> 4 : 0;
   const int frow = two ? 16 * q + (lane & 15) : 32 * q + lane;      // feature within the tile
   const int srow = two ? 64 * bank + frow : frow;                   // row of the raw stage
-  const uint32_t raw0 = smem_u32(smem + pl.off_raw) + (uint32_t)srow * T::PITCH;
+  // block-FP8: two 128-byte column halves per bank, one behind the other
+  const uint32_t raw0 = smem_u32(smem + pl.off_raw) +
+                        (T::BOXES == 2 && two ? (uint32_t)(16384 * bank + 128 * frow) : (uint32_t)srow * T::PITCH);
+  const uint32_t half_stride = two ? 8192u : 16384u;
   const uint32_t sw = (uint32_t)srow & 7u;
   const int kb64 = p.k >> 6;                                        // 64-k steps of the whole K
   const int subs = pl.subs, sub_shift = subs == 4 ? 2 : 1;
@@ -514,7 +572,7 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
     for (int rs = rs_lo; rs < rs_hi; ++rs) {
       const uint32_t sc = sc_next;
       if (SIDE && rs + 1 < rs_hi) sc_next = fetch_side(rs + 1);
-      if (!mbar_wait(&bar.full_r[slot], ph, spin)) {
+      if (!dq_wait(&bar.full_r[slot], ph, spin)) {
         if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 500 + slot);
         spin = 1;
       }
@@ -523,12 +581,13 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
       if (4 * rs + C < kb64) {
         const uint32_t taddr = tcol + (uint32_t)(32 * subs * at.s);
         DqRow<FMT> row;
-        row.load(raw0 + (uint32_t)slot * T::STAGE, C, T::WIDE ? 0 : (int)(mis >> 2), T::WIDE ? 0u : mis & 2u, sw, sc);
+        row.load(raw0 + (uint32_t)slot * T::STAGE, C, T::WIDE ? 0 : (int)(mis >> 2),
+                 T::BOXES == 2 ? half_stride : T::WIDE ? 0u : mis & 2u, sw, sc);
         bool ok = true;
 #pragma unroll 1
         for (int i = 0; i < 2; ++i) {
           ok = row.half(C, i, [&](int at_pair, const uint32_t (&v)[8]) {
-            if (i == 0 && at_pair == 0 && at.use > 0 && !mbar_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
+            if (i == 0 && at_pair == 0 && at.use > 0 && !dq_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
               if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 520 + at.s);
               spin = 1;
             }
@@ -537,23 +596,23 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
         }
         // every byte of the raw stage this warp needs has been read
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.empty_r[slot]);
+        dq_arrive(&bar.empty_r[slot]);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.full[at.s]);
+        dq_arrive(&bar.full[at.s]);
         if (FMT == HQ_FMT_MXFP4 && !ok && n_ok) report_status(p.status, HQ_DEV_SCALE_RANGE, 600);
       } else {
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.empty_r[slot]);
+        dq_arrive(&bar.empty_r[slot]);
         // the K tail ends inside this group's stage: nothing to add, but the stage counts its arrivals
         if (local < slice_stages) {
-          if (at.use > 0 && !mbar_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
+          if (at.use > 0 && !dq_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
             if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 521);
             spin = 1;
           }
           __syncwarp();
-          if (lane == 0) mbar_arrive(&bar.full[at.s]);
+          dq_arrive(&bar.full[at.s]);
         }
       }
       if (!T::WIDE) mis = (mis + T::SB) & (pl.raw_tma ? 15u : 2u);
@@ -655,7 +714,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       const uint32_t idesc = make_idesc_f16(__shfl_sync(0xffffffffu, max(16, (t.count + 15) & ~15), 0));
       const int buf = pl.nbuf == 2 ? tcount & 1 : 0;
       const int use = pl.nbuf == 2 ? tcount >> 1 : tcount;
-      if (use > 0 && !mbar_wait_backoff(&bar.acc_empty[buf], (use - 1) & 1, spin)) {
+      if (use > 0 && !dq_wait(&bar.acc_empty[buf], (use - 1) & 1, spin)) {
         if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 300 + buf);
         spin = 1;
       }
@@ -663,7 +722,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       const uint32_t d0 = tmem_u + (uint32_t)(buf * pl.tn);
       for (int j = 0; j < slice_subs; j += pl.subs, ++it) {
         const DqSlot at = dq_slot(pl, it);
-        if (!mbar_wait(&bar.full[at.s], at.use & 1, spin)) {
+        if (!dq_wait(&bar.full[at.s], at.use & 1, spin)) {
           if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 310 + at.s);
           spin = 1;
         }
@@ -708,7 +767,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       float sc = 1.f;
       if (FMT == HQ_FMT_FP8_BLOCK)
         sc = __ldg((bank == 0 ? p.fp8_tile_scale : p.fp8_tile_scale_up) + (int64_t)t.expert * p.fp8_nb + t.n0 / 128);
-      if (!mbar_wait_backoff(&bar.acc_full[buf], use & 1, spin)) {
+      if (!dq_wait(&bar.acc_full[buf], use & 1, spin)) {
         if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 400 + buf);
         spin = 1;
         failed = true;                 // nothing is stored once a wait has run out
@@ -768,7 +827,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         else columns([](float f) { return f; });
         tc_fence_before();               // the buffer is read out: the next tile may accumulate into it
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.acc_empty[buf]);
+        dq_arrive(&bar.acc_empty[buf]);
       } else {
         // ---- split K: token column c is finished by CTA c / cpc of the cluster ------------------------
         const int cpc = (t.count + S - 1) / S;
@@ -798,7 +857,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.acc_empty[buf]);
+        dq_arrive(&bar.acc_empty[buf]);
         if (lane < S) dq_arrive_remote(dq_mapa(redf_u, (uint32_t)lane));
         if (!dq_wait_cluster(bar.red_full, tcount & 1, spin)) {
           if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 420);
@@ -819,31 +878,44 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         if (lane < S) dq_arrive_remote(dq_mapa(rede_u, (uint32_t)lane));
       }
     }
-  } else if (warp == 1 + kDqEpilogueWarps) {
+  } else if (warp == 1 + kDqEpilogueWarps || (pl.x_tma && warp == 3 + kDqEpilogueWarps)) {
     // =========================== raw weight bytes, as boxes =============================================
     if (pl.raw_tma) {
       uint32_t spin = kDqSpin;
       int slot = 0, ph = 0;
       bool wrapped = false, stop = false;
       const int banks = two ? 2 : 1;
-      constexpr uint32_t BANK1 = 64u * T::PITCH;
+      // One round {wait, arrive, copy} is a chain of some five hundred cycles whatever it copies: two warps take the
+      // stages in turn (the second token warp has nothing to do when one box holds a stage's tokens)
+      // (65,536 x 4,096 at 16 rows, one warp and a box per 64 k before: MXFP4 68 -> 57 us, FP8 64 -> 55).  A slot's
+      // parity stays unambiguous: stages are consumed in order, so a warp that has issued stage i - 2 knows that the
+      // use of its slot before the last one (stage i - 2 nr) is long over.
+      const int helpers = pl.x_tma ? 2 : 1, me = warp == 1 + kDqEpilogueWarps ? 0 : 1;
+      int turn = 0;
       for (int w = first; w < n_tiles && !stop; w += step) {
         const DqTile t = dq_tile(p, pl, pref, w, n_nt, fw);
         const int row = t.expert * p.n + t.n0;
         for (int rs = rs_lo; rs < rs_hi; ++rs) {
-          if (wrapped && !mbar_wait(&bar.empty_r[slot], ph ^ 1, spin)) {
+          const bool mine = helpers == 1 || (turn & 1) == me;
+          ++turn;
+          if (!mine) {
+            if (++slot == pl.nr) { slot = 0; ph ^= 1; wrapped = true; }
+            continue;
+          }
+          if (wrapped && !dq_wait(&bar.empty_r[slot], ph ^ 1, spin)) {
             if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 560 + slot);
             stop = true;               // nothing more is issued: the target may still be in use
             break;
           }
-          if (lane == 0) mbar_arrive_expect_tx(&bar.full_r[slot], (uint32_t)T::STAGE);
-          __syncwarp();
+          dq_arrive_expect(&bar.full_r[slot], (uint32_t)T::STAGE);
           const uint32_t dst = smem_u32(smem + pl.off_raw) + (uint32_t)slot * T::STAGE;
           const int x = ((rs * T::SB) & ~15) / 2;            // 16-bit elements
-          for (int b = 0; b < banks; ++b)
-#pragma unroll
-            for (int i = 0; i < T::BOXES; ++i)
-              dq_tma_2d(dst + (uint32_t)(i * 128 * T::PITCH) + b * BANK1, b ? &tm_wu : &tm_w, x + i * 64, row, &bar.full_r[slot]);
+          for (int b = 0; b < banks; ++b) {
+            if constexpr (T::BOXES == 2)
+              dq_tma_3d(dst + b * 16384u, b ? &tm_wu : &tm_w, 0, row, 2 * rs, &bar.full_r[slot]);
+            else
+              dq_tma_2d(dst + b * (64u * T::PITCH), b ? &tm_wu : &tm_w, x, row, &bar.full_r[slot]);
+          }
           if (++slot == pl.nr) { slot = 0; ph ^= 1; wrapped = true; }
         }
       }
@@ -861,19 +933,24 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         for (int w = first; w < n_tiles && !stop; w += step) {
           const DqTile t = dq_tile(p, pl, pref, w, n_nt, fw);
           // whole boxes, then pieces of 16 rows (rows behind the tile's last may be copied along: never looked at)
-          const int boxes = p.expert_bounds != nullptr ? t.count / pl.x_box : 1;
-          const int pieces = p.expert_bounds != nullptr ? (t.count - boxes * pl.x_box + 15) >> 4 : 0;
+          const int boxes = t.count / pl.x_box;
+          const int pieces = (t.count - boxes * pl.x_box + 15) >> 4;
           const uint32_t bytes = (uint32_t)(boxes * pl.x_box + 16 * pieces) * 128u;
           for (int j = 0; j < slice_subs; j += pl.subs, ++it) {
             const DqSlot at = dq_slot(pl, it);
-            if (at.use > 0 && !mbar_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
+            if (at.use > 0 && !dq_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
               if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 540 + at.s);
               stop = true;
               break;
             }
+            if (pl.x_stage) {
+              dq_arrive_expect(&bar.full[at.s], (uint32_t)pl.subs * sub_bytes);
+              dq_tma_3d(smem_u32(smem) + (uint32_t)(at.s * pl.subs) * sub_bytes, &tm_x, 0, t.row_start, 4 * rs_lo + j,
+                        &bar.full[at.s]);
+              continue;
+            }
             const int n_sub = min(pl.subs, slice_subs - j);
-            if (lane == 0) mbar_arrive_expect_tx(&bar.full[at.s], bytes * (uint32_t)n_sub);
-            __syncwarp();
+            dq_arrive_expect(&bar.full[at.s], bytes * (uint32_t)n_sub);
             for (int c = 0; c < n_sub; ++c) {
               const int x = (4 * rs_lo + j + c) * 64;
               uint32_t dst = smem_u32(smem) + (uint32_t)(at.s * pl.subs + c) * sub_bytes;
@@ -896,7 +973,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       auto hand_over = [&]() {
         fence_proxy_async_smem();     // the copies are visible to the tensor core (async proxy)
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.full[dq_slot(pl, done).s]);
+        dq_arrive(&bar.full[dq_slot(pl, done).s]);
         ++done;
       };
       for (int w = first; w < n_tiles; w += step, ++tcount) {
@@ -911,7 +988,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         named_bar_sync(1, 32 * kDqTokenWarps);
         for (int j = 0; j < slice_subs; j += pl.subs, ++it) {
           const DqSlot at = dq_slot(pl, it);
-          if (at.use > 0 && !mbar_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
+          if (at.use > 0 && !dq_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
             if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 540 + at.s);
             spin = 1;
           }
@@ -947,7 +1024,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const int rows_valid = min(fw, p.n - t.n0);
         const int64_t tile_off = ((int64_t)t.expert * p.n + t.n0) * p.w_row_bytes;
         for (int rs = rs_lo; rs < rs_hi; ++rs) {
-          if (wrapped && !mbar_wait(&bar.empty_r[slot], ph ^ 1, spin)) {
+          if (wrapped && !dq_wait(&bar.empty_r[slot], ph ^ 1, spin)) {
             if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 570 + slot);
             spin = 1;
           }

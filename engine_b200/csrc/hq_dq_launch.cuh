@@ -7,6 +7,10 @@ namespace hq {
 
 bool f8_encode_2d(CUtensorMap* map, CUtensorMapDataType type, const void* base, uint64_t inner, uint64_t rows,
                   uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_rows, CUtensorMapSwizzle swz);
+// a [rows, 64 * blocks] matrix of 16-bit elements as (64 columns, rows, column blocks): a box is `box_rows` rows of
+// `box_blocks` column blocks, one block behind the other in shared memory, each of 128-byte swizzled rows
+bool encode_column_blocks(CUtensorMap* map, const void* base, uint64_t blocks, uint64_t rows, uint64_t row_stride_bytes,
+                          uint32_t box_rows, uint32_t box_blocks);
 
 // Cycles of one 64-k step of a tile, fitted to sweeps of tile widths on this part: the instructions that expand 128 x 64
 // weights, then half a cycle per token column.  A tile costs a start-up; without a second accumulator buffer its
@@ -153,17 +157,27 @@ int32_t launch_dq(const GroupedParams& p, int64_t rows, cudaStream_t stream) {
     const uint64_t wrows = (uint64_t)p.n_experts * (uint64_t)p.n;
     const CUtensorMapSwizzle swz = T::SWZ ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE;
     const uint32_t box_rows = p.w_up != nullptr ? 64 : 128;
-    if (!f8_encode_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.w, (uint64_t)p.w_row_bytes / 2, wrows,
-                      (uint64_t)p.w_row_bytes, T::PITCH / 2, box_rows, swz))
+    if constexpr (T::BOXES == 2) {
+      const uint64_t blocks = (uint64_t)p.w_row_bytes / 128;
+      if (!encode_column_blocks(&tm_w, p.w, blocks, wrows, (uint64_t)p.w_row_bytes, box_rows, 2) ||
+          (p.w_up != nullptr && !encode_column_blocks(&tm_wu, p.w_up, blocks, wrows, (uint64_t)p.w_row_bytes, box_rows, 2)))
+        return HQ_ERR_CUDA;
+    } else if (!f8_encode_2d(&tm_w, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.w, (uint64_t)p.w_row_bytes / 2, wrows,
+                             (uint64_t)p.w_row_bytes, T::PITCH / 2, box_rows, swz) ||
+               (p.w_up != nullptr && !f8_encode_2d(&tm_wu, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.w_up, (uint64_t)p.w_row_bytes / 2,
+                                                   wrows, (uint64_t)p.w_row_bytes, T::PITCH / 2, box_rows, swz))) {
       return HQ_ERR_CUDA;
-    if (p.w_up != nullptr && !f8_encode_2d(&tm_wu, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.w_up, (uint64_t)p.w_row_bytes / 2,
-                                           wrows, (uint64_t)p.w_row_bytes, T::PITCH / 2, box_rows, swz))
-      return HQ_ERR_CUDA;
+    }
   }
   pl.x_tma = p.x_rows == nullptr;
   if (pl.x_tma) {
-    pl.x_box = p.expert_bounds != nullptr && pl.tn > 64 ? 64 : pl.tn;
-    if (!f8_encode_2d(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.x, (uint64_t)p.k, (uint64_t)rows, (uint64_t)p.x_stride * 2,
+    pl.x_stage = p.expert_bounds == nullptr || pl.tn <= 64;
+    pl.x_box = 64;
+    if (pl.x_stage) {
+      if (!encode_column_blocks(&tm_x, p.x, (uint64_t)p.k / 64, (uint64_t)rows, (uint64_t)p.x_stride * 2, (uint32_t)pl.tn,
+                                (uint32_t)pl.subs))
+        return HQ_ERR_CUDA;
+    } else if (!f8_encode_2d(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.x, (uint64_t)p.k, (uint64_t)rows, (uint64_t)p.x_stride * 2,
                       64, (uint32_t)pl.x_box, CU_TENSOR_MAP_SWIZZLE_128B) ||
         !f8_encode_2d(&tm_x16, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.x, (uint64_t)p.k, (uint64_t)rows,
                       (uint64_t)p.x_stride * 2, 64, 16, CU_TENSOR_MAP_SWIZZLE_128B))
