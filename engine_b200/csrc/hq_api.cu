@@ -7,6 +7,12 @@ using namespace hq;
 
 namespace {
 
+int32_t check_router(const hq_router_args& a) {
+  if (a.n_experts < 1 || a.n_experts > 1024) return HQ_ERR_SHAPE;
+  if (a.top_k < 1 || a.top_k > 32 || a.top_k > a.n_experts) return HQ_ERR_SHAPE;
+  if (a.score_mode < 0 || a.score_mode > 2 || a.weight_mode < 0 || a.weight_mode > 2) return HQ_ERR_FORMAT;
+  return HQ_OK;
+}
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 bool valid_dtype(int d) { return d == HQ_DT_F32 || d == HQ_DT_F16 || d == HQ_DT_BF16; }
 
@@ -289,11 +295,9 @@ int32_t hq_router_topk(const void* logits, int32_t logits_dtype, int64_t n_rows,
   if (n_rows == 0) return HQ_OK;
   if (logits == nullptr || ids_out == nullptr || weights_out == nullptr) return HQ_ERR_NULL;
   if (!valid_dtype(logits_dtype)) return HQ_ERR_FORMAT;
-  if (args->n_experts < 1 || args->n_experts > 1024) return HQ_ERR_SHAPE;
-  if (args->top_k < 1 || args->top_k > 32 || args->top_k > args->n_experts) return HQ_ERR_SHAPE;
-  if (args->score_mode < 0 || args->score_mode > 2 || args->weight_mode < 0 || args->weight_mode > 2)
-    return HQ_ERR_FORMAT;
-  return launch_router(logits, logits_dtype, n_rows, *args, 1, 1, 0, ids_out, weights_out, (cudaStream_t)stream);
+  const int32_t bad = check_router(*args);
+  if (bad != HQ_OK) return bad;
+  return launch_router(RouterCall{logits, logits_dtype, n_rows, *args, 1, 1, 0, ids_out, weights_out}, (cudaStream_t)stream);
 }
 
 int32_t hq_router_topk_grouped(const void* logits, int32_t logits_dtype, int64_t n_rows, const hq_router_args* args,
@@ -311,12 +315,10 @@ int32_t hq_router_topk_grouped(const void* logits, int32_t logits_dtype, int64_t
   if (n_rows == 0) return HQ_OK;
   if (logits == nullptr || ids_out == nullptr || weights_out == nullptr) return HQ_ERR_NULL;
   if (!valid_dtype(logits_dtype)) return HQ_ERR_FORMAT;
-  if (args->n_experts < 1 || args->n_experts > 1024) return HQ_ERR_SHAPE;
-  if (args->top_k < 1 || args->top_k > 32 || args->top_k > args->n_experts) return HQ_ERR_SHAPE;
-  if (args->score_mode < 0 || args->score_mode > 2 || args->weight_mode < 0 || args->weight_mode > 2)
-    return HQ_ERR_FORMAT;
-  return launch_router(logits, logits_dtype, n_rows, *args, n_group, topk_group, group_score_mode, ids_out, weights_out,
-                       (cudaStream_t)stream);
+  const int32_t bad = check_router(*args);
+  if (bad != HQ_OK) return bad;
+  return launch_router(RouterCall{logits, logits_dtype, n_rows, *args, n_group, topk_group, group_score_mode, ids_out,
+                                  weights_out}, (cudaStream_t)stream);
 }
 
 int64_t hq_moe_dispatch_workspace_bytes(int64_t n_tokens, int32_t top_k, int32_t n_experts) {
@@ -397,14 +399,15 @@ int32_t hq_moe_gather_forward(const hq_weight* w, const hq_weight* w_up, const h
   p.x = x; p.x_dtype = x_dtype; p.x_stride = w->k;
   p.y = out; p.y_dtype = out_dtype;
   p.y_stride = (has_act && w_up == nullptr) ? w->n / 2 : w->n;
-  p.tiles = ws + l.off_tiles8;
+  p.tiles = ws + l.off_tiles;
+  p.tile_rows = l.tile_rows;
   p.tile_count = ws;
   p.expert_bounds = expert_bounds;
   p.x_rows = x_rows;
   p.y_rows = y_rows;
   if (has_act) p.act = *act; else p.act.act = HQ_ACT_NONE;
   p.status = status_dev;
-  return launch_gemv(p, (int)l.max_tiles8, (cudaStream_t)stream);
+  return launch_gemv(p, (int)l.max_tiles, (cudaStream_t)stream);
 }
 
 // ---- block-FP8 layers with FP8 activations (codes + 1 x 128 scales) ------------------------------------
@@ -904,9 +907,17 @@ int32_t hq_moe_layer_forward(const hq_moe_layer* layer, const void* logits, int3
   int32_t* st = (int32_t*)(ws + p.off_st);
   int32_t* inv = (int32_t*)(ws + p.off_inv);
   void* dws = ws + p.off_dws;
-  rc = hq_router_topk(logits, logits_dtype, n_tokens, &layer->router, ids, wts, stream);
-  if (rc != HQ_OK) return rc;
-  rc = hq_moe_dispatch_build(ids, n_tokens, (int32_t)p.k, (int32_t)p.e, bounds, sa, st, inv, dws, p.dws_bytes, stream);
+  if (n_tokens <= kRouteDispatchRows && p.e <= 256) {
+    // few tokens: one block routes them and builds the tables
+    rc = check_router(layer->router);
+    if (rc != HQ_OK) return rc;
+    rc = launch_route_dispatch(RouterCall{logits, logits_dtype, n_tokens, layer->router, 1, 1, 0, ids, wts}, bounds, sa, st,
+                               inv, (int32_t*)dws, (cudaStream_t)stream);
+  } else {
+    rc = hq_router_topk(logits, logits_dtype, n_tokens, &layer->router, ids, wts, stream);
+    if (rc != HQ_OK) return rc;
+    rc = hq_moe_dispatch_build(ids, n_tokens, (int32_t)p.k, (int32_t)p.e, bounds, sa, st, inv, dws, p.dws_bytes, stream);
+  }
   if (rc != HQ_OK) return rc;
   const void* xin = x;
   int32_t xin_dtype = x_dtype, xin_layout = HQ_ROWS_PER_TOKEN;

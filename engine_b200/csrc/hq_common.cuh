@@ -93,6 +93,33 @@ __device__ __forceinline__ void bulk_g2s_hint(void* dst_smem, const void* src_gm
 }
 
 // ---- named barrier among a subset of warps --------------------------------
+// Programmatic dependent launch: the kernel after this one in the stream may start its CTAs as ours retire (and
+// this kernel may have been started that way): everything that does not depend on the previous kernel -- barrier
+// set-up, the first weight stages -- then overlaps its tail.  Whatever reads activations, the scratch or
+// dispatch tables, or writes outputs, first waits for the previous kernel to have completed.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// launch of a kernel that calls pdl_wait() before it touches memory, in clusters of `cluster` blocks
+template <typename... K, typename... A>
+inline int32_t launch_pdl(void (*kern)(K...), dim3 grid, int threads, size_t smem, cudaStream_t stream, int cluster,
+                          const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
+}
+
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }

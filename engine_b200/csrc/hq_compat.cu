@@ -24,10 +24,7 @@ void complain(const char* symbol, int32_t rc) {
 // ---- scratch for the calls that need dispatch tables -----------------------------------------------
 constexpr int kCompatMaxAssign = 65536;
 constexpr int kCompatMaxExperts = 512;
-constexpr int64_t kCompatWsWords = 4 + (int64_t)(kCompatMaxAssign / kDispatchChunk) * kCompatMaxExperts +
-                                   2 * ((int64_t)kCompatMaxAssign / 8 + kCompatMaxExperts) +
-                                   2 * ((int64_t)kCompatMaxAssign / 128 + kCompatMaxExperts) +
-                                   2 * ((int64_t)kCompatMaxAssign / 256 + kCompatMaxExperts);
+constexpr int64_t kCompatWsWords = 4 + 2 * ((int64_t)kCompatMaxAssign / 8 + kCompatMaxExperts);
 constexpr int64_t kCompatWords = (kCompatMaxExperts + 64) + 3 * (int64_t)kCompatMaxAssign + kCompatWsWords + 64;
 static __device__ __align__(256) int32_t g_compat_scratch[kCompatWords];
 

@@ -17,6 +17,8 @@ __global__ void __launch_bounds__(256) weighted_reduce_kernel(const TY* __restri
                                                               const int32_t* __restrict__ row_map,
                                                               const TO* __restrict__ addend, TO* __restrict__ out,
                                                               int top_k, int64_t hidden) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t t = blockIdx.x;
   __shared__ float sw[64];
   __shared__ int64_t srow[64];
@@ -66,9 +68,8 @@ static int32_t launch_wr(const void* y, const float* w, const int32_t* row_map, 
                          int64_t n_tokens, int top_k, int64_t hidden, cudaStream_t stream) {
   constexpr int V = 16 / sizeof(TY);
   dim3 grid((unsigned)n_tokens, (unsigned)((hidden + 256 * V - 1) / (256 * V)));
-  weighted_reduce_kernel<TY, TO><<<grid, 256, 0, stream>>>((const TY*)y, w, row_map, (const TO*)addend, (TO*)out,
-                                                          top_k, hidden);
-  return cudaGetLastError() == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
+  return launch_pdl(weighted_reduce_kernel<TY, TO>, grid, 256, 0, stream, 1, (const TY*)y, w, row_map, (const TO*)addend,
+                    (TO*)out, top_k, hidden);
 }
 
 int32_t launch_weighted_reduce(const void* y, int y_dtype, const float* w, const int32_t* row_map,
@@ -202,6 +203,8 @@ __global__ void __launch_bounds__(256) fp8_quant_rows_kernel(const void* __restr
                                                              const int32_t* __restrict__ n_valid, int64_t n_rows,
                                                              int kgroups, uint8_t* __restrict__ codes,
                                                              float* __restrict__ scales) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int chunks = (kgroups + 3) / 4;
   const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int64_t limit = n_valid != nullptr ? min((int64_t)*n_valid, n_rows) : n_rows;   // rows the map is defined for
@@ -251,9 +254,8 @@ int32_t launch_fp8_quant_rows(const void* x, int x_dtype, int64_t x_stride, cons
                               cudaStream_t stream) {
   const int64_t items = n_rows * ((k / 128 + 3) / 4);
   if (items == 0) return HQ_OK;
-  fp8_quant_rows_kernel<<<(unsigned)((items + 7) / 8), 256, 0, stream>>>(x, x_dtype, x_stride, row_map, n_valid,
-                                                                        n_rows, (int)(k / 128), codes, scales);
-  return cudaGetLastError() == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
+  return launch_pdl(fp8_quant_rows_kernel, dim3((unsigned)((items + 7) / 8)), 256, 0, stream, 1, x, x_dtype, x_stride, row_map,
+                    n_valid, n_rows, (int)(k / 128), codes, scales);
 }
 
 int32_t launch_fp8_vector_dequant(const uint8_t* codes, const float* scales, int64_t n, void* out, int out_dtype,
@@ -285,6 +287,8 @@ int32_t launch_fp8_block_dequant(const uint8_t* codes, const float* scales, int6
 __global__ void __launch_bounds__(256) convert_kernel(const void* __restrict__ src, int src_dtype,
                                                       void* __restrict__ dst, int dst_dtype, int64_t n, int vec_ok,
                                                       int32_t* __restrict__ status) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (i0 >= n) return;
   float v[8];
@@ -333,9 +337,8 @@ int32_t launch_convert(const void* src, int src_dtype, void* dst, int dst_dtype,
   if (n == 0) return HQ_OK;
   const int64_t threads = (n + 7) / 8;
   const int vec_ok = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
-  convert_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(src, src_dtype, dst, dst_dtype, n, vec_ok,
-                                                                        status);
-  return cudaGetLastError() == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
+  return launch_pdl(convert_kernel, dim3((unsigned)((threads + 255) / 256)), 256, 0, stream, 1, src, src_dtype, dst, dst_dtype,
+                    n, vec_ok, status);
 }
 
 // a finite value beyond the f16 range is clamped to +-65504 (inf / NaN pass through)
@@ -367,8 +370,8 @@ __global__ void __launch_bounds__(256) gather_rows_f16_kernel(const void* __rest
                                                               const int32_t* __restrict__ row_map,
                                                               const int32_t* __restrict__ n_valid, int64_t n_rows, int k8,
                                                               uint16_t* __restrict__ out, int32_t* __restrict__ status) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_launch_dependents();
+  pdl_wait();
   // a warp per row, four 8-element chunks of it in flight per lane
   const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= n_rows || (n_valid != nullptr && row >= (int64_t)*n_valid)) return;
@@ -404,12 +407,8 @@ __global__ void __launch_bounds__(256) gather_rows_f16_kernel(const void* __rest
 int32_t launch_gather_rows_f16(const void* x, int dtype, int64_t x_stride, const int32_t* row_map, const int32_t* n_valid,
                                int64_t n_rows, int64_t k, void* out, int32_t* status, cudaStream_t stream) {
   if (n_rows == 0) return HQ_OK;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((n_rows + 7) / 8));
-  cfg.blockDim = dim3(256);
-  cfg.stream = stream;
-  return cudaLaunchKernelEx(&cfg, gather_rows_f16_kernel, x, dtype, x_stride, row_map, n_valid, n_rows, (int)(k / 8),
-                            (uint16_t*)out, status) == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
+  return launch_pdl(gather_rows_f16_kernel, dim3((unsigned)((n_rows + 7) / 8)), 256, 0, stream, 1, x, dtype, x_stride, row_map,
+                    n_valid, n_rows, (int)(k / 8), (uint16_t*)out, status);
 }
 
 // ---- gated activations --------------------------------------------------------------

@@ -559,7 +559,7 @@ static int32_t launch_cfg(const GemvParams& p, int n_y_max, int max_rows, cudaSt
 
 int32_t launch_gemv(const GemvParams& p, int n_y_max, cudaStream_t stream) {
   // most activation rows any work item of this launch can have
-  const int max_rows = p.tiles != nullptr ? 8 : (p.m < 8 ? p.m : 8);
+  const int max_rows = p.tiles != nullptr ? p.tile_rows : (p.m < 8 ? p.m : 8);
   // chunk sizes keep every bulk copy (one row segment) at 2 KiB or more
   switch (p.format) {
     case HQ_FMT_Q8_0:

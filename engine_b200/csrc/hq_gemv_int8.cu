@@ -13,9 +13,9 @@
 // the accumulator as floats through a bias constant (no conversion instruction), are multiplied by the
 // block's d, summed over the four blocks of a group and scaled once by the group's activation scale.
 //
-// Layout of the work: persistent CTAs (one per SM) walk items of 16 output rows.  Two producer warps stream
-// the item's row segments (2176 bytes = 64 blocks per bulk async copy; copies below 2 KiB cannot keep HBM
-// busy) into a shared-memory ring with mbarrier completion.  The consumer warps each take groups of
+// Layout of the work: persistent CTAs (one per SM) walk items of 16, 32 or 64 output rows.  Two producer warps
+// stream the item's row segments (2176 bytes = 64 blocks per bulk async copy for 16 rows) into a shared-memory ring
+// with mbarrier completion.  The sixteen consumer warps each take one group of
 // four blocks (136 bytes, 8-byte aligned) of every stage, so the misaligned block payloads are fetched
 // with a fixed pattern of 8- and 4-byte loads and four funnel shifts per row.  Within an MMA the k order
 // is free as long as both operands agree: lane t owns payload bytes 8t..8t+7 of a block, and reads the
@@ -28,17 +28,17 @@
 
 namespace hq {
 
-#ifndef HQ_Q8_GROUPS_PER_WARP
-#define HQ_Q8_GROUPS_PER_WARP 2
-#endif
-constexpr int kQ8GroupsPerWarp = HQ_Q8_GROUPS_PER_WARP;   // 128-element groups a warp takes from every stage
-constexpr int kQ8Warps = 16 / kQ8GroupsPerWarp;  // consumer warps
+constexpr int kQ8Warps = 16;                     // consumer warps, one group of a stage each
 constexpr int kQ8Consumers = kQ8Warps * 32;
 constexpr int kQ8Producers = 2;                  // producer warps: a bulk-copy instruction holds its warp for ~50
                                                  // cycles per active lane, so the 16 row copies of a stage are
                                                  // split over two warps
 constexpr int kQ8Threads = kQ8Consumers + 32 * (kQ8Producers + 1);   // + producers + the reducing warp
-constexpr int kQ8RT = 16;
+constexpr int kQ8RT = 16;                        // output rows of one MMA tile
+// A work item is RS such tiles (RS = 1, 2 or 4), a stage 16 / RS groups of every row: with K short of 16 groups (an
+// expert's 768 or 2048 columns) the warps that would have no group take further rows instead, and a stage stays one
+// ring slot full of bytes.  (Sixteen warps of one group each, instead of eight of two, and the taller items: Llama-3-8B
+// block Q4_K_M at 4 rows 104 -> 96 us; 128 experts of 768 x 2048 Q4_K, top 8, 64 tokens 308 -> 296 us.)
 
 // Stage geometry per format.  A stage holds KC columns of 16 weight rows = 16 groups of GK columns; a group is
 // the unit a consumer warp works on (Q8_0: four 34-byte blocks = 136 bytes; Q4_K: one 144-byte super-block)
@@ -49,34 +49,38 @@ struct I8Traits;
 template <>
 struct I8Traits<HQ_FMT_Q8_0> {
   static constexpr int KC = 2048, GK = 128, GROUP_BYTES = 136;
-  static constexpr int SEG = KC / 32 * 34, PITCH = SEG + 32, STAGE_BYTES = kQ8RT * PITCH;
   __host__ __device__ static constexpr int64_t row_bytes(int64_t k) { return k / 32 * 34; }
   static constexpr bool kSubSums = false;
 };
 template <>
 struct I8Traits<HQ_FMT_Q4_K> {
   static constexpr int KC = 4096, GK = 256, GROUP_BYTES = 144;
-  static constexpr int SEG = KC / 256 * 144, PITCH = SEG + 32, STAGE_BYTES = kQ8RT * PITCH;
   __host__ __device__ static constexpr int64_t row_bytes(int64_t k) { return k / 256 * 144; }
   static constexpr bool kSubSums = true;     // per 32-element sub-block sums of the staged bytes (the min term)
 };
 constexpr int kQ8MaxStages = 8;
 constexpr int kQ8SmemBudget = 227 * 1024 - 256;   // dynamic part; a few static words come on top
-constexpr int kQ8XGroups = 8;                    // 16-byte registers a thread prefetches activations into
+constexpr int kQ8XGroups = 4;                    // 16-byte registers a thread prefetches activations into
 constexpr uint32_t kQ8Spin = 1u << 22;
 constexpr int kQ8Magic = 0x4B400000;             // 1.5 * 2^23 as f32 bits: magic + n reads as 12582912.f + n
 template <>
 struct I8Traits<HQ_FMT_FP8_BLOCK> {
   // e4m3 codes, one byte per weight: a 128-column group is 128 bytes and shares one weight-block scale
   static constexpr int KC = 2048, GK = 128, GROUP_BYTES = 128;
-  static constexpr int SEG = KC, PITCH = SEG + 32, STAGE_BYTES = kQ8RT * PITCH;
   __host__ __device__ static constexpr int64_t row_bytes(int64_t k) { return k; }
   static constexpr bool kSubSums = false;
 };
-static_assert(I8Traits<HQ_FMT_Q8_0>::SEG >= 2048 && I8Traits<HQ_FMT_Q8_0>::SEG % 16 == 0, "bulk copy size");
-static_assert(I8Traits<HQ_FMT_Q4_K>::SEG >= 2048 && I8Traits<HQ_FMT_Q4_K>::SEG % 16 == 0, "bulk copy size");
-static_assert(I8Traits<HQ_FMT_Q8_0>::PITCH % 128 == 32 && I8Traits<HQ_FMT_Q4_K>::PITCH % 128 == 32, "row pitch");
 static_assert(I8Traits<HQ_FMT_Q8_0>::KC / I8Traits<HQ_FMT_Q8_0>::GK == 16 && I8Traits<HQ_FMT_Q4_K>::KC / I8Traits<HQ_FMT_Q4_K>::GK == 16, "16 groups per stage");
+// a stage of an item of RS row tiles
+template <int FMT, int RS>
+struct I8Stage {
+  static constexpr int KC = I8Traits<FMT>::KC / RS;      // columns
+  static constexpr int SEG = (int)I8Traits<FMT>::row_bytes(I8Traits<FMT>::KC) / RS;
+  static constexpr int PITCH = SEG % 128 == 32 ? SEG : SEG + 32;
+  static constexpr int ROWS = kQ8RT * RS;
+  static constexpr int BYTES = ROWS * PITCH;
+  static_assert(SEG % 16 == 0 && PITCH % 64 == 32, "bulk copies; 8-byte loads of 4 rows x 4 lanes cover all banks");
+};
 
 // shared-memory plan of one launch (computed on the host)
 struct Q8Layout {
@@ -107,13 +111,6 @@ __device__ __forceinline__ void mma_e4m3_16832(float (&d)[4], uint32_t a0, uint3
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-
-// Programmatic dependent launch: the kernel after this one in the stream may start its CTAs as ours retire (and
-// this kernel may have been started that way): everything that does not depend on the previous kernel -- barrier
-// set-up, the first weight stages -- then overlaps its tail.  Whatever reads activations, the scratch or
-// dispatch tables, or writes outputs, first waits for the previous kernel to have completed.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // two f32 lanes per instruction (sm_100): the accumulator pairs of one weight row share every factor
 __device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
@@ -505,23 +502,11 @@ template <int NCS>
 __device__ __forceinline__ void q4k_group(float (&acc)[NCS][4], uint32_t pa, uint32_t pb, uint32_t da, uint32_t db,
                                           uint32_t xq, uint32_t cs_stride, uint32_t sx, uint32_t xs,
                                           uint32_t xs_cs_stride, int t) {
-  // ---- all shared loads first ----
+  // ---- weight bytes ----
   const uint4 hA = lds128(da), hB = lds128(db);     // {d | dmin, 12 bytes of 6-bit scales and minima}
   uint2 qA[4], qB[4];
   qA[0] = lds64<16>(pa); qA[1] = lds64<48>(pa); qA[2] = lds64<80>(pa); qA[3] = lds64<112>(pa);
   qB[0] = lds64<16>(pb); qB[1] = lds64<48>(pb); qB[2] = lds64<80>(pb); qB[3] = lds64<112>(pb);
-  uint2 xb[NCS][8];
-  uint2 sxv[NCS];
-  uint32_t xsa[NCS], xsb[NCS];
-#pragma unroll
-  for (int c = 0; c < NCS; ++c) {
-    const uint32_t xc = xq + c * cs_stride;
-    xb[c][0] = lds64<0>(xc);   xb[c][1] = lds64<32>(xc);  xb[c][2] = lds64<64>(xc);  xb[c][3] = lds64<96>(xc);
-    xb[c][4] = lds64<128>(xc); xb[c][5] = lds64<160>(xc); xb[c][6] = lds64<192>(xc); xb[c][7] = lds64<224>(xc);
-    sxv[c] = lds64(sx + 32u * c);
-    xsa[c] = lds32<0>(xs + c * xs_cs_stride);
-    xsb[c] = lds32<8>(xs + c * xs_cs_stride);
-  }
   // ---- 6-bit scales and minima, four to a word (sub-blocks 0-3 and 4-7) ----
   uint32_t scA[2], scB[2], mnA[2], mnB[2];
   scA[0] = hA.y & 0x3F3F3F3Fu; mnA[0] = hA.z & 0x3F3F3F3Fu;
@@ -546,13 +531,20 @@ __device__ __forceinline__ void q4k_group(float (&acc)[NCS][4], uint32_t pa, uin
   const uint32_t mB = t == 0 ? mnB[0] : (t == 1 ? mnB[1] : 0u);
 #pragma unroll
   for (int c = 0; c < NCS; ++c) {
+    // (a set's activations are loaded here: two sets of them at once do not fit the registers of 20 warps)
+    uint2 xb[8];
+    const uint32_t xc = xq + c * cs_stride;
+    xb[0] = lds64<0>(xc);   xb[1] = lds64<32>(xc);  xb[2] = lds64<64>(xc);  xb[3] = lds64<96>(xc);
+    xb[4] = lds64<128>(xc); xb[5] = lds64<160>(xc); xb[6] = lds64<192>(xc); xb[7] = lds64<224>(xc);
+    const uint2 sxv = lds64(sx + 32u * c);
+    const uint32_t xsa = lds32<0>(xs + c * xs_cs_stride), xsb = lds32<8>(xs + c * xs_cs_stride);
     int isum[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int ch = j >> 1;
       int d[4];
-      if (j & 1) mma_s8_16832(d, aH[ch][0], bH[ch][0], aH[ch][1], bH[ch][1], xb[c][j].x, xb[c][j].y, 0);
-      else       mma_s8_16832(d, aL[ch][0], bL[ch][0], aL[ch][1], bL[ch][1], xb[c][j].x, xb[c][j].y, 0);
+      if (j & 1) mma_s8_16832(d, aH[ch][0], bH[ch][0], aH[ch][1], bH[ch][1], xb[j].x, xb[j].y, 0);
+      else       mma_s8_16832(d, aL[ch][0], bL[ch][0], aL[ch][1], bL[ch][1], xb[j].x, xb[j].y, 0);
       const int sa = (int)((scA[j >> 2] >> (8 * (j & 3))) & 0xFFu);
       const int sb = (int)((scB[j >> 2] >> (8 * (j & 3))) & 0xFFu);
       isum[0] += sa * d[0];
@@ -562,9 +554,9 @@ __device__ __forceinline__ void q4k_group(float (&acc)[NCS][4], uint32_t pa, uin
     }
     // |isum| <= 8 * 63 * 32 * 15 * 128 < 2^31
     int ma[4] = {0, 0, 0, 0}, mb[4] = {0, 0, 0, 0};
-    mma_s8_16832_acc(ma, mA, mB, 0u, 0u, xsa[c], 0u);
-    mma_s8_16832_acc(mb, mA, mB, 0u, 0u, xsb[c], 0u);
-    const float s0 = __uint_as_float(sxv[c].x), s1 = __uint_as_float(sxv[c].y);
+    mma_s8_16832_acc(ma, mA, mB, 0u, 0u, xsa, 0u);
+    mma_s8_16832_acc(mb, mA, mB, 0u, 0u, xsb, 0u);
+    const float s0 = __uint_as_float(sxv.x), s1 = __uint_as_float(sxv.y);
     const float v0 = dA * (float)isum[0] - nA * (float)(32 * ma[0] + mb[0]);
     const float v1 = dA * (float)isum[1] - nA * (float)(32 * ma[1] + mb[1]);
     const float v2 = dB * (float)isum[2] - nB * (float)(32 * ma[2] + mb[2]);
@@ -579,12 +571,14 @@ __device__ __forceinline__ void q4k_group(float (&acc)[NCS][4], uint32_t pa, uin
 // ---- the kernel ------------------------------------------------------------------------------------
 // NCS = column sets per block: 1 when every work item has at most 4 activation rows (columns 0-3 hold the
 // leading terms, 4-7 the remainders), 2 for up to 8 rows (set 0 = leading terms, set 1 = remainders).
-template <int FMT, int NCS>
+template <int FMT, int NCS, int RS>
 __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvParams p, const Q8Layout lay) {
   using T = I8Traits<FMT>;
+  using ST = I8Stage<FMT, RS>;
   constexpr int WK = kQ8Warps;
-  constexpr int RT = kQ8RT;
-  constexpr int KC = T::KC;
+  constexpr int WG = WK / RS;                  // groups of a stage (warps of a row tile)
+  constexpr int RT = kQ8RT * RS;
+  constexpr int KC = ST::KC;
   const int NSTAGE = lay.nstage;
   extern __shared__ __align__(128) uint8_t smem[];
 
@@ -668,9 +662,9 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
                                 T::row_bytes(k_lo + chunk * KC);
           if (lane == 0) mbar_arrive_expect_tx(&full[s], bytes * (uint32_t)my_rows);
           __syncwarp();
-          uint8_t* dst = smem + s * T::STAGE_BYTES + pw * RPP * T::PITCH;
+          uint8_t* dst = smem + s * ST::BYTES + pw * RPP * ST::PITCH;
           if (lane < my_rows)
-            bulk_g2s_hint(dst + lane * T::PITCH, wsrc + (int64_t)lane * row_bytes, bytes, &full[s], policy);
+            bulk_g2s_hint(dst + lane * ST::PITCH, wsrc + (int64_t)lane * row_bytes, bytes, &full[s], policy);
           if (++s == NSTAGE) {
             s = 0;
             ++round;
@@ -699,40 +693,46 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
         spin = 1;
         failed = true;                 // nothing is stored for an item whose partial sums never arrived
       }
-      float v[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-      for (int b = 0; b < 2; ++b)
-        if (b < p.n_banks) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            float sum = 0.f;
-#pragma unroll
-            for (int j = 0; j < WK; ++j) sum += rbuf[((b * WK + j) * 4 + i) * 32 + lane];
-            if (NCS == 1 && FMT == HQ_FMT_FP8_BLOCK) {
-              // two-row layout of the three e4m3 terms: columns 2, 3 and 4, 5 sit one and two lanes further on
-              const float s1 = __shfl_down_sync(0xffffffffu, sum, 1), s2 = __shfl_down_sync(0xffffffffu, sum, 2);
-              sum += s1 + s2;
-            } else if (NCS == 1) {
-              // four-row layout: the remainder columns 4..7 sit two lanes further on
-              sum += __shfl_down_sync(0xffffffffu, sum, 2);
-            }
-            v[b][i] = sum;
-          }
-        }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&red_free[rb]);
-      if (S > 1) {
-        // split K: the slice sums of an item meet in global memory and are added when the kernel ends
-        const int nb = p.n_banks;
-        float* mine = lay.partials + ((int64_t)w * S + slice) * (nb * 128);
+      WorkItem ti = wi;
+#pragma unroll 1
+      for (int rt = 0; rt < RS; ++rt, ti.n0 += kQ8RT) {
+        float v[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
         for (int b = 0; b < 2; ++b)
-          if (b < nb) {
+          if (b < p.n_banks) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) __stcg(mine + (b * 4 + i) * 32 + lane, v[b][i]);
+            for (int i = 0; i < 4; ++i) {
+              float sum = 0.f;
+#pragma unroll
+              for (int j = 0; j < WG; ++j) sum += rbuf[((b * WK + rt * WG + j) * 4 + i) * 32 + lane];
+              if (NCS == 1 && FMT == HQ_FMT_FP8_BLOCK) {
+                // two-row layout of the three e4m3 terms: columns 2, 3 and 4, 5 sit one and two lanes further on
+                const float s1 = __shfl_down_sync(0xffffffffu, sum, 1), s2 = __shfl_down_sync(0xffffffffu, sum, 2);
+                sum += s1 + s2;
+              } else if (NCS == 1) {
+                // four-row layout: the remainder columns 4..7 sit two lanes further on
+                sum += __shfl_down_sync(0xffffffffu, sum, 2);
+              }
+              v[b][i] = sum;
+            }
           }
-      } else {
-        gemv_store_item(p, wi, g, 2 * t, !failed && (NCS > 1 || t < (FMT == HQ_FMT_FP8_BLOCK ? 1 : 2)), v);
+        if (rt == RS - 1) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&red_free[rb]);
+        }
+        if (S > 1) {
+          // split K: the slice sums of an item meet in global memory and are added when the kernel ends
+          const int nb = p.n_banks;
+          float* mine = lay.partials + (((int64_t)w * S + slice) * RS + rt) * (nb * 128);
+#pragma unroll
+          for (int b = 0; b < 2; ++b)
+            if (b < nb) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) __stcg(mine + (b * 4 + i) * 32 + lane, v[b][i]);
+            }
+        } else {
+          gemv_store_item(p, ti, g, 2 * t, !failed && (NCS > 1 || t < (FMT == HQ_FMT_FP8_BLOCK ? 1 : 2)), v);
+        }
       }
       ++item;
     }
@@ -751,10 +751,11 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
   constexpr int kTerms = FMT == HQ_FMT_FP8_BLOCK ? 3 : 2;
   const int tstride = FMT == HQ_FMT_FP8_BLOCK ? 2 : (ncols >> 1);
   // this lane's staged column (column g of every set), its group within a stage, its scale-table columns
-  const uint32_t xq_lane = smem_u32(xq) + (uint32_t)g * xpitch + (uint32_t)T::GK * warp + 8u * t;
-  const uint32_t sx_lane = smem_u32(sx) + (uint32_t)warp * ncols * 4u + 8u * t;
+  const int rtile = warp / WG, wgrp = warp - rtile * WG;     // this warp's row tile and group of every stage
+  const uint32_t xq_lane = smem_u32(xq) + (uint32_t)g * xpitch + (uint32_t)T::GK * wgrp + 8u * t;
+  const uint32_t sx_lane = smem_u32(sx) + (uint32_t)wgrp * ncols * 4u + 8u * t;
   uint8_t* xsub = smem + lay.off_xs;     // Q4_K: sub-block sums [group][column][16]
-  const uint32_t xs_lane = smem_u32(xsub) + ((uint32_t)warp * ncols + g) * 16u + 4u * (t & 1);
+  const uint32_t xs_lane = smem_u32(xsub) + ((uint32_t)wgrp * ncols + g) * 16u + 4u * (t & 1);
 
   Q8XPrefetch pf;
   bool pf_valid = false;
@@ -836,41 +837,31 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
 #pragma unroll
         for (int bank = 0; bank < 2; ++bank) {
           if (bank >= p.n_banks) break;
-          // block-FP8: the 128 x 128 weight-block scales of this warp's groups, fetched before the wait for the stage
-          float wsv[kQ8GroupsPerWarp];
-          if (FMT == HQ_FMT_FP8_BLOCK) {
-            const float* fsc = reinterpret_cast<const float*>(bank == 0 ? p.scales : p.scales_up) +
-                               (int64_t)wi.expert * p.scale_expert_stride +
-                               (int64_t)(wi.n0 / 128) * ((p.k + 127) / 128) + k_chunk / 128;
-#pragma unroll
-            for (int gi = 0; gi < kQ8GroupsPerWarp; ++gi) {
-              const int grp = warp + gi * WK;
-              wsv[gi] = grp < ngroups ? __ldg(fsc + grp) : 0.f;
-            }
-          }
+          // block-FP8: the 128 x 128 weight-block scale of this warp's group, fetched before the wait for the stage
+          float wsv = 0.f;
+          if (FMT == HQ_FMT_FP8_BLOCK && wgrp < ngroups)
+            wsv = __ldg(reinterpret_cast<const float*>(bank == 0 ? p.scales : p.scales_up) +
+                        (int64_t)wi.expert * p.scale_expert_stride +
+                        (int64_t)((wi.n0 + kQ8RT * rtile) / 128) * ((p.k + 127) / 128) + k_chunk / 128 + wgrp);
           if (!mbar_wait(&full[s], phase, spin)) {
             // bounded wait ran out: flag it and carry on (every warp still reaches every barrier)
             if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 200 + s);
             spin = 1;
           }
-#pragma unroll
-          for (int gi = 0; gi < kQ8GroupsPerWarp; ++gi) {
-            const int grp = warp + gi * WK;
-            if (grp < ngroups) {
-              const uint32_t da = smem_u32(smem + s * T::STAGE_BYTES) + (uint32_t)g * T::PITCH +
-                                  (uint32_t)T::GROUP_BYTES * grp;
-              const uint32_t db = da + 8u * T::PITCH;
-              const uint32_t gq = kx / T::GK + gi * WK;      // group index inside the staged activations, less `warp`
-              if (FMT == HQ_FMT_Q8_0) {
-                q8_group<NCS>(acc[bank], da + 8u * t, db + 8u * t, da, db, xq_lane + gq * T::GK, cs_stride,
-                              sx_lane + gq * (uint32_t)ncols * 4u);
-              } else if (FMT == HQ_FMT_FP8_BLOCK) {
-                fp8_group<NCS>(acc[bank], da + 8u * t, db + 8u * t, xq_lane + gq * T::GK, cs_stride,
-                               sx_lane + gq * (uint32_t)ncols * 4u, wsv[gi]);
-              } else {
-                q4k_group<NCS>(acc[bank], da + 8u * t, db + 8u * t, da, db, xq_lane + gq * T::GK, cs_stride,
-                               sx_lane + gq * (uint32_t)ncols * 4u, xs_lane + gq * (uint32_t)ncols * 16u, 128u, t);
-              }
+          if (wgrp < ngroups) {
+            const uint32_t da = smem_u32(smem + s * ST::BYTES) + (uint32_t)(kQ8RT * rtile + g) * ST::PITCH +
+                                (uint32_t)T::GROUP_BYTES * wgrp;
+            const uint32_t db = da + 8u * ST::PITCH;
+            const uint32_t gq = kx / T::GK;      // group index inside the staged activations, less this warp's own
+            if (FMT == HQ_FMT_Q8_0) {
+              q8_group<NCS>(acc[bank], da + 8u * t, db + 8u * t, da, db, xq_lane + gq * T::GK, cs_stride,
+                            sx_lane + gq * (uint32_t)ncols * 4u);
+            } else if (FMT == HQ_FMT_FP8_BLOCK) {
+              fp8_group<NCS>(acc[bank], da + 8u * t, db + 8u * t, xq_lane + gq * T::GK, cs_stride,
+                             sx_lane + gq * (uint32_t)ncols * 4u, wsv);
+            } else {
+              q4k_group<NCS>(acc[bank], da + 8u * t, db + 8u * t, da, db, xq_lane + gq * T::GK, cs_stride,
+                             sx_lane + gq * (uint32_t)ncols * 4u, xs_lane + gq * (uint32_t)ncols * 16u, 128u, t);
             }
           }
           __syncwarp();
@@ -927,32 +918,34 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
       __threadfence();
       const int nb = p.n_banks;
       int idx = 0;
-      for (int w = w_begin; w < w_end; w += w_step, ++idx) {
-        if (idx % (kQ8Threads / 32) != warp) continue;
-        const WorkItem wi = get_item<RT>(p, w, n_rt);
-        if (wi.nrows <= 0) continue;
-        const float* all = lay.partials + (int64_t)w * S * (nb * 128);
-        float v[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      for (int w = w_begin; w < w_end; w += w_step)
+        for (int rt = 0; rt < RS; ++rt, ++idx) {
+          if (idx % (kQ8Threads / 32) != warp) continue;
+          WorkItem wi = get_item<RT>(p, w, n_rt);
+          if (wi.nrows <= 0) continue;
+          wi.n0 += kQ8RT * rt;
+          const float* all = lay.partials + ((int64_t)w * S * RS + rt) * (nb * 128);
+          float v[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-        for (int b = 0; b < 2; ++b)
-          if (b < nb) {
-            // every load of a bank is issued before the first sum needs one (at most eight slices)
-            float part[8][4];
+          for (int b = 0; b < 2; ++b)
+            if (b < nb) {
+              // every load of a bank is issued before the first sum needs one (at most eight slices)
+              float part[8][4];
 #pragma unroll
-            for (int sl = 0; sl < 8; ++sl)
+              for (int sl = 0; sl < 8; ++sl)
 #pragma unroll
-              for (int i = 0; i < 4; ++i)
-                part[sl][i] = sl < S ? __ldcg(all + (sl * nb + b) * 128 + i * 32 + lane) : 0.f;
+                for (int i = 0; i < 4; ++i)
+                  part[sl][i] = sl < S ? __ldcg(all + (sl * RS * nb + b) * 128 + i * 32 + lane) : 0.f;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              float sum = 0.f;
+              for (int i = 0; i < 4; ++i) {
+                float sum = 0.f;
 #pragma unroll
-              for (int sl = 0; sl < 8; ++sl) sum += part[sl][i];   // slice order; absent slices add +0
-              v[b][i] = sum;
+                for (int sl = 0; sl < 8; ++sl) sum += part[sl][i];   // slice order; absent slices add +0
+                v[b][i] = sum;
+              }
             }
-          }
-        gemv_store_item(p, wi, g, 2 * t, NCS > 1 || t < (FMT == HQ_FMT_FP8_BLOCK ? 1 : 2), v);
-      }
+          gemv_store_item(p, wi, g, 2 * t, NCS > 1 || t < (FMT == HQ_FMT_FP8_BLOCK ? 1 : 2), v);
+        }
     }
   }
 }
@@ -979,7 +972,7 @@ static int q8_fixed_bytes(int ncols, int xk, int n_banks) {
 }
 template <int FMT>
 static int q8_ring_stages(int ncols, int xk, int n_banks) {
-  return (kQ8SmemBudget - q8_fixed_bytes<FMT>(ncols, xk, n_banks)) / I8Traits<FMT>::STAGE_BYTES;
+  return (kQ8SmemBudget - q8_fixed_bytes<FMT>(ncols, xk, n_banks)) / I8Stage<FMT, 1>::BYTES;
 }
 template <int FMT>
 static Q8Split q8_split_plan(int64_t n, int64_t k, int64_t n_y, int n_banks, bool expert_indexed, int ncols) {
@@ -1020,9 +1013,10 @@ int64_t gemv_int8_workspace_bytes(int format, int64_t n, int64_t k, int64_t m) {
   return 0;
 }
 
-template <int FMT, int NCS>
-static int32_t launch_q8_cfg(const GemvParams& p, int n_y_max, int max_rows, cudaStream_t stream) {
+template <int FMT, int NCS, int RS>
+static int32_t launch_q8_rs(const GemvParams& p, int n_y_max, int max_rows, cudaStream_t stream) {
   using T = I8Traits<FMT>;
+  using ST = I8Stage<FMT, RS>;
   Q8Layout lay{};
   lay.ncols = 8 * NCS;
   Q8Split sp = q8_split_plan<FMT>(p.n, p.k, n_y_max, p.n_banks, p.tiles != nullptr, lay.ncols);
@@ -1040,7 +1034,7 @@ static int32_t launch_q8_cfg(const GemvParams& p, int n_y_max, int max_rows, cud
   // K range when it fits -- then a persistent CTA quantizes its activations once), give every remaining byte
   // to the ring.
   const int esz = dtype_size(p.x_dtype);
-  const int k_round = (sp.slice_k + T::KC - 1) / T::KC * T::KC;
+  const int k_round = (sp.slice_k + ST::KC - 1) / ST::KC * ST::KC;
   const int candidates[3] = {k_round, 8192 < k_round ? 8192 : k_round, 4096 < k_round ? 4096 : k_round};
   for (int c = 0; c < 3; ++c) {
     lay.xk = candidates[c];
@@ -1051,10 +1045,10 @@ static int32_t launch_q8_cfg(const GemvParams& p, int n_y_max, int max_rows, cud
     const int red_bytes = 2 * p.n_banks * kQ8Warps * 4 * 32 * 4;
     const int bar_bytes = (2 * kQ8MaxStages + 4) * 8 + 16;
     const int fixed = lay.x_bytes + sx_bytes + xs_bytes + red_bytes + bar_bytes;
-    int nst = (kQ8SmemBudget - fixed) / T::STAGE_BYTES;
+    int nst = (kQ8SmemBudget - fixed) / ST::BYTES;
     if (nst > kQ8MaxStages) nst = kQ8MaxStages;
     lay.nstage = nst;
-    lay.off_x = nst * T::STAGE_BYTES;
+    lay.off_x = nst * ST::BYTES;
     lay.off_sx = lay.off_x + lay.x_bytes;
     lay.off_xs = lay.off_sx + sx_bytes;
     lay.off_red = lay.off_xs + xs_bytes;
@@ -1066,7 +1060,7 @@ static int32_t launch_q8_cfg(const GemvParams& p, int n_y_max, int max_rows, cud
   // columns one register prefetch can hold, in whole 256-column steps
   const int sub = (kQ8XGroups * kQ8Consumers * 16) / (max_rows * esz) / 256 * 256;   // 16 bytes per register
   lay.xk_sub = sub < lay.xk ? sub : lay.xk;
-  auto kern = gemv_int8_kernel<FMT, NCS>;
+  auto kern = gemv_int8_kernel<FMT, NCS, RS>;
   static bool attr_done[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return HQ_ERR_CUDA;
@@ -1075,7 +1069,7 @@ static int32_t launch_q8_cfg(const GemvParams& p, int n_y_max, int max_rows, cud
       return HQ_ERR_CUDA;
     attr_done[dev] = true;
   }
-  const int64_t items = (int64_t)n_y_max * ((p.n + kQ8RT - 1) / kQ8RT);
+  const int64_t items = (int64_t)n_y_max * ((p.n + ST::ROWS - 1) / ST::ROWS);
   int64_t streams = sm_count() / sp.kslices;
   if (streams < 1) streams = 1;
   if (streams > items) streams = items;
@@ -1092,6 +1086,15 @@ static int32_t launch_q8_cfg(const GemvParams& p, int n_y_max, int max_rows, cud
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, p, lay) == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
+}
+
+// Row tiles per item: as many as the groups of K leave consumer warps for.  A call that splits K has long rows: one.
+template <int FMT, int NCS>
+static int32_t launch_q8_cfg(const GemvParams& p, int n_y_max, int max_rows, cudaStream_t stream) {
+  const int groups = p.k / I8Traits<FMT>::GK;
+  if (groups <= 4) return launch_q8_rs<FMT, NCS, 4>(p, n_y_max, max_rows, stream);
+  if (groups <= 8) return launch_q8_rs<FMT, NCS, 2>(p, n_y_max, max_rows, stream);
+  return launch_q8_rs<FMT, NCS, 1>(p, n_y_max, max_rows, stream);
 }
 
 int32_t launch_gemv_int8(const GemvParams& p, int n_y_max, int max_rows, cudaStream_t stream) {

@@ -34,7 +34,7 @@ __device__ __forceinline__ WorkItem get_item(const GemvParams& p, int w, int n_r
   if (p.tiles != nullptr) {
     it.expert = p.tiles[2 * it.y];
     it.row0 = p.tiles[2 * it.y + 1];
-    it.nrows = min(8, p.expert_bounds[it.expert + 1] - it.row0);
+    it.nrows = min(p.tile_rows, p.expert_bounds[it.expert + 1] - it.row0);
   } else {
     it.expert = 0;
     it.row0 = 8 * it.y;

@@ -27,7 +27,8 @@ struct GemvParams {
   void* y;
   int y_dtype;
   int64_t y_stride;             // elements
-  // expert-indexed mode: work items of <= 8 sorted rows of one expert
+  // expert-indexed mode: work items of <= tile_rows sorted rows of one expert
+  int tile_rows;                // 4 or 8
   const int32_t* tiles;         // [n_items][2] = (expert, first sorted row)
   const int32_t* tile_count;    // device word holding n_items
   const int32_t* expert_bounds; // [E+1]
@@ -147,16 +148,13 @@ int32_t launch_mxfp8_quant_rows(const void* x, int x_dtype, int64_t x_stride, co
                                 cudaStream_t stream);
 
 // ---- dispatch tables (hq_dispatch.cu) -------------------------------------------
-constexpr int kDispatchChunk = 1024;  // flat assignments per block
+// sorted rows of one expert in a work item of the decode kernels: 8, or 4 when a call has no more tokens than that (the
+// Q8_0 / Q4_K kernel then needs half the activation columns)
+constexpr int kDecodeShortTile = 4;
 struct DispatchLayout {
-  int64_t n_blocks;      // ceil(T*k / kDispatchChunk)
-  int64_t off_counts;    // int32 words
-  int64_t off_tiles8;    // int32 words, [max8][2]
-  int64_t max_tiles8;
-  int64_t off_tiles128;  // int32 words, [max128][2]
-  int64_t max_tiles128;
-  int64_t off_tiles256;  // int32 words, [max256][2]
-  int64_t max_tiles256;
+  int tile_rows;         // rows of a work item
+  int64_t off_tiles;     // int32 words, [max_tiles][2]
+  int64_t max_tiles;
   int64_t total_words;
 };
 DispatchLayout dispatch_layout(int64_t n_tokens, int top_k, int n_experts);
@@ -169,8 +167,20 @@ int32_t launch_dispatch_noalloc(const uint32_t* ids, int64_t n_tokens, int top_k
                                 cudaStream_t stream);
 
 // ---- router (hq_router.cu) --------------------------------------------------------
-int32_t launch_router(const void* logits, int dtype, int64_t n_rows, const hq_router_args& a, int n_group,
-                      int topk_group, int group_mode, uint32_t* ids, float* weights, cudaStream_t stream);
+struct RouterCall {
+  const void* logits;
+  int dtype;
+  int64_t n_rows;
+  hq_router_args a;
+  int n_group, topk_group, group_mode;
+  uint32_t* ids;
+  float* weights;
+};
+int32_t launch_router(const RouterCall& c, cudaStream_t stream);
+// router and dispatch tables in one launch: at most kRouteDispatchRows rows and 256 experts
+constexpr int kRouteDispatchRows = 32;
+int32_t launch_route_dispatch(const RouterCall& c, int32_t* bounds, int32_t* sorted_assign, int32_t* sorted_token,
+                              int32_t* inv_perm, int32_t* ws, cudaStream_t stream);
 
 // ---- elementwise / reduce (hq_elementwise.cu) --------------------------------------
 int32_t launch_weighted_reduce(const void* y, int y_dtype, const float* w, const int32_t* row_map,

@@ -120,3 +120,18 @@ def test_fp8_one_and_two_rows_on_the_fp8_warp_mma(m, x_dtype):
     x[m - 1, 5] = np.nan
     y2 = layer.forward_raw(T.to_dev(x, torch.float32, DEV), torch.float32).cpu().numpy()
     assert np.all(~np.isfinite(y2[m - 1]))
+
+
+@pytest.mark.parametrize("m", [1, 4, 5, 8])
+@pytest.mark.parametrize("n", [31, 100])
+@pytest.mark.parametrize("fmt,k", [("Q4_K", 256), ("Q4_K", 1024), ("Q4_K", 1280), ("Q4_K", 2048), ("Q4_K", 2304),
+                                   ("Q8_0", 512), ("Q8_0", 1024), ("Q8_0", 1280)])
+def test_tall_items_of_short_rows(fmt, n, k, m):
+    # up to four groups of K: items of 64 output rows, up to eight: 32, else 16; n cuts the last item short
+    layer, deq, rng = _layer(fmt, n, k, 40 + k)
+    x = T.to_dev(rng.standard_normal((m, k)).astype(np.float32), torch.bfloat16, DEV)
+    y = layer.forward_raw(x, torch.float32)
+    torch.cuda.synchronize()
+    assert layer.device_status()[0] == 0
+    want = M.dense_forward(x.to(torch.float32).cpu().numpy(), deq, None)
+    assert T.rel_l2(y.cpu().numpy(), want) <= 1e-3
