@@ -17,6 +17,7 @@ SCORE_RAW, SCORE_SOFTMAX, SCORE_SIGMOID = 0, 1, 2
 WEIGHT_SCORE, WEIGHT_SOFTMAX, WEIGHT_SIGMOID = 0, 1, 2
 ACT_NONE, ACT_SWIGLU, ACT_GPTOSS = 0, 1, 2
 DEV_OK, DEV_WAIT_TIMEOUT, DEV_BAD_INDEX, DEV_SCALE_RANGE, DEV_F16_RANGE = 0, 1, 2, 3, 4
+WEIGHT_F16_SCALES = 1
 ROWS_PER_TOKEN, ROWS_PER_SLOT, ROWS_SORTED = 0, 1, 2
 CFG_MOE_TENSOR_MIN_ROWS, CFG_DENSE_TENSOR_MIN_ROWS, CFG_SPIN_LIMIT, CFG_TEST_SKIP_PRODUCER = 0, 1, 2, 3
 CFG_FP8_LOAD_BURST, CFG_FP8_L2_PREFETCH = 4, 5
@@ -25,7 +26,7 @@ CFG_FP8_LOAD_BURST, CFG_FP8_L2_PREFETCH = 4, 5
 class HqWeight(C.Structure):
     _fields_ = [("format", C.c_int32), ("n_experts", C.c_int32), ("n", C.c_int64), ("k", C.c_int64),
                 ("data", C.c_void_p), ("scales", C.c_void_p), ("bias", C.c_void_p),
-                ("bias_dtype", C.c_int32), ("reserved", C.c_int32),
+                ("bias_dtype", C.c_int32), ("flags", C.c_int32),
                 ("fp8_tile_scale", C.c_void_p), ("fp8_rel_scale", C.c_void_p)]
 
 
@@ -104,6 +105,7 @@ SIGNATURES = {
     "hq_config_get": (_I64, [_I32]),
     "hq_convert": (_I32, [_P, _I32, _P, _I32, _I64, _P]),
     "hq_convert_status": (_I32, [_P, _I32, _P, _I32, _I64, _P, _P]),
+    "hq_tensor_path": (_I32, [C.POINTER(HqWeight), _I64, _I32]),
     "hq_gather_rows_f16": (_I32, [_P, _I32, _I64, _P, _P, _I64, _I64, _P, _P, _P]),
     "hq_probe_tensor_peak": (_I32, [_I32, _I32, _I32, _P, C.POINTER(C.c_double), _P]),
     "hq_gated_act": (_I32, [_P, _P, _I32, _I64, _I32, C.POINTER(HqActArgs), _P, _P]),

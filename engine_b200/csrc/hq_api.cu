@@ -94,14 +94,21 @@ void fill_grouped(GroupedParams& g, const hq_weight* w, const hq_weight* w_up) {
   g.fp8_kb = (int)((w->k + 127) / 128);
 }
 
-// Row counts from which a call goes to the tensor-core grouped GEMM.  Q8_0's decode kernel streams at HBM speed,
-// so re-reading the weights once per 8 rows stays cheaper than expanding them for longer: four times the
-// configured thresholds.
-int64_t dense_tensor_min_rows(int format) {
-  return g_cfg[HQ_CFG_DENSE_TENSOR_MIN_ROWS] * (format == HQ_FMT_Q8_0 ? 4 : 1);
+// Row counts from which a call goes to the tensor-core GEMM.  Q8_0's decode kernel streams at HBM speed, so re-reading
+// the weights once per 8 rows stays cheaper than expanding them for longer: four times the configured thresholds.  MXFP4
+// with block scales the f16 operand holds (HQ_WEIGHT_F16_SCALES): from the first row on at the default settings -- the
+// expanded weights are exact there, both kernels round activations to f16, and the decode kernel, bounded by its
+// instructions, is slower at every count (us, decode against tensor: 14,336 x 4,096 at 1 row 22.7 : 17.3, 4,096 x 14,336
+// at 8 rows 64 : 19; 128 experts of 2,880 x 2,880, top 4: 1 token 56 : 54, 16 tokens 413 : 273, 128 tokens 1,224 : 637).
+bool dense_tensor_rows(const hq_weight* w, int64_t m) {
+  const int64_t cfg = g_cfg[HQ_CFG_DENSE_TENSOR_MIN_ROWS];
+  if (w->format == HQ_FMT_MXFP4 && (w->flags & HQ_WEIGHT_F16_SCALES) != 0 && cfg <= 9) return m >= 1;
+  return m >= cfg * (w->format == HQ_FMT_Q8_0 ? 4 : 1);
 }
-int64_t moe_tensor_min_rows(int format) {
-  return g_cfg[HQ_CFG_MOE_TENSOR_MIN_ROWS] * (format == HQ_FMT_Q8_0 ? 4 : 1);
+bool moe_tensor_rows(const hq_weight* w, int64_t rows) {
+  const int64_t cfg = g_cfg[HQ_CFG_MOE_TENSOR_MIN_ROWS];
+  if (w->format == HQ_FMT_MXFP4 && (w->flags & HQ_WEIGHT_F16_SCALES) != 0 && cfg <= 8) return rows >= 1;
+  return rows >= cfg * (w->format == HQ_FMT_Q8_0 ? 4 : 1) * (int64_t)w->n_experts;
 }
 
 // the tensor-core kernel takes f16 activation rows (it copies them into its operand tiles); hosts holding bf16 or
@@ -177,7 +184,7 @@ int64_t hq_linear_workspace_bytes(const hq_weight* w, int64_t m) {
   if (check_weight(w) != HQ_OK || m <= 0) return 0;
   if (w->n_experts != 1) return 0;
   if ((w->format == HQ_FMT_Q4_K || w->format == HQ_FMT_FP8_BLOCK || w->format == HQ_FMT_Q8_0) &&
-      m >= dense_tensor_min_rows(w->format))
+      dense_tensor_rows(w, m))
     return 0;   // tensor-core path
   return gemv_int8_workspace_bytes(w->format, w->n, w->k, m);
 }
@@ -194,7 +201,7 @@ int32_t hq_linear_forward_ws(const hq_weight* w, const void* x, int32_t x_dtype,
   if (!aligned16(x) || (x_stride * dtype_size(x_dtype)) % 16 != 0) return HQ_ERR_ALIGN;
   if (x_stride < w->k || y_stride < w->n) return HQ_ERR_SHAPE;
   if (workspace != nullptr && (workspace_bytes < 0 || ((uintptr_t)workspace & 255u) != 0)) return HQ_ERR_ALIGN;
-  if (m >= dense_tensor_min_rows(w->format) && w->n_experts == 1 && tensor_path_ok(w, nullptr, x_dtype, x_stride)) {
+  if (dense_tensor_rows(w, m) && w->n_experts == 1 && tensor_path_ok(w, nullptr, x_dtype, x_stride)) {
     GroupedParams g{};
     fill_grouped(g, w, nullptr);
     g.m = (int)m;
@@ -244,7 +251,8 @@ int32_t hq_linear_glu_forward(const hq_weight* w_gate, const hq_weight* w_up, co
   if (!aligned16(x) || (x_stride * dtype_size(x_dtype)) % 16 != 0) return HQ_ERR_ALIGN;
   const int64_t n_out = w_up != nullptr ? w_gate->n : w_gate->n / 2;
   if (x_stride < w_gate->k || y_stride < n_out) return HQ_ERR_SHAPE;
-  if (m >= dense_tensor_min_rows(w_gate->format) && tensor_path_ok(w_gate, w_up, x_dtype, x_stride)) {
+  if (dense_tensor_rows(w_gate, m) && (w_up == nullptr || dense_tensor_rows(w_up, m)) &&
+      tensor_path_ok(w_gate, w_up, x_dtype, x_stride)) {
     GroupedParams g{};
     fill_grouped(g, w_gate, w_up);
     g.m = (int)m;
@@ -380,7 +388,8 @@ int32_t hq_moe_gather_forward(const hq_weight* w, const hq_weight* w_up, const h
   const int32_t* x_rows =
       x_layout == HQ_ROWS_PER_TOKEN ? sorted_token : (x_layout == HQ_ROWS_PER_SLOT ? sorted_assign : nullptr);
   const int32_t* y_rows = out_layout == HQ_ROWS_PER_SLOT ? sorted_assign : nullptr;
-  if (n_tokens * top_k >= moe_tensor_min_rows(w->format) * (int64_t)w->n_experts && tensor_path_ok(w, w_up, x_dtype, w->k)) {
+  if (moe_tensor_rows(w, n_tokens * top_k) && (w_up == nullptr || moe_tensor_rows(w_up, n_tokens * top_k)) &&
+      tensor_path_ok(w, w_up, x_dtype, w->k)) {
     GroupedParams g{};
     fill_grouped(g, w, w_up);
     g.x = x; g.x_dtype = x_dtype; g.x_stride = w->k;
@@ -795,6 +804,11 @@ int32_t hq_fp8_scale_prepare(const float* scales, int32_t n_experts, int64_t n, 
                                   (cudaStream_t)stream);
 }
 
+int32_t hq_tensor_path(const hq_weight* w, int64_t rows, int32_t dense) {
+  if (check_weight(w) != HQ_OK || !tensor_path_ok(w, nullptr, HQ_DT_F16, w->k)) return 0;
+  return (dense != 0 ? dense_tensor_rows(w, rows) : moe_tensor_rows(w, rows)) ? 1 : 0;
+}
+
 int32_t hq_convert_status(const void* src, int32_t src_dtype, void* dst, int32_t dst_dtype, int64_t n_elems,
                           int32_t* status_dev, void* stream) {
   if (n_elems < 0) return HQ_ERR_SHAPE;
@@ -861,8 +875,8 @@ int32_t plan_moe_layer(const hq_moe_layer* l, int64_t n_tokens, int32_t x_dtype,
   if (l->act.act == HQ_ACT_NONE) return HQ_ERR_FORMAT;
   p.rows = p.t * p.k;
   // the tensor-core kernel takes f16 rows and copies them fastest in expert order: one pass converts and permutes
-  p.gather_x = p.rows >= moe_tensor_min_rows(l->gate->format) * p.e &&
-             tensor_path_ok(l->gate, l->up, HQ_DT_F16, l->gate->k);
+  p.gather_x = moe_tensor_rows(l->gate, p.rows) && (l->up == nullptr || moe_tensor_rows(l->up, p.rows)) &&
+               tensor_path_ok(l->gate, l->up, HQ_DT_F16, l->gate->k);
   int64_t o = 0;
   p.off_ids = o;    o += up256(p.rows * 4);
   p.off_w = o;      o += up256(p.rows * 4);

@@ -113,14 +113,6 @@ PyObject* py_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return reinterpret_cast<PyObject*>(l);
 }
 
-// the library's own rule for sending a call to the tensor-core GEMM (rows of f16)
-bool tensor_path(const hq_weight& w, int64_t rows, bool dense) {
-  if (w.k % 64 != 0 || (w.format == HQ_FMT_FP8_BLOCK && w.k % 128 != 0)) return false;
-  const int64_t mult = w.format == HQ_FMT_Q8_0 ? 4 : 1;
-  if (dense) return rows >= mult * hq_config_get(HQ_CFG_DENSE_TENSOR_MIN_ROWS);
-  return rows >= mult * hq_config_get(HQ_CFG_MOE_TENSOR_MIN_ROWS) * w.n_experts;
-}
-
 // rows of a [.., k] activation as the library reads them
 struct Rows {
   at::Tensor hold;
@@ -210,7 +202,7 @@ PyObject* py_linear(PyObject*, PyObject* const* p, Py_ssize_t n) {
   const cudaStream_t s = stream_of(a);
   const at::ScalarType od = dtype_or(p[2], a.scalar_type());
   Rows x = rows_of(a, l->w.k);
-  if (tensor_path(l->w, x.m, true)) to_f16(x, l->w.k, a, l->status_ptr(), s);
+  if (hq_tensor_path(&l->w, x.m, 1)) to_f16(x, l->w.k, a, l->status_ptr(), s);
   return THPVariable_Wrap(run_linear(l, a, od, x, s));
   HQ_CATCH
 }
@@ -225,7 +217,7 @@ PyObject* py_qkv(PyObject*, PyObject* const* p, Py_ssize_t n) {
   const cudaStream_t s = stream_of(a);
   const at::ScalarType od = dtype_or(p[4], a.scalar_type());
   Rows x = rows_of(a, l[0]->w.k);
-  if (tensor_path(l[0]->w, x.m, true)) to_f16(x, l[0]->w.k, a, l[0]->status_ptr(), s);
+  if (hq_tensor_path(&l[0]->w, x.m, 1)) to_f16(x, l[0]->w.k, a, l[0]->status_ptr(), s);
   PyObject* out = PyTuple_New(3);
   if (out == nullptr) return nullptr;
   for (int i = 0; i < 3; ++i) {
@@ -252,7 +244,7 @@ PyObject* py_glu(PyObject*, PyObject* const* p, Py_ssize_t n) {
   const cudaStream_t s = stream_of(a);
   const at::ScalarType od = dtype_or(p[4], a.scalar_type());
   Rows x = rows_of(a, g->w.k);
-  if (tensor_path(g->w, x.m, true)) to_f16(x, g->w.k, a, g->status_ptr(), s);
+  if (hq_tensor_path(&g->w, x.m, 1)) to_f16(x, g->w.k, a, g->status_ptr(), s);
   at::Tensor y = out_like(a, g->w.n, od);
   check(hq_linear_glu_forward(&g->w, &u->w, act, x.ptr, x.dtype, x.stride, y.data_ptr(), dt_code(od), g->w.n, x.m,
                               g->status_ptr(), s),

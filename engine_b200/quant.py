@@ -97,19 +97,9 @@ def gather_rows_f16(x: torch.Tensor, row_map: torch.Tensor, n_valid: torch.Tenso
 
 
 def tensor_path_expected(layer, n_rows_total: int, dense: bool) -> bool:
-    """Mirror of the C-side rule that sends a call to the tensor-core grouped GEMM (prefill-sized row counts,
-    K % 64 == 0; Q8_0 from four times the configured row thresholds, because its decode kernel streams at HBM
-    speed).  Used only to decide whether to hand activations over as f16, which that kernel copies into its
-    operand tiles without a conversion pass."""
-    if layer.k % 64:
-        return False
-    if layer.format == L.FMT_FP8_BLOCK and layer.k % 128:
-        return False
-    lib = L.lib()
-    mult = 4 if layer.format == L.FMT_Q8_0 else 1
-    if dense:
-        return n_rows_total >= mult * lib.hq_config_get(L.CFG_DENSE_TENSOR_MIN_ROWS)
-    return n_rows_total >= mult * lib.hq_config_get(L.CFG_MOE_TENSOR_MIN_ROWS) * layer.n_experts
+    """Whether the library sends a call to the tensor-core GEMM, given f16 rows (hq_tensor_path)."""
+    w = layer._weight_struct()
+    return bool(L.lib().hq_tensor_path(C.byref(w), n_rows_total, int(dense)))
 
 
 class QuantMethod:
@@ -388,11 +378,15 @@ class MXFP4Layer(QuantMethod):
         if self.k % 32 or tuple(scales.shape[-2:]) != (self.n, self.k // 32):
             raise L.HqError("MXFP4: K must be a multiple of 32 and scales [.., N, K/32]")
         self.bias = None if bias is None else bias.contiguous()
+        # block scales the f16 operands of the tensor cores hold exactly (2^-14 .. 2^13, or zero): looked at once here
+        odd = (self.scales - 1).view(torch.uint8)          # 0 -> 255, so one comparison covers 1 .. 112
+        self._f16_scales = not bool(((odd < 112) | ((odd > 139) & (odd < 255))).any())
 
     def _weight_struct(self):
         return L.HqWeight(self.format, self.n_experts, self.n, self.k, self.blocks.data_ptr(),
                           self.scales.data_ptr(), 0 if self.bias is None else self.bias.data_ptr(),
-                          0 if self.bias is None else dt_code(self.bias.dtype), 0)
+                          0 if self.bias is None else dt_code(self.bias.dtype),
+                          L.WEIGHT_F16_SCALES if self._f16_scales else 0)
 
     def _3d_input_is_per_slot(self):
         return True

@@ -94,6 +94,11 @@ extern "C" {
  * exact byte layout the reference keeps on the device (hanzo-quant
  * kernels/mmvq_gguf/mmvq_gguf.cu:134-170, src/blockwise_fp8/mod.rs:24-30,
  * src/mxfp4/mod.rs:29-41).  Expert e starts at data + e*N*row_bytes. */
+/* hq_weight.flags.  MXFP4: every block scale is zero or within 2^-14 .. 2^13 (e8m0 byte 0 or 113 .. 140), which the host
+ * has checked once.  The f16 operands of the tensor-core GEMM hold such scales exactly, so that kernel then serves calls
+ * of any row count; without the flag a small call stays on the decode kernel, which applies scales in f32. */
+#define HQ_WEIGHT_F16_SCALES 1
+
 typedef struct hq_weight {
   int32_t format;      /* HQ_FMT_* */
   int32_t n_experts;   /* 1 for a dense layer */
@@ -103,7 +108,7 @@ typedef struct hq_weight {
   const void* scales;  /* FP8: f32 [E, ceil(N/128), ceil(K/128)]; MXFP4: u8 [E, N, K/32]; else NULL */
   const void* bias;    /* optional [E, N] in bias_dtype, or NULL */
   int32_t bias_dtype;  /* HQ_DT_* */
-  int32_t reserved;
+  int32_t flags;       /* HQ_WEIGHT_* bits, 0 by default */
   /* FP8 only, optional: tables written once per layer by hq_fp8_scale_prepare.  With them the
    * prefill-sized calls run on the tensor cores; without them every call takes the decode kernel. */
   const void* fp8_tile_scale;  /* f32 [E, ceil(N/128)] */
@@ -485,6 +490,11 @@ int32_t hq_fp8_block_dequant(const uint8_t* codes, const float* scales, int64_t 
  * element, hanzo-quant/kernels/blockwise_fp8/blockwise_fp8_gemm.cu:47-124). */
 int32_t hq_fp8_scale_prepare(const float* scales, int32_t n_experts, int64_t n, int64_t k, float* tile_scale_out,
                              float* rel_scale_out, void* stream);
+
+/* 1 when a call on this layer with `rows` activation rows (dense = 0: rows = n_tokens * top_k assignments over the
+ * expert bank) runs on the tensor-core GEMM provided the activations are f16, else 0.  Hosts use it to decide whether to
+ * convert (hq_convert_status) or gather (hq_gather_rows_f16) first. */
+int32_t hq_tensor_path(const hq_weight* w, int64_t rows, int32_t dense);
 
 /* Elementwise dtype conversion (f32 / f16 / bf16).  The prefill-sized calls run on the tensor cores only
  * when the activations are f16 (their rows are copied straight into the operand tiles); a host holding

@@ -38,7 +38,7 @@ pub struct hq_weight {
     pub scales: *const c_void,
     pub bias: *const c_void,
     pub bias_dtype: i32,
-    pub reserved: i32,
+    pub flags: i32,
     pub fp8_tile_scale: *const c_void,
     pub fp8_rel_scale: *const c_void,
 }

@@ -61,3 +61,25 @@ def test_expert_rows_cut_into_equal_tiles(per_expert):
     want = np.einsum("tk,tsnk->tsn", x.float().cpu().numpy(), deq[ids])
     assert layer.device_status()[0] == 0
     assert T.rel_l2(got, want) <= 1e-3
+
+
+@pytest.mark.parametrize("m", [1, 8])
+@pytest.mark.parametrize("byte", [112, 113, 140, 141])
+def test_mxfp4_rows_by_scale_range(byte, m):
+    # e8m0 bytes 113 .. 140 are exact f16 operands: any row count takes the tensor cores; beyond, few rows do not
+    from engine_b200 import _lib as L
+    from engine_b200.quant import MXFP4Layer, tensor_path_expected
+    n, k = 192, 320
+    g = torch.Generator().manual_seed(byte)
+    blocks = torch.randint(0, 256, (n, k // 2), generator=g, dtype=torch.uint8)
+    scales = torch.randint(113, 141, (n, k // 32), generator=g, dtype=torch.uint8)
+    scales[5, 3], scales[7, 1] = byte, 0
+    layer = MXFP4Layer(blocks.to(DEV), scales.to(DEV))
+    inside = 113 <= byte <= 140
+    assert bool(layer._weight_struct().flags & L.WEIGHT_F16_SCALES) == inside
+    assert tensor_path_expected(layer, m, dense=True) == inside
+    x = torch.randn((m, k), generator=g).to(DEV, torch.bfloat16)
+    got = layer.forward_raw(x, torch.float32)
+    assert layer.device_status()[0] == 0
+    want = x.double() @ layer.dequantize_w().double().t()
+    assert float((got.double() - want).norm() / want.norm()) <= 1e-5
