@@ -34,11 +34,11 @@
 #include <cuda.h>
 
 #include "hq_dequant.cuh"
+#include "hq_warp_issue.cuh"
 
 namespace hq {
 
-constexpr uint32_t kDqSpin = 1u << 16;       // polls of a wait, each suspended for up to kDqSuspendNs
-constexpr uint32_t kDqSuspendNs = 20000;
+constexpr uint32_t kDqSpin = 1u << 16;       // polls of a wait, each suspended for a while
 constexpr int kDqMaxTokens = 256;
 constexpr int kDqExpandWarps = 16;
 constexpr int kDqTokenWarps = 2;
@@ -390,7 +390,7 @@ __device__ __forceinline__ bool dq_wait_cluster(uint64_t* bar, uint32_t parity, 
         "selp.u32 %0, 1, 0, p;\n"
         "}\n"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(kDqSuspendNs)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(kWaitSuspendNs)
         : "memory");
     if (ok) return true;
   }
@@ -421,78 +421,6 @@ __device__ __forceinline__ void dq_mma64(uint32_t d, uint32_t a, uint64_t b, uin
       "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void dq_commit(uint64_t* bar) {
-  asm volatile(
-      "{\n"
-      ".reg .pred e;\n"
-      "elect.sync _|e, 0xffffffff;\n"
-      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
-      "}\n" ::"r"(smem_u32(bar))
-      : "memory");
-}
-
-// box copies by the elected lane of a whole warp
-__device__ __forceinline__ void dq_tma_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
-  asm volatile(
-      "{\n"
-      ".reg .pred e;\n"
-      "elect.sync _|e, 0xffffffff;\n"
-      "@e cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n"
-      "}\n" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ void dq_tma_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile(
-      "{\n"
-      ".reg .pred e;\n"
-      "elect.sync _|e, 0xffffffff;\n"
-      "@e cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
-      "}\n" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// Bounded wait whose polls suspend the warp for long: twenty-odd warps that poll at the default rate keep the barrier unit
-// busy enough to slow down the arrivals and copy instructions of the others.
-__device__ __forceinline__ bool dq_wait(uint64_t* bar, uint32_t parity, uint32_t spin_limit) {
-  for (uint32_t i = 0; i < spin_limit; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(kDqSuspendNs)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-// mbarrier arrivals by the elected lane of a whole warp, as a predicated instruction: a branch for one lane costs the
-// other roles' warps instruction fetches (and this one several hundred cycles when it misses)
-__device__ __forceinline__ void dq_arrive(uint64_t* bar) {
-  asm volatile(
-      "{\n"
-      ".reg .pred e;\n"
-      "elect.sync _|e, 0xffffffff;\n"
-      "@e mbarrier.arrive.shared::cta.b64 _, [%0];\n"
-      "}\n" ::"r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ void dq_arrive_expect(uint64_t* bar, uint32_t bytes) {
-  asm volatile(
-      "{\n"
-      ".reg .pred e;\n"
-      "elect.sync _|e, 0xffffffff;\n"
-      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
-      "}\n" ::"r"(smem_u32(bar)),
-      "r"(bytes)
-      : "memory");
-}
-
 constexpr int kDqMaxStages = 8, kDqMaxRaw = 12;
 constexpr int kDqNumBars = 2 * kDqMaxStages + 2 * kDqMaxRaw + 4 + 2;   // operand ring, raw ring, accumulators, exchange
 struct DqBars {
@@ -572,7 +500,7 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
     for (int rs = rs_lo; rs < rs_hi; ++rs) {
       const uint32_t sc = sc_next;
       if (SIDE && rs + 1 < rs_hi) sc_next = fetch_side(rs + 1);
-      if (!dq_wait(&bar.full_r[slot], ph, spin)) {
+      if (!warp_wait(&bar.full_r[slot], ph, spin)) {
         if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 500 + slot);
         spin = 1;
       }
@@ -587,7 +515,7 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
 #pragma unroll 1
         for (int i = 0; i < 2; ++i) {
           ok = row.half(C, i, [&](int at_pair, const uint32_t (&v)[8]) {
-            if (i == 0 && at_pair == 0 && at.use > 0 && !dq_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
+            if (i == 0 && at_pair == 0 && at.use > 0 && !warp_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
               if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 520 + at.s);
               spin = 1;
             }
@@ -596,23 +524,23 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
         }
         // every byte of the raw stage this warp needs has been read
         __syncwarp();
-        dq_arrive(&bar.empty_r[slot]);
+        warp_arrive(&bar.empty_r[slot]);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        dq_arrive(&bar.full[at.s]);
+        warp_arrive(&bar.full[at.s]);
         if (FMT == HQ_FMT_MXFP4 && !ok && n_ok) report_status(p.status, HQ_DEV_SCALE_RANGE, 600);
       } else {
         __syncwarp();
-        dq_arrive(&bar.empty_r[slot]);
+        warp_arrive(&bar.empty_r[slot]);
         // the K tail ends inside this group's stage: nothing to add, but the stage counts its arrivals
         if (local < slice_stages) {
-          if (at.use > 0 && !dq_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
+          if (at.use > 0 && !warp_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
             if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 521);
             spin = 1;
           }
           __syncwarp();
-          dq_arrive(&bar.full[at.s]);
+          warp_arrive(&bar.full[at.s]);
         }
       }
       if (!T::WIDE) mis = (mis + T::SB) & (pl.raw_tma ? 15u : 2u);
@@ -714,7 +642,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       const uint32_t idesc = make_idesc_f16(__shfl_sync(0xffffffffu, max(16, (t.count + 15) & ~15), 0));
       const int buf = pl.nbuf == 2 ? tcount & 1 : 0;
       const int use = pl.nbuf == 2 ? tcount >> 1 : tcount;
-      if (use > 0 && !dq_wait(&bar.acc_empty[buf], (use - 1) & 1, spin)) {
+      if (use > 0 && !warp_wait(&bar.acc_empty[buf], (use - 1) & 1, spin)) {
         if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 300 + buf);
         spin = 1;
       }
@@ -722,7 +650,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       const uint32_t d0 = tmem_u + (uint32_t)(buf * pl.tn);
       for (int j = 0; j < slice_subs; j += pl.subs, ++it) {
         const DqSlot at = dq_slot(pl, it);
-        if (!dq_wait(&bar.full[at.s], at.use & 1, spin)) {
+        if (!warp_wait(&bar.full[at.s], at.use & 1, spin)) {
           if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 310 + at.s);
           spin = 1;
         }
@@ -735,9 +663,9 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           bdesc += sub_bytes >> 4;
           a0 += 32;
         }
-        dq_commit(&bar.empty[at.s]);
+        warp_commit(&bar.empty[at.s]);
       }
-      dq_commit(&bar.acc_full[buf]);
+      warp_commit(&bar.acc_full[buf]);
     }
     __syncwarp();
   } else if (warp <= kDqEpilogueWarps) {
@@ -767,7 +695,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       float sc = 1.f;
       if (FMT == HQ_FMT_FP8_BLOCK)
         sc = __ldg((bank == 0 ? p.fp8_tile_scale : p.fp8_tile_scale_up) + (int64_t)t.expert * p.fp8_nb + t.n0 / 128);
-      if (!dq_wait(&bar.acc_full[buf], use & 1, spin)) {
+      if (!warp_wait(&bar.acc_full[buf], use & 1, spin)) {
         if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 400 + buf);
         spin = 1;
         failed = true;                 // nothing is stored once a wait has run out
@@ -827,7 +755,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         else columns([](float f) { return f; });
         tc_fence_before();               // the buffer is read out: the next tile may accumulate into it
         __syncwarp();
-        dq_arrive(&bar.acc_empty[buf]);
+        warp_arrive(&bar.acc_empty[buf]);
       } else {
         // ---- split K: token column c is finished by CTA c / cpc of the cluster ------------------------
         const int cpc = (t.count + S - 1) / S;
@@ -857,7 +785,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         }
         tc_fence_before();
         __syncwarp();
-        dq_arrive(&bar.acc_empty[buf]);
+        warp_arrive(&bar.acc_empty[buf]);
         if (lane < S) dq_arrive_remote(dq_mapa(redf_u, (uint32_t)lane));
         if (!dq_wait_cluster(bar.red_full, tcount & 1, spin)) {
           if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 420);
@@ -902,19 +830,19 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
             if (++slot == pl.nr) { slot = 0; ph ^= 1; wrapped = true; }
             continue;
           }
-          if (wrapped && !dq_wait(&bar.empty_r[slot], ph ^ 1, spin)) {
+          if (wrapped && !warp_wait(&bar.empty_r[slot], ph ^ 1, spin)) {
             if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 560 + slot);
             stop = true;               // nothing more is issued: the target may still be in use
             break;
           }
-          dq_arrive_expect(&bar.full_r[slot], (uint32_t)T::STAGE);
+          warp_arrive_expect(&bar.full_r[slot], (uint32_t)T::STAGE);
           const uint32_t dst = smem_u32(smem + pl.off_raw) + (uint32_t)slot * T::STAGE;
           const int x = ((rs * T::SB) & ~15) / 2;            // 16-bit elements
           for (int b = 0; b < banks; ++b) {
             if constexpr (T::BOXES == 2)
-              dq_tma_3d(dst + b * 16384u, b ? &tm_wu : &tm_w, 0, row, 2 * rs, &bar.full_r[slot]);
+              warp_tma_3d(dst + b * 16384u, b ? &tm_wu : &tm_w, 0, row, 2 * rs, &bar.full_r[slot]);
             else
-              dq_tma_2d(dst + b * (64u * T::PITCH), b ? &tm_wu : &tm_w, x, row, &bar.full_r[slot]);
+              warp_tma_2d(dst + b * (64u * T::PITCH), b ? &tm_wu : &tm_w, x, row, &bar.full_r[slot]);
           }
           if (++slot == pl.nr) { slot = 0; ph ^= 1; wrapped = true; }
         }
@@ -938,26 +866,26 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           const uint32_t bytes = (uint32_t)(boxes * pl.x_box + 16 * pieces) * 128u;
           for (int j = 0; j < slice_subs; j += pl.subs, ++it) {
             const DqSlot at = dq_slot(pl, it);
-            if (at.use > 0 && !dq_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
+            if (at.use > 0 && !warp_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
               if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 540 + at.s);
               stop = true;
               break;
             }
             if (pl.x_stage) {
-              dq_arrive_expect(&bar.full[at.s], (uint32_t)pl.subs * sub_bytes);
-              dq_tma_3d(smem_u32(smem) + (uint32_t)(at.s * pl.subs) * sub_bytes, &tm_x, 0, t.row_start, 4 * rs_lo + j,
+              warp_arrive_expect(&bar.full[at.s], (uint32_t)pl.subs * sub_bytes);
+              warp_tma_3d(smem_u32(smem) + (uint32_t)(at.s * pl.subs) * sub_bytes, &tm_x, 0, t.row_start, 4 * rs_lo + j,
                         &bar.full[at.s]);
               continue;
             }
             const int n_sub = min(pl.subs, slice_subs - j);
-            dq_arrive_expect(&bar.full[at.s], bytes * (uint32_t)n_sub);
+            warp_arrive_expect(&bar.full[at.s], bytes * (uint32_t)n_sub);
             for (int c = 0; c < n_sub; ++c) {
               const int x = (4 * rs_lo + j + c) * 64;
               uint32_t dst = smem_u32(smem) + (uint32_t)(at.s * pl.subs + c) * sub_bytes;
               int row = t.row_start;
               for (int i = 0; i < boxes; ++i, row += pl.x_box, dst += (uint32_t)pl.x_box * 128u)
-                dq_tma_2d(dst, &tm_x, x, row, &bar.full[at.s]);
-              for (int i = 0; i < pieces; ++i, row += 16, dst += 2048u) dq_tma_2d(dst, &tm_x16, x, row, &bar.full[at.s]);
+                warp_tma_2d(dst, &tm_x, x, row, &bar.full[at.s]);
+              for (int i = 0; i < pieces; ++i, row += 16, dst += 2048u) warp_tma_2d(dst, &tm_x16, x, row, &bar.full[at.s]);
             }
           }
         }
@@ -973,7 +901,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       auto hand_over = [&]() {
         fence_proxy_async_smem();     // the copies are visible to the tensor core (async proxy)
         __syncwarp();
-        dq_arrive(&bar.full[dq_slot(pl, done).s]);
+        warp_arrive(&bar.full[dq_slot(pl, done).s]);
         ++done;
       };
       for (int w = first; w < n_tiles; w += step, ++tcount) {
@@ -988,7 +916,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         named_bar_sync(1, 32 * kDqTokenWarps);
         for (int j = 0; j < slice_subs; j += pl.subs, ++it) {
           const DqSlot at = dq_slot(pl, it);
-          if (at.use > 0 && !dq_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
+          if (at.use > 0 && !warp_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
             if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 540 + at.s);
             spin = 1;
           }
@@ -1024,7 +952,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const int rows_valid = min(fw, p.n - t.n0);
         const int64_t tile_off = ((int64_t)t.expert * p.n + t.n0) * p.w_row_bytes;
         for (int rs = rs_lo; rs < rs_hi; ++rs) {
-          if (wrapped && !dq_wait(&bar.empty_r[slot], ph ^ 1, spin)) {
+          if (wrapped && !warp_wait(&bar.empty_r[slot], ph ^ 1, spin)) {
             if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 570 + slot);
             spin = 1;
           }

@@ -100,7 +100,7 @@ struct Fp8GroupedParams {
   void* y;                      // plain mode output
   int y_dtype;
   int64_t y_stride;
-  bool y_vec_ok;                // set by the launcher: output row segments can be written with 16-byte stores
+  bool y_pair_ok;               // set by the launcher: 16-bit outputs can be written two at a time
   uint8_t* hq;                  // gated mode output: e4m3 codes [n_rows, N] ...
   float* hs;                    // ... and scales [n_rows, N/128] of act(gate) * up, expert-sorted
   hq_act_args act;
@@ -109,7 +109,6 @@ struct Fp8GroupedParams {
   int32_t* status;
   uint32_t spin_limit;          // polls per bounded wait (0 = default)
   int test_skip_producer;       // test hook: the TMA warp issues nothing, so every consumer wait runs out
-  int load_burst;               // 128-column blocks the TMA warp requests together: 1, 2 or 4 (0 = default)
   int load_burst_prefetch_off;  // 1 = do not pull weight rows into L2 ahead of the operand copies
   int l2_prefetch;              // set by the launcher
 };

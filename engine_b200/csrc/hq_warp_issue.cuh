@@ -1,0 +1,87 @@
+// Copies, arrivals, commits and waits issued by a whole warp: the instruction is predicated on the lane elect.sync picks,
+// the warp does not branch.  From a branch for one lane a tcgen05.mma costs about 75 cycles and a commit 125, whatever the
+// width; a round {wait, arrive, copy} of an issuing warp stays a chain of about five hundred cycles, so what a round copies
+// should be large, or several warps take the rounds in turn.
+#pragma once
+#include <cuda.h>
+
+#include "hq_common.cuh"
+
+namespace hq {
+
+constexpr uint32_t kWaitSuspendNs = 20000;
+
+// Bounded wait whose polls suspend the warp for long: twenty-odd warps that poll at the default rate keep the barrier unit
+// busy enough to slow down the arrivals and copy instructions of the others.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, uint32_t spin_limit) {
+  for (uint32_t i = 0; i < spin_limit; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(kWaitSuspendNs)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+// mbarrier arrivals by the elected lane of a whole warp, as a predicated instruction: a branch for one lane costs the
+// other roles' warps instruction fetches (and this one several hundred cycles when it misses)
+__device__ __forceinline__ void warp_arrive(uint64_t* bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e mbarrier.arrive.shared::cta.b64 _, [%0];\n"
+      "}\n" ::"r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void warp_arrive_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
+      "}\n" ::"r"(smem_u32(bar)),
+      "r"(bytes)
+      : "memory");
+}
+
+// box copies by the elected lane of a whole warp
+__device__ __forceinline__ void warp_tma_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n"
+      "}\n" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void warp_tma_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
+      "}\n" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
+      : "memory");
+}
+
+// tcgen05.commit by the elected lane
+__device__ __forceinline__ void warp_commit(uint64_t* bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(smem_u32(bar))
+      : "memory");
+}
+
+}  // namespace hq
