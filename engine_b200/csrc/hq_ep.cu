@@ -141,7 +141,8 @@ __global__ void __launch_bounds__(256) ep_unpack_meta_kernel(const hq_ep_layout 
 }
 
 // dst row r = src row row_map[r] for r < *n_valid: e4m3 codes (k bytes) and their k / 128 scales, each side with
-// its own row stride.  One warp per row.
+// its own row stride.  One warp per row, four 16-byte loads in flight per lane.  Bound by the codes written (the sources
+// are re-read from L2, once per slot of a token).
 __global__ void __launch_bounds__(256) fp8_gather_rows_kernel(const uint8_t* __restrict__ src_codes,
                                                               int64_t src_code_stride,
                                                               const uint8_t* __restrict__ src_scales,
@@ -150,6 +151,8 @@ __global__ void __launch_bounds__(256) fp8_gather_rows_kernel(const uint8_t* __r
                                                               const int32_t* __restrict__ n_valid, int64_t n_rows,
                                                               int k, uint8_t* __restrict__ codes,
                                                               float* __restrict__ scales) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   const int64_t limit = n_valid != nullptr ? min((int64_t)*n_valid, n_rows) : n_rows;
@@ -157,7 +160,15 @@ __global__ void __launch_bounds__(256) fp8_gather_rows_kernel(const uint8_t* __r
   const int64_t src = row_map != nullptr ? (int64_t)row_map[row] : row;
   const uint4* sc = reinterpret_cast<const uint4*>(src_codes + src * src_code_stride);
   uint4* dc = reinterpret_cast<uint4*>(codes + row * k);
-  for (int i = lane; i < k / 16; i += 32) dc[i] = sc[i];
+  for (int i0 = lane; i0 < k / 16; i0 += 128) {
+    uint4 v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + 32 * j < k / 16) v[j] = sc[i0 + 32 * j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + 32 * j < k / 16) dc[i0 + 32 * j] = v[j];
+  }
   const float* ss = reinterpret_cast<const float*>(src_scales + src * src_scale_stride);
   for (int i = lane; i < k / 128; i += 32) scales[row * (k / 128) + i] = ss[i];
 }
@@ -270,10 +281,9 @@ int32_t launch_fp8_gather_rows(const void* src_codes, int64_t src_code_stride, c
                                int64_t src_scale_stride, const int32_t* row_map, const int32_t* n_valid,
                                int64_t n_rows, int64_t k, uint8_t* codes, float* scales, cudaStream_t stream) {
   if (n_rows == 0) return HQ_OK;
-  fp8_gather_rows_kernel<<<(unsigned)((n_rows + 7) / 8), 256, 0, stream>>>(
-      (const uint8_t*)src_codes, src_code_stride, (const uint8_t*)src_scales, src_scale_stride, row_map, n_valid,
-      n_rows, (int)k, codes, scales);
-  return cudaGetLastError() == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
+  return launch_pdl(fp8_gather_rows_kernel, dim3((unsigned)((n_rows + 7) / 8)), 256, 0, stream, 1, (const uint8_t*)src_codes,
+                    src_code_stride, (const uint8_t*)src_scales, src_scale_stride, row_map, n_valid, n_rows, (int)k, codes,
+                    scales);
 }
 
 int32_t launch_ep_push(const void* send, void* const* peers, int world, int rank, int64_t slab_bytes,

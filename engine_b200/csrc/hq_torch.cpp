@@ -445,14 +445,28 @@ PyObject* py_moe_fp8(PyObject*, PyObject* const* p, Py_ssize_t n) {
   const Tables tb(sc, r.t, r.k, e);
   const int64_t xq = sc.add(rows * hidden), xsc = sc.add(rows * (hidden / 128) * 4), hq = sc.add(rows * inter),
                 hs = sc.add(rows * (inter / 128) * 4), y = sc.add(rows * d->w.n * (yd == at::kFloat ? 4 : 2));
+  // A token's row stands in the sorted order once per slot.  Quantizing it each time is bound by the divisions (4,096 tokens x
+  // 8 slots x 7,168: 270 us); from about a thousand rows the tokens are quantized once and their codes copied (launch and copy
+  // cost less than the divisions saved).
+  const bool once = r.k > 1 && rows >= 1024;
+  const int64_t tq = once ? sc.add(r.t * hidden) : 0, ts = once ? sc.add(r.t * (hidden / 128) * 4) : 0;
   sc.alloc(x);
   const int32_t* bounds = (const int32_t*)(sc.base + tb.bounds);
   at::Tensor out = out_like(xs, d->w.n, od);
   const at::Tensor add = addend(p[7], od, out.numel());
   tb.build(sc, r.id_ptr(), r.t, r.k, e, s);
-  check(hq_fp8_quant_rows_n(x.data_ptr(), dt_code(x.scalar_type()), hidden, (const int32_t*)(sc.base + tb.st), bounds + e, rows,
-                            hidden, sc.base + xq, (float*)(sc.base + xsc), s),
-        "hq_fp8_quant_rows_n");
+  if (once) {
+    check(hq_fp8_quant_rows(x.data_ptr(), dt_code(x.scalar_type()), hidden, nullptr, r.t, hidden, sc.base + tq,
+                            (float*)(sc.base + ts), s),
+          "hq_fp8_quant_rows");
+    check(hq_fp8_gather_rows(sc.base + tq, hidden, (const float*)(sc.base + ts), hidden / 128 * 4, (const int32_t*)(sc.base + tb.st),
+                             bounds + e, rows, hidden, sc.base + xq, (float*)(sc.base + xsc), s),
+          "hq_fp8_gather_rows");
+  } else {
+    check(hq_fp8_quant_rows_n(x.data_ptr(), dt_code(x.scalar_type()), hidden, (const int32_t*)(sc.base + tb.st), bounds + e,
+                              rows, hidden, sc.base + xq, (float*)(sc.base + xsc), s),
+          "hq_fp8_quant_rows_n");
+  }
   check(hq_moe_fp8_gate_up_forward(&g->w, &u->w, act, sc.base + xq, (const float*)(sc.base + xsc), r.t, r.k, bounds,
                                    sc.base + hq, (float*)(sc.base + hs), g->status_ptr(), s),
         "hq_moe_fp8_gate_up_forward");
