@@ -139,3 +139,25 @@ def test_bounded_wait_runs_out_and_the_call_returns():
     torch.cuda.synchronize()
     assert layer.device_status()[0] == 0
     assert bool(torch.isfinite(y2).all())
+
+
+@pytest.mark.parametrize("m", [15, 16, 17, 32, 33, 48, 49, 96, 97, 143, 144, 145, 289])
+def test_token_tile_edges(m):
+    # tiles of 16 .. 144 tokens: one to nine 16-token groups over three epilogue warps, the next tile at 145 and 289
+    import engine_b200 as hq
+    n, k = 128, 512
+    rng = T.rng_for(9, 7)
+    arrays, deq = T.make_weight("FP8", rng, n, k)
+    layer = T.make_layer("FP8", arrays, k, DEV)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    codes, scales = hq.fp8_quantize_rows(T.to_dev(x, torch.float32, DEV))
+    y = layer.forward_fp8_rows(codes, scales, torch.float32)
+    torch.cuda.synchronize()
+    assert layer.device_status()[0] == 0
+    assert T.rel_l2(y.cpu().numpy(), M.dense_forward(_qdq(x), deq, None)) <= 1e-5
+
+
+def test_tokens_quantized_once_from_a_thousand_rows():
+    # 520 tokens x 2 slots: codes gathered into expert order, padding slots among them
+    got, want = _expert_block_case(8, 2, 512, 512, 520, 8, pad_slot=True)
+    assert T.rel_l2(got, want) <= 2e-3

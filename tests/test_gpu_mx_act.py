@@ -172,3 +172,18 @@ def test_bounded_wait_runs_out_and_the_call_returns():
     y2 = layer.forward_mx_rows(codes, scales, torch.float32)
     torch.cuda.synchronize()
     assert layer.device_status()[0] == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(40, 192, 4096), (40, 192, 6144), (130, 200, 256), (130, 384, 256), (9, 576, 2944)])
+def test_tiles_of_128_and_192_weight_rows(m, n, k):
+    # K = 6144 leaves no three stages of 192-row tiles, N = 200 would pad too far: 128-row tiles; the others 192
+    import engine_b200 as hq
+    rng = T.rng_for(11, 12)
+    arrays, deq = T.make_weight("MXFP4", rng, n, k)
+    layer = T.make_layer("MXFP4", arrays, k, DEV)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    codes, scales = hq.mxfp8_quantize_rows(T.to_dev(x, torch.float32, DEV))
+    y = layer.forward_mx_rows(codes, scales, torch.float32)
+    torch.cuda.synchronize()
+    assert layer.device_status()[0] == 0
+    assert T.rel_l2(y.cpu().numpy(), M.dense_forward(_qdq(x), deq, None)) <= 1e-5
