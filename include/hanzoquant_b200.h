@@ -133,7 +133,9 @@ int32_t hq_status_read(const int32_t* status_dev, int32_t out_host[4], void* str
 /* Tuning knobs (process-wide, read at call time).  HQ_CFG_MOE_TENSOR_MIN_ROWS: expert projections run on the
  * tensor-core grouped GEMM when n_tokens*top_k >= value * n_experts (default 8; 0 = always when the shape
  * allows, a huge value = never).  HQ_CFG_DENSE_TENSOR_MIN_ROWS: same switch for hq_linear_forward's m
- * (default 9).  Shapes the grouped GEMM does not cover (Q8_0, K % 64 != 0) always take the decode kernel. */
+ * (default 9).  Q8_0 goes there from four times either value; MXFP4 with HQ_WEIGHT_F16_SCALES from the first row while
+ * the value is at its default or below.  hq_tensor_path answers for a layer and a row count.  Shapes the tensor-core GEMM
+ * does not cover (K % 64 != 0) always take the decode kernel. */
 #define HQ_CFG_MOE_TENSOR_MIN_ROWS 0
 #define HQ_CFG_DENSE_TENSOR_MIN_ROWS 1
 /* HQ_CFG_SPIN_LIMIT: polls a kernel spends on one bounded wait before it gives up, leaves HQ_DEV_WAIT_TIMEOUT in
