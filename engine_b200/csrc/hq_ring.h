@@ -1,0 +1,29 @@
+// Which slot and which barrier phase a stage of a ring of buffers uses, and which stages a copying warp waits for before its
+// CTA exits.  Plain arithmetic, the same on the host (tests/test_ring_protocol.py) and in the kernels.
+//
+// A slot's barrier tells "use u is complete" from "use u - 1 is" by one parity bit, so a wait for use u is only sound while
+// use u - 1 is known to be complete and use u + 1 cannot be: otherwise the bit reads the wrong way round, as complete too
+// early or as incomplete for good.
+#pragma once
+
+#ifdef __CUDACC__
+#define HQ_RING_FN __host__ __device__ __forceinline__
+#else
+#define HQ_RING_FN inline
+#endif
+
+namespace hq {
+
+HQ_RING_FN int ring_slot(int stage, int slots) { return stage % slots; }
+HQ_RING_FN int ring_parity(int stage, int slots) { return (stage / slots) & 1; }
+
+// The stages whose copies a warp waits for when it has left its loop in front of stage `next` (the length of the sequence, or
+// where a wait ran out): its own -- those with stage % warps == me -- among the last `slots`.  They are the last uses of their
+// slots, so no later copy moves their barriers on, and the warp issued them, so the use before is known to be complete.
+// A slot's older stages were consumed before its last one was issued.  (A warp that waits for its last two stages whatever the
+// ring's length polls, with three slots, one that another warp has used again by then.)
+HQ_RING_FN bool ring_drains(int stage, int next, int slots, int warps, int me) {
+  return stage >= 0 && stage < next && stage >= next - slots && stage % warps == me;
+}
+
+}  // namespace hq

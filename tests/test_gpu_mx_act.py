@@ -187,3 +187,27 @@ def test_tiles_of_128_and_192_weight_rows(m, n, k):
     torch.cuda.synchronize()
     assert layer.device_status()[0] == 0
     assert T.rel_l2(y.cpu().numpy(), M.dense_forward(_qdq(x), deq, None)) <= 1e-5
+
+
+@pytest.mark.parametrize("n,k", [(3072, 3008), (3072, 4096), (2048, 6144), (2048, 7936), (1920, 9920)])
+def test_launches_end_when_the_ring_is_two_or_three_stages(n, k):
+    # K from 3,008 (tiles of 192 weight rows) and 5,888 (128): three stages, from 7,936: two.  At least two items per CTA, so
+    # that slots are used again up to the end; a wait that outlives the work costs 50 ms and more, and is reported.
+    import engine_b200 as hq
+    m = 2560
+    rng = T.rng_for(11, 13)
+    arrays, deq = T.make_weight("MXFP4", rng, n, k)
+    layer = T.make_layer("MXFP4", arrays, k, DEV)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    codes, scales = hq.mxfp8_quantize_rows(T.to_dev(x, torch.float32, DEV))
+    y = layer.forward_mx_rows(codes, scales, torch.float32)
+    marks = [torch.cuda.Event(enable_timing=True) for _ in range(21)]
+    marks[0].record()
+    for mark in marks[1:]:
+        layer.forward_mx_rows(codes, scales, torch.float32)
+        assert layer.device_status()[0] == 0
+        mark.record()
+    torch.cuda.synchronize()
+    assert max(a.elapsed_time(b) for a, b in zip(marks, marks[1:])) < 50.0
+    rows = rng.choice(m, 200, replace=False)
+    assert T.rel_l2(y.cpu().numpy()[rows], M.dense_forward(_qdq(x[rows]), deq, None)) <= 1e-5

@@ -1,0 +1,163 @@
+"""Host model of the barrier protocols of the GEMM kernels' rings: mbarriers with arrival counts, transaction bytes and one
+parity bit, the roles as coroutines that a random scheduler advances one step at a time, copies and MMAs that complete
+some time after they were issued (MMAs in order).  The index arithmetic under test is the kernels' own
+(engine_b200/csrc/hq_ring.h, compiled for the host).  A run is right when every role reaches its end, nothing is written
+that has not been read, and no barrier is arrived on more often than its count."""
+import ctypes as C
+import os
+import random
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def ring(tmp_path_factory):
+    out = tmp_path_factory.mktemp("ring")
+    src, lib = str(out / "ring.cpp"), str(out / "ring.so")
+    with open(src, "w") as f:
+        f.write('#include "hq_ring.h"\n'
+                'extern "C" int slot(int i, int n) { return hq::ring_slot(i, n); }\n'
+                'extern "C" int parity(int i, int n) { return hq::ring_parity(i, n); }\n'
+                'extern "C" int drains(int i, int next, int n, int w, int me) { return hq::ring_drains(i, next, n, w, me); }\n')
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(ROOT, "engine_b200", "csrc"), src, "-o", lib],
+                   check=True)
+    return C.CDLL(lib)
+
+
+class Wrong(Exception):
+    pass
+
+
+class Bar:
+    def __init__(self, count):
+        self.count = self.pending = count
+        self.done, self.tx = 0, 0             # completed phases; bytes still expected in this one
+
+    def arrive(self, expect=0):
+        if self.pending == 0:
+            raise Wrong("arrival beyond the count")
+        self.pending -= 1
+        self.tx += expect
+        self._turn()
+
+    def complete(self, n):
+        self.tx -= n
+        self._turn()
+
+    def _turn(self):
+        if self.pending == 0 and self.tx == 0:
+            self.done, self.pending = self.done + 1, self.count
+
+    def passed(self, parity):
+        """What a wait on the parity bit sees: the phase running now is not of this parity."""
+        return (self.done & 1) != parity
+
+
+class Machine:
+    """Roles yield None (a step) or a barrier and the parity they wait for."""
+
+    def __init__(self, seed):
+        self.rng, self.roles, self.copies, self.mmas = random.Random(seed), {}, [], []
+
+    def role(self, name, gen):
+        self.roles[name] = [gen, None]
+
+    def run(self):
+        while True:
+            ready = [n for n, (_, w) in self.roles.items() if w is None or w[0].passed(w[1])]
+            acts = [("role", n) for n in ready] + [("copy", i) for i in range(len(self.copies))] + \
+                   ([("mma", 0)] if self.mmas else [])
+            if not acts:
+                if self.roles:
+                    raise Wrong("stuck: " + ", ".join(sorted(self.roles)))
+                return
+            kind, which = self.rng.choice(acts)
+            if kind == "copy":
+                self.copies.pop(which)()
+            elif kind == "mma":
+                self.mmas.pop(0)()
+            else:
+                slot = self.roles[which]
+                try:
+                    slot[1] = next(slot[0])
+                except StopIteration:
+                    del self.roles[which]
+
+
+# ---- block-scaled expert GEMM: two copy warps that take the stages in turn --------------------------------------------
+
+def block_scaled(ring, slots, stages, seed, drain):
+    m = Machine(seed)
+    full, empty = [Bar(1 + 1) for _ in range(slots)], [Bar(1) for _ in range(slots)]
+    held = [None] * slots                     # the stage whose bytes lie in the slot and have not been read
+
+    def copy_warp(me):
+        for i in range(stages):
+            if i % 2 != me:
+                continue
+            s = ring.slot(i, slots)
+            if i >= slots:
+                yield empty[s], ring.parity(i - slots, slots)
+            if held[s] is not None:
+                raise Wrong("copy over an unread stage")
+            held[s] = i
+            full[s].arrive(1)
+            m.copies.append(lambda s=s: full[s].complete(1))
+            yield None
+        for i in drain(stages, slots, me):
+            yield full[ring.slot(i, slots)], ring.parity(i, slots)
+
+    def scale_warps(me):
+        for i in range(me, stages, 2):
+            s = ring.slot(i, slots)
+            if i >= slots:
+                yield empty[s], ring.parity(i - slots, slots)
+            full[s].arrive()
+            yield None
+
+    def mma_warp():
+        def finish(s, i):
+            if held[s] != i:
+                raise Wrong("multiplied the wrong stage")
+            held[s] = None
+            empty[s].arrive()
+        for i in range(stages):
+            s = ring.slot(i, slots)
+            yield full[s], ring.parity(i, slots)
+            m.mmas.append(lambda s=s, i=i: finish(s, i))
+            yield None
+
+    for me in (0, 1):
+        m.role(f"copy {me}", copy_warp(me))
+        m.role(f"scale {me}", scale_warps(me))
+    m.role("mma", mma_warp())
+    m.run()
+    if m.copies:
+        raise Wrong("copies in flight at the end")
+
+
+def kernel_drain(ring):
+    return lambda stages, slots, me: [i for i in range(stages - 1, -1, -1) if ring.drains(i, stages, slots, 2, me)]
+
+
+@pytest.mark.parametrize("slots", [2, 3, 4, 5, 6])
+@pytest.mark.parametrize("stages", [1, 2, 3, 5, 8, 13, 24, 39])
+def test_block_scaled_gemm_ends(ring, slots, stages):
+    for seed in range(40):
+        block_scaled(ring, slots, stages, seed, kernel_drain(ring))
+
+
+def test_the_model_finds_a_wait_that_a_later_use_has_overtaken(ring):
+    # each warp's own last two stages whatever the ring's length: with two and three slots one of them has been used again
+    own = lambda stages, slots, me: [i for i in range(stages - 1, -1, -1) if i % 2 == me][:2]
+    for slots, found in ((2, True), (3, True), (4, False), (6, False)):
+        stuck = 0
+        for seed in range(100):
+            try:
+                block_scaled(ring, slots, 24, seed, own)
+            except Wrong:
+                stuck += 1
+        assert (stuck > 0) == found, (slots, stuck)
