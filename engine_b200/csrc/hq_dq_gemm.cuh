@@ -469,7 +469,7 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
   const int subs = pl.subs, sub_shift = subs == 4 ? 2 : 1;
   const int my_stage = C >> sub_shift, my_sub = C & (subs - 1);     // stage within the raw stage, step within the stage
   const int stages_per_raw = 4 >> sub_shift;
-  const int slice_stages = (min(kb64, 4 * rs_hi) - 4 * rs_lo + subs - 1) >> sub_shift;
+  const int slice_stages = (dq_walk_steps(subs, pl.ns, min(kb64, 4 * rs_hi) - 4 * rs_lo) + subs - 1) >> sub_shift;
   const uint32_t tcol = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(512 - 32 * subs * pl.ns + 32 * my_sub);
   uint32_t spin = kDqSpin;
   int slot = 0, ph = 0, it0 = 0;
@@ -533,7 +533,7 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
       } else {
         __syncwarp();
         warp_arrive(&bar.empty_r[slot]);
-        // the K tail ends inside this group's stage: nothing to add, but the stage counts its arrivals
+        // the K tail ends inside or in front of this group's stage: nothing to add, but the stage counts its arrivals
         if (local < slice_stages) {
           if (at.use > 0 && !warp_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
             if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 521);
@@ -635,7 +635,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
     const uint32_t sub_bytes = (uint32_t)pl.tn * 128u, b0 = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
     const int a_col = 512 - 32 * pl.subs * pl.ns;
-    const int slice_subs = min(kb64, 4 * rs_hi) - 4 * rs_lo;
+    const int slice_subs = min(kb64, 4 * rs_hi) - 4 * rs_lo, walk_subs = dq_walk_steps(pl.subs, pl.ns, slice_subs);
     int it = 0, tcount = 0;
     for (int w = first; w < n_tiles; w += step, ++tcount) {
       const DqTile t = dq_tile(p, pl, pref, w, n_nt, fw);
@@ -648,7 +648,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       }
       tc_fence_after();
       const uint32_t d0 = tmem_u + (uint32_t)(buf * pl.tn);
-      for (int j = 0; j < slice_subs; j += pl.subs, ++it) {
+      for (int j = 0; j < walk_subs; j += pl.subs, ++it) {
         const DqSlot at = dq_slot(pl, it);
         if (!warp_wait(&bar.full[at.s], at.use & 1, spin)) {
           if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 310 + at.s);
@@ -852,7 +852,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     // =========================== activation rows ========================================================
     dq_pdl_wait();
     const uint32_t sub_bytes = (uint32_t)pl.tn * 128u;
-    const int slice_subs = min(kb64, 4 * rs_hi) - 4 * rs_lo;
+    const int slice_subs = min(kb64, 4 * rs_hi) - 4 * rs_lo, walk_subs = dq_walk_steps(pl.subs, pl.ns, slice_subs);
     uint32_t spin = kDqSpin;
     int it = 0;
     if (pl.x_tma) {
@@ -864,12 +864,16 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           const int boxes = t.count / pl.x_box;
           const int pieces = (t.count - boxes * pl.x_box + 15) >> 4;
           const uint32_t bytes = (uint32_t)(boxes * pl.x_box + 16 * pieces) * 128u;
-          for (int j = 0; j < slice_subs; j += pl.subs, ++it) {
+          for (int j = 0; j < walk_subs; j += pl.subs, ++it) {
             const DqSlot at = dq_slot(pl, it);
             if (at.use > 0 && !warp_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
               if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 540 + at.s);
               stop = true;
               break;
+            }
+            if (j >= slice_subs) {      // a stage without products
+              warp_arrive(&bar.full[at.s]);
+              continue;
             }
             if (pl.x_stage) {
               warp_arrive_expect(&bar.full[at.s], (uint32_t)pl.subs * sub_bytes);
@@ -914,7 +918,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           rows[r] = (uint32_t)(p.x_rows ? __ldg(p.x_rows + sp) : sp) * x_stride16;
         }
         named_bar_sync(1, 32 * kDqTokenWarps);
-        for (int j = 0; j < slice_subs; j += pl.subs, ++it) {
+        for (int j = 0; j < walk_subs; j += pl.subs, ++it) {
           const DqSlot at = dq_slot(pl, it);
           if (at.use > 0 && !warp_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
             if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 540 + at.s);

@@ -37,8 +37,8 @@ bool dq_smem_plan(DqPlan& pl, int n_experts, bool expert_indexed) {
   const int fixed = rows + pref + kDqNumBars * 8 + 16 + 1024;
   pl.ns = (512 - pl.nbuf * pl.tn) / (32 * pl.subs);
   if (pl.ns > 4) pl.ns = 4;
-  // two slots at least: a group of expanding warps meets every stage (subs = 4) or every second one (subs = 2), so its
-  // slot is never two uses behind, which one parity bit could not tell from none
+  // two slots at least: a group of expanding warps meets every stage (subs = 4) or, dq_walk_steps sees to it, every second one
+  // (subs = 2), so its slot is never two uses behind, which one parity bit could not tell from none
   const int min_ns = 2;
   for (;; --pl.ns) {
     if (pl.ns < min_ns) return false;
@@ -133,6 +133,16 @@ bool dq_plan(const GroupedParams& p, int64_t rows, DqPlan& best, int& grid) {
     }
   }
   return best_cost >= 0.0;
+}
+
+template <int FMT>
+bool dq_plan_query(const GroupedParams& p, int64_t rows, int32_t* out) {
+  DqPlan pl{};
+  int grid = 0;
+  if (!dq_plan<FMT>(p, rows, pl, grid)) return false;
+  const int32_t v[8] = {pl.tn, pl.subs, pl.ns, pl.nr, pl.nbuf, pl.kslices, grid, pl.smem};
+  for (int i = 0; i < 8; ++i) out[i] = v[i];
+  return true;
 }
 
 template <int FMT>

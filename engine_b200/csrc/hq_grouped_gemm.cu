@@ -60,4 +60,28 @@ int32_t launch_grouped_gemm(const GroupedParams& p, int64_t rows, cudaStream_t s
   }
 }
 
+template <int FMT>
+static bool plan_query(int format, const GroupedParams& p, int64_t rows, int32_t* out) {
+  if (format == FMT) return dq_plan_query<FMT>(p, rows, out);
+  if constexpr (FMT < HQ_FMT_Q3_K) return plan_query<FMT + 1>(format, p, rows, out);
+  return false;
+}
+
 }  // namespace hq
+
+// Test aid, not part of the public header: the plan of a call with `rows` activation rows (or assignments, with more than one
+// expert), `gated` = a gate and an up bank.  Eight words as in dq_plan_query; 0 = there is one.
+extern "C" int32_t hq_dq_gemm_plan(int32_t format, int64_t n, int64_t k, int32_t n_experts, int32_t gated, int64_t rows,
+                                   int32_t* out) {
+  hq::GroupedParams p{};
+  static const int32_t some_bounds = 0;
+  p.format = format;
+  p.n = (int)n;
+  p.k = (int)k;
+  p.n_experts = n_experts;
+  p.m = (int)rows;
+  p.w_up = gated ? out : nullptr;
+  p.expert_bounds = n_experts > 1 ? &some_bounds : nullptr;
+  return rows > 0 && hq::grouped_gemm_supported(format, n, k) && hq::plan_query<HQ_FMT_Q8_0>(format, p, rows, out)
+             ? HQ_OK : HQ_ERR_SHAPE;
+}

@@ -79,6 +79,10 @@ bool grouped_gemm_supported(int format, int64_t n, int64_t k);
 int32_t launch_grouped_gemm(const GroupedParams& p, int64_t rows, cudaStream_t stream);
 template <int FMT>
 int32_t launch_dq(const GroupedParams& p, int64_t rows, cudaStream_t stream);
+// the plan such a launch would take: token columns, 64-k steps per operand stage, operand slots, raw slots, accumulators, K
+// slices, CTAs, shared memory (host arithmetic)
+template <int FMT>
+bool dq_plan_query(const GroupedParams& p, int64_t rows, int32_t* out);
 int32_t launch_fp8_scale_prepare(const float* scales, int64_t n_groups, int kb, float* tile_scale, float* rel_scale,
                                  cudaStream_t stream);
 

@@ -17,7 +17,7 @@ DEV = "cuda:0"
 @pytest.mark.parametrize("fmt,n,k", [("Q4_K", 200, 1280), ("FP8", 576, 640), ("MXFP4", 130, 320)])
 def test_token_tile_edges(fmt, n, k, m):
     # MXFP4: K = 320 ends in a stage with one 64-k step; FP8: N = 576 ends in half a 128-row scale block, K = 640 in half
-    # a 256-k stage; few features: K is cut into slices
+    # a 256-k stage; few features: K is cut into slices, no CTA meets a second tile
     got, want = run_case(fmt, n, k, m, torch.float16, torch.float32, 700 + m, bias=True)
     assert T.rel_l2(got, want) <= TOL[fmt]
 
@@ -83,3 +83,54 @@ def test_mxfp4_rows_by_scale_range(byte, m):
     assert layer.device_status()[0] == 0
     want = x.double() @ layer.dequantize_w().double().t()
     assert float((got.double() - want).norm() / want.norm()) <= 1e-5
+
+
+def _plan(fmt, n, k, experts, rows):
+    import ctypes as C
+    from engine_b200 import _lib as L
+    out = (C.c_int32 * 8)()
+    f = L.lib().hq_dq_gemm_plan
+    f.argtypes = [C.c_int32, C.c_int64, C.c_int64, C.c_int32, C.c_int32, C.c_int64, C.c_void_p]
+    assert f({"FP8": L.FMT_FP8_BLOCK, "MXFP4": L.FMT_MXFP4}[fmt], n, k, experts, 0, rows, out) == 0
+    return dict(zip(("tn", "subs", "ns", "nr", "nbuf", "kslices", "grid"), out))
+
+
+def _odd_tiles_on_two_slots(fmt, n, k, experts, rows):
+    """The case is what its name says: tiles with an odd number of stages, two operand slots, a second tile for every CTA."""
+    pl = _plan(fmt, n, k, experts, rows)
+    assert (pl["subs"], pl["ns"], pl["kslices"]) == (2, 2, 1) and -(-k // 128) % 2 == 1, pl
+    tiles = experts if experts > 1 else -(-rows // pl["tn"])
+    assert tiles * (-(-n // 128)) >= 2 * pl["grid"], pl
+
+
+@pytest.mark.parametrize("fmt,n,k,m", [("FP8", 5120, 1408, 2048), ("MXFP4", 3584, 320, 2432), ("FP8", 3584, 640, 2432)])
+def test_odd_stage_counts_over_several_tiles(fmt, n, k, m):
+    _odd_tiles_on_two_slots(fmt, n, k, 1, m)
+    rng = T.rng_for(8, k)
+    arrays, deq = T.make_weight(fmt, rng, n, k)
+    layer = T.make_layer(fmt, arrays, k, DEV)
+    x = T.to_dev(rng.standard_normal((m, k)).astype(np.float32), torch.float16, DEV)
+    y = layer.forward_raw(x, torch.float32)
+    for _ in range(20):
+        assert torch.equal(layer.forward_raw(x, torch.float32), y)
+    assert layer.device_status()[0] == 0
+    assert T.rel_l2(y.cpu().numpy(), M.dense_forward(x.float().cpu().numpy(), deq, None)) <= TOL[fmt]
+
+
+def test_odd_stage_counts_over_several_expert_tiles():
+    # rows gathered in token order
+    e, n, k, topk, t = 16, 3072, 320, 2, 1200
+    _odd_tiles_on_two_slots("MXFP4", n, k, e, t * topk)
+    rng = T.rng_for(8, 2)
+    arrays, deq = T.make_weight("MXFP4", rng, n, k, experts=e)
+    layer = T.make_layer("MXFP4", arrays, k, DEV)
+    x = T.to_dev(rng.standard_normal((t, k)).astype(np.float32), torch.float16, DEV)
+    ids = np.stack([rng.choice(e, size=topk, replace=False) for _ in range(t)]).astype(np.int32)
+    ids_dev = T.to_dev(ids, torch.int32, DEV)
+    y = layer.gather_forward_raw(x, ids_dev, torch.float32)
+    for _ in range(20):
+        assert torch.equal(layer.gather_forward_raw(x, ids_dev, torch.float32), y)
+    assert layer.device_status()[0] == 0
+    some = rng.choice(t, 100, replace=False)
+    want = np.einsum("tk,tsnk->tsn", x.float().cpu().numpy()[some], deq[ids[some]])
+    assert T.rel_l2(y.cpu().numpy()[some], want) <= TOL["MXFP4"]

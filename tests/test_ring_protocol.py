@@ -21,7 +21,8 @@ def ring(tmp_path_factory):
         f.write('#include "hq_ring.h"\n'
                 'extern "C" int slot(int i, int n) { return hq::ring_slot(i, n); }\n'
                 'extern "C" int parity(int i, int n) { return hq::ring_parity(i, n); }\n'
-                'extern "C" int drains(int i, int next, int n, int w, int me) { return hq::ring_drains(i, next, n, w, me); }\n')
+                'extern "C" int drains(int i, int next, int n, int w, int me) { return hq::ring_drains(i, next, n, w, me); }\n'
+                'extern "C" int walk(int subs, int n, int steps) { return hq::dq_walk_steps(subs, n, steps); }\n')
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(ROOT, "engine_b200", "csrc"), src, "-o", lib],
                    check=True)
     return C.CDLL(lib)
@@ -161,3 +162,109 @@ def test_the_model_finds_a_wait_that_a_later_use_has_overtaken(ring):
             except Wrong:
                 stuck += 1
         assert (stuck > 0) == found, (slots, stuck)
+
+
+# ---- dequantizing GEMM: raw ring, four expanding groups, operand ring --------------------------------------------------
+
+def dequantizing(ring, slots, raw_slots, subs, steps, tiles, seed, walk):
+    """`steps` 64-k steps per tile; a raw stage holds four, an operand stage `subs`."""
+    m = Machine(seed)
+    tile_stages, raw_stages = -(-walk(subs, slots, steps) // subs), -(-steps // 4)
+    full, empty = [Bar(subs + 1) for _ in range(slots)], [Bar(1) for _ in range(slots)]
+    full_r, empty_r = [Bar(1) for _ in range(raw_slots)], [Bar(4) for _ in range(raw_slots)]
+    acc_full, acc_empty = [Bar(1) for _ in range(2)], [Bar(1) for _ in range(2)]
+    operand = {}                              # (slot, step within the stage) -> stage written and not multiplied yet
+
+    def raw_warp(me):
+        for r in range(tiles * raw_stages):
+            if r % 2 != me:
+                continue
+            s = ring.slot(r, raw_slots)
+            if r >= raw_slots:
+                yield empty_r[s], ring.parity(r - raw_slots, raw_slots)
+            full_r[s].arrive(1)
+            m.copies.append(lambda s=s: full_r[s].complete(1))
+            yield None
+
+    def group(c):
+        stage, sub = c // subs, c % subs
+        for t in range(tiles):
+            for rs in range(raw_stages):
+                r = t * raw_stages + rs
+                yield full_r[ring.slot(r, raw_slots)], ring.parity(r, raw_slots)
+                local = rs * (4 // subs) + stage
+                i = t * tile_stages + local
+                s = ring.slot(i, slots)
+                live = 4 * rs + c < steps
+                if not live:
+                    empty_r[ring.slot(r, raw_slots)].arrive()
+                    if local >= tile_stages:
+                        continue
+                if i >= slots:
+                    yield empty[s], ring.parity(i - slots, slots)
+                if live:
+                    if operand.get((s, sub)) is not None:
+                        raise Wrong("expanded over an unread operand")
+                    operand[s, sub] = i
+                    empty_r[ring.slot(r, raw_slots)].arrive()
+                    yield None
+                full[s].arrive()
+
+    def token_warp():
+        for i in range(tiles * tile_stages):
+            s = ring.slot(i, slots)
+            if i >= slots:
+                yield empty[s], ring.parity(i - slots, slots)
+            full[s].arrive(1)
+            m.copies.append(lambda s=s: full[s].complete(1))
+            yield None
+
+    def mma_warp():
+        def finish(s, i, n):
+            for sub in range(n):
+                if operand.pop((s, sub), None) != i:
+                    raise Wrong("multiplied the wrong operand")
+            empty[s].arrive()
+        for t in range(tiles):
+            if t >= 2:
+                yield acc_empty[t % 2], ring.parity(t - 2, 2)
+            for j in range(tile_stages):
+                i = t * tile_stages + j
+                s = ring.slot(i, slots)
+                yield full[s], ring.parity(i, slots)
+                m.mmas.append(lambda s=s, i=i, n=min(subs, steps - j * subs): finish(s, i, n))
+                yield None
+            m.mmas.append(lambda t=t: acc_full[t % 2].arrive())
+
+    def epilogue():
+        for t in range(tiles):
+            yield acc_full[t % 2], ring.parity(t, 2)
+            yield None
+            acc_empty[t % 2].arrive()
+
+    for me in (0, 1):
+        m.role(f"raw {me}", raw_warp(me))
+    for c in range(4):
+        m.role(f"group {c}", group(c))
+    for name, gen in (("tokens", token_warp()), ("mma", mma_warp()), ("epilogue", epilogue())):
+        m.role(name, gen)
+    m.run()
+
+
+@pytest.mark.parametrize("steps", [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 22, 45])
+@pytest.mark.parametrize("slots,raw_slots,subs", [(2, 2, 2), (2, 5, 2), (3, 3, 2), (4, 2, 2), (2, 2, 4), (4, 4, 4)])
+def test_dequantizing_gemm_rings(ring, slots, raw_slots, subs, steps):
+    for seed in range(30):
+        dequantizing(ring, slots, raw_slots, subs, steps, 5, seed, ring.walk)
+
+
+def test_the_model_finds_a_slot_two_uses_behind(ring):
+    # tiles walked for their own stages only: wrong with two slots and an odd number of them
+    for slots, steps, found in ((2, 5, True), (2, 10, True), (2, 45, True), (2, 8, False), (3, 5, False), (3, 45, False)):
+        wrong = 0
+        for seed in range(300):
+            try:
+                dequantizing(ring, slots, 5, 2, steps, 5, seed, lambda subs, n, k: k)
+            except Wrong:
+                wrong += 1
+        assert (wrong > 0) == found, (slots, steps, wrong)
