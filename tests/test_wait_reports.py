@@ -1,0 +1,34 @@
+"""Every bounded wait of the kernels leaves HQ_DEV_WAIT_TIMEOUT in the status word when it runs out: a wait that gives up in
+silence hides a stall of many milliseconds behind a right result.  Read from the source: no such wait can be made to run out
+on the GPU one by one."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "engine_b200", "csrc")
+WAIT = re.compile(r"\b(warp_wait|warp_drain|mbar_wait|mbar_wait_backoff|dq_wait_cluster)\s*\(")
+DEFINITION = re.compile(r"__device__ __forceinline__ bool \w+\(")
+
+
+def silent_waits(text):
+    """Lines with a wait whose result is not followed by a report within the branch it opens."""
+    lines = text.split("\n")
+    inside, out = False, []                   # inside: the body of one of the wait functions themselves
+    for i, line in enumerate(lines):
+        if DEFINITION.search(line):
+            inside = True
+        if not inside and WAIT.search(line.split("//")[0]) and "report_status" not in " ".join(lines[i:i + 4]):
+            out.append(i + 1)
+        if line.startswith("}"):
+            inside = False
+    return out
+
+
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))))
+def test_a_wait_that_runs_out_is_reported(name):
+    assert silent_waits(open(os.path.join(CSRC, name)).read()) == []
+
+
+def test_a_silent_wait_is_found():
+    assert silent_waits("  for (;;)\n    if (!warp_wait(&full[i], 0, spin)) break;\n  }\n  next();\n  done();\n") == [2]
