@@ -448,7 +448,7 @@ __device__ __forceinline__ DqSlot dq_slot(const DqPlan& pl, int i) {
   return r;
 }
 
-template <int FMT>
+template <int FMT, bool ODD>
 __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const DqPlan& pl, uint8_t* smem, int n_tiles,
                                                 int n_nt, int rs_lo, int rs_hi, int first, int step, uint32_t tmem_base,
                                                 int C, int q, int lane) {
@@ -469,7 +469,7 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
   const int subs = pl.subs, sub_shift = subs == 4 ? 2 : 1;
   const int my_stage = C >> sub_shift, my_sub = C & (subs - 1);     // stage within the raw stage, step within the stage
   const int stages_per_raw = 4 >> sub_shift;
-  const int slice_stages = (dq_walk_steps(subs, pl.ns, min(kb64, 4 * rs_hi) - 4 * rs_lo) + subs - 1) >> sub_shift;
+  const int slice_stages = (dq_walk_steps(ODD, min(kb64, 4 * rs_hi) - 4 * rs_lo) + subs - 1) >> sub_shift;
   const uint32_t tcol = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(512 - 32 * subs * pl.ns + 32 * my_sub);
   uint32_t spin = kDqSpin;
   int slot = 0, ph = 0, it0 = 0;
@@ -550,8 +550,10 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
   }
 }
 
-template <int FMT>
-__global__ void __launch_bounds__(DqTraits<FMT>::THREADS, 1) 
+// ODD: some tiles have an odd number of operand stages and there are two slots for them (dq_walk_steps).  An instance of its own,
+// because the kernel is sensitive to its code: with the walk decided at run time other shapes ran 0.3 to 1.3 % slower.
+template <int FMT, bool ODD>
+__global__ void __launch_bounds__(DqTraits<FMT>::THREADS, 1)
 dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_wu,
                const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_x16, const GroupedParams p,
                const DqPlan pl) {
@@ -635,7 +637,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
     const uint32_t sub_bytes = (uint32_t)pl.tn * 128u, b0 = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
     const int a_col = 512 - 32 * pl.subs * pl.ns;
-    const int slice_subs = min(kb64, 4 * rs_hi) - 4 * rs_lo, walk_subs = dq_walk_steps(pl.subs, pl.ns, slice_subs);
+    const int slice_subs = min(kb64, 4 * rs_hi) - 4 * rs_lo, walk_subs = dq_walk_steps(ODD, slice_subs);
     int it = 0, tcount = 0;
     for (int w = first; w < n_tiles; w += step, ++tcount) {
       const DqTile t = dq_tile(p, pl, pref, w, n_nt, fw);
@@ -852,7 +854,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     // =========================== activation rows ========================================================
     dq_pdl_wait();
     const uint32_t sub_bytes = (uint32_t)pl.tn * 128u;
-    const int slice_subs = min(kb64, 4 * rs_hi) - 4 * rs_lo, walk_subs = dq_walk_steps(pl.subs, pl.ns, slice_subs);
+    const int slice_subs = min(kb64, 4 * rs_hi) - 4 * rs_lo, walk_subs = dq_walk_steps(ODD, slice_subs);
     uint32_t spin = kDqSpin;
     int it = 0;
     if (pl.x_tma) {
@@ -871,7 +873,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
               stop = true;
               break;
             }
-            if (j >= slice_subs) {      // a stage without products
+            if (ODD && j >= slice_subs) {      // a stage without products
               warp_arrive(&bar.full[at.s]);
               continue;
             }
@@ -988,7 +990,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     // =========================== expansion ==============================================================
     const int ew = warp - T::FIRST_EXPAND;
     const int quarter = warp & 3;      // the tensor-memory lane quarter a warp may write
-    dq_expand_warps<FMT>(p, pl, smem, n_tiles, n_nt, rs_lo, rs_hi, first, step, tmem_base, ew >> 2, quarter, lane);
+    dq_expand_warps<FMT, ODD>(p, pl, smem, n_tiles, n_nt, rs_lo, rs_hi, first, step, tmem_base, ew >> 2, quarter, lane);
   }
 
   tc_fence_before();

@@ -74,7 +74,7 @@ int dq_max_clusters(int s) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, dq_gemm_kernel<FMT>, &cfg) != cudaSuccess || n < 1) {
+    if (cudaOccupancyMaxActiveClusters(&n, dq_gemm_kernel<FMT, false>, &cfg) != cudaSuccess || n < 1) {
       cudaGetLastError();
       n = sm_count() / s * 3 / 4;
       if (n < 1) n = 1;
@@ -145,20 +145,22 @@ bool dq_plan_query(const GroupedParams& p, int64_t rows, int32_t* out) {
   return true;
 }
 
-template <int FMT>
-int32_t launch_dq(const GroupedParams& p, int64_t rows, cudaStream_t stream) {
-  auto kern = dq_gemm_kernel<FMT>;
-  static bool attr_done[64] = {};
+// lets the kernel have its shared memory, once per device
+template <int FMT, bool ODD>
+bool dq_kernel_ready() {
+  static bool done[64] = {};
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return HQ_ERR_CUDA;
-  if (dev < 64 && !attr_done[dev]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kDqSmem) != cudaSuccess) return HQ_ERR_CUDA;
-    attr_done[dev] = true;
-  }
-  DqPlan pl{};
-  int grid = 0;
-  if (!dq_plan<FMT>(p, rows, pl, grid)) return HQ_ERR_SHAPE;
-  if (grid <= 0) return HQ_OK;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  if (dev < 64 && done[dev]) return true;
+  if (cudaFuncSetAttribute(dq_gemm_kernel<FMT, ODD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDqSmem) != cudaSuccess)
+    return false;
+  if (dev < 64) done[dev] = true;
+  return true;
+}
+
+template <int FMT, bool ODD>
+int32_t launch_dq_plan(const GroupedParams& p, DqPlan& pl, int grid, int64_t rows, cudaStream_t stream) {
+  if (!dq_kernel_ready<FMT, ODD>()) return HQ_ERR_CUDA;
   using T = DqTraits<FMT>;
   CUtensorMap tm_w{}, tm_wu{}, tm_x{}, tm_x16{};
   pl.raw_tma = T::WIDE || (p.w_row_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(p.w) & 15u) == 0 &&
@@ -206,7 +208,24 @@ int32_t launch_dq(const GroupedParams& p, int64_t rows, cudaStream_t stream) {
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pl.kslices > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, tm_w, tm_wu, tm_x, tm_x16, p, pl) == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
+  return cudaLaunchKernelEx(&cfg, dq_gemm_kernel<FMT, ODD>, tm_w, tm_wu, tm_x, tm_x16, p, pl) == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
+}
+
+template <int FMT>
+int32_t launch_dq(const GroupedParams& p, int64_t rows, cudaStream_t stream) {
+  if (!dq_kernel_ready<FMT, false>()) return HQ_ERR_CUDA;      // the plan asks how many clusters of it fit
+  DqPlan pl{};
+  int grid = 0;
+  if (!dq_plan<FMT>(p, rows, pl, grid)) return HQ_ERR_SHAPE;
+  if (grid <= 0) return HQ_OK;
+  // The GGML types have whole raw stages only (K % 256 == 0), which is an even number of operand stages.  So have all K slices
+  // but the last.
+  if constexpr (FMT == HQ_FMT_FP8_BLOCK || FMT == HQ_FMT_MXFP4) {
+    const int per = ((p.k + 255) / 256 + pl.kslices - 1) / pl.kslices;
+    if (dq_odd_on_two_slots(pl.subs, pl.ns, p.k / 64 - 4 * per * (pl.kslices - 1)))
+      return launch_dq_plan<FMT, true>(p, pl, grid, rows, stream);
+  }
+  return launch_dq_plan<FMT, false>(p, pl, grid, rows, stream);
 }
 
 }  // namespace hq

@@ -26,14 +26,15 @@ HQ_RING_FN bool ring_drains(int stage, int next, int slots, int warps, int me) {
   return stage >= 0 && stage < next && stage >= next - slots && stage % warps == me;
 }
 
-// Dequantizing GEMM: the 64-k steps for which its roles walk the operand stages of a tile of `steps` (`subs` per stage).  A group
-// of expanding warps serves every stage (four steps each), or every second one of a tile (two steps): then the group of the odd
-// ones would get from its last stage of a tile to its first of the next three stages on when a tile has an odd number.  Its wait
-// in front of stage j (stage j - slots consumed) needs stage j - 2 slots to be known as consumed, and the one in front of stage
-// j - 3 has shown that of stage j - 3 - slots: enough with three slots, one short with two.  Such a tile is walked for one
-// more stage, without products.
-HQ_RING_FN int dq_walk_steps(int subs, int slots, int steps) {
-  return subs == 2 && slots == 2 ? (steps + 3) & ~3 : steps;
+// Dequantizing GEMM, tiles of `steps` 64-k steps, `subs` of them per operand stage.  A group of expanding warps serves every
+// stage (subs = 4), or every second one of a tile (subs = 2): then the group of the odd ones gets from its last stage of a tile to
+// its first of the next three stages on when a tile has an odd number.  Its wait in front of stage j (stage j - slots consumed)
+// needs stage j - 2 slots to be known as consumed, and the one in front of stage j - 3 has shown that of stage j - 3 - slots:
+// enough with three slots, one short with two.  There a tile is walked for one more stage, without products.
+HQ_RING_FN bool dq_odd_on_two_slots(int subs, int slots, int steps) {
+  return subs == 2 && slots == 2 && (((steps + 1) >> 1) & 1) != 0;
 }
+// ... the steps for which the roles walk a tile, `odd`: the above of any of the launch's K slices
+HQ_RING_FN int dq_walk_steps(bool odd, int steps) { return odd ? (steps + 3) & ~3 : steps; }
 
 }  // namespace hq

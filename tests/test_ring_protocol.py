@@ -22,7 +22,8 @@ def ring(tmp_path_factory):
                 'extern "C" int slot(int i, int n) { return hq::ring_slot(i, n); }\n'
                 'extern "C" int parity(int i, int n) { return hq::ring_parity(i, n); }\n'
                 'extern "C" int drains(int i, int next, int n, int w, int me) { return hq::ring_drains(i, next, n, w, me); }\n'
-                'extern "C" int walk(int subs, int n, int steps) { return hq::dq_walk_steps(subs, n, steps); }\n')
+                'extern "C" int walk(int subs, int n, int steps) {\n'
+                '  return hq::dq_walk_steps(hq::dq_odd_on_two_slots(subs, n, steps), steps); }\n')
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(ROOT, "engine_b200", "csrc"), src, "-o", lib],
                    check=True)
     return C.CDLL(lib)
