@@ -28,8 +28,8 @@
 // partial sums are exchanged through distributed shared memory (each CTA finishes a share of the tile's tokens) and
 // added in rank order, so the result does not depend on timing and no scratch is needed.
 //
-// Every wait is bounded; after a time-out the status word is set, nothing more is stored and the kernel reaches its
-// normal exit.  No multicast, no peer memory.
+// Every wait is bounded; after a time-out the status word is set, nothing more is stored, the copy warps wait (bounded) for what
+// they have issued and the kernel reaches its normal exit.  No multicast, no peer memory.
 #pragma once
 #include <cuda.h>
 
@@ -849,6 +849,17 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           if (++slot == pl.nr) { slot = 0; ph ^= 1; wrapped = true; }
         }
       }
+      // No copy may still be writing the CTA's shared memory when it exits: the stages ring_drain names, walked as it does (written
+      // out here and for the tokens: of the forms tried the one that left other code as fast as it was).
+      const int next = stop ? turn - 1 : turn;
+#pragma unroll 1
+      for (int i = next - pl.nr; i < next; ++i) {
+        if (i >= 0 && (i & (helpers - 1)) == me && !warp_wait(&bar.full_r[slot], ph ^ 1, spin)) {
+          if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 580 + me);
+          spin = 1;
+        }
+        if (++slot == pl.nr) { slot = 0; ph ^= 1; }
+      }
     }
   } else if (warp < 2 + kDqEpilogueWarps + kDqTokenWarps) {
     // =========================== activation rows ========================================================
@@ -893,6 +904,14 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
                 warp_tma_2d(dst, &tm_x, x, row, &bar.full[at.s]);
               for (int i = 0; i < pieces; ++i, row += 16, dst += 2048u) warp_tma_2d(dst, &tm_x16, x, row, &bar.full[at.s]);
             }
+          }
+        }
+#pragma unroll 1
+        for (int i = max(0, it - pl.ns); i < it; ++i) {      // ... and the last stages of tokens
+          const DqSlot at = dq_slot(pl, i);
+          if (!warp_wait(&bar.full[at.s], at.use & 1, spin)) {
+            if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 590 + at.s);
+            spin = 1;
           }
         }
       }

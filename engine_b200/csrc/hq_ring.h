@@ -18,12 +18,21 @@ HQ_RING_FN int ring_slot(int stage, int slots) { return stage % slots; }
 HQ_RING_FN int ring_parity(int stage, int slots) { return (stage / slots) & 1; }
 
 // The stages whose copies a warp waits for when it has left its loop in front of stage `next` (the length of the sequence, or
-// where a wait ran out): its own -- those with stage % warps == me -- among the last `slots`.  They are the last uses of their
-// slots, so no later copy moves their barriers on, and the warp issued them, so the use before is known to be complete.
-// A slot's older stages were consumed before its last one was issued.  (A warp that waits for its last two stages whatever the
-// ring's length polls, with three slots, one that another warp has used again by then.)
-HQ_RING_FN bool ring_drains(int stage, int next, int slots, int warps, int me) {
-  return stage >= 0 && stage < next && stage >= next - slots && stage % warps == me;
+// where a wait ran out): its own -- of `warps` (1 or 2) that take the stages in turn -- among the last `slots`.  They are the last
+// uses of their slots, so no later copy moves their barriers on, and the warp issued them, so the use before is known to be
+// complete.  A slot's older stages were consumed before its last one was issued.  (A warp that waits for its last two stages
+// whatever the ring's length polls, with three slots, one that another warp has used again by then.)
+// `slot`, `parity`: the slot stage `next` would take, the parity of its last use.  False: a wait ran out.
+template <typename Wait>
+HQ_RING_FN bool ring_drain(int next, int slots, int slot, int parity, int warps, int me, Wait wait) {
+#ifdef __CUDACC__
+#pragma unroll 1
+#endif
+  for (int i = next - slots; i < next; ++i) {
+    if (i >= 0 && (i & (warps - 1)) == me && !wait(slot, parity)) return false;
+    if (++slot == slots) { slot = 0; parity ^= 1; }
+  }
+  return true;
 }
 
 // Dequantizing GEMM, tiles of `steps` 64-k steps, `subs` of them per operand stage.  A group of expanding warps serves every

@@ -30,14 +30,11 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, uint32
   }
   return false;
 }
-// No copy may still be writing a CTA's shared memory when it exits: bounded wait of copying warp `me` of `warps`, which has left
-// its loop in front of stage `next`, for the stages ring_drains names (bar[slot] completes with a stage's copies).  False: a
-// wait ran out.
-__device__ __forceinline__ bool warp_drain(uint64_t* bar, int next, int slots, int warps, int me, uint32_t spin_limit) {
-  for (int i = next - 1; i >= 0 && i >= next - slots; --i)
-    if (ring_drains(i, next, slots, warps, me) && !warp_wait(&bar[ring_slot(i, slots)], ring_parity(i, slots), spin_limit))
-      return false;
-  return true;
+// No copy may still be writing a CTA's shared memory when it exits: bounded wait of a copying warp for the stages ring_drain
+// names (bar[slot] completes with a stage's copies).  On the normal path whoever reads the stages waits for the same.
+__device__ __forceinline__ bool warp_drain(uint64_t* bar, int next, int slots, int slot, int parity, int warps, int me,
+                                           uint32_t spin_limit) {
+  return ring_drain(next, slots, slot, parity, warps, me, [&](int s, int ph) { return warp_wait(&bar[s], ph, spin_limit); });
 }
 // mbarrier arrivals by the elected lane of a whole warp, as a predicated instruction: a branch for one lane costs the
 // other roles' warps instruction fetches (and this one several hundred cycles when it misses)

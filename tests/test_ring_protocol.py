@@ -21,7 +21,10 @@ def ring(tmp_path_factory):
         f.write('#include "hq_ring.h"\n'
                 'extern "C" int slot(int i, int n) { return hq::ring_slot(i, n); }\n'
                 'extern "C" int parity(int i, int n) { return hq::ring_parity(i, n); }\n'
-                'extern "C" int drains(int i, int next, int n, int w, int me) { return hq::ring_drains(i, next, n, w, me); }\n'
+                'extern "C" int drain(int next, int n, int s, int ph, int w, int me, int* out) {\n'
+                '  int k = 0;\n'
+                '  hq::ring_drain(next, n, s, ph, w, me, [&](int a, int b) { out[k++] = 2 * a + b; return true; });\n'
+                '  return k; }\n'
                 'extern "C" int walk(int subs, int n, int steps) {\n'
                 '  return hq::dq_walk_steps(hq::dq_odd_on_two_slots(subs, n, steps), steps); }\n')
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(ROOT, "engine_b200", "csrc"), src, "-o", lib],
@@ -109,8 +112,8 @@ def block_scaled(ring, slots, stages, seed, drain):
             full[s].arrive(1)
             m.copies.append(lambda s=s: full[s].complete(1))
             yield None
-        for i in drain(stages, slots, me):
-            yield full[ring.slot(i, slots)], ring.parity(i, slots)
+        for s, parity in drain(stages, slots, me):
+            yield full[s], parity
 
     def scale_warps(me):
         for i in range(me, stages, 2):
@@ -141,8 +144,21 @@ def block_scaled(ring, slots, stages, seed, drain):
         raise Wrong("copies in flight at the end")
 
 
-def kernel_drain(ring):
-    return lambda stages, slots, me: [i for i in range(stages - 1, -1, -1) if ring.drains(i, stages, slots, 2, me)]
+def kernel_drain(ring, copy_warps=2):
+    def drain(stages, slots, me):
+        out = (C.c_int * slots)()
+        n = ring.drain(stages, slots, ring.slot(stages, slots), ring.parity(stages, slots) ^ 1, copy_warps, me, out)
+        return [(v // 2, v % 2) for v in out[:n]]
+    return drain
+
+
+@pytest.mark.parametrize("slots", range(2, 13))
+def test_the_last_use_of_every_slot_is_drained_once(ring, slots):
+    for stages in range(40):
+        last = [(i % slots, i // slots % 2) for i in range(max(0, stages - slots), stages)]
+        assert kernel_drain(ring, 1)(stages, slots, 0) == last
+        halves = [kernel_drain(ring, 2)(stages, slots, me) for me in (0, 1)]
+        assert sorted(halves[0] + halves[1]) == sorted(last)
 
 
 @pytest.mark.parametrize("slots", [2, 3, 4, 5, 6])
@@ -154,7 +170,10 @@ def test_block_scaled_gemm_ends(ring, slots, stages):
 
 def test_the_model_finds_a_wait_that_a_later_use_has_overtaken(ring):
     # each warp's own last two stages whatever the ring's length: with two and three slots one of them has been used again
-    own = lambda stages, slots, me: [i for i in range(stages - 1, -1, -1) if i % 2 == me][:2]
+    def own(stages, slots, me):
+        last = [i for i in range(stages - 1, -1, -1) if i % 2 == me][:2]
+        return [(i % slots, i // slots % 2) for i in last]
+
     for slots, found in ((2, True), (3, True), (4, False), (6, False)):
         stuck = 0
         for seed in range(100):
@@ -186,6 +205,8 @@ def dequantizing(ring, slots, raw_slots, subs, steps, tiles, seed, walk):
             full_r[s].arrive(1)
             m.copies.append(lambda s=s: full_r[s].complete(1))
             yield None
+        for s, parity in kernel_drain(ring)(tiles * raw_stages, raw_slots, me):
+            yield full_r[s], parity
 
     def group(c):
         stage, sub = c // subs, c % subs
@@ -219,6 +240,8 @@ def dequantizing(ring, slots, raw_slots, subs, steps, tiles, seed, walk):
             full[s].arrive(1)
             m.copies.append(lambda s=s: full[s].complete(1))
             yield None
+        for s, parity in kernel_drain(ring, 1)(tiles * tile_stages, slots, 0):
+            yield full[s], parity
 
     def mma_warp():
         def finish(s, i, n):

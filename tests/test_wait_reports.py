@@ -32,3 +32,15 @@ def test_a_wait_that_runs_out_is_reported(name):
 
 def test_a_silent_wait_is_found():
     assert silent_waits("  for (;;)\n    if (!warp_wait(&full[i], 0, spin)) break;\n  }\n  next();\n  done();\n") == [2]
+
+
+@pytest.mark.parametrize("name", ["hq_dq_gemm.cuh", "hq_fp8_grouped.cu", "hq_mx_grouped.cu"])
+def test_copies_are_waited_for_by_the_warps_that_issue_them(name):
+    # after a time-out nobody else waits for a stage any more: the rings box copies signal are drained before the CTA exits,
+    # by warp_drain or by a loop over the last stages of the sequence
+    text = open(os.path.join(CSRC, name)).read()
+    rings = set(re.findall(r"warp_tma_[23]d\([^;]*&([\w.]+)\[", text, re.S))
+    drained = set(re.findall(r"warp_drain\(([\w.]+),", text))
+    for loop in re.findall(r"for \(int i = [^;]*(?:next|it) - pl\.n[rs]\)?;.*?warp_wait\(&([\w.]+)\[", text, re.S):
+        drained.add(loop)
+    assert rings and rings <= drained, (rings, drained)
