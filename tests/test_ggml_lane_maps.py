@@ -3,9 +3,9 @@ oracle's dequantizers: which bytes, shifts and masks give which weight.
 
 * `hq::gm_decode_span` (engine_b200/csrc/hq_gemv_ggml_mma.cu): lane t of a quad decodes the four weights 4t..4t+3 of
   every 16-weight group of a 256-weight span from one 32-bit word of code bits (+ one of high bits);
-* `hq::fetch_a` / `emit_*` (engine_b200/csrc/hq_grouped_gemm.cu): a producer thread expands 16 consecutive weights
-  (quarter q of a 64-weight stage) from four or five aligned words, funnel-shifted when the block starts in the
-  middle of a word.
+* `hq::DqRow` / `emit_*` (engine_b200/csrc/hq_dq_gemm.cuh, hq_dequant.cuh): a thread of the dequantizing GEMM expands the
+  64 weights 64c.. of one row's 256-weight stage, in two halves, from 16-byte loads of the stage's copy; rows that are no
+  multiple of 16 bytes long start somewhere behind the copy's first byte.
 
 The restatement uses f32 products in the oracle's order, so a correct mapping reproduces the oracle bit for bit.  It
 is how the mappings were settled before the kernels first ran; the kernels themselves are compared with the oracle by
@@ -133,103 +133,135 @@ def test_decode_kernel_lane_map(fmt):
         assert np.array_equal(decode_span(fmt, raw[r]), want[r]), fmt
 
 
-# ---- the grouped GEMM's producers: 16 consecutive weights per thread ------------------------------------------------
+# ---- the dequantizing GEMM: 64 weights of a row's 256-weight stage per thread ----------------------------------------
 
-def _words(buf, addr, n):
-    return [int.from_bytes(bytes(buf[addr + 4 * i:addr + 4 * i + 4]).ljust(4, b"\0"), "little") for i in range(n)]
+STAGE_BYTES = {"Q8_0": 272, "Q4_K": 144, "Q6_K": 210, "Q5_K": 176, "Q4_0": 144, "Q5_0": 176, "Q4_1": 160, "Q5_1": 192,
+               "Q2_K": 84, "Q3_K": 110}
+NARROW = ("Q6_K", "Q2_K", "Q3_K")
+
+
+def _words(b, at, n, ws=0):
+    """dq_lds_words: whole 16-byte units from a 16-byte boundary on, the first `ws` words dropped"""
+    assert at % 16 == 0 and 0 <= ws < 4
+    return [_ld32(b, at + 4 * i) for i in range(4 * ((n + ws + 3) // 4))][ws:ws + n]
 
 
 def _funnel(lo, hi, sh):
     return ((lo | (hi << 32)) >> sh) & 0xFFFFFFFF
 
 
-def _five_words(buf, p):
-    """the 16 bytes at the 2-byte aligned address p as four aligned words, a fifth when p is 2 bytes off"""
-    mis = p & 2
-    w = _words(buf, p - mis, 4) + [_words(buf, p - mis + 16, 1)[0] if mis else 0]
-    return [_funnel(w[i], w[i + 1], 8 * mis) for i in range(4)]
+def _join(w, sh):
+    """16 consecutive bytes from four or five words, `sh` bits into the first"""
+    return [_funnel(w[i], w[i + 1] if sh else 0, sh) for i in range(4)]
 
 
-def producer_row(fmt, buf, base, k):
-    """`buf`: bytes of a 16-byte aligned tensor, `base`: offset of the row in it."""
-    out = np.zeros(k, f32)
-    for k0 in range(0, k, 64):
-        for q in range(4):
-            pos = (k0 & 255) + 16 * q
-            h, j, u = pos >> 7, (pos >> 5) & 3, (pos >> 4) & 1
-            o = k0 + 16 * q
-            if fmt == "Q5_K":
-                blk = base + 176 * (k0 >> 8)
-                c, hi = (k0 & 255) >> 6, q >> 1
-                hdr = _words(buf, blk, 4)
-                qw = _words(buf, blk + 48 + 32 * c + 16 * (q & 1), 4)
-                hw = _words(buf, blk + 16 + 16 * (q & 1), 4)
-                jj = 2 * c + hi
-                sc, mn = _k4_scale_min(hdr, jj)
-                d, dmin = _f16(buf, blk), _f16(buf, blk + 2)
-                for i in range(4):
-                    vm = (((qw[i] >> 4) if hi else qw[i]) & 0x0F0F0F0F) | (((hw[i] >> jj) & 0x01010101) << 4)
-                    for t, code in enumerate(_bytes4(vm)):
-                        out[o + 4 * i + t] = f32(d * sc) * f32(code) - f32(dmin * mn)
-            elif fmt == "Q2_K":
-                blk = base + 84 * (k0 >> 8)
-                qw = _words(buf, blk + 16 + 32 * h + 16 * u, 4)
-                s = int(buf[blk + 8 * h + 2 * j + u])
-                d, dmin = _f16(buf, blk + 80), _f16(buf, blk + 82)
-                for i in range(4):
-                    for t, code in enumerate(_bytes4((qw[i] >> (2 * j)) & 0x03030303)):
-                        out[o + 4 * i + t] = f32(f32(d) * f32(s & 15)) * f32(code) - f32(f32(dmin) * f32(s >> 4))
-            elif fmt in ("Q6_K", "Q3_K"):
+def stage_quarter(fmt, b, c, ws, mis):
+    """b: a row of the stage's copy; the stage starts 4 ws + mis bytes behind its beginning.  -> weights 64c .. 64c + 63"""
+    out = []
+
+    def put(codes, factor, zero=0, less=0.0):
+        out.extend(factor * f32(code - zero) - f32(less) for word in codes for code in _bytes4(word))
+
+    sh, h, odd = 8 * mis, c >> 1, 2 * (c & 1)
+    if fmt in ("Q4_K", "Q5_K"):
+        hdr, w = _words(b, 0, 4), _words(b, (16 if fmt == "Q4_K" else 48) + 32 * c, 8)
+        fifth = _words(b, 16, 8) if fmt == "Q5_K" else [0] * 8
+        d, dmin = _f16(b, 0), _f16(b, 2)
+        y, z, x = hdr[1:]
+        s = (x & 0x0F0F0F0F) | ((y >> 2) & 0x30303030) if h else y & 0x3F3F3F3F
+        m = ((x >> 4) & 0x0F0F0F0F) | ((z >> 2) & 0x30303030) if h else z & 0x3F3F3F3F
+        s, m = s >> (16 * (c & 1)), m >> (16 * (c & 1))
+        for i in range(2):
+            sc, mn = (s >> (8 * i)) & 0xFF, (m >> (8 * i)) & 0xFF
+            put([((w[j] >> (4 * i)) & 0x0F0F0F0F) | (((fifth[j] >> (2 * c + i)) & 0x01010101) << 4) for j in range(8)],
+                f32(d * sc), 0, dmin * mn)
+    elif fmt == "Q8_0":
+        w = _words(b, (68 * c) & ~15, 17, c)
+        for d, first in ((w[0] & 0xFFFF, _join(w[0:5], 16) + _join(w[4:9], 16)), (w[8] >> 16, w[9:17])):
+            d = f32(np.array([d], np.uint16).view(np.float16)[0])
+            put([word ^ 0x80808080 for word in first], d, 128)
+    elif fmt in ("Q6_K", "Q3_K"):
+        if fmt == "Q6_K":
+            lo, hi = _words(b, 64 * h, 17, ws), _words(b, 128 + 32 * h, 9, ws)
+            at = 192 + 4 * c + 4 * ws
+            scales, d, zero = _funnel(_ld32(b, at), _ld32(b, at + 4), sh), _f16(b, 208 + 4 * ws + mis), 32
+        else:
+            lo, hi = _words(b, 32 + 32 * h, 9, ws), _words(b, 0, 9, ws)
+            at = 96 + 4 * ws
+            nib = _funnel(_ld32(b, at + 4 * (c & 1)), _ld32(b, at + 4 * (c & 1) + 4), sh) >> (0 if c < 2 else 4)
+            top = _funnel(_ld32(b, at + 8), _ld32(b, at + 12), sh) >> (2 * c)
+            scales, d, zero = (nib & 0x0F0F0F0F) | ((top & 0x03030303) << 4), _f16(b, 108 + 4 * ws + mis), 4
+        for i in range(2):
+            j = odd + i
+            for u in range(2):
+                lw = _join(lo[(8 * i if fmt == "Q6_K" else 0) + 4 * u:][:5], sh)
+                hw = _join(hi[4 * u:][:5], sh)
+                sc = (scales >> (16 * i + 8 * u)) & 0xFF
                 if fmt == "Q6_K":
-                    blk = base + 210 * (k0 >> 8)
-                    lw = _five_words(buf, blk + 64 * h + 32 * (j & 1) + 16 * u)
-                    hw = _five_words(buf, blk + 128 + 32 * h + 16 * u)
-                    d, sc = _f16(buf, blk + 208), int(np.int8(buf[blk + 192 + 8 * h + 2 * j + u]))
-                    for i in range(4):
-                        nib = (lw[i] if j < 2 else (lw[i] >> 4)) & 0x0F0F0F0F
-                        w6 = nib | (((hw[i] >> (2 * j)) & 0x03030303) << 4)
-                        for t, code in enumerate(_bytes4(w6)):
-                            out[o + 4 * i + t] = f32(d) * f32(sc) * f32(code - 32)
+                    codes = [((lw[t] >> (2 * (j & 2))) & 0x0F0F0F0F) | (((hw[t] >> (2 * j)) & 0x03030303) << 4) for t in range(4)]
+                    sc = int(np.int8(np.uint8(sc)))
                 else:
-                    blk = base + 110 * (k0 >> 8)
-                    lw = _five_words(buf, blk + 32 + 32 * h + 16 * u)
-                    hw = _five_words(buf, blk + 16 * u)
-                    s16 = 8 * h + 2 * j + u
-                    a, b = s16 >> 2, s16 & 3
-                    nib, top = int(buf[blk + 96 + 4 * (a & 1) + b]), int(buf[blk + 104 + b])
-                    sc6 = ((nib & 15) if a < 2 else (nib >> 4)) | (((top >> (2 * a)) & 3) << 4)
-                    d = _f16(buf, blk + 108)
-                    for i in range(4):
-                        w3 = ((lw[i] >> (2 * j)) & 0x03030303) | (((hw[i] >> (4 * h + j)) & 0x01010101) << 2)
-                        for t, code in enumerate(_bytes4(w3)):
-                            out[o + 4 * i + t] = f32(f32(d) * f32(sc6 - 32)) * f32(code - 4)
+                    codes = [((lw[t] >> (2 * j)) & 0x03030303) | (((hw[t] >> (4 * h + j)) & 0x01010101) << 2) for t in range(4)]
+                    sc -= 32
+                put(codes, f32(d) * f32(sc), zero)
+    elif fmt == "Q2_K":
+        w, scales, dd = _words(b, 16 + 32 * h, 8, ws), _ld32(b, 4 * c + 4 * ws), 80 + 4 * ws
+        d, dmin = _f16(b, dd), _f16(b, dd + 2)
+        for i in range(2):
+            for u in range(2):
+                sb = (scales >> (16 * i + 8 * u)) & 0xFF
+                put([(w[4 * u + t] >> (2 * (odd + i))) & 0x03030303 for t in range(4)], f32(d) * f32(sb & 15), 0,
+                    f32(dmin) * f32(sb >> 4))
+    else:
+        five, has_min = fmt in ("Q5_0", "Q5_1"), fmt in ("Q4_1", "Q5_1")
+        size = {"Q4_0": 18, "Q5_0": 22, "Q4_1": 20, "Q5_1": 24}[fmt]
+        zero = 0 if has_min else (16 if five else 8)
+        if fmt != "Q5_1":
+            n = {"Q4_0": 9, "Q5_0": 11, "Q4_1": 10}[fmt]
+            w = _words(b, (2 * size * c) & ~15, n, ((2 * size * c) & 15) >> 2)
+        for i in range(2):
+            qh, m = 0, 0
+            if fmt == "Q4_0":
+                d, q = (w[0] & 0xFFFF, _join(w[0:5], 16)) if i == 0 else (w[4] >> 16, w[5:9])
+            elif fmt == "Q5_0":
+                d, qh, q = ((w[0] & 0xFFFF, _funnel(w[0], w[1], 16), _join(w[1:6], 16)) if i == 0
+                            else (w[5] >> 16, w[6], w[7:11]))
+            elif fmt == "Q4_1":
+                d, m, q = w[5 * i] & 0xFFFF, w[5 * i] >> 16, w[5 * i + 1:5 * i + 5]
             else:
-                five, has_min = fmt in ("Q5_0", "Q5_1"), fmt in ("Q4_1", "Q5_1")
-                bb = 18 + 4 * five + 2 * has_min
-                zero = 0 if has_min else (16 if five else 8)
-                blk = base + bb * ((k0 >> 5) + (q >> 1))
-                half = q & 1
-                w = _five_words(buf, blk + bb - 16)
-                d, m = _f16(buf, blk), (_f16(buf, blk + 2) if has_min else 0.0)
-                qh_at = blk + (4 if has_min else 2) + 2 * half
-                ext = (int(buf[qh_at]) | int(buf[qh_at + 1]) << 8) if five else 0
-                for i in range(4):
-                    vm = ((w[i] >> 4) if half else w[i]) & 0x0F0F0F0F
-                    if five:
-                        vm |= _spread4(ext >> (4 * i)) << 4
-                    for t, code in enumerate(_bytes4(vm)):
-                        out[o + 4 * i + t] = f32(d) * f32(code - zero) + f32(m)
-    return out
+                head = [_ld32(b, 48 * c + 24 * i + 4 * t) for t in range(6)]
+                d, m, qh, q = head[0] & 0xFFFF, head[0] >> 16, head[1], head[2:]
+            d, m = (f32(np.array([v], np.uint16).view(np.float16)[0]) for v in (d, m))
+            for half in range(2):
+                ext = (qh >> 16) if half else (qh & 0xFFFF)
+                codes = [((q[t] >> (4 * half)) & 0x0F0F0F0F) | ((_spread4(ext >> (4 * t)) << 4) if five else 0) for t in range(4)]
+                put(codes, d, zero, -m)
+    return np.array(out, f32)
 
 
-@pytest.mark.parametrize("fmt", ["Q6_K", "Q5_K", "Q4_0", "Q5_0", "Q4_1", "Q5_1", "Q2_K", "Q3_K"])
-def test_grouped_gemm_producer_map(fmt):
-    # K = 768: three super-blocks per row, so Q6_K / Q3_K rows (630 / 330 bytes) alternate between word-aligned and two
-    # bytes off, and so do the 18- / 22-byte blocks of Q4_0 / Q5_0 inside a row
+@pytest.mark.parametrize("boxes", [True, False])
+@pytest.mark.parametrize("fmt", sorted(STAGE_BYTES))
+def test_dequantizing_gemm_row_map(fmt, boxes):
+    # three super-blocks per row: rows of Q6_K / Q3_K (630 / 330 bytes) and Q2_K (252) start at every even or fourth byte of a
+    # 16-byte unit.  Their stages are copied from the 16-byte boundary at or below the block (boxes) or from the 4-byte one
+    if fmt not in NARROW and not boxes:
+        pytest.skip("every stage starts on a 16-byte boundary")
     rng = np.random.Generator(np.random.PCG64(12))
-    k = 768
-    raw = F.ggml_random_blocks(fmt, rng, 4, k)
-    want = F.GGML_DEQUANT[fmt](raw, k)
-    flat, row_bytes = raw.reshape(-1), raw.shape[1]
+    k, size = 768, STAGE_BYTES[fmt]
+    if fmt in ("Q8_0", "Q4_K"):
+        w = rng.normal(0.0, 0.02, (4, k)).astype(f32)
+        raw = F.q8_0_quantize(w) if fmt == "Q8_0" else F.q4_k_quantize(w)
+        want = F.q8_0_dequant(raw, k) if fmt == "Q8_0" else F.q4_k_dequant(raw, k)
+    else:
+        raw = F.ggml_random_blocks(fmt, rng, 4, k)
+        want = F.GGML_DEQUANT[fmt](raw, k)
+    flat = np.concatenate([raw.reshape(-1), np.full(64, 0xA5, np.uint8)])
+    assert raw.shape[1] == 3 * size
     for r in range(4):
-        assert np.array_equal(producer_row(fmt, flat, r * row_bytes, k), want[r]), (fmt, r)
+        got = np.zeros(k, f32)
+        for rs in range(3):
+            at = (3 * r + rs) * size
+            off = at & (15 if boxes else 3)
+            for c in range(4):
+                got[256 * rs + 64 * c:][:64] = stage_quarter(fmt, flat[at - off:], c, off >> 2, off & 2)
+        assert np.array_equal(got, want[r].reshape(-1)), (fmt, r)
