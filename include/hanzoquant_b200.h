@@ -138,9 +138,11 @@ int32_t hq_status_read(const int32_t* status_dev, int32_t out_host[4], void* str
  * does not cover (K % 64 != 0) always take the decode kernel. */
 #define HQ_CFG_MOE_TENSOR_MIN_ROWS 0
 #define HQ_CFG_DENSE_TENSOR_MIN_ROWS 1
-/* HQ_CFG_SPIN_LIMIT: polls a kernel spends on one bounded wait before it gives up, leaves HQ_DEV_WAIT_TIMEOUT in
- * the status word and stops storing results (default 1 << 22; read by the FP8 expert GEMM).
- * HQ_CFG_TEST_SKIP_PRODUCER: test hook, 0 by default.  With 1 the FP8 expert GEMM's copy-issuing warp issues
+/* HQ_CFG_SPIN_LIMIT: how long a bounded wait goes on before the kernel leaves HQ_DEV_WAIT_TIMEOUT in the status word and
+ * stops storing results (default 1 << 22).  Read by the FP8 and MXFP4 expert GEMMs over 8-bit activations, whose polls suspend
+ * their warp for up to 20 us and which give up after value / 64 + 1 of them (1.3 s at most at the default), and by
+ * hq_ep_barrier, which polls `value` times.  The other kernels' limits are constants.
+ * HQ_CFG_TEST_SKIP_PRODUCER: test hook, 0 by default.  With 1 the copy-issuing warps of those two GEMMs issue
  * nothing, so every wait of the other warps runs out: the way to see the time-out path return without anything
  * left in flight (no copy and no MMA is issued in that launch). */
 #define HQ_CFG_SPIN_LIMIT 2
