@@ -439,7 +439,6 @@ static void fill_fp8_native(Fp8GroupedParams& g, const hq_weight* w) {
   g.bias_dtype = w->bias_dtype;
   g.spin_limit = (uint32_t)g_cfg[HQ_CFG_SPIN_LIMIT];
   g.test_skip_producer = (int)g_cfg[HQ_CFG_TEST_SKIP_PRODUCER];
-  g.load_burst_prefetch_off = g_cfg[HQ_CFG_FP8_L2_PREFETCH] == 0;
 }
 
 int32_t hq_fp8_quant_rows(const void* x, int32_t x_dtype, int64_t x_stride, const int32_t* row_map, int64_t n_rows,

@@ -20,9 +20,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
@@ -61,17 +58,6 @@ __device__ __forceinline__ uint32_t make_idesc_f16(int tile_n) {
 __device__ __forceinline__ uint32_t swz(int r, int c) {
   return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4));
 }
-__device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-      "}\n" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]),
                "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
@@ -82,13 +68,12 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 // ---- expansion of 16 consecutive weights: the raw fields picked out of a block (hq_dq_gemm.cuh) -> eight f16 pairs in
 // natural k order
 struct RawA {
-  uint4 hdr;          // Q4_K / Q5_K: super-block header {d, dmin, 12 scale bytes}; Q8_0, Q4_0 ..: .x = fifth payload word
-  uint4 q;            // Q4_K / Q5_K: 16 nibble bytes; FP8: 16 codes; MXFP4: .x/.y = 8 nibble bytes; else payload words
-  uint32_t aux;       // FP8: relative block scale (f32 bits); MXFP4: e8m0 byte; Q8_0 ..: d (f16 bits) | shift << 16
-  uint4 ext;          // Q6_K: .x / .y = fifth word of the low-nibble / high-bit bytes, .z = d (f16 bits) |
-                      // scale byte << 16, .w = shifts (low-nibble bytes | high-bit bytes << 8); Q5_K: the 16 bytes
-                      // of fifth bits; Q5_0 / Q5_1: .x = the 16 fifth bits of this half block; Q3_K: as Q6_K with
-                      // the code words in q and the hmask words in hdr, .z = d | 6-bit scale << 16
+  uint4 hdr;          // Q8_0, Q4_0 ..: .x = fifth payload word, .y = m (f16 bits); Q6_K: words of high bits; Q3_K: of hmask
+  uint4 q;            // FP8: 16 codes; MXFP4: .x/.y = 8 nibble bytes; else payload words
+  uint32_t aux;       // FP8: relative block scale (f32 bits); MXFP4: e8m0 byte; Q8_0, Q4_0 ..: d (f16 bits) | shift << 16
+                      // [| half block << 24]; Q6_K, Q3_K: bit pair [| hmask bit << 8]
+  uint4 ext;          // Q6_K, Q3_K: .x / .y = fifth words of q / hdr, .z = d (f16 bits) | scale << 16, .w = shifts (of q |
+                      // of hdr << 8); Q5_0 / Q5_1: .x = the 16 fifth bits of this half block
 };
 
 // Q4_K, Q5_K, Q2_K: w = d * s * code - dmin * m with the integer scale s and minimum m of the sub-block.  A code byte

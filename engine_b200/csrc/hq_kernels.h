@@ -113,8 +113,6 @@ struct Fp8GroupedParams {
   int32_t* status;
   uint32_t spin_limit;          // polls per bounded wait (0 = default)
   int test_skip_producer;       // test hook: the TMA warp issues nothing, so every consumer wait runs out
-  int load_burst_prefetch_off;  // 1 = do not pull weight rows into L2 ahead of the operand copies
-  int l2_prefetch;              // set by the launcher
 };
 bool fp8_grouped_supported(int64_t n, int64_t k);
 int32_t launch_fp8_grouped(const Fp8GroupedParams& p, cudaStream_t stream);
