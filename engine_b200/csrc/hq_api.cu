@@ -94,8 +94,13 @@ void fill_grouped(GroupedParams& g, const hq_weight* w, const hq_weight* w_up) {
   g.fp8_kb = (int)((w->k + 127) / 128);
 }
 
-// Row counts from which a call goes to the tensor-core GEMM.  Q8_0's decode kernel streams at HBM speed, so re-reading
-// the weights once per 8 rows stays cheaper than expanding them for longer: four times the configured thresholds.  MXFP4
+// Row counts from which a call goes to the tensor-core GEMM: where a decode kernel, which serves up to 8 rows with one pass over
+// the weights, starts its second pass (9 rows, or 8 per expert).  Q8_0, whose decode kernel is the fastest per pass, from four
+// times that.  These lines were drawn against an earlier GEMM and now lie late (us, decode : tensor, bf16 activations, the
+// conversion to f16 included): Q8_0 4,096 x 4,096 at 8 rows 13.4 : 12.0, at 16 24.3 : 13.9, at 32 44.4 : 14.1, 65,536 x
+// 4,096 at 16 121 : 67; Q4_K 4,096 x 4,096 at 4 10.0 : 11.7, at 8 14.3 : 11.8, 65,536 x 4,096 at 8 59.6 : 70.4, at 16
+// 116 : 70; FP8 65,536 x 4,096 at 2 55.7 : 57.1, at 4 65.2 : 57.4; 128 Q4_K experts of 2,048 x 768, top 8, at 16 tokens
+// 158 : 137, at 64 230 : 190, at 128 (the line) 307 : 192.  MXFP4
 // with block scales the f16 operand holds (HQ_WEIGHT_F16_SCALES): from the first row on at the default settings -- the
 // expanded weights are exact there, both kernels round activations to f16, and the decode kernel, bounded by its
 // instructions, is slower at every count (us, decode against tensor: 14,336 x 4,096 at 1 row 22.7 : 17.3, 4,096 x 14,336
