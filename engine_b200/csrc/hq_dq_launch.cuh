@@ -56,6 +56,19 @@ bool dq_smem_plan(DqPlan& pl, int n_experts, bool expert_indexed) {
   return true;
 }
 
+// lets the kernel have its shared memory, once per device
+template <int FMT, bool ODD>
+bool dq_kernel_ready() {
+  static bool done[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  if (dev < 64 && done[dev]) return true;
+  if (cudaFuncSetAttribute(dq_gemm_kernel<FMT, ODD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDqSmem) != cudaSuccess)
+    return false;
+  if (dev < 64) done[dev] = true;
+  return true;
+}
+
 // CTA clusters of `s` CTAs (one per SM) the device can hold at once
 template <int FMT>
 int dq_max_clusters(int s) {
@@ -74,7 +87,9 @@ int dq_max_clusters(int s) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, dq_gemm_kernel<FMT, false>, &cfg) != cudaSuccess || n < 1) {
+    // (without the attribute the query fails, and the answer would be the guess below for good)
+    if (!dq_kernel_ready<FMT, false>() ||
+        cudaOccupancyMaxActiveClusters(&n, dq_gemm_kernel<FMT, false>, &cfg) != cudaSuccess || n < 1) {
       cudaGetLastError();
       n = sm_count() / s * 3 / 4;
       if (n < 1) n = 1;
@@ -145,19 +160,6 @@ bool dq_plan_query(const GroupedParams& p, int64_t rows, int32_t* out) {
   return true;
 }
 
-// lets the kernel have its shared memory, once per device
-template <int FMT, bool ODD>
-bool dq_kernel_ready() {
-  static bool done[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return false;
-  if (dev < 64 && done[dev]) return true;
-  if (cudaFuncSetAttribute(dq_gemm_kernel<FMT, ODD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDqSmem) != cudaSuccess)
-    return false;
-  if (dev < 64) done[dev] = true;
-  return true;
-}
-
 template <int FMT, bool ODD>
 int32_t launch_dq_plan(const GroupedParams& p, DqPlan& pl, int grid, int64_t rows, cudaStream_t stream) {
   if (!dq_kernel_ready<FMT, ODD>()) return HQ_ERR_CUDA;
@@ -213,7 +215,6 @@ int32_t launch_dq_plan(const GroupedParams& p, DqPlan& pl, int grid, int64_t row
 
 template <int FMT>
 int32_t launch_dq(const GroupedParams& p, int64_t rows, cudaStream_t stream) {
-  if (!dq_kernel_ready<FMT, false>()) return HQ_ERR_CUDA;      // the plan asks how many clusters of it fit
   DqPlan pl{};
   int grid = 0;
   if (!dq_plan<FMT>(p, rows, pl, grid)) return HQ_ERR_SHAPE;
