@@ -42,10 +42,10 @@ MS = [1, 2, 4, 8]
 UNIT = "tokens/s"
 
 # DRAM bytes over algorithmic bytes from the ncu captures under profiles/
-NCU_TRAFFIC_RATIO_GEMV = 563.3 / 558.2      # hq::gemv_int8_kernel, 4096 -> 128256
-NCU_TRAFFIC_RATIO_FP8 = 1573.4 / 1515.6     # hq::fp8_grouped_kernel, routed gate/up + down, 32 experts x 128 rows
-NCU_TRAFFIC_RATIO_MX = 527.3 / 543.2        # hq::mx_grouped_kernel, gate/up + down, 32 experts x 256 rows
-NCU_TRAFFIC_RATIO_Q4K = 118.8 / 181.3       # hq::grouped_gemm_kernel<Q4_K>, gate/up + down, 32 experts x 256 rows
+NCU_TRAFFIC_RATIO_GEMV = 562.2 / 558.2      # hq::gemv_int8_kernel, 4096 -> 128256, mean of M = 1, 2, 4, 8
+NCU_TRAFFIC_RATIO_FP8 = 1546.8 / 1515.6     # hq::fp8_grouped_kernel, routed gate/up + down, 32 experts x 128 rows
+NCU_TRAFFIC_RATIO_MX = 525.0 / 543.2        # hq::mx_grouped_kernel, gate/up + down, 32 experts x 256 rows
+NCU_TRAFFIC_RATIO_Q4K = 148.4 / 181.4       # hq::dq_gemm_kernel<Q4_K>, gate/up + down, 32 experts x 256 rows
                                             # (below 1: most of the f32 output rows are still in L2 at the end)
 
 
@@ -430,7 +430,7 @@ def gemv_measure(args, torch, dev, rank, world, dist, with_cpu=True):
                      "frac": round(achieved / peaks["hbm_gbs"], 4),
                      "frac_of_nominal_8tbs": round(achieved / 8000.0, 4),
                      "traffic": int(NCU_TRAFFIC_RATIO_GEMV * step_bytes / launches_per_step),
-                     "traffic_note": "algorithmic bytes x 1.009 (ncu dram bytes / algorithmic bytes of the "
+                     "traffic_note": "algorithmic bytes x 1.007 (ncu dram bytes / algorithmic bytes of the "
                                      "4096x128256 launch)",
                      "peak_kind": peaks["kind"], "kernel": "hq::gemv_int8_kernel<Q8_0>",
                      "launch_ms_sum": round(kern_ms, 4), "bytes_per_step": step_bytes,
@@ -621,14 +621,15 @@ def run_moe(args):
 
     # launches of this library's kernels per step (the collectives' own kernels are not counted)
     if ep is not None:
-        launches_per_step = 1 + 1 + 1 + 3 + (3 if (fp8 or mx) else 2) + 1 + 1 + \
-            (4 if (shared is not None and fp8) else 0)
-    elif fp8:
-        launches_per_step = 1 + 3 + 3 + 1 + (4 if shared is not None else 0)
-    elif mx:
-        launches_per_step = 1 + 3 + 1 + 2 + 1          # router, dispatch build, row quantizer, two GEMMs, reduce
+        # router, pack, unpack, dispatch tables, [row gather,] two GEMMs, two reduces (pushes and barriers not counted)
+        launches_per_step = 1 + 1 + 1 + 1 + (3 if (fp8 or mx) else 2) + 1 + 1
     else:
-        launches_per_step = 1 + 3 + 1 + 2 + 1
+        # router, dispatch tables, row quantizer or gather, two GEMMs, reduce
+        launches_per_step = 6
+        if not (fp8 or mx):        # up to 32 tokens the first two are one launch; the decode kernels read rows where they are
+            launches_per_step -= int(t_local <= 32 and e <= 256) + int(not hq.quant.tensor_path_expected(experts.down, t_local * k, False))
+    if shared is not None and fp8:
+        launches_per_step += 3                         # row quantizer, two GEMMs
 
     for w in range(max(args.warmup, 3)):
         out = step(w)
@@ -874,10 +875,9 @@ def run_moe(args):
                              "algorithmic_bytes": abytes,
                              "hbm_gbs": round(abytes / (gemm_ms / 1e3) / 1e9, 1),
                              "hbm_frac_of_measured": round(abytes / (gemm_ms / 1e3) / 1e9 / peaks["hbm_gbs"], 4),
-                             "note": "at 128 rows per expert every weight byte feeds one token tile and every token "
-                                     "tile is fetched once per weight tile: ncu shows DRAM at 30 % and the tensor "
-                                     "pipe at 24 % while the SMs pull 6.2 TB/s from L2, the ceiling this kernel "
-                                     "and a copy-only build of it settle at"})
+                             "note": "at 128 rows per expert every weight byte feeds one token tile: what bounds the "
+                                     "kernel is the fold of every 128-column block by its scales (ncu, 32 experts: "
+                                     "3.3 TB/s of DRAM, tensor pipe 20 %, issue slots 49 %)"})
                 if NCU_TRAFFIC_RATIO_FP8 is not None:
                     roof["traffic"] = int(NCU_TRAFFIC_RATIO_FP8 * abytes / 2)
                     roof["traffic_note"] = "per launch: algorithmic bytes x the ncu dram/algorithmic ratio"
@@ -893,10 +893,7 @@ def run_moe(args):
                              "traffic": int(NCU_TRAFFIC_RATIO_MX * abytes / 2),
                              "traffic_note": "per launch: algorithmic bytes x the ncu dram/algorithmic ratio"})
             else:
-                rows_per_expert = rows_here / max(1, e_l)
-                ts_k = cfg["fmt"] == "MXFP4" or (cfg["fmt"] == "Q4_K" and rows_per_expert < 192)
-                roof["kernel"] = ("hq::grouped_gemm_ts_kernel" if ts_k else "hq::grouped_gemm_kernel") + \
-                                 " (gate/up + down)"
+                roof["kernel"] = "hq::dq_gemm_kernel x2 (gate/up with the gated activation; down); few rows: the decode kernel"
                 bits = 4.5 if cfg["fmt"] == "Q4_K" else 4.25
                 # every weight once, f16 token rows in, f16 intermediate out and in again, f32 rows out
                 abytes = int(3 * e_l * i_ * h * bits / 8) + t_local * h * 2 + rows_here * (4 * i_ + 4 * h)
