@@ -96,7 +96,7 @@ def test_expert_block_tile_edges_and_padding_slots():
 
 @pytest.mark.parametrize("dt", ["bfloat16", "float16"])
 def test_expert_block_16_bit_rows(dt):
-    # 16-bit output: the down projection's rows leave through the shared-memory transpose as 16-bit values
+    # 16-bit output: the down projection's lanes trade halves of token pairs and store two features at a time
     out_dtype = getattr(torch, dt)
     got, want = _expert_block_case(8, 2, 512, 512, 333, 5, out_dtype=out_dtype)
     tol = 2e-3 + (4.5e-3 if dt == "bfloat16" else 6e-4)     # + two roundings of the output dtype (rows, result)

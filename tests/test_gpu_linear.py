@@ -77,7 +77,7 @@ def test_q8_0_prefill_rows_on_the_tensor_cores(m, dt):
 @pytest.mark.parametrize("k", [768, 2048])
 def test_q6_k_prefill_rows_on_the_tensor_cores(m, k):
     # K = 768 has three super-blocks per row, so rows alternate between 4-byte aligned and 2 bytes off: both forms
-    # of the producers' word loads are exercised
+    # of the expanding warps' word loads are exercised
     got, want = run_case("Q6_K", 1000, k, m, torch.bfloat16, torch.float32, 70 + m)
     assert T.rel_l2(got, want) <= 1e-3
 
@@ -95,10 +95,10 @@ def test_further_ggml_types_any_row_count(fmt, dt):
 @pytest.mark.parametrize("m", [9, 130, 600])
 @pytest.mark.parametrize("k", [768, 2048])
 def test_further_ggml_types_prefill_rows_on_the_tensor_cores(fmt, m, k):
-    # the blocks are expanded to f16 by the producer warps (Q5_K / Q2_K: d sc q - dmin m in split f16 arithmetic;
+    # the blocks are expanded to f16 (Q5_K / Q2_K: d sc q - dmin m in split f16 arithmetic;
     # Q4_0 / Q5_0 / Q4_1 / Q5_1: (q - zero) x d [+ m] rounded once; Q3_K: (q - 4) x (d scale)) and multiplied by
     # tcgen05; K = 768 gives Q4_0 / Q5_0 rows whose 18- / 22-byte blocks alternate between 4-byte aligned and 2 bytes
-    # off, and Q3_K rows of 330 bytes that do the same: both forms of the producers' word loads
+    # off, and Q3_K rows of 330 bytes that do the same: both forms of the expanding warps' word loads
     got, want = run_case(fmt, 1000, k, m, torch.bfloat16, torch.float32, 90 + m)
     assert T.rel_l2(got, want) <= 1e-3
 

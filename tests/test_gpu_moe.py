@@ -206,7 +206,7 @@ def test_moe_block_q6_k_gate_and_up(t):
 @pytest.mark.parametrize("fmt", ["Q5_K", "Q4_0", "Q5_0", "Q4_1", "Q5_1", "Q2_K", "Q3_K"])
 @pytest.mark.parametrize("t", [3, 200])
 def test_moe_block_further_ggml_types(fmt, t):
-    # decode rows (the warp-MMA decode kernel) and prefill rows (the tcgen05 grouped GEMM: 200 tokens x top-2 over 4
+    # decode rows (the warp-MMA decode kernel) and prefill rows (the dequantizing GEMM: 200 tokens x top-2 over 4
     # experts is 100 rows per expert)
     got, want = _moe_case(fmt, t, 4, 2, 256, 256, False, L.ACT_SWIGLU, 40 + t)
     assert T.rel_l2(got, want) <= 1e-3
@@ -272,7 +272,7 @@ def test_fp8_quantizers_bit_exact():
     assert got == [[0, 0, 1, 1, 2], [0, 0, 1, 1, 2], [3, 3, 4, 4, 5], [3, 3, 4, 4, 5], [6, 6, 7, 7, 8]]
 
 
-# ---- tensor-core (tcgen05) grouped GEMM: forced on, checked against the oracle and the decode kernel ----------
+# ---- dequantizing tensor-core GEMM: forced on, checked against the oracle and the decode kernel ----------
 
 @pytest.fixture
 def tensor_path():
@@ -308,7 +308,7 @@ def test_tensor_path_dense(tensor_path, fmt, n, k, m):
 @pytest.mark.parametrize("fmt,k,n", [("Q4_K", 512, 192), ("FP8", 256, 128), ("MXFP4", 128, 144)])
 def test_tensor_path_gather_forward(tensor_path, fmt, k, n):
     rng = T.rng_for(5, k + n)
-    e, t, topk = 5, 300, 2          # expert 4 gets nothing, expert 0 gets several 128-row tiles
+    e, t, topk = 5, 300, 2          # expert 4 gets nothing, expert 0 several token tiles
     arrays, deq = T.make_weight(fmt, rng, n, k, experts=e)
     layer = T.make_layer(fmt, arrays, k, DEV)
     p = np.array([0.7, 0.15, 0.1, 0.05, 0.0])
@@ -333,7 +333,7 @@ def test_tensor_path_moe_blocks(tensor_path):
 
 
 def test_tensor_path_wide_token_tiles(tensor_path):
-    # enough rows per expert on average for the 256-token tiles (f16 rows copied with cp.async)
+    # several hundred rows per expert: wide token tiles, rows gathered with cp.async
     rng = T.rng_for(5, 91)
     e, t, topk, k, n = 4, 700, 2, 256, 192
     arrays, deq = T.make_weight("Q4_K", rng, n, k, experts=e)
@@ -355,8 +355,8 @@ def test_tensor_path_wide_token_tiles(tensor_path):
 
 
 def test_tensor_path_short_k_and_partial_feature_tiles(tensor_path):
-    # the kernel that expands the weights into tensor memory, at its edges: K of one, three and five 64-column
-    # stages (fewer stages than producer groups: a group's next stage lies in a later tile), 64-feature gate/up
+    # the dequantizing GEMM at its edges: K of one, three and five 64-column steps (fewer steps than groups of
+    # expanding warps: some serve no stage of a tile), 64-feature gate/up
     # tiles with a partly filled last tile, a 128-lane tile with 64 valid rows, token tiles with a few rows
     got, want = _moe_case("MXFP4", 300, 8, 4, 64, 192, True, L.ACT_GPTOSS, 41, limit=7.0)
     assert T.rel_l2(got, want) <= 2e-3
