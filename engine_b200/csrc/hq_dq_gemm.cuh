@@ -91,9 +91,7 @@ struct DqPlan {
   int nr;             // raw stages in shared memory
   int kslices;        // CTAs (cluster size) per tile
   int cpc;            // split K: most token columns a CTA of the cluster finishes
-  int x_tma;          // token rows lie in tile order: copied as boxes
-  int x_stage;        // ... one box per stage (tn rows, every 64-k step); else boxes of x_box rows, and 16 for the rest
-  int x_box;
+  int x_tma;          // token rows lie in tile order: one box per operand stage
   int raw_tma;        // raw rows copied as boxes (else in 4-byte pieces)
   int off_raw, off_recv, off_rows, off_pref, off_bar, smem;
 };
@@ -336,6 +334,14 @@ struct DqRow {
   }
 };
 
+// Token boxes: a stage's 64-k steps of 16, 32, .. rows, so that an expert's tile of whatever size is one copy (dense calls: the
+// first map, rows of the plan's tile).  A copy instruction costs its warp some 250 cycles: with boxes of 64 and 16 rows and one
+// step each a stage of 128 tokens took six, 1,500 cycles for 1,000 cycles of products (128 experts of 768 x 2,048 Q4_K, 4,096
+// tokens: gated launch 365 us so, 265 with one box; down launch 237, 172).
+struct DqTokenMaps {
+  CUtensorMap m[kDqMaxTokens / 16];
+};
+
 // ---- work items --------------------------------------------------------------------------------------------------
 struct DqTile {
   int expert, row_start, count, n0;
@@ -351,12 +357,12 @@ __device__ __forceinline__ DqTile dq_tile(const GroupedParams& p, const DqPlan& 
     t.count = min(pl.rows_per_tile, p.m - t.row_start);
     return t;
   }
-  int lo = 0, hi = p.n_experts - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (pref[mid] <= tt) lo = mid; else hi = mid - 1;
-  }
-  const int base = __ldg(p.expert_bounds + lo), cnt = __ldg(p.expert_bounds + lo + 1) - base;
+  // the last expert whose tiles start at or in front of tile tt; called by whole warps
+  int before = 0;
+  for (int e = 1 + (threadIdx.x & 31); e < p.n_experts; e += 32) before += pref[e] <= tt ? 1 : 0;
+  const int lo = __reduce_add_sync(0xffffffffu, before);
+  const int32_t* rows = pref + p.n_experts + 1;
+  const int base = rows[lo], cnt = rows[lo + 1] - base;
   // an expert's rows are cut into equal tiles (multiples of 16 rows)
   const int nt = pref[lo + 1] - pref[lo], j = tt - pref[lo];
   const int per = ((cnt + nt - 1) / nt + 15) & ~15;
@@ -364,6 +370,11 @@ __device__ __forceinline__ DqTile dq_tile(const GroupedParams& p, const DqPlan& 
   t.row_start = base + j * per;
   t.count = max(0, min(per, cnt - j * per));
   return t;
+}
+
+// rows of a tile's tokens in shared memory: the distance between the 64-k steps of a stage
+__device__ __forceinline__ int dq_box_rows(const GroupedParams& p, const DqPlan& pl, const DqTile& t) {
+  return p.expert_bounds != nullptr ? max(16, (t.count + 15) & ~15) : pl.tn;
 }
 
 __device__ __forceinline__ void dq_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -555,8 +566,7 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
 template <int FMT, bool ODD>
 __global__ void __launch_bounds__(DqTraits<FMT>::THREADS, 1)
 dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_wu,
-               const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_x16, const GroupedParams p,
-               const DqPlan pl) {
+               const __grid_constant__ DqTokenMaps tm_x, const GroupedParams p, const DqPlan pl) {
   using T = DqTraits<FMT>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -599,8 +609,11 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   if (p.expert_bounds != nullptr) {
     dq_pdl_wait();                 // the routing tables come from the previous kernels
     for (int e = tid; e < p.n_experts; e += T::THREADS) {
-      const int cnt = __ldg(p.expert_bounds + e + 1) - __ldg(p.expert_bounds + e);
-      pref[e + 1] = (cnt + pl.tn - 1) / pl.tn;
+      const int lo = __ldg(p.expert_bounds + e), hi = __ldg(p.expert_bounds + e + 1);
+      pref[e + 1] = (hi - lo + pl.tn - 1) / pl.tn;
+      int32_t* rows = pref + p.n_experts + 1;      // the experts' first rows behind their first tiles
+      rows[e] = lo;
+      if (e == p.n_experts - 1) rows[e + 1] = hi;
     }
     if (tid == 0) pref[0] = 0;
     __syncthreads();
@@ -635,13 +648,14 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     // tensor core needs for 128 columns.)
     uint32_t spin = kDqSpin;
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
-    const uint32_t sub_bytes = (uint32_t)pl.tn * 128u, b0 = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
+    const uint32_t step_bytes = (uint32_t)pl.tn * 128u, b0 = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
     const int a_col = 512 - 32 * pl.subs * pl.ns;
     const int slice_subs = min(kb64, 4 * rs_hi) - 4 * rs_lo, walk_subs = dq_walk_steps(ODD, slice_subs);
     int it = 0, tcount = 0;
     for (int w = first; w < n_tiles; w += step, ++tcount) {
       const DqTile t = dq_tile(p, pl, pref, w, n_nt, fw);
       const uint32_t idesc = make_idesc_f16(__shfl_sync(0xffffffffu, max(16, (t.count + 15) & ~15), 0));
+      const uint32_t sub_bytes = __shfl_sync(0xffffffffu, (uint32_t)dq_box_rows(p, pl, t) * 128u, 0);
       const int buf = pl.nbuf == 2 ? tcount & 1 : 0;
       const int use = pl.nbuf == 2 ? tcount >> 1 : tcount;
       if (use > 0 && !warp_wait(&bar.acc_empty[buf], (use - 1) & 1, spin)) {
@@ -657,7 +671,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           spin = 1;
         }
         tc_fence_after();
-        uint64_t bdesc = make_smem_desc(b0 + (uint32_t)(at.s * pl.subs) * sub_bytes);
+        uint64_t bdesc = make_smem_desc(b0 + (uint32_t)(at.s * pl.subs) * step_bytes);
         uint32_t a0 = tmem_u + (uint32_t)(a_col + 32 * pl.subs * at.s);
         const int n_sub = min(pl.subs, slice_subs - j);
         for (int c = 0; c < n_sub; ++c) {
@@ -864,7 +878,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   } else if (warp < 2 + kDqEpilogueWarps + kDqTokenWarps) {
     // =========================== activation rows ========================================================
     dq_pdl_wait();
-    const uint32_t sub_bytes = (uint32_t)pl.tn * 128u;
+    const uint32_t step_bytes = (uint32_t)pl.tn * 128u;
     const int slice_subs = min(kb64, 4 * rs_hi) - 4 * rs_lo, walk_subs = dq_walk_steps(ODD, slice_subs);
     uint32_t spin = kDqSpin;
     int it = 0;
@@ -873,10 +887,10 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         bool stop = false;
         for (int w = first; w < n_tiles && !stop; w += step) {
           const DqTile t = dq_tile(p, pl, pref, w, n_nt, fw);
-          // whole boxes, then pieces of 16 rows (rows behind the tile's last may be copied along: never looked at)
-          const int boxes = t.count / pl.x_box;
-          const int pieces = (t.count - boxes * pl.x_box + 15) >> 4;
-          const uint32_t bytes = (uint32_t)(boxes * pl.x_box + 16 * pieces) * 128u;
+          // (rows behind the tile's last are copied along: other experts' or zeros, in accumulator columns nobody reads)
+          const int box = dq_box_rows(p, pl, t);
+          const uint32_t bytes = (uint32_t)(pl.subs * box) * 128u;
+          const CUtensorMap* map = &tm_x.m[p.expert_bounds != nullptr ? (box >> 4) - 1 : 0];
           for (int j = 0; j < walk_subs; j += pl.subs, ++it) {
             const DqSlot at = dq_slot(pl, it);
             if (at.use > 0 && !warp_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
@@ -888,22 +902,9 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
               warp_arrive(&bar.full[at.s]);
               continue;
             }
-            if (pl.x_stage) {
-              warp_arrive_expect(&bar.full[at.s], (uint32_t)pl.subs * sub_bytes);
-              warp_tma_3d(smem_u32(smem) + (uint32_t)(at.s * pl.subs) * sub_bytes, &tm_x, 0, t.row_start, 4 * rs_lo + j,
+            warp_arrive_expect(&bar.full[at.s], bytes);
+            warp_tma_3d(smem_u32(smem) + (uint32_t)(at.s * pl.subs) * step_bytes, map, 0, t.row_start, 4 * rs_lo + j,
                         &bar.full[at.s]);
-              continue;
-            }
-            const int n_sub = min(pl.subs, slice_subs - j);
-            warp_arrive_expect(&bar.full[at.s], bytes * (uint32_t)n_sub);
-            for (int c = 0; c < n_sub; ++c) {
-              const int x = (4 * rs_lo + j + c) * 64;
-              uint32_t dst = smem_u32(smem) + (uint32_t)(at.s * pl.subs + c) * sub_bytes;
-              int row = t.row_start;
-              for (int i = 0; i < boxes; ++i, row += pl.x_box, dst += (uint32_t)pl.x_box * 128u)
-                warp_tma_2d(dst, &tm_x, x, row, &bar.full[at.s]);
-              for (int i = 0; i < pieces; ++i, row += 16, dst += 2048u) warp_tma_2d(dst, &tm_x16, x, row, &bar.full[at.s]);
-            }
           }
         }
 #pragma unroll 1
@@ -939,6 +940,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           rows[r] = (uint32_t)(p.x_rows ? __ldg(p.x_rows + sp) : sp) * x_stride16;
         }
         named_bar_sync(1, 32 * kDqTokenWarps);
+        const uint32_t sub_bytes = (uint32_t)dq_box_rows(p, pl, t) * 128u;
         for (int j = 0; j < walk_subs; j += pl.subs, ++it) {
           const DqSlot at = dq_slot(pl, it);
           if (at.use > 0 && !warp_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
@@ -947,7 +949,7 @@ dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           }
           const int n_sub = min(pl.subs, slice_subs - j);
           for (int c = 0; c < n_sub; ++c) {
-            uint32_t dst = dst_thread + (uint32_t)(at.s * pl.subs + c) * sub_bytes;
+            uint32_t dst = dst_thread + (uint32_t)(at.s * pl.subs) * step_bytes + (uint32_t)c * sub_bytes;
             const uint4* src = reinterpret_cast<const uint4*>(p.x) + ((uint32_t)(4 * rs_lo + j + c) * 8u + (uint32_t)chunk);
 #pragma unroll 8
             for (int r = row0; r < t.count; r += 8, dst += 1024u)

@@ -32,7 +32,7 @@ bool dq_smem_plan(DqPlan& pl, int n_experts, bool expert_indexed) {
   const int stage = pl.subs * pl.tn * 128;
   pl.cpc = (pl.tn + pl.kslices - 1) / pl.kslices;
   const int recv = pl.kslices > 1 ? pl.kslices * pl.cpc * 512 : 0;
-  const int pref = expert_indexed ? ((n_experts + 1) * 4 + 15) & ~15 : 16;
+  const int pref = expert_indexed ? (2 * (n_experts + 1) * 4 + 15) & ~15 : 16;
   const int rows = 2 * kDqMaxTokens * 4;
   const int fixed = rows + pref + kDqNumBars * 8 + 16 + 1024;
   pl.ns = (512 - pl.nbuf * pl.tn) / (32 * pl.subs);
@@ -164,7 +164,8 @@ template <int FMT, bool ODD>
 int32_t launch_dq_plan(const GroupedParams& p, DqPlan& pl, int grid, int64_t rows, cudaStream_t stream) {
   if (!dq_kernel_ready<FMT, ODD>()) return HQ_ERR_CUDA;
   using T = DqTraits<FMT>;
-  CUtensorMap tm_w{}, tm_wu{}, tm_x{}, tm_x16{};
+  CUtensorMap tm_w{}, tm_wu{};
+  DqTokenMaps tm_x{};
   pl.raw_tma = T::WIDE || (p.w_row_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(p.w) & 15u) == 0 &&
                            (reinterpret_cast<uintptr_t>(p.w_up) & 15u) == 0);
   if (pl.raw_tma) {
@@ -185,17 +186,11 @@ int32_t launch_dq_plan(const GroupedParams& p, DqPlan& pl, int grid, int64_t row
   }
   pl.x_tma = p.x_rows == nullptr;
   if (pl.x_tma) {
-    pl.x_stage = p.expert_bounds == nullptr || pl.tn <= 64;
-    pl.x_box = 64;
-    if (pl.x_stage) {
-      if (!encode_column_blocks(&tm_x, p.x, (uint64_t)p.k / 64, (uint64_t)rows, (uint64_t)p.x_stride * 2, (uint32_t)pl.tn,
-                                (uint32_t)pl.subs))
+    const int first = p.expert_bounds != nullptr ? 16 : pl.tn;
+    for (int box = first; box <= pl.tn; box += 16)
+      if (!encode_column_blocks(&tm_x.m[(box - first) / 16], p.x, (uint64_t)p.k / 64, (uint64_t)rows, (uint64_t)p.x_stride * 2,
+                                (uint32_t)box, (uint32_t)pl.subs))
         return HQ_ERR_CUDA;
-    } else if (!f8_encode_2d(&tm_x, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.x, (uint64_t)p.k, (uint64_t)rows, (uint64_t)p.x_stride * 2,
-                      64, (uint32_t)pl.x_box, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !f8_encode_2d(&tm_x16, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.x, (uint64_t)p.k, (uint64_t)rows,
-                      (uint64_t)p.x_stride * 2, 64, 16, CU_TENSOR_MAP_SWIZZLE_128B))
-      return HQ_ERR_CUDA;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
@@ -210,7 +205,7 @@ int32_t launch_dq_plan(const GroupedParams& p, DqPlan& pl, int grid, int64_t row
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pl.kslices > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, dq_gemm_kernel<FMT, ODD>, tm_w, tm_wu, tm_x, tm_x16, p, pl) == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
+  return cudaLaunchKernelEx(&cfg, dq_gemm_kernel<FMT, ODD>, tm_w, tm_wu, tm_x, p, pl) == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
 }
 
 template <int FMT>

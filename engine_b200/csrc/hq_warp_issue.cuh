@@ -12,9 +12,25 @@ namespace hq {
 
 constexpr uint32_t kWaitSuspendNs = 20000;
 
+__device__ __forceinline__ bool warp_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Bounded wait whose polls suspend the warp for long: twenty-odd warps that poll at the default rate keep the barrier unit
-// busy enough to slow down the arrivals and copy instructions of the others.
+// busy enough to slow down the arrivals and copy instructions of the others.  A plain test goes first: on a phase that is
+// complete already, the usual case in a ring that runs ahead, it takes 66 cycles, a try_wait with a time limit 100 to 127
+// (65,536 x 4,096 at 16 rows on the dequantizing GEMM: Q4_K 69.9 -> 67.2 us, FP8 55.1 -> 52.8).
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, uint32_t spin_limit) {
+  if (warp_test(bar, parity)) return true;
   for (uint32_t i = 0; i < spin_limit; ++i) {
     uint32_t ok;
     asm volatile(
