@@ -97,6 +97,35 @@ __device__ __forceinline__ AffineH2 make_affine(uint32_t d_dmin, uint32_t s, uin
   r.ml = __float2half2_rn(m1 - __half2float(mh));
   return r;
 }
+__device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+__device__ __forceinline__ __half2 bits_h2(uint32_t b) { return *reinterpret_cast<const __half2*>(&b); }
+// The same of two sub-blocks at a time, their scales and minima the bytes of s4 / m4 that `pick` (a permute selector that pairs
+// each with 0x64) names: words {d | dmin, ...} -> {d twice, scales, minus the minima, their remainders}, a sub-block per half.
+// HIGH: the second sub-block's codes come 16 times too large, as high nibbles where they lie, and its scale is a sixteenth.
+// All exact but the rounding of dmin * m to its leading part, as in make_affine; 11 instructions instead of 2 x 15.
+template <bool HIGH>
+__device__ __forceinline__ void affine_pair(uint32_t* w, uint32_t s4, uint32_t m4, uint32_t pick) {
+  const __half2 one = bits_h2(0x64006400u);      // 1024
+  __half2 s = __hsub2(bits_h2(__byte_perm(s4, 0x64646464u, pick)), one);
+  if (HIGH) s = __hmul2(s, bits_h2(0x2C003C00u));      // 1, 1 / 16
+  const __half2 m = __hsub2(bits_h2(__byte_perm(m4, 0x64646464u, pick)), one);
+  const __half2 dmin = __hneg2(bits_h2(__byte_perm(w[0], 0u, 0x3232)));
+  const __half2 mh = __hmul2(dmin, m);
+  w[0] = __byte_perm(w[0], 0u, 0x1010);
+  w[1] = h2_bits(s);
+  w[2] = h2_bits(mh);
+  w[3] = h2_bits(__hfma2(dmin, m, __hneg2(mh)));
+}
+__device__ __forceinline__ AffineH2 affine_of(const uint32_t* w, int i) {
+  const uint32_t pick = i ? 0x3232u : 0x1010u;
+  AffineH2 r;
+  r.s = bits_h2(__byte_perm(w[1], 0u, pick));
+  r.cs = __hmul2(r.s, bits_h2(0xE400E400u));      // -1024
+  r.d = bits_h2(w[0]);
+  r.mh = bits_h2(__byte_perm(w[2], 0u, pick));
+  r.ml = bits_h2(__byte_perm(w[3], 0u, pick));
+  return r;
+}
 // four code bytes -> two f16 pairs
 __device__ __forceinline__ void affine4(const AffineH2& a, uint32_t codes, uint32_t& o01, uint32_t& o23) {
   uint32_t p01 = __byte_perm(codes, 0x64646464u, 0x4140);

@@ -148,8 +148,7 @@ struct DqRow {
       if constexpr (FMT == HQ_FMT_Q5_K) dq_lds_shifted<8, 0>(w + 12, addr + 16);
       uint32_t s4, m4;
       k_scales(w[1], w[2], w[3], c >= 2, s4, m4);
-      w[1] = s4 >> (16 * (c & 1));      // scale and minimum of the first half in the low byte, of the second above it
-      w[2] = m4 >> (16 * (c & 1));
+      affine_pair<FMT == HQ_FMT_Q4_K>(w, s4, m4, (c & 1) ? 0x4342u : 0x4140u);
     } else if constexpr (FMT == HQ_FMT_Q8_0) {
       // two 34-byte blocks {f16 d, int8 q[32]} from byte 68 c on
       dq_lds_words<17>(w, addr + ((68 * c) & ~15), c);
@@ -198,13 +197,15 @@ struct DqRow {
     uint32_t o[8];
     bool ok = true;
     if constexpr (FMT == HQ_FMT_Q4_K || FMT == HQ_FMT_Q5_K) {
-      const AffineH2 f = make_affine(w[0], (w[1] >> (8 * i)) & 0xFFu, (w[2] >> (8 * i)) & 0xFFu);
+      const AffineH2 f = affine_of(w, i);
+      const uint32_t nibbles = 0x0F0F0F0Fu << (4 * i);      // Q4_K: the second half's codes stay 16 times too large
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          uint32_t codes = (w[4 + 4 * u + j] >> (4 * i)) & 0x0F0F0F0Fu;
-          if constexpr (FMT == HQ_FMT_Q5_K) codes |= ((w[12 + 4 * u + j] >> (2 * c + i)) & 0x01010101u) << 4;
+          uint32_t codes;
+          if constexpr (FMT == HQ_FMT_Q4_K) codes = w[4 + 4 * u + j] & nibbles;
+          else codes = ((w[4 + 4 * u + j] >> (4 * i)) & 0x0F0F0F0Fu) | (((w[12 + 4 * u + j] >> (2 * c + i)) & 0x01010101u) << 4);
           affine4(f, codes, o[2 * j], o[2 * j + 1]);
         }
         put(8 * u, o);

@@ -46,6 +46,34 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, uint32
   }
   return false;
 }
+// The same for the loops whose instruction count matters: no branch the compiler has to treat as divergent (its convergence
+// barriers are instructions too), the outcome as a value.  Whole converged warps only.
+__device__ __forceinline__ uint32_t warp_wait_uni(uint32_t bar, uint32_t parity, uint32_t spin_limit) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      ".reg .u32 n;\n"
+      "mov.u32 %0, 1;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "vote.sync.all.pred p, p, 0xffffffff;\n"
+      "@p bra.uni DONE;\n"
+      "mov.u32 n, %3;\n"
+      "POLL:\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %4;\n"
+      "vote.sync.all.pred p, p, 0xffffffff;\n"
+      "@p bra.uni DONE;\n"
+      "setp.gt.u32 q, n, 1;\n"
+      "sub.u32 n, n, 1;\n"
+      "@q bra.uni POLL;\n"
+      "mov.u32 %0, 0;\n"
+      "DONE:\n"
+      "}\n"
+      : "=&r"(ok)
+      : "r"(bar), "r"(parity), "r"(spin_limit), "r"(kWaitSuspendNs)
+      : "memory");
+  return ok;
+}
 // No copy may still be writing a CTA's shared memory when it exits: bounded wait of a copying warp for the stages ring_drain
 // names (bar[slot] completes with a stage's copies).  On the normal path whoever reads the stages waits for the same.
 __device__ __forceinline__ bool warp_drain(uint64_t* bar, int next, int slots, int slot, int parity, int warps, int me,
@@ -54,15 +82,16 @@ __device__ __forceinline__ bool warp_drain(uint64_t* bar, int next, int slots, i
 }
 // mbarrier arrivals by the elected lane of a whole warp, as a predicated instruction: a branch for one lane costs the
 // other roles' warps instruction fetches (and this one several hundred cycles when it misses)
-__device__ __forceinline__ void warp_arrive(uint64_t* bar) {
+__device__ __forceinline__ void warp_arrive_at(uint32_t bar) {
   asm volatile(
       "{\n"
       ".reg .pred e;\n"
       "elect.sync _|e, 0xffffffff;\n"
       "@e mbarrier.arrive.shared::cta.b64 _, [%0];\n"
-      "}\n" ::"r"(smem_u32(bar))
+      "}\n" ::"r"(bar)
       : "memory");
 }
+__device__ __forceinline__ void warp_arrive(uint64_t* bar) { warp_arrive_at(smem_u32(bar)); }
 __device__ __forceinline__ void warp_arrive_expect(uint64_t* bar, uint32_t bytes) {
   asm volatile(
       "{\n"
