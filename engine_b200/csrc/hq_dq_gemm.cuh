@@ -358,10 +358,11 @@ __device__ __forceinline__ DqTile dq_tile(const GroupedParams& p, const DqPlan& 
     t.count = min(pl.rows_per_tile, p.m - t.row_start);
     return t;
   }
-  // the last expert whose tiles start at or in front of tile tt; called by whole warps
-  int before = 0;
-  for (int e = 1 + (threadIdx.x & 31); e < p.n_experts; e += 32) before += pref[e] <= tt ? 1 : 0;
-  const int lo = __reduce_add_sync(0xffffffffu, before);
+  int lo = 0, hi = p.n_experts - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (pref[mid] <= tt) lo = mid; else hi = mid - 1;
+  }
   const int32_t* rows = pref + p.n_experts + 1;
   const int base = rows[lo], cnt = rows[lo + 1] - base;
   // an expert's rows are cut into equal tiles (multiples of 16 rows)
