@@ -13,27 +13,32 @@
 // the accumulator as floats through a bias constant (no conversion instruction), are multiplied by the
 // block's d, summed over the four blocks of a group and scaled once by the group's activation scale.
 //
-// Layout of the work: persistent CTAs (one per SM) walk items of 16, 32 or 64 output rows.  Two producer warps
+// Layout of the work: persistent CTAs (one per SM) walk items of 16, 32 or 64 output rows.  Four producer warps
 // stream the item's row segments (2176 bytes = 64 blocks per bulk async copy for 16 rows) into a shared-memory ring
 // with mbarrier completion.  The sixteen consumer warps each take one group of
 // four blocks (136 bytes, 8-byte aligned) of every stage, so the misaligned block payloads are fetched
 // with a fixed pattern of 8- and 4-byte loads and four funnel shifts per row.  Within an MMA the k order
 // is free as long as both operands agree: lane t owns payload bytes 8t..8t+7 of a block, and reads the
 // same eight positions of the staged activations with one 8-byte load.  Partial sums of the K slices
-// meet in shared memory and are added in warp order by a warp of their own: results are
+// meet in shared memory and are added in warp order by four warps of their own: results are
 // bit-reproducible.
+// What a short item costs besides its groups decides (us, one reducing warp and two producers before: 4,096 x 4,096 Q4_K, one
+// row 7.3 -> 6.1; 65,536 x 4,096 Q4_K 48.6 -> 40.3; 128 experts of 768 x 2,048, 64 tokens 231 -> 154): items are looked up
+// one ahead, dense calls of up to eight rows without a division, and the waits of the consumer warps leave no branch behind.
 //
 // Algorithmic bytes per launch: N*K*34/32 (weights) + M*K*sizeof(x) + M*N*sizeof(y).
 #include "hq_gemv_shared.cuh"
+#include "hq_warp_issue.cuh"
 
 namespace hq {
 
 constexpr int kQ8Warps = 16;                     // consumer warps, one group of a stage each
 constexpr int kQ8Consumers = kQ8Warps * 32;
-constexpr int kQ8Producers = 2;                  // producer warps: a bulk-copy instruction holds its warp for ~50
-                                                 // cycles per active lane, so the 16 row copies of a stage are
-                                                 // split over two warps
-constexpr int kQ8Threads = kQ8Consumers + 32 * (kQ8Producers + 1);   // + producers + the reducing warp
+constexpr int kQ8Producers = 4;                  // producer warps: a bulk-copy instruction holds its warp for ~50
+                                                 // cycles per active lane, so the 16 to 64 row copies of a stage are
+                                                 // split over four warps
+constexpr int kQ8Reducers = 4;                   // reducing warps, one accumulator value of every lane each
+constexpr int kQ8Threads = kQ8Consumers + 32 * (kQ8Producers + kQ8Reducers);
 constexpr int kQ8RT = 16;                        // output rows of one MMA tile
 // A work item is RS such tiles (RS = 1, 2 or 4), a stage 16 / RS groups of every row: with K short of 16 groups (an
 // expert's 768 or 2048 columns) the warps that would have no group take further rows instead, and a stage stays one
@@ -61,7 +66,7 @@ struct I8Traits<HQ_FMT_Q4_K> {
 constexpr int kQ8MaxStages = 8;
 constexpr int kQ8SmemBudget = 227 * 1024 - 256;   // dynamic part; a few static words come on top
 constexpr int kQ8XGroups = 4;                    // 16-byte registers a thread prefetches activations into
-constexpr uint32_t kQ8Spin = 1u << 22;
+constexpr uint32_t kQ8Spin = 1u << 16;           // polls of a wait, each suspended for a while
 constexpr int kQ8Magic = 0x4B400000;             // 1.5 * 2^23 as f32 bits: magic + n reads as 12582912.f + n
 template <>
 struct I8Traits<HQ_FMT_FP8_BLOCK> {
@@ -618,25 +623,36 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
 
-  if (tid == 0) {
-    for (int s = 0; s < NSTAGE; ++s) {
-      mbar_init(&full[s], kQ8Producers);
-      mbar_init(&empty[s], WK);
+  // The producer warps set up the barriers and start copying; the others clear the staged activations meanwhile (columns
+  // beyond an item's row count must read as zero) and meet them at a barrier the producers do not wait at.
+  const bool producer = warp >= WK && warp < WK + kQ8Producers;
+  if (producer) {
+    if (tid == kQ8Consumers) {
+      for (int s = 0; s < NSTAGE; ++s) {
+        mbar_init(&full[s], kQ8Producers);
+        mbar_init(&empty[s], WK);
+      }
+      for (int b = 0; b < 2; ++b) {
+        mbar_init(&red_full[b], WK);
+        mbar_init(&red_free[b], kQ8Reducers);
+      }
+      fence_barrier_init();
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&red_full[b], WK);
-      mbar_init(&red_free[b], 1);
-    }
-    fence_barrier_init();
+    named_bar_sync(3, 32 * kQ8Producers);
+    asm volatile("bar.arrive 2, %0;" ::"n"(kQ8Threads) : "memory");
+  } else {
+    for (int i = warp < WK ? tid : tid - 32 * kQ8Producers; i < lay.x_bytes / 16; i += kQ8Threads - 32 * kQ8Producers)
+      reinterpret_cast<uint4*>(smem + lay.off_x)[i] = make_uint4(0, 0, 0, 0);
+    named_bar_sync(2, kQ8Threads);
   }
-  // zero the staged activations once: columns beyond an item's row count must read as zero
-  for (int i = tid; i < lay.x_bytes / 16; i += kQ8Threads)
-    reinterpret_cast<uint4*>(smem + lay.off_x)[i] = make_uint4(0, 0, 0, 0);
-  __syncthreads();
-
   const int64_t row_bytes = T::row_bytes(p.k);
 
-  if (warp >= WK && warp < WK + kQ8Producers) {
+  float* red = reinterpret_cast<float*>(smem + lay.off_red);   // [2 buffers][banks][warps][4][32]
+  const int g = lane >> 2, t = lane & 3;
+
+  // 768 threads x 80 registers at launch = 512 x 96 + 256 x 48
+  if (producer) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
     // ================= producer warps: stream weight row segments ================================
     const int pw = warp - WK;
     constexpr int RPP = RT / kQ8Producers;      // rows per producer warp
@@ -644,8 +660,9 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
     uint64_t policy;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
     int s = 0, round = 0;
-    for (int w = w_begin; w < w_end; w += w_step) {
-      const WorkItem wi = get_item<RT>(p, w, n_rt);
+    WorkItem wi = get_item<RT>(p, w_begin, n_rt), nx;
+    for (int w = w_begin; w < w_end; w += w_step, wi = nx) {
+      nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt);      // fetched an item ahead
       if (wi.nrows <= 0) continue;
       const int rows_valid = min(RT, p.n - wi.n0);
       const int my_rows = max(0, min(RPP, rows_valid - pw * RPP));
@@ -675,21 +692,26 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
         }
       }
     }
-  }
-
-  float* red = reinterpret_cast<float*>(smem + lay.off_red);   // [2 buffers][banks][warps][4][32]
-  const int g = lane >> 2, t = lane & 3;
-
-  if (warp == WK + kQ8Producers) {
-    // ================= reducing warp: adds the K-split partial sums in warp order and writes ======
+    } else if (warp >= WK) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    // ================= reducing warps: add the K-split partial sums in warp order and write ======
+    // Each takes one of a lane's four accumulator values: output row g (+ 8), activation row 2 t (+ 1).  One warp for all
+    // four bound short items (RS = 2 or 4): Q4_K experts of 768 x 2,048, 64 tokens, 6,700 cycles an item.
     pdl_wait();
+    const int vi = warp - (WK + kQ8Producers);
+    const int row = g + 8 * (vi >> 1), col = 2 * t + (vi & 1);
+    const bool owner = NCS > 1 || t < (FMT == HQ_FMT_FP8_BLOCK ? 1 : 2);
     uint32_t spin = kQ8Spin;
     int item = 0;
-    for (int w = w_begin; w < w_end; w += w_step) {
-      const WorkItem wi = get_item<RT>(p, w, n_rt);
+    WorkItem wi = get_item<RT>(p, w_begin, n_rt), nx;
+    for (int w = w_begin; w < w_end; w += w_step, wi = nx) {
+      nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt);
       if (wi.nrows <= 0) continue;
       const int rb = item & 1;
-      const float* rbuf = red + rb * (p.n_banks * WK * 4 * 32);
+      const float* rbuf = red + rb * (p.n_banks * WK * 4 * 32) + vi * 32 + lane;
+      const bool mine = owner && col < wi.nrows;
+      int64_t yrow = wi.row0 + col;
+      if (mine && p.y_rows != nullptr && S == 1) yrow = p.y_rows[wi.row0 + col];
       bool failed = false;
       if (!mbar_wait_backoff(&red_full[rb], (item >> 1) & 1, spin)) {
         if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 310 + rb);
@@ -699,49 +721,42 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
       WorkItem ti = wi;
 #pragma unroll 1
       for (int rt = 0; rt < RS; ++rt, ti.n0 += kQ8RT) {
-        float v[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        float v[2] = {0.f, 0.f};
 #pragma unroll
         for (int b = 0; b < 2; ++b)
           if (b < p.n_banks) {
+            float sum = 0.f;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              float sum = 0.f;
-#pragma unroll
-              for (int j = 0; j < WG; ++j) sum += rbuf[((b * WK + rt * WG + j) * 4 + i) * 32 + lane];
-              if (NCS == 1 && FMT == HQ_FMT_FP8_BLOCK) {
-                // two-row layout of the three e4m3 terms: columns 2, 3 and 4, 5 sit one and two lanes further on
-                const float s1 = __shfl_down_sync(0xffffffffu, sum, 1), s2 = __shfl_down_sync(0xffffffffu, sum, 2);
-                sum += s1 + s2;
-              } else if (NCS == 1) {
-                // four-row layout: the remainder columns 4..7 sit two lanes further on
-                sum += __shfl_down_sync(0xffffffffu, sum, 2);
-              }
-              v[b][i] = sum;
+            for (int j = 0; j < WG; ++j) sum += rbuf[(b * WK + rt * WG + j) * 128];
+            if (NCS == 1 && FMT == HQ_FMT_FP8_BLOCK) {
+              // two-row layout of the three e4m3 terms: columns 2, 3 and 4, 5 sit one and two lanes further on
+              const float s1 = __shfl_down_sync(0xffffffffu, sum, 1), s2 = __shfl_down_sync(0xffffffffu, sum, 2);
+              sum += s1 + s2;
+            } else if (NCS == 1) {
+              // four-row layout: the remainder columns 4..7 sit two lanes further on
+              sum += __shfl_down_sync(0xffffffffu, sum, 2);
             }
+            v[b] = sum;
           }
         if (rt == RS - 1) {
           __syncwarp();
-          if (lane == 0) mbar_arrive(&red_free[rb]);
+          warp_arrive(&red_free[rb]);
         }
         if (S > 1) {
           // split K: the slice sums of an item meet in global memory and are added when the kernel ends
           const int nb = p.n_banks;
-          float* mine = lay.partials + (((int64_t)w * S + slice) * RS + rt) * (nb * 128);
-#pragma unroll
-          for (int b = 0; b < 2; ++b)
-            if (b < nb) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i) __stcg(mine + (b * 4 + i) * 32 + lane, v[b][i]);
-            }
+          float* part = lay.partials + (((int64_t)w * S + slice) * RS + rt) * (nb * 128) + vi * 32 + lane;
+          __stcg(part, v[0]);
+          if (nb == 2) __stcg(part + 128, v[1]);
         } else {
-          gemv_store_item(p, ti, g, 2 * t, !failed && (NCS > 1 || t < (FMT == HQ_FMT_FP8_BLOCK ? 1 : 2)), v);
+          gemv_store_value(p, ti.expert, ti.n0 + row, mine && !failed, yrow, v[0], v[1]);
         }
       }
       ++item;
     }
-  }
-
-  if (warp < WK) {
+    if (S > 1) asm volatile("bar.arrive 4, %0;" ::"n"(kQ8Consumers + 32 * kQ8Reducers) : "memory");
+  } else {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
   pdl_wait();
   // ================= consumer warps ================================================================
   uint8_t* xq = smem + lay.off_x;
@@ -764,19 +779,19 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
   bool pf_valid = false;
   int staged_y = -1;        // activation rows currently staged (valid when n_super == 1)
   int staged_rows = 0;
-  {
-    const WorkItem w0 = get_item<RT>(p, w_begin, n_rt);
-    if (w0.nrows > 0) {
-      q8_x_prefetch(pf, p, w0.row0, w0.nrows, k_lo, min(xk_sub, k_hi - k_lo), tid);
-      pf_valid = true;
-    }
+  WorkItem wi = get_item<RT>(p, w_begin, n_rt), nx;
+  if (wi.nrows > 0) {
+    q8_x_prefetch(pf, p, wi.row0, wi.nrows, k_lo, min(xk_sub, k_hi - k_lo), tid);
+    pf_valid = true;
   }
 
+  // (a wait that runs out makes `spin` 0: the waits left poll once, every warp still reaches every barrier, and it is reported
+  // at the end; the reducing warps keep what never arrived from being stored)
   uint32_t spin = kQ8Spin;
   int s = 0, item = 0;
   uint32_t phase = 0;
-  for (int w = w_begin; w < w_end; w += w_step) {
-    const WorkItem wi = get_item<RT>(p, w, n_rt);
+  for (int w = w_begin; w < w_end; w += w_step, wi = nx) {
+    nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt);      // fetched an item ahead
     if (wi.nrows <= 0) continue;
     float acc[2][NCS][4];
 #pragma unroll
@@ -823,7 +838,6 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
           q8_x_prefetch(pf, p, wi.row0, wi.nrows, k_base + kXK, min(xk_sub, k_hi - k_base - kXK), tid);
           pf_valid = true;
         } else if (w + w_step < w_end) {
-          const WorkItem nx = get_item<RT>(p, w + w_step, n_rt);
           if (nx.nrows > 0 && (n_super > 1 || nx.y != wi.y)) {
             q8_x_prefetch(pf, p, nx.row0, nx.nrows, k_lo, min(xk_sub, k_hi - k_lo), tid);
             pf_valid = true;
@@ -846,11 +860,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
             wsv = __ldg(reinterpret_cast<const float*>(bank == 0 ? p.scales : p.scales_up) +
                         (int64_t)wi.expert * p.scale_expert_stride +
                         (int64_t)((wi.n0 + kQ8RT * rtile) / 128) * ((p.k + 127) / 128) + k_chunk / 128 + wgrp);
-          if (!mbar_wait(&full[s], phase, spin)) {
-            // bounded wait ran out: flag it and carry on (every warp still reaches every barrier)
-            if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 200 + s);
-            spin = 1;
-          }
+          spin = warp_wait_uni(smem_u32(&full[s]), phase, spin) ? spin : 0u;
           if (wgrp < ngroups) {
             const uint32_t da = smem_u32(smem + s * ST::BYTES) + (uint32_t)(kQ8RT * rtile + g) * ST::PITCH +
                                 (uint32_t)T::GROUP_BYTES * wgrp;
@@ -880,12 +890,8 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
     // ---- hand the K-split partials to the reducing warp (two buffers) ----------------------------------
     const int rb = item & 1;
     float* rbuf = red + rb * (p.n_banks * WK * 4 * 32);
-    if (item >= 2) {
-      if (!mbar_wait(&red_free[rb], ((item >> 1) - 1) & 1, spin)) {
-        if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 300 + rb);
-        spin = 1;
-      }
-    }
+    // (the first two items wait for the phase before a barrier's first, which counts as complete)
+    spin = warp_wait_uni(smem_u32(&red_free[rb]), ((item >> 1) - 1) & 1, spin) ? spin : 0u;
 #pragma unroll
     for (int b = 0; b < 2; ++b)
       if (b < p.n_banks) {
@@ -899,31 +905,31 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
         }
       }
     __syncwarp();
-    if (lane == 0) mbar_arrive(&red_full[rb]);
+    warp_arrive(&red_full[rb]);
     ++item;
   }
-  }   // consumer warps
+  if (spin == 0u && lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 200);
+
 
   if (S > 1) {
     // ---- split K: whichever CTA of an item stream finishes last adds the slice sums of the stream's items, in
     // slice order (so the result does not depend on who that is), and leaves the counter at zero ---------------
     __shared__ int last_flag;
-    pdl_wait();
-    __syncthreads();
+    named_bar_sync(4, kQ8Consumers + 32 * kQ8Reducers);      // the reducing warps have written the CTA's slice sums
     if (tid == 0) {
       __threadfence();
       const int old = atomicAdd(lay.counters + r0, 1);
       last_flag = old == S - 1;
       if (last_flag) lay.counters[r0] = 0;
     }
-    __syncthreads();
+    named_bar_sync(1, kQ8Consumers);
     if (last_flag) {
       __threadfence();
       const int nb = p.n_banks;
       int idx = 0;
       for (int w = w_begin; w < w_end; w += w_step)
         for (int rt = 0; rt < RS; ++rt, ++idx) {
-          if (idx % (kQ8Threads / 32) != warp) continue;
+          if (idx % WK != warp) continue;
           WorkItem wi = get_item<RT>(p, w, n_rt);
           if (wi.nrows <= 0) continue;
           wi.n0 += kQ8RT * rt;
@@ -951,6 +957,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
         }
     }
   }
+  }   // consumer warps
 }
 
 // ---- host launcher -----------------------------------------------------------------------------

@@ -29,7 +29,7 @@ struct WorkItem {
 template <int RT>
 __device__ __forceinline__ WorkItem get_item(const GemvParams& p, int w, int n_rt) {
   WorkItem it;
-  it.y = w / n_rt;
+  it.y = p.tiles == nullptr && p.m <= 8 ? 0 : w / n_rt;
   it.n0 = (w - it.y * n_rt) * RT;
   if (p.tiles != nullptr) {
     it.expert = p.tiles[2 * it.y];
@@ -89,6 +89,27 @@ __device__ __forceinline__ void gemv_store_item(const GemvParams& p, const WorkI
       }
     }
   }
+}
+
+// The same for one value per lane and bank: output row n of activation row `yrow`; `mine`: the lane has one to write.  Lane
+// 4 g + t holds row n0 + g (+ 8), so the up row of an interleaved pair sits four lanes further on.
+__device__ __forceinline__ void gemv_store_value(const GemvParams& p, int expert, int n, bool mine, int64_t yrow, float v,
+                                                 float u) {
+  const bool n_ok = n < p.n;
+  if (n_ok && p.bias != nullptr) v += load_as_float(p.bias, p.bias_dtype, (int64_t)expert * p.n + n);
+  if (n_ok && p.n_banks == 2 && p.bias_up != nullptr) u += load_as_float(p.bias_up, p.bias_dtype, (int64_t)expert * p.n + n);
+  int64_t out_n = n;
+  bool write = n_ok && mine;
+  if (p.act.act != HQ_ACT_NONE) {
+    if (p.n_banks == 2) {
+      v = gated(v, u, p.act);
+    } else {
+      v = gated(v, __shfl_down_sync(0xffffffffu, v, 4), p.act);
+      write = write && (n & 1) == 0;
+      out_n = n >> 1;
+    }
+  }
+  if (write) store_from_float(p.y, p.y_dtype, yrow * p.y_stride + out_n, v);
 }
 
 // ---- cp.async pieces of the kernels that stage weight rows through shared memory --------------------------------
