@@ -74,6 +74,22 @@ __device__ __forceinline__ uint32_t warp_wait_uni(uint32_t bar, uint32_t parity,
       : "memory");
   return ok;
 }
+// Remembers a wait that ran out (`spin` 0) in a word of shared memory, without a branch.
+//
+// An MMA-issuing warp must not branch on its waits' outcome: where the compiler has to take control flow for divergent, the
+// operands of tcgen05.mma move from vector to uniform registers for every instruction, 120 to 140 cycles an MMA instead of 40
+// to 70.  Such a warp keeps issuing after a time-out, on whatever its stages hold, and leaves this word for the warps that
+// would store the products.
+__device__ __forceinline__ void warp_mark_late(uint32_t word, uint32_t spin) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.eq.u32 q, %1, 0;\n"
+      "@q st.shared.u32 [%0], 1;\n"
+      "}\n" ::"r"(word),
+      "r"(spin)
+      : "memory");
+}
 // No copy may still be writing a CTA's shared memory when it exits: bounded wait of a copying warp for the stages ring_drain
 // names (bar[slot] completes with a stage's copies).  On the normal path whoever reads the stages waits for the same.
 __device__ __forceinline__ bool warp_drain(uint64_t* bar, int next, int slots, int slot, int parity, int warps, int me,
@@ -122,6 +138,36 @@ __device__ __forceinline__ void warp_tma_2d(uint32_t dst, const CUtensorMap* map
       "@e cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
       "}\n" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
+      : "memory");
+}
+
+// 128 k of block-scaled products, kind::mxf8f6f4: four MMAs of K = 32, 32 bytes along the swizzled rows of both operands and one
+// scale byte (instruction descriptor bits [4,6) of B, [29,31) of A) apart.  One election for the four: with one each, and their
+// operands made one by one, an MMA took 101 to 140 cycles to issue where the tensor core needs 44 (48 columns) to 96 (192).
+__device__ __forceinline__ void warp_mx_mma128(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb,
+                                               uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, e;\n"
+      ".reg .b64 a1, b1;\n"
+      ".reg .b32 i1;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "setp.ne.b32 p, %6, 0;\n"
+      "@e tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], %1, %2, %3, [%4], [%5], p;\n"
+      "add.s64 a1, %1, 2;\n"
+      "add.s64 b1, %2, 2;\n"
+      "add.u32 i1, %3, 0x20000010;\n"
+      "@e tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], a1, b1, i1, [%4], [%5], 1;\n"
+      "add.s64 a1, %1, 4;\n"
+      "add.s64 b1, %2, 4;\n"
+      "add.u32 i1, %3, 0x40000020;\n"
+      "@e tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], a1, b1, i1, [%4], [%5], 1;\n"
+      "add.s64 a1, %1, 6;\n"
+      "add.s64 b1, %2, 6;\n"
+      "add.u32 i1, %3, 0x60000030;\n"
+      "@e tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], a1, b1, i1, [%4], [%5], 1;\n"
+      "}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
       : "memory");
 }
 
