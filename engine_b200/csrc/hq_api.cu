@@ -857,10 +857,45 @@ int32_t hq_probe_tensor_peak(int32_t kind, int32_t n, int32_t iters, int32_t* st
 namespace {
 struct MoeLayerPlan {
   int64_t t, k, e, hidden, inter, rows;
-  bool interleaved, gather_x;
-  int64_t off_ids, off_w, off_bounds, off_sa, off_st, off_inv, off_dws, dws_bytes, off_x16, off_h, off_y, total;
+  bool interleaved, gather_x, terms;
+  int64_t off_ids, off_w, off_bounds, off_sa, off_st, off_inv, off_dws, dws_bytes, off_x16, off_xs, off_h, off_hq, off_hs, off_y, total;
 };
 int64_t up256(int64_t v) { return (v + 255) / 256 * 256; }
+
+// MXFP4 layers with few rows per expert go to the block-scaled MMA with three e4m3 terms per activation (hq_mx_rows.cu): among
+// the banks the f16-expanding GEMM takes, one interleaved gate/up bank, up to kMxRowsPerExpert rows per expert on average.
+// Both forms of the activations are exact, so the line lies where the times meet (us, f16 GEMM : this; 32 experts of 2,880 x
+// 2,880, top 4): 16 rows an expert 188 : 158, 24 rows 191 : 168, 32 rows 196 : 194, 50 rows 218 : 235; 128 experts of 1,600 x
+// 1,600 at 28 rows 271 : 278.
+constexpr int64_t kMxRowsPerExpert = 24;
+bool mx_rows_bank(const hq_weight* w, int64_t rows) {
+  return w->format == HQ_FMT_MXFP4 && moe_tensor_rows(w, rows) && mx_rows_supported(w->n, w->k, rows, w->n_experts) &&
+         aligned16(w->scales) && (reinterpret_cast<uintptr_t>(w->data) & 31u) == 0;
+}
+bool mx_rows_layer(const hq_moe_layer* l, int64_t rows) {
+  return l->up == nullptr && rows <= kMxRowsPerExpert * l->gate->n_experts && (l->gate->flags & HQ_WEIGHT_F16_SCALES) != 0 &&
+         (l->down->flags & HQ_WEIGHT_F16_SCALES) != 0 && mx_rows_bank(l->gate, rows) && mx_rows_bank(l->down, rows);
+}
+void fill_mx_rows(MxRowsParams& g, const hq_weight* w, const uint8_t* xq, const uint8_t* xs, int64_t rows, void* y, int y_dtype,
+                  int64_t y_stride, const int32_t* bounds, int32_t* status) {
+  g.n = (int)w->n;
+  g.k = (int)w->k;
+  g.m = (int)rows;
+  g.n_experts = w->n_experts;
+  g.w = w->data;
+  g.w_scales = (const uint8_t*)w->scales;
+  g.bias = w->bias;
+  g.bias_dtype = w->bias_dtype;
+  g.xq = xq;
+  g.xs = xs;
+  g.n_rows = rows;
+  g.y = y;
+  g.y_dtype = y_dtype;
+  g.y_stride = y_stride;
+  g.act.act = HQ_ACT_NONE;
+  g.expert_bounds = bounds;
+  g.status = status;
+}
 int32_t plan_moe_layer(const hq_moe_layer* l, int64_t n_tokens, int32_t x_dtype, MoeLayerPlan& p) {
   if (l == nullptr || l->gate == nullptr || l->down == nullptr) return HQ_ERR_NULL;
   int32_t rc = check_weight(l->gate);
@@ -880,6 +915,7 @@ int32_t plan_moe_layer(const hq_moe_layer* l, int64_t n_tokens, int32_t x_dtype,
   // the tensor-core kernel takes f16 rows and copies them fastest in expert order: one pass converts and permutes
   p.gather_x = moe_tensor_rows(l->gate, p.rows) && (l->up == nullptr || moe_tensor_rows(l->up, p.rows)) &&
                tensor_path_ok(l->gate, l->up, HQ_DT_F16, l->gate->k);
+  p.terms = mx_rows_layer(l, p.rows);
   int64_t o = 0;
   p.off_ids = o;    o += up256(p.rows * 4);
   p.off_w = o;      o += up256(p.rows * 4);
@@ -889,8 +925,11 @@ int32_t plan_moe_layer(const hq_moe_layer* l, int64_t n_tokens, int32_t x_dtype,
   p.off_inv = o;    o += up256(p.rows * 4);
   p.dws_bytes = hq_moe_dispatch_workspace_bytes(p.t, (int32_t)p.k, (int32_t)p.e);
   p.off_dws = o;    o += up256(p.dws_bytes);
-  p.off_x16 = o;    o += p.gather_x ? up256(p.rows * p.hidden * 2) : 0;
+  p.off_x16 = o;    o += p.terms ? up256(3 * p.rows * p.hidden) : p.gather_x ? up256(p.rows * p.hidden * 2) : 0;
+  p.off_xs = o;     o += p.terms ? up256(3 * p.rows * (p.hidden / 32)) : 0;
   p.off_h = o;      o += up256(p.rows * p.inter * 2);
+  p.off_hq = o;     o += p.terms ? up256(3 * p.rows * p.inter) : 0;
+  p.off_hs = o;     o += p.terms ? up256(3 * p.rows * (p.inter / 32)) : 0;
   p.off_y = o;      o += up256(p.rows * p.hidden * 4);
   p.total = o;
   return HQ_OK;
@@ -936,6 +975,25 @@ int32_t hq_moe_layer_forward(const hq_moe_layer* layer, const void* logits, int3
     rc = hq_moe_dispatch_build(ids, n_tokens, (int32_t)p.k, (int32_t)p.e, bounds, sa, st, inv, dws, p.dws_bytes, stream);
   }
   if (rc != HQ_OK) return rc;
+  void* h = ws + p.off_h;
+  void* y = ws + p.off_y;
+  if (p.terms) {
+    if (!aligned16(x) || (p.hidden * dtype_size(x_dtype)) % 16 != 0) return HQ_ERR_ALIGN;
+    const cudaStream_t s = (cudaStream_t)stream;
+    rc = launch_mx_terms(x, x_dtype, p.hidden, st, bounds + p.e, p.rows, p.hidden, ws + p.off_x16, ws + p.off_xs, s);
+    if (rc != HQ_OK) return rc;
+    MxRowsParams g{};
+    fill_mx_rows(g, layer->gate, ws + p.off_x16, ws + p.off_xs, p.rows, h, HQ_DT_F16, p.inter, bounds, status_dev);
+    g.act = layer->act;
+    rc = launch_mx_rows(g, s);
+    if (rc != HQ_OK) return rc;
+    rc = launch_mx_terms(h, HQ_DT_F16, p.inter, nullptr, bounds + p.e, p.rows, p.inter, ws + p.off_hq, ws + p.off_hs, s);
+    if (rc != HQ_OK) return rc;
+    fill_mx_rows(g, layer->down, ws + p.off_hq, ws + p.off_hs, p.rows, y, HQ_DT_F32, p.hidden, bounds, status_dev);
+    rc = launch_mx_rows(g, s);
+    if (rc != HQ_OK) return rc;
+    return hq_moe_weighted_reduce(y, HQ_DT_F32, wts, inv, shared_addend, out, out_dtype, n_tokens, (int32_t)p.k, p.hidden, stream);
+  }
   const void* xin = x;
   int32_t xin_dtype = x_dtype, xin_layout = HQ_ROWS_PER_TOKEN;
   if (p.gather_x) {
@@ -945,11 +1003,9 @@ int32_t hq_moe_layer_forward(const hq_moe_layer* layer, const void* logits, int3
     xin_dtype = HQ_DT_F16;
     xin_layout = HQ_ROWS_SORTED;
   }
-  void* h = ws + p.off_h;
   rc = hq_moe_gather_forward(layer->gate, layer->up, &layer->act, xin, xin_dtype, xin_layout, n_tokens,
                              (int32_t)p.k, bounds, sa, st, dws, h, HQ_DT_F16, HQ_ROWS_SORTED, status_dev, stream);
   if (rc != HQ_OK) return rc;
-  void* y = ws + p.off_y;
   rc = hq_moe_gather_forward(layer->down, nullptr, nullptr, h, HQ_DT_F16, HQ_ROWS_SORTED, n_tokens, (int32_t)p.k,
                              bounds, sa, st, dws, y, HQ_DT_F32, HQ_ROWS_SORTED, status_dev, stream);
   if (rc != HQ_OK) return rc;

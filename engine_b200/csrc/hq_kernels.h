@@ -117,6 +117,30 @@ struct Fp8GroupedParams {
 bool fp8_grouped_supported(int64_t n, int64_t k);
 int32_t launch_fp8_grouped(const Fp8GroupedParams& p, cudaStream_t stream);
 
+// ---- MXFP4 weights against few 16-bit rows, three e4m3 terms per activation, on the block-scaled MMA (hq_mx_rows.cu) ------
+struct MxRowsParams {
+  int n, k, m;                  // m: dense rows (used when expert_bounds == nullptr)
+  int n_experts;
+  const void* w;                // packed e2m1 nibbles [E, N, K/2]
+  const uint8_t* w_scales;      // e8m0 [E, N, K/32]
+  const void* bias;             // [E, N] or nullptr
+  int bias_dtype;
+  const uint8_t* xq;            // terms [3 * n_rows, K] of rows in expert-sorted order (launch_mx_terms)
+  const uint8_t* xs;            // e8m0 [3 * n_rows, K/32]
+  int64_t n_rows;
+  void* y;                      // [rows, N], or with a gated activation of interleaved rows [rows, N/2]
+  int y_dtype;
+  int64_t y_stride;
+  hq_act_args act;
+  const int32_t* expert_bounds; // [E+1]
+  const int32_t* y_rows;        // sorted row -> output row (nullptr = identity)
+  int32_t* status;
+};
+bool mx_rows_supported(int64_t n, int64_t k, int64_t rows, int n_experts);
+int32_t launch_mx_rows(const MxRowsParams& p, cudaStream_t stream);
+int32_t launch_mx_terms(const void* x, int x_dtype, int64_t x_stride, const int32_t* row_map, const int32_t* n_valid,
+                        int64_t n_rows, int64_t k, uint8_t* codes, uint8_t* scales, cudaStream_t stream);
+
 // ---- MXFP4 expert GEMM with MXFP8 activations on tcgen05 kind::mxf8f6f4.block_scale (hq_mx_grouped.cu) ------
 struct MxGroupedParams {
   int n, k, m;                  // m: dense rows (used when expert_bounds == nullptr)

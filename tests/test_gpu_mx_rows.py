@@ -1,0 +1,83 @@
+"""MXFP4 expert layers with few 16-bit rows per expert on the block-scaled MMA (three e4m3 terms per activation), against the
+oracle's dequantized weights.  The products are exact and the sums f32, so what separates the f32 output from the oracle is the
+f16 rounding of the intermediate, which the oracle applies too: a value next to a rounding boundary may fall to either side,
+2^-11 of itself, so the tolerance of the MXFP4 layers (2e-3) holds with a wide margin."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+from oracle import moe as M
+from tests import hq_testlib as T
+
+DEV = "cuda:0"
+
+
+def _layer(e, h, i, seed):
+    import engine_b200 as hq
+    from engine_b200 import _lib as L
+    rng = T.rng_for(31, seed)
+    gu_a, gu = T.make_weight("MXFP4", rng, 2 * i, h, experts=e)
+    d_a, d = T.make_weight("MXFP4", rng, h, i, experts=e)
+    gub = T.to_dev(rng.normal(0, 0.02, (e, 2 * i)).astype(np.float32), torch.bfloat16, DEV)
+    db = T.to_dev(rng.normal(0, 0.02, (e, h)).astype(np.float32), torch.bfloat16, DEV)
+    experts = hq.MoEExperts(T.make_layer("MXFP4", d_a, i, DEV, db), gate_up_proj=T.make_layer("MXFP4", gu_a, h, DEV, gub),
+                            act=L.ACT_GPTOSS, limit=7.0)
+
+    def want(x, ids, w):
+        return M.moe_layer(x, ids, w, None, None, d, L.ACT_GPTOSS, gate_up_bank=gu, gate_up_bias=gub.float().cpu().numpy(),
+                           down_bias=db.float().cpu().numpy(), limit=7.0, h_round=lambda a: a.astype(np.float16).astype(np.float32))
+    return experts, want, rng
+
+
+def _run(experts, x, logits, k):
+    import engine_b200 as hq
+    from engine_b200 import _lib as L
+    rcfg = hq.MoeRouterTopKConfig(k, L.SCORE_SOFTMAX, L.WEIGHT_SCORE, True)
+    y = experts.forward_layer(x, T.to_dev(logits, torch.float32, DEV), rcfg, out_dtype=torch.float32)
+    torch.cuda.synchronize()
+    assert experts.gate_up.device_status()[0] == 0
+    return y.cpu().numpy()
+
+
+# K of 128 (one block), 192 and 320 (a last block that overlaps the one before by a half), 2880 (an odd number of blocks); N of
+# 192 .. 704, whole tiles of 128 and not; 1 .. 24 rows per expert on average: one column group, 16 and 17 tokens, tiles of 96
+# columns, experts without a token
+@pytest.mark.parametrize("t,e,k,h,i,dtype", [(1, 4, 2, 128, 128, torch.bfloat16), (5, 4, 4, 192, 320, torch.float16),
+                                             (16, 2, 2, 256, 192, torch.float32), (17, 2, 2, 320, 448, torch.bfloat16),
+                                             (6, 32, 4, 576, 704, torch.bfloat16), (24, 4, 4, 320, 128, torch.float32),
+                                             (23, 4, 3, 2880, 192, torch.bfloat16), (90, 16, 4, 192, 2880, torch.float16)])
+def test_layer_matches_the_oracle(t, e, k, h, i, dtype):
+    from engine_b200 import _lib as L
+    experts, want, rng = _layer(e, h, i, t)
+    x = T.to_dev(rng.standard_normal((t, h)).astype(np.float32), dtype, DEV)
+    logits = rng.standard_normal((t, e)).astype(np.float32)
+    ids, w = M.router_topk(logits, k, L.SCORE_SOFTMAX, L.WEIGHT_SCORE, True)
+    got = _run(experts, x, logits, k)
+    assert T.rel_l2(got, want(x.float().cpu().numpy(), ids, w)) <= 2e-3
+    assert np.array_equal(got, _run(experts, x, logits, k))
+
+
+def test_wide_ranges_and_values_that_are_not_finite():
+    # a block's largest value 2^20 times its others, values no f16 holds, a zero block; then a NaN and an infinity, each of which
+    # may reach its own token only
+    from engine_b200 import _lib as L
+    t, e, k, h, i = 7, 4, 4, 256, 128
+    experts, want, rng = _layer(e, h, i, 99)
+    x = rng.standard_normal((t, h)).astype(np.float32)
+    x[1, 40] = 2.0 ** 20
+    x[2] *= 2.0 ** -30
+    x[3, 64:128] = 0.0
+    x[4, 9] = -1.0e5
+    xd = T.to_dev(x, torch.bfloat16, DEV)
+    logits = rng.standard_normal((t, e)).astype(np.float32)
+    ids, w = M.router_topk(logits, k, L.SCORE_SOFTMAX, L.WEIGHT_SCORE, True)
+    got, ref = _run(experts, xd, logits, k), want(xd.float().cpu().numpy(), ids, w)
+    for row in range(t):
+        assert T.rel_l2(got[row], ref[row]) <= 2e-3, row
+    xd[5, 17] = float("nan")
+    xd[6, 200] = float("inf")
+    bad = _run(experts, xd, logits, k)
+    assert np.array_equal(bad[:5], got[:5])
+    assert not np.isfinite(bad[5:]).all(axis=1).any()
