@@ -484,7 +484,22 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
   const int stages_per_raw = 4 >> sub_shift;
   const int slice_stages = (dq_walk_steps(ODD, min(kb64, 4 * rs_hi) - 4 * rs_lo) + subs - 1) >> sub_shift;
   const uint32_t tcol = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(512 - 32 * subs * pl.ns + 32 * my_sub);
+  // What binds these warps is the number of their instructions, so a wait should leave no branch behind (warp_wait_uni: `spin`
+  // becomes 0 when one runs out, which is reported at the end).  65,536 x 4,096 at 16 rows, us, with the branches and without:
+  // FP8 51.0 : 49.8, MXFP4 54.8 : 52.8, Q5_K 75.0 : 72.8; Q4_K 61.6 : 64.9 and Q6_K 94.6 : 94.8, which leave no register free.
+  // (The first use of a slot waits for the phase before its first, which counts as complete.)
+  constexpr bool BRANCH = FMT == HQ_FMT_Q4_K || !T::WIDE;
   uint32_t spin = kDqSpin;
+  auto await = [&](uint64_t* b, uint32_t parity, int tag) {
+    if constexpr (BRANCH) {
+      if (!warp_wait(b, parity, spin)) {
+        if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, tag);
+        spin = 1;
+      }
+    } else {
+      spin = warp_wait_uni(smem_u32(b), parity, spin) ? spin : 0u;
+    }
+  };
   int slot = 0, ph = 0, it0 = 0;
   // scales that do not travel with the raw bytes: MXFP4 e8m0 pairs, FP8 relative block scales; fetched a stage ahead
   constexpr bool SIDE = FMT == HQ_FMT_MXFP4 || FMT == HQ_FMT_FP8_BLOCK;
@@ -513,10 +528,7 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
     for (int rs = rs_lo; rs < rs_hi; ++rs) {
       const uint32_t sc = sc_next;
       if (SIDE && rs + 1 < rs_hi) sc_next = fetch_side(rs + 1);
-      if (!warp_wait(&bar.full_r[slot], ph, spin)) {
-        if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 500 + slot);
-        spin = 1;
-      }
+      await(&bar.full_r[slot], ph, 500 + slot);
       const int local = (rs - rs_lo) * stages_per_raw + my_stage;        // operand stage within this tile
       const DqSlot at = dq_slot(pl, it0 + local);
       if (4 * rs + C < kb64) {
@@ -528,10 +540,7 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
 #pragma unroll 1
         for (int i = 0; i < 2; ++i) {
           ok = row.half(C, i, [&](int at_pair, const uint32_t (&v)[8]) {
-            if (i == 0 && at_pair == 0 && at.use > 0 && !warp_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
-              if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 520 + at.s);
-              spin = 1;
-            }
+            if (i == 0 && at_pair == 0) await(&bar.empty[at.s], (at.use - 1) & 1, 520 + at.s);
             tmem_st8(taddr + 16 * i + at_pair, v);
           }) && ok;
         }
@@ -548,10 +557,7 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
         warp_arrive(&bar.empty_r[slot]);
         // the K tail ends inside or in front of this group's stage: nothing to add, but the stage counts its arrivals
         if (local < slice_stages) {
-          if (at.use > 0 && !warp_wait(&bar.empty[at.s], (at.use - 1) & 1, spin)) {
-            if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 521);
-            spin = 1;
-          }
+          await(&bar.empty[at.s], (at.use - 1) & 1, 521);
           __syncwarp();
           warp_arrive(&bar.full[at.s]);
         }
@@ -561,6 +567,7 @@ __device__ __forceinline__ void dq_expand_warps(const GroupedParams& p, const Dq
     }
     it0 += slice_stages;
   }
+  if (!BRANCH && spin == 0u && lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 500 + C);
 }
 
 // ODD: some tiles have an odd number of operand stages and there are two slots for them (dq_walk_steps).  An instance of its own,
