@@ -414,6 +414,7 @@ int32_t hq_moe_gather_forward(const hq_weight* w, const hq_weight* w_up, const h
   p.y = out; p.y_dtype = out_dtype;
   p.y_stride = (has_act && w_up == nullptr) ? w->n / 2 : w->n;
   p.tiles = ws + l.off_tiles;
+  p.item_rows = ws + l.off_rows;
   p.tile_rows = l.tile_rows;
   p.tile_count = ws;
   p.expert_bounds = expert_bounds;

@@ -32,9 +32,10 @@ __device__ __forceinline__ WorkItem get_item(const GemvParams& p, int w, int n_r
   it.y = p.tiles == nullptr && p.m <= 8 ? 0 : w / n_rt;
   it.n0 = (w - it.y * n_rt) * RT;
   if (p.tiles != nullptr) {
-    it.expert = p.tiles[2 * it.y];
-    it.row0 = p.tiles[2 * it.y + 1];
-    it.nrows = min(p.tile_rows, p.expert_bounds[it.expert + 1] - it.row0);
+    const int2 v = *reinterpret_cast<const int2*>(p.tiles + 2 * it.y);
+    it.expert = v.x;
+    it.row0 = v.y;
+    it.nrows = p.item_rows[it.y];
   } else {
     it.expert = 0;
     it.row0 = 8 * it.y;

@@ -30,6 +30,7 @@ struct GemvParams {
   // expert-indexed mode: work items of <= tile_rows sorted rows of one expert
   int tile_rows;                // 4 or 8
   const int32_t* tiles;         // [n_items][2] = (expert, first sorted row)
+  const int32_t* item_rows;     // [n_items]
   const int32_t* tile_count;    // device word holding n_items
   const int32_t* expert_bounds; // [E+1]
   const int32_t* x_rows;        // sorted row -> activation row (nullptr = identity)
@@ -178,7 +179,8 @@ int32_t launch_mxfp8_quant_rows(const void* x, int x_dtype, int64_t x_stride, co
 constexpr int kDecodeShortTile = 4;
 struct DispatchLayout {
   int tile_rows;         // rows of a work item
-  int64_t off_tiles;     // int32 words, [max_tiles][2]
+  int64_t off_tiles;     // int32 words, [max_tiles][2]: expert, first sorted row
+  int64_t off_rows;      // [max_tiles]: rows of the item (a look at the expert's bounds would wait for the first word)
   int64_t max_tiles;
   int64_t total_words;
 };

@@ -30,9 +30,9 @@ __device__ __forceinline__ uint32_t order_key(float v) {
   return (b & 0x80000000u) ? ~b : b | 0x80000000u;
 }
 
-// groups_sm: n_experts floats of shared memory of this warp, read with n_group > 1 only
+// groups_sm: n_experts floats of shared memory of this warp, read with n_group > 1 only; ids_sm: if given, the ids go there too
 template <int NV>
-__device__ __forceinline__ void route_row(const RouterCall& c, int64_t row, int lane, float* groups_sm) {
+__device__ __forceinline__ void route_row(const RouterCall& c, int64_t row, int lane, float* groups_sm, uint32_t* ids_sm = nullptr) {
   const hq_router_args& a = c.a;
   const int E = a.n_experts;
   float raw[NV], score[NV];
@@ -148,6 +148,7 @@ __device__ __forceinline__ void route_row(const RouterCall& c, int64_t row, int 
   if (mine) {
     if (a.expert_scale != nullptr) my_w *= a.expert_scale[my_id];
     c.weights[row * a.top_k + lane] = my_w;
+    if (ids_sm != nullptr) ids_sm[row * a.top_k + lane] = my_id;
     c.ids[row * a.top_k + lane] = my_id;
   }
 }

@@ -252,7 +252,7 @@ int32_t hq_moe_dispatch_build(const uint32_t* ids, int64_t n_tokens, int32_t top
 /* Same tables for hosts that have no device memory to spare for a workspace and may not allocate any:
  * engines whose own pool already owns all of HBM, or code that runs where the CUDA runtime must not be
  * asked for memory.  This entry point has no counterpart in the reference.  The scratch it needs sits in a
- * fixed array inside the library (about 70 KB per GPU, held until the process exits), so it only accepts
+ * fixed array inside the library (about 100 KB per GPU, held until the process exits), so it only accepts
  * n_tokens*top_k <= 65536 and n_experts <= 512 and answers HQ_ERR_TOO_LARGE beyond that.  It calls no
  * allocator of any kind.  The first call on a device looks up the array's device address (with lazy module
  * loading that is also when the driver backs the array with memory, so it can fail with HQ_ERR_CUDA on a GPU
