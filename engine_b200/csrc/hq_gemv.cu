@@ -557,6 +557,11 @@ static int32_t launch_cfg(const GemvParams& p, int n_y_max, int max_rows, cudaSt
   return cudaGetLastError() == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
 }
 
+bool gemv_is_int8(const GemvParams& p) {
+  return p.format == HQ_FMT_Q8_0 || p.format == HQ_FMT_Q4_K ||
+         (p.format == HQ_FMT_FP8_BLOCK && p.tiles == nullptr && p.m <= 2 && p.k % 256 == 0 && p.n % 16 == 0);
+}
+
 int32_t launch_gemv(const GemvParams& p, int n_y_max, cudaStream_t stream) {
   // most activation rows any work item of this launch can have
   const int max_rows = p.tiles != nullptr ? p.tile_rows : (p.m < 8 ? p.m : 8);

@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
   const int NSTAGE = lay.nstage;
   extern __shared__ __align__(128) uint8_t smem[];
 
-  pdl_launch_dependents();
+  if (p.pdl != kPdlFirst) pdl_launch_dependents();
   if (p.tiles != nullptr) pdl_wait();    // the item list itself comes from the previous kernel
   const int n_rt = (p.n + RT - 1) / RT;
   const int n_y = p.tiles != nullptr ? p.tile_count[0] : (p.m + 7) / 8;
@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
     // ================= reducing warps: add the K-split partial sums in warp order and write ======
     // Each takes one of a lane's four accumulator values: output row g (+ 8), activation row 2 t (+ 1).  One warp for all
     // four bound short items (RS = 2 or 4): Q4_K experts of 768 x 2,048, 64 tokens, 6,700 cycles an item.
-    pdl_wait();
+    if (p.pdl != kPdlNext) pdl_wait();
     const int vi = warp - (WK + kQ8Producers);
     const int row = g + 8 * (vi >> 1), col = 2 * t + (vi & 1);
     const bool owner = NCS > 1 || t < (FMT == HQ_FMT_FP8_BLOCK ? 1 : 2);
@@ -757,7 +757,8 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
     if (S > 1) asm volatile("bar.arrive 4, %0;" ::"n"(kQ8Consumers + 32 * kQ8Reducers) : "memory");
   } else {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
-  pdl_wait();
+  if (p.pdl != kPdlNext) pdl_wait();
+  if (p.pdl == kPdlFirst) pdl_launch_dependents();
   // ================= consumer warps ================================================================
   uint8_t* xq = smem + lay.off_x;
   float* sx = reinterpret_cast<float*>(smem + lay.off_sx);
@@ -958,6 +959,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
     }
   }
   }   // consumer warps
+  if (p.pdl == kPdlNext) pdl_wait();
 }
 
 // ---- host launcher -----------------------------------------------------------------------------

@@ -7,8 +7,16 @@
 
 namespace hq {
 
+// How a launch takes part in programmatic dependent launch.  kPdlPlain: the next kernel may start at once, and whatever depends on
+// the kernel before waits for it.  Neighbouring launches that do not depend on one another (the projections of one activation) run
+// into one another with the other two: kPdlFirst lets the next kernel start only when the kernels before itself are complete,
+// so that a kPdlNext launch behind it may read and write without waiting; it waits before it ends, which keeps the order of
+// completion for the kernels behind it.
+constexpr int kPdlPlain = 0, kPdlFirst = 1, kPdlNext = 2;
+
 // ---- decode mat-vec (hq_gemv.cu) ----------------------------------------------
 struct GemvParams {
+  int pdl;                     // kPdl*; all but kPdlPlain in the integer kernel only (gemv_is_int8)
   int format;
   int n, k, m;                 // m: dense activation rows (ignored when tiles != nullptr)
   int n_banks;                 // 1, or 2 = gate bank + up bank feeding one gated activation
@@ -41,6 +49,8 @@ struct GemvParams {
   int64_t workspace_bytes;
 };
 int32_t launch_gemv(const GemvParams& p, int grid_y, cudaStream_t stream);
+// whether such a dense call goes to the integer kernel
+bool gemv_is_int8(const GemvParams& p);
 // scratch bytes the Q8_0 / Q4_K decode kernel wants for a dense [m, k] x [n, k] call (0 = none)
 int64_t gemv_int8_workspace_bytes(int format, int64_t n, int64_t k, int64_t m);
 

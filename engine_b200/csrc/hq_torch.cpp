@@ -14,6 +14,10 @@
 
 #include "../../include/hanzoquant_b200.h"
 
+// three projections of one activation with a status word each (hq_api.cu; not part of the public header)
+extern "C" int32_t hq_linear_qkv_run(const hq_weight* const w[3], const void* x, int32_t x_dtype, int64_t x_stride,
+                                     void* const y[3], int32_t y_dtype, int64_t m, int32_t* const status_dev[3], void* stream);
+
 namespace {
 
 PyObject* g_error = nullptr;      // engine_b200._lib.HqError
@@ -78,6 +82,10 @@ struct Layer {
   std::unordered_map<int64_t, int64_t>* need;                  // rows -> scratch bytes
   std::unordered_map<void*, at::Tensor>* scratch;              // stream -> zero-filled scratch
   int32_t* status_ptr() const { return status->data_ptr<int32_t>(); }
+  int64_t scratch_bytes(int64_t m) {
+    auto it = need->find(m);
+    return it != need->end() ? it->second : (*need)[m] = hq_linear_workspace_bytes(&w, m);
+  }
 };
 PyTypeObject LayerType = {PyVarObject_HEAD_INIT(nullptr, 0) "engine_b200._hqtorch.Layer", sizeof(Layer)};
 
@@ -160,8 +168,7 @@ at::Tensor run_linear(Layer* l, const at::Tensor& a, at::ScalarType out_dtype, R
   at::Tensor y = out_like(a, l->w.n, out_dtype);
   void* ws = nullptr;
   int64_t ws_bytes = 0;
-  auto it = l->need->find(x.m);
-  const int64_t need = it != l->need->end() ? it->second : (*l->need)[x.m] = hq_linear_workspace_bytes(&l->w, x.m);
+  const int64_t need = l->scratch_bytes(x.m);
   if (need > 0) {
     at::Tensor& t = (*l->scratch)[s];
     if (!t.defined() || t.numel() < need) t = at::zeros({need}, a.options().dtype(at::kByte));
@@ -218,6 +225,22 @@ PyObject* py_qkv(PyObject*, PyObject* const* p, Py_ssize_t n) {
   const at::ScalarType od = dtype_or(p[4], a.scalar_type());
   Rows x = rows_of(a, l[0]->w.k);
   if (hq_tensor_path(&l[0]->w, x.m, 1)) to_f16(x, l[0]->w.k, a, l[0]->status_ptr(), s);
+  bool scratch = false;
+  for (int i = 0; i < 3; ++i) scratch = scratch || l[i]->scratch_bytes(x.m) > 0 || l[i]->w.k != l[0]->w.k;
+  if (!scratch) {
+    at::Tensor y[3];
+    const hq_weight* w[3];
+    void* yp[3];
+    int32_t* status[3];
+    for (int i = 0; i < 3; ++i) {
+      y[i] = out_like(a, l[i]->w.n, od);
+      w[i] = &l[i]->w;
+      yp[i] = y[i].data_ptr();
+      status[i] = l[i]->status_ptr();
+    }
+    check(hq_linear_qkv_run(w, x.ptr, x.dtype, x.stride, yp, dt_code(od), x.m, status, s), "hq_linear_qkv_forward");
+    return Py_BuildValue("(NNN)", THPVariable_Wrap(y[0]), THPVariable_Wrap(y[1]), THPVariable_Wrap(y[2]));
+  }
   PyObject* out = PyTuple_New(3);
   if (out == nullptr) return nullptr;
   for (int i = 0; i < 3; ++i) {
