@@ -243,6 +243,8 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   const int NSTAGE = lay.nstage;
   extern __shared__ __align__(128) uint8_t smem[];
 
+  pdl_launch_dependents();
+  if (p.tiles != nullptr) pdl_wait();      // the item list itself comes from the previous kernel
   const int n_rt = (p.n + RT - 1) / RT;
   const int n_y = p.tiles != nullptr ? p.tile_count[0] : (p.m + 7) / 8;
   const int total = n_y * n_rt;
@@ -331,6 +333,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
 
   if (warp == kConsumerWarps + kProducerWarps) {
     // ================= reducing warp: adds the K-split partial sums in warp order and writes ==========
+    pdl_wait();
     uint32_t spin = kSpinLimit;
     int item = 0;
     for (int w = w_begin; w < w_end; w += w_step) {
@@ -366,6 +369,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   }
 
   // ================= consumer warps ============================================
+  pdl_wait();
   const int wk = warp;
   __half* xs = reinterpret_cast<__half*>(smem + lay.off_x);
   const int XP = lay.xk + 16;                 // f16 elements per staged activation row
@@ -553,8 +557,7 @@ static int32_t launch_cfg(const GemvParams& p, int n_y_max, int max_rows, cudaSt
   const int64_t items = (int64_t)n_y_max * ((p.n + L::RT - 1) / L::RT);
   const int64_t grid = items < sm_count() ? items : sm_count();
   if (grid <= 0) return HQ_OK;
-  kern<<<(unsigned)grid, kGemvThreads, lay.total, stream>>>(p, lay);
-  return cudaGetLastError() == cudaSuccess ? HQ_OK : HQ_ERR_CUDA;
+  return launch_pdl(kern, dim3((unsigned)grid), kGemvThreads, (size_t)lay.total, stream, 1, p, lay);
 }
 
 bool gemv_is_int8(const GemvParams& p) {
