@@ -16,6 +16,7 @@
 //
 // Algorithmic bytes per launch: N*K*bits/8 (weights) + M*K*sizeof(x) + M*N*sizeof(y).
 #include "hq_gemv_shared.cuh"
+#include "hq_warp_issue.cuh"
 
 namespace hq {
 
@@ -23,7 +24,7 @@ constexpr int kConsumerWarps = 13;
 constexpr int kConsumerThreads = kConsumerWarps * 32;
 constexpr int kProducerWarps = 2;   // a bulk-copy instruction holds its warp ~50 cycles per active lane: split the rows
 constexpr int kGemvThreads = kConsumerThreads + 32 * (kProducerWarps + 1);   // + producers + the reducing warp
-constexpr uint32_t kSpinLimit = 1u << 22;
+constexpr uint32_t kSpinLimit = 1u << 16;
 
 // shared-memory plan of one launch (computed on the host)
 struct GemvLayout {
@@ -304,7 +305,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
         const uint32_t bytes = (uint32_t)F::seg_bytes(kc_len);
         for (int bank = 0; bank < p.n_banks; ++bank) {
           if (round > 0) {
-            if (!mbar_wait_backoff(&empty[s], (round - 1) & 1, spin)) {
+            if (!warp_wait(&empty[s], (round - 1) & 1, spin)) {
               // give up waiting but keep the control flow intact: results are invalid and flagged
               if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 100 + s);
               spin = 1;
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
       const int rb = item & 1;
       const float* rbuf = red + rb * (p.n_banks * kConsumerWarps * 4 * 32);
       bool failed = false;
-      if (!mbar_wait_backoff(&red_full[rb], (item >> 1) & 1, spin)) {
+      if (!warp_wait(&red_full[rb], (item >> 1) & 1, spin)) {
         if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 310 + rb);
         spin = 1;
         failed = true;                 // nothing is stored for an item whose partial sums never arrived
@@ -380,19 +381,19 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   bool pf_valid = false;
   int staged_y = -1;        // activation rows currently in shared memory (valid when n_super == 1)
   int staged_rows = 0;
-  {
-    const WorkItem w0 = get_item<RT>(p, w_begin, n_rt);
-    if (w0.nrows > 0) {
-      x_prefetch(pf, p, w0.row0, w0.nrows, 0, min(xk_sub, p.k), tid);
-      pf_valid = true;
-    }
+  WorkItem wi = get_item<RT>(p, w_begin, n_rt), nx;
+  if (wi.nrows > 0) {
+    x_prefetch(pf, p, wi.row0, wi.nrows, 0, min(xk_sub, p.k), tid);
+    pf_valid = true;
   }
 
+  // (a wait that runs out makes `spin` 0: the waits left poll once, every warp still reaches every barrier, and it is reported
+  // at the end)
   uint32_t spin = kSpinLimit;
-  int s = 0, it = 0, item = 0;
+  int s = 0, item = 0, wrot = wk;
   uint32_t phase = 0;
-  for (int w = w_begin; w < w_end; w += w_step) {
-    const WorkItem wi = get_item<RT>(p, w, n_rt);
+  for (int w = w_begin; w < w_end; w += w_step, wi = nx) {
+    nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt);      // looked up an item ahead
     if (wi.nrows <= 0) continue;
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
     for (int sc = 0; sc < n_super; ++sc) {
@@ -418,7 +419,6 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
           x_prefetch(pf, p, wi.row0, wi.nrows, k_base + kXK, min(xk_sub, p.k - k_base - kXK), tid);
           pf_valid = true;
         } else if (w + w_step < w_end) {
-          const WorkItem nx = get_item<RT>(p, w + w_step, n_rt);
           if (nx.nrows > 0 && (n_super > 1 || nx.y != wi.y)) {
             x_prefetch(pf, p, nx.row0, nx.nrows, 0, min(xk_sub, p.k), tid);
             pf_valid = true;
@@ -433,14 +433,9 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
 #pragma unroll
         for (int bank = 0; bank < 2; ++bank) {
           if (bank >= p.n_banks) break;
-          if (!mbar_wait(&full[s], phase, spin)) {
-            // bounded wait ran out: flag it and carry on (every warp still reaches every barrier)
-            if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 200 + s);
-            spin = 1;
-          }
-          ++it;
+          spin = warp_wait_uni(smem_u32(&full[s]), phase, spin) ? spin : 0u;
           // the units of a stage do not divide evenly among the warps: rotate who gets the extra one
-          const int wrot = (wk + it) % WK;
+          wrot = wrot + 1 == WK ? 0 : wrot + 1;
           const uint32_t rowA = smem_u32(smem + s * L::STAGE_BYTES) + (uint32_t)g * L::PITCH;
           const uint32_t rowB = rowA + 8u * L::PITCH;
           const uint32_t xs_c = xs_g + 2u * kx;
@@ -494,12 +489,8 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
     // ---- hand the K-split partials to the reducing warp (two buffers) ----------------------------------
     const int rb = item & 1;
     float* rbuf = red + rb * (p.n_banks * kConsumerWarps * 4 * 32);
-    if (item >= 2) {
-      if (!mbar_wait(&red_free[rb], ((item >> 1) - 1) & 1, spin)) {
-        if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 300 + rb);
-        spin = 1;
-      }
-    }
+    // (the first two items wait for the phase before a barrier's first, which counts as complete)
+    spin = warp_wait_uni(smem_u32(&red_free[rb]), ((item >> 1) - 1) & 1, spin) ? spin : 0u;
 #pragma unroll
     for (int b = 0; b < 2; ++b)
       if (b < p.n_banks) {
@@ -510,6 +501,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
     if (lane == 0) mbar_arrive(&red_full[rb]);
     ++item;
   }
+  if (spin == 0u && lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 200);
 }
 
 // ---- host launcher ------------------------------------------------------------
