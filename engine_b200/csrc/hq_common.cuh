@@ -170,6 +170,23 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
+// a / b rounded to nearest for many a and one b > 0: with y = 1 / b rounded to nearest and q within an ulp of the quotient,
+// q + (a - b q) y in two fused operations is the rounded quotient (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990); a first such step brings a y, two ulps off at worst, to within
+// one.  The sign is put back for a = -0.  Six instructions of the full-rate pipe and no branch.  b from 2^-60 up: there a
+// remainder can underflow only where the quotient is below 2^-40, which the callers' 8-bit formats round to zero either way.
+struct DivideBy {
+  float b, y;
+  bool fast;
+  __device__ __forceinline__ float quick(float a) const {      // where `fast`, and a is finite
+    float q = a * y;
+    q = fmaf(fmaf(-q, b, a), y, q);
+    q = fmaf(fmaf(-q, b, a), y, q);
+    return __uint_as_float(__float_as_uint(q) | (__float_as_uint(a) & 0x80000000u));
+  }
+};
+__device__ __forceinline__ DivideBy divide_by(float b) { return DivideBy{b, __frcp_rn(b), b >= 8.6736174e-19f && b < 3.0e38f}; }
+
 // value conversion for the three activation/output dtypes that cross the ABI
 template <typename T>
 __device__ __forceinline__ float to_float(T v);
