@@ -210,4 +210,15 @@ __device__ __forceinline__ void store_from_float(void* p, int dtype, int64_t i, 
 
 __host__ __device__ __forceinline__ int dtype_size(int dtype) { return dtype == HQ_DT_F32 ? 4 : 2; }
 
+// eight consecutive values as they are stored (16 bytes of 16-bit ones, 32 of f32; 16-byte aligned), and one of them
+template <typename T>
+__device__ __forceinline__ void load8(const T* p, uint4 (&r)[sizeof(T) / 2]) {
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(T) / 2); ++i) r[i] = __ldg(reinterpret_cast<const uint4*>(p) + i);
+}
+template <typename T>
+__device__ __forceinline__ float elem8(const uint4 (&r)[sizeof(T) / 2], int i) {
+  return to_float<T>(reinterpret_cast<const T*>(r)[i]);
+}
+
 }  // namespace hq
