@@ -341,7 +341,7 @@ int32_t launch_route_dispatch(const RouterCall& rc, int32_t* bounds, int32_t* so
 // their own pool (a serving engine that sizes its KV cache to whatever is free), or the call is made from
 // a place where asking the CUDA runtime for memory is not allowed.  For them the work-item
 // lists live in a fixed array inside the library image.  It is sized for kNoAllocMaxAssignments
-// assignments and kNoAllocMaxExperts experts (about 70 KB), exists once per GPU that loads the library
+// assignments and kNoAllocMaxExperts experts (about 100 KB), exists once per GPU that loads the library
 // and is shared by every call: two calls that overlap on the GPU (different streams, or graphs replayed
 // concurrently) race on it.  Nothing in it has to start at zero -- every word that is read is written
 // first by the same call.

@@ -508,7 +508,7 @@ __device__ __forceinline__ void q4k_group(float (&acc)[NCS][4], uint32_t pa, uin
                                           uint32_t xq, uint32_t cs_stride, uint32_t sx, uint32_t xs,
                                           uint32_t xs_cs_stride, int t) {
   // The chunks are the outer loop: with all unpacked nibbles of the super-block kept for a second column set the registers
-  // of 19 warps did not suffice (290 bytes of spills; 14,336 x 4,096 at 8 rows 35 against 23 us, 64-token MoE
+  // did not suffice (290 bytes of spills; 14,336 x 4,096 at 8 rows 35 against 23 us, 64-token MoE
   // layer of 128 experts 270 against 232).
   const uint4 hA = lds128(da), hB = lds128(db);     // {d | dmin, 12 bytes of 6-bit scales and minima}
   // ---- 6-bit scales and minima, four to a word (sub-blocks 0-3 and 4-7) ----

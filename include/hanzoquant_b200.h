@@ -189,9 +189,9 @@ int32_t hq_linear_forward_ws(const hq_weight* w, const void* x, int32_t x_dtype,
  * hanzo-quant/src/lib.rs:1116-1160; gguf/fast_mmvq.rs:463-700; kernel mmvq_gguf.cu:788-900).  w_up NULL = the rows
  * of w_gate interleave gate / up and y has n / 2 columns.  Any format; m >= 9 takes the tensor-core kernel when the
  * activations are f16.
- * hq_linear_qkv_forward: the three attention projections of one activation in one call (three back-to-back
- * launches; the reference's fused_qkv kernel, gguf/fast_mmvq.rs:702-925, saves the same host work).  q / k / v are
- * [m, n_q] / [m, n_k] / [m, n_v], dense.
+ * hq_linear_qkv_forward: the three attention projections of one activation in one call: three launches, which run into
+ * one another on the integer decode kernel (the reference's fused_qkv kernel, gguf/fast_mmvq.rs:702-925, saves the same
+ * host work).  q / k / v are [m, n_q] / [m, n_k] / [m, n_v], dense.
  * hq_dense_gemv: unquantized weights W [n, k] in f16 / bf16 / f32, 1..8 activation rows: launch_gemv_{bf16,f16,f32}
  * (hanzo-quant/src/gemv/mod.rs:120-185, kernels/gemv/gemv.cu:51-282).  k % 8 == 0, W rows 16-byte aligned. */
 int32_t hq_linear_glu_forward(const hq_weight* w_gate, const hq_weight* w_up, const hq_act_args* act, const void* x,

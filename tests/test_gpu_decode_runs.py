@@ -1,0 +1,44 @@
+"""Decode paths that run several small launches into one another: dispatch tables built by comparison (up to 256 assignments)
+and by sorting above, with the rows that their work items carry; query, key and value projections of one activation."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+from tests import hq_testlib as T
+from tests.test_gpu_dispatch import test_tables_match_a_stable_sort as tables_match
+
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("e", [1, 33, 256, 1024, 4096])
+@pytest.mark.parametrize("t,k", [(1, 8), (4, 8), (31, 8), (32, 8), (256, 1), (257, 1), (33, 8)])
+def test_tables_around_the_line(t, k, e):
+    tables_match(t, k, e)
+
+
+@pytest.mark.parametrize("t,k,e", [(3, 8, 128), (32, 8, 16), (40, 8, 16)])
+def test_items_carry_their_rows(t, k, e):
+    from engine_b200.quant import moe_dispatch_build
+    ids = torch.from_numpy(T.rng_for(13, t).integers(0, e // 2, (t, k)).astype(np.int32)).to(DEV)
+    tab = moe_dispatch_build(ids, e)
+    w = 4 if t <= 4 else 8
+    ws, b = tab.workspace.view(torch.int32).tolist(), tab.expert_bounds.tolist()
+    want = [min(w, b[x + 1] - r) for x in range(e) for r in range(b[x], b[x + 1], w)]
+    at = 4 + 2 * ((t * k + w - 1) // w + e)
+    assert ws[at:at + ws[0]] == want
+
+
+@pytest.mark.parametrize("fmts", [("Q8_0",) * 3, ("Q4_K",) * 3, ("FP8",) * 3])
+@pytest.mark.parametrize("m", [1, 2, 3, 8, 9])
+def test_a_run_of_projections_is_the_separate_calls(fmts, m):
+    import engine_b200 as hq
+    rng = T.rng_for(13, 9)
+    k = 1024
+    layers = [T.make_layer(f, T.make_weight(f, rng, n, k)[0], k, DEV) for f, n in zip(fmts, (1024, 256, 384))]
+    for i in range(3):                                    # several in a row: each run's first launch follows the last's last
+        x = T.to_dev(rng.standard_normal((m, k)).astype(np.float32), torch.bfloat16, DEV)
+        outs = hq.try_fused_quantized_qkv(x, *layers, out_dtype=torch.float32)
+        for o, layer in zip(outs, layers):
+            assert torch.equal(o, layer.forward_raw(x, torch.float32))
