@@ -847,7 +847,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
         named_bar_sync(1, kQ8Consumers);
       }
       // stages of this epoch, counted from the slice's first column (an epoch is a whole number of stages)
-      const int c0 = (k_base - k_lo) / KC, c1 = (k_base - k_lo + k_len + KC - 1) / KC;
+      const int c0 = (int)((unsigned)(k_base - k_lo) / KC), c1 = (int)((unsigned)(k_base - k_lo + k_len + KC - 1) / KC);
       for (int chunk = c0; chunk < c1; ++chunk) {
         const int k_chunk = k_lo + chunk * KC;
         const int ngroups = min(KC, k_hi - k_chunk) / T::GK;   // groups in this stage
@@ -855,12 +855,14 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
 #pragma unroll
         for (int bank = 0; bank < 2; ++bank) {
           if (bank >= p.n_banks) break;
-          // block-FP8: the 128 x 128 weight-block scale of this warp's group, fetched before the wait for the stage
+          // block-FP8: the 128 x 128 weight-block scale of this warp's group, fetched before the wait for the stage.  (Its indexes
+          // are unsigned: signed divisions by 128 cost 3 % of 65,536 x 4,096 at one row, 55.9 us against 54.2.)
           float wsv = 0.f;
           if (FMT == HQ_FMT_FP8_BLOCK && wgrp < ngroups)
             wsv = __ldg(reinterpret_cast<const float*>(bank == 0 ? p.scales : p.scales_up) +
                         (int64_t)wi.expert * p.scale_expert_stride +
-                        (int64_t)((wi.n0 + kQ8RT * rtile) / 128) * ((p.k + 127) / 128) + k_chunk / 128 + wgrp);
+                        (int64_t)((unsigned)(wi.n0 + kQ8RT * rtile) >> 7) * (int)((unsigned)(p.k + 127) >> 7) +
+                        (int)((unsigned)k_chunk >> 7) + wgrp);
           spin = warp_wait_uni(smem_u32(&full[s]), phase, spin) ? spin : 0u;
           if (wgrp < ngroups) {
             const uint32_t da = smem_u32(smem + s * ST::BYTES) + (uint32_t)(kQ8RT * rtile + g) * ST::PITCH +
