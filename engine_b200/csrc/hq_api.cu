@@ -891,27 +891,29 @@ int32_t hq_probe_tensor_peak(int32_t kind, int32_t n, int32_t iters, int32_t* st
 namespace {
 struct MoeLayerPlan {
   int64_t t, k, e, hidden, inter, rows;
-  bool interleaved, gather_x, terms;
+  bool interleaved, gather_x;
+  int terms;       // of an activation on the block-scaled MMA, or 0: another kernel
   int64_t off_ids, off_w, off_bounds, off_sa, off_st, off_inv, off_dws, dws_bytes, off_x16, off_xs, off_h, off_hq, off_hs, off_y, total;
 };
 int64_t up256(int64_t v) { return (v + 255) / 256 * 256; }
 
-// MXFP4 layers with few rows per expert go to the block-scaled MMA with three e4m3 terms per activation (hq_mx_rows.cu): among
+// MXFP4 layers with few rows per expert go to the block-scaled MMA with three e5m2 terms per activation (hq_mx_rows.cu): among
 // the banks the f16-expanding GEMM takes, one interleaved gate/up bank, up to kMxRowsPerExpert rows per expert on average.
-// Both forms of the activations are exact, so the line lies where the times meet (us, f16 GEMM : this; 32 experts of 2,880 x
+// Both forms hold a 16-bit activation exactly, so the line lies where the times meet (us, f16 GEMM : this; 32 experts of 2,880 x
 // 2,880, top 4): 16 rows an expert 188 : 158, 24 rows 191 : 168, 32 rows 196 : 194, 50 rows 218 : 235; 128 experts of 1,600 x
-// 1,600 at 28 rows 271 : 278.
+// 1,600 at 28 rows 271 : 278.  (f32 rows, four terms: 32 experts 182 at 16 rows and 188 at 24, so the line holds for them too.)
 constexpr int64_t kMxRowsPerExpert = 24;
-bool mx_rows_bank(const hq_weight* w, int64_t rows) {
-  return w->format == HQ_FMT_MXFP4 && moe_tensor_rows(w, rows) && mx_rows_supported(w->n, w->k, rows, w->n_experts) &&
+bool mx_rows_bank(const hq_weight* w, int64_t rows, int terms) {
+  return w->format == HQ_FMT_MXFP4 && moe_tensor_rows(w, rows) && mx_rows_supported(w->n, w->k, rows, w->n_experts, terms) &&
          aligned16(w->scales) && (reinterpret_cast<uintptr_t>(w->data) & 31u) == 0;
 }
-bool mx_rows_layer(const hq_moe_layer* l, int64_t rows) {
+bool mx_rows_layer(const hq_moe_layer* l, int64_t rows, int terms) {
   return l->up == nullptr && rows <= kMxRowsPerExpert * l->gate->n_experts && (l->gate->flags & HQ_WEIGHT_F16_SCALES) != 0 &&
-         (l->down->flags & HQ_WEIGHT_F16_SCALES) != 0 && mx_rows_bank(l->gate, rows) && mx_rows_bank(l->down, rows);
+         (l->down->flags & HQ_WEIGHT_F16_SCALES) != 0 && mx_rows_bank(l->gate, rows, terms) &&
+         mx_rows_bank(l->down, rows, 3);
 }
-void fill_mx_rows(MxRowsParams& g, const hq_weight* w, const uint8_t* xq, const uint8_t* xs, int64_t rows, void* y, int y_dtype,
-                  int64_t y_stride, const int32_t* bounds, int32_t* status) {
+void fill_mx_rows(MxRowsParams& g, const hq_weight* w, int terms, const uint8_t* xq, const uint8_t* xs, int64_t rows, void* y,
+                  int y_dtype, int64_t y_stride, const int32_t* bounds, int32_t* status) {
   g.n = (int)w->n;
   g.k = (int)w->k;
   g.m = (int)rows;
@@ -920,6 +922,7 @@ void fill_mx_rows(MxRowsParams& g, const hq_weight* w, const uint8_t* xq, const 
   g.w_scales = (const uint8_t*)w->scales;
   g.bias = w->bias;
   g.bias_dtype = w->bias_dtype;
+  g.terms = terms;
   g.xq = xq;
   g.xs = xs;
   g.n_rows = rows;
@@ -949,7 +952,7 @@ int32_t plan_moe_layer(const hq_moe_layer* l, int64_t n_tokens, int32_t x_dtype,
   // the tensor-core kernel takes f16 rows and copies them fastest in expert order: one pass converts and permutes
   p.gather_x = moe_tensor_rows(l->gate, p.rows) && (l->up == nullptr || moe_tensor_rows(l->up, p.rows)) &&
                tensor_path_ok(l->gate, l->up, HQ_DT_F16, l->gate->k);
-  p.terms = mx_rows_layer(l, p.rows);
+  p.terms = mx_rows_layer(l, p.rows, mx_terms(x_dtype)) ? mx_terms(x_dtype) : 0;
   int64_t o = 0;
   p.off_ids = o;    o += up256(p.rows * 4);
   p.off_w = o;      o += up256(p.rows * 4);
@@ -959,8 +962,8 @@ int32_t plan_moe_layer(const hq_moe_layer* l, int64_t n_tokens, int32_t x_dtype,
   p.off_inv = o;    o += up256(p.rows * 4);
   p.dws_bytes = hq_moe_dispatch_workspace_bytes(p.t, (int32_t)p.k, (int32_t)p.e);
   p.off_dws = o;    o += up256(p.dws_bytes);
-  p.off_x16 = o;    o += p.terms ? up256(3 * p.rows * p.hidden) : p.gather_x ? up256(p.rows * p.hidden * 2) : 0;
-  p.off_xs = o;     o += p.terms ? up256(3 * p.rows * (p.hidden / 32)) : 0;
+  p.off_x16 = o;    o += p.terms ? up256(p.terms * p.rows * p.hidden) : p.gather_x ? up256(p.rows * p.hidden * 2) : 0;
+  p.off_xs = o;     o += p.terms ? up256(p.terms * p.rows * (p.hidden / 32)) : 0;
   p.off_h = o;      o += up256(p.rows * p.inter * 2);
   p.off_hq = o;     o += p.terms ? up256(3 * p.rows * p.inter) : 0;
   p.off_hs = o;     o += p.terms ? up256(3 * p.rows * (p.inter / 32)) : 0;
@@ -1017,13 +1020,13 @@ int32_t hq_moe_layer_forward(const hq_moe_layer* layer, const void* logits, int3
     rc = launch_mx_terms(x, x_dtype, p.hidden, st, bounds + p.e, p.rows, p.hidden, ws + p.off_x16, ws + p.off_xs, s);
     if (rc != HQ_OK) return rc;
     MxRowsParams g{};
-    fill_mx_rows(g, layer->gate, ws + p.off_x16, ws + p.off_xs, p.rows, h, HQ_DT_F16, p.inter, bounds, status_dev);
+    fill_mx_rows(g, layer->gate, p.terms, ws + p.off_x16, ws + p.off_xs, p.rows, h, HQ_DT_F16, p.inter, bounds, status_dev);
     g.act = layer->act;
     rc = launch_mx_rows(g, s);
     if (rc != HQ_OK) return rc;
     rc = launch_mx_terms(h, HQ_DT_F16, p.inter, nullptr, bounds + p.e, p.rows, p.inter, ws + p.off_hq, ws + p.off_hs, s);
     if (rc != HQ_OK) return rc;
-    fill_mx_rows(g, layer->down, ws + p.off_hq, ws + p.off_hs, p.rows, y, HQ_DT_F32, p.hidden, bounds, status_dev);
+    fill_mx_rows(g, layer->down, mx_terms(HQ_DT_F16), ws + p.off_hq, ws + p.off_hs, p.rows, y, HQ_DT_F32, p.hidden, bounds, status_dev);
     rc = launch_mx_rows(g, s);
     if (rc != HQ_OK) return rc;
     return hq_moe_weighted_reduce(y, HQ_DT_F32, wts, inv, shared_addend, out, out_dtype, n_tokens, (int32_t)p.k, p.hidden, stream);

@@ -128,7 +128,7 @@ struct Fp8GroupedParams {
 bool fp8_grouped_supported(int64_t n, int64_t k);
 int32_t launch_fp8_grouped(const Fp8GroupedParams& p, cudaStream_t stream);
 
-// ---- MXFP4 weights against few 16-bit rows, three e4m3 terms per activation, on the block-scaled MMA (hq_mx_rows.cu) ------
+// ---- MXFP4 weights against few rows, three or four e5m2 terms per activation, on the block-scaled MMA (hq_mx_rows.cu) -----
 struct MxRowsParams {
   int n, k, m;                  // m: dense rows (used when expert_bounds == nullptr)
   int n_experts;
@@ -136,8 +136,9 @@ struct MxRowsParams {
   const uint8_t* w_scales;      // e8m0 [E, N, K/32]
   const void* bias;             // [E, N] or nullptr
   int bias_dtype;
-  const uint8_t* xq;            // terms [3 * n_rows, K] of rows in expert-sorted order (launch_mx_terms)
-  const uint8_t* xs;            // e8m0 [3 * n_rows, K/32]
+  int terms;                    // of an activation: mx_terms of the type the rows had
+  const uint8_t* xq;            // terms [terms * n_rows, K] of rows in expert-sorted order (launch_mx_terms)
+  const uint8_t* xs;            // e8m0 [terms * n_rows, K/32]
   int64_t n_rows;
   void* y;                      // [rows, N], or with a gated activation of interleaved rows [rows, N/2]
   int y_dtype;
@@ -147,7 +148,8 @@ struct MxRowsParams {
   const int32_t* y_rows;        // sorted row -> output row (nullptr = identity)
   int32_t* status;
 };
-bool mx_rows_supported(int64_t n, int64_t k, int64_t rows, int n_experts);
+int mx_terms(int x_dtype);       // 3 for 16-bit types, 4 for f32
+bool mx_rows_supported(int64_t n, int64_t k, int64_t rows, int n_experts, int terms);
 int32_t launch_mx_rows(const MxRowsParams& p, cudaStream_t stream);
 int32_t launch_mx_terms(const void* x, int x_dtype, int64_t x_stride, const int32_t* row_map, const int32_t* n_valid,
                         int64_t n_rows, int64_t k, uint8_t* codes, uint8_t* scales, cudaStream_t stream);

@@ -1,4 +1,4 @@
-"""MXFP4 expert layers with few 16-bit rows per expert on the block-scaled MMA (three e4m3 terms per activation), against the
+"""MXFP4 expert layers with few rows per expert on the block-scaled MMA (three or four e5m2 terms per activation), against the
 oracle's dequantized weights.  The products are exact and the sums f32, so what separates the f32 output from the oracle is the
 f16 rounding of the intermediate, which the oracle applies too: a value next to a rounding boundary may fall to either side,
 2^-11 of itself, so the tolerance of the MXFP4 layers (2e-3) holds with a wide margin."""
@@ -81,3 +81,56 @@ def test_wide_ranges_and_values_that_are_not_finite():
     bad = _run(experts, xd, logits, k)
     assert np.array_equal(bad[:5], got[:5])
     assert not np.isfinite(bad[5:]).all(axis=1).any()
+
+
+def _layer_with_dead_columns(e, h, i, seed):
+    """Every 32-block's first weight of the gate/up bank is zero; the bank's other weights are 2^12 times the usual."""
+    import engine_b200 as hq
+    from engine_b200 import _lib as L
+    from oracle import formats as F
+    rng = T.rng_for(31, seed)
+    gu_a, _ = T.make_weight("MXFP4", rng, 2 * i, h, experts=e)
+    d_a, d = T.make_weight("MXFP4", rng, h, i, experts=e)
+    blocks, scales = gu_a["blocks"].copy(), gu_a["scales"] + 12
+    blocks.reshape(-1, 16)[:, 0] &= 0xF0
+    gu = F.mxfp4_dequant(blocks.reshape(-1, h // 2), scales.reshape(-1, h // 32)).reshape(e, 2 * i, h)
+    assert (gu[..., ::32] == 0).all() and scales.min() >= 113 and scales.max() <= 140
+    experts = hq.MoEExperts(T.make_layer("MXFP4", d_a, i, DEV), gate_up_proj=T.make_layer("MXFP4", {"blocks": blocks, "scales": scales}, h, DEV),
+                            act=L.ACT_GPTOSS, limit=7.0)
+    return experts, gu.astype(np.float64), d.astype(np.float64), rng
+
+
+def _exact(x, ids, w, gu, d):
+    """The layer in 64 bits, no value rounded."""
+    out = np.zeros((x.shape[0], d.shape[1]))
+    for t in range(x.shape[0]):
+        for e, weight in zip(ids[t], w[t]):
+            both = gu[e] @ x[t].astype(np.float64)
+            g, u = np.minimum(both[0::2], 7.0), np.clip(both[1::2], -7.0, 7.0)
+            out[t] += float(weight) * (d[e] @ ((u + 1.0) * g / (1.0 + np.exp(-1.702 * g))))
+    return out
+
+
+# a block's largest value meets a zero weight, so its others are all there is, `down` binades below it: with terms that drop bits
+# there, the error shows in full.  The f16-expanding GEMM behind the separate calls holds an f16 activation exactly; both round
+# the intermediate to f16, which is what their distance from 64 bits then is (2^-12 of each value, 1.5e-4 and more with the
+# sums' signs; 1e-3 leaves room for sums that cancel).  `small`: the others are f16 values without a subnormal.
+@pytest.mark.parametrize("down", [6, 14, 18, 20])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+def test_small_values_beside_a_large_one_keep_their_bits(down, dtype):
+    import engine_b200 as hq
+    from engine_b200 import _lib as L
+    t, e, k, h, i = 12, 4, 4, 256, 192
+    experts, gu, d, rng = _layer_with_dead_columns(e, h, i, 7 + down)
+    x = np.sign(rng.standard_normal((t, h))) * rng.uniform(1.0, 2.0, (t, h)) * 2.0 ** (7 - down)
+    x[:, ::32] = 200.0
+    xd = T.to_dev(x.astype(np.float32), dtype, DEV)
+    logits = rng.standard_normal((t, e)).astype(np.float32)
+    ids, w = M.router_topk(logits, k, L.SCORE_SOFTMAX, L.WEIGHT_SCORE, True)
+    want = _exact(xd.float().cpu().numpy(), ids, w, gu, d)
+    got = _run(experts, xd, logits, k)
+    top = hq.moe_router_topk(T.to_dev(logits, torch.float32, DEV), hq.MoeRouterTopKConfig(k, L.SCORE_SOFTMAX, L.WEIGHT_SCORE, True))
+    split = experts.forward(xd, top.values, top.indices, out_dtype=torch.float32).cpu().numpy()
+    err, err_gemm = T.rel_l2(got, want), T.rel_l2(split, want)
+    print(f"down {down} {dtype}: {err:.2e}, f16 GEMM {err_gemm:.2e}")
+    assert err <= 1e-3 and err <= 1.1 * err_gemm
