@@ -446,8 +446,7 @@ int32_t hq_moe_gather_forward(const hq_weight* w, const hq_weight* w_up, const h
   p.x = x; p.x_dtype = x_dtype; p.x_stride = w->k;
   p.y = out; p.y_dtype = out_dtype;
   p.y_stride = (has_act && w_up == nullptr) ? w->n / 2 : w->n;
-  p.tiles = ws + l.off_tiles;
-  p.item_rows = ws + l.off_rows;
+  p.tiles = ws + kItemsAt;
   p.tile_rows = l.tile_rows;
   p.tile_count = ws;
   p.expert_bounds = expert_bounds;
@@ -455,7 +454,7 @@ int32_t hq_moe_gather_forward(const hq_weight* w, const hq_weight* w_up, const h
   p.y_rows = y_rows;
   if (has_act) p.act = *act; else p.act.act = HQ_ACT_NONE;
   p.status = status_dev;
-  return launch_gemv(p, (int)l.max_tiles, (cudaStream_t)stream);
+  return launch_gemv(p, (int)l.max_items, (cudaStream_t)stream);
 }
 
 // ---- block-FP8 layers with FP8 activations (codes + 1 x 128 scales) ------------------------------------

@@ -26,21 +26,10 @@ constexpr int kDispatchCluster = 8;
 // assignments up to which one block does it all: its 32 warps walk 128 each, as long as a cluster's start takes
 constexpr int64_t kDispatchOneBlock = 4096;
 
-DispatchLayout dispatch_layout(int64_t n_tokens, int top_k, int n_experts) {
-  DispatchLayout l;
-  const int64_t total = n_tokens * top_k;
-  l.tile_rows = n_tokens <= kDecodeShortTile ? kDecodeShortTile : 8;
-  l.off_tiles = 4;
-  l.max_tiles = (total + l.tile_rows - 1) / l.tile_rows + n_experts;
-  l.off_rows = l.off_tiles + 2 * l.max_tiles;
-  l.total_words = l.off_rows + l.max_tiles;
-  return l;
-}
-
 struct DispatchCall {
   const uint32_t* ids;
   int total, top_k, n_experts, tile_rows;
-  int32_t *bounds, *sorted_assign, *sorted_token, *inv_perm, *header, *tiles, *item_rows;
+  int32_t *bounds, *sorted_assign, *sorted_token, *inv_perm, *header, *items;
 };
 
 // warps that own a run: as many as histogram rows fit
@@ -116,9 +105,7 @@ static __device__ __forceinline__ void dispatch_few(const DispatchCall& c, const
   if (tid == kDispatchSmall) {
     c.header[0] = before;
   } else {
-    c.tiles[2 * before] = (int32_t)e;
-    c.tiles[2 * before + 1] = pos;
-    c.item_rows[before] = min(c.tile_rows, n - at);
+    put_decode_item(c.items, before, (int32_t)e, pos, min(c.tile_rows, n - at));
   }
 }
 
@@ -247,12 +234,8 @@ static __device__ __forceinline__ void dispatch_block(const DispatchCall& c, int
   // work items: a warp per expert, lanes over its items
   for (int e = rank * 32 + warp; e < E; e += 32 * n_ranks) {
     const int r = start[e], n = count[e];
-    int32_t* t = c.tiles + 2 * (int64_t)tile0[e];
-    for (int i = lane; i * c.tile_rows < n; i += 32) {
-      t[2 * i] = e;
-      t[2 * i + 1] = r + i * c.tile_rows;
-      c.item_rows[tile0[e] + i] = min(c.tile_rows, n - i * c.tile_rows);
-    }
+    for (int i = lane; i * c.tile_rows < n; i += 32)
+      put_decode_item(c.items, tile0[e] + i, e, r + i * c.tile_rows, min(c.tile_rows, n - i * c.tile_rows));
   }
   if (n_ranks > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -307,7 +290,7 @@ static DispatchCall dispatch_call(const uint32_t* ids, int64_t n_tokens, int top
                                   int32_t* sorted_assign, int32_t* sorted_token, int32_t* inv_perm, int32_t* ws) {
   const DispatchLayout l = dispatch_layout(n_tokens, top_k, n_experts);
   return DispatchCall{ids, (int)(n_tokens * top_k), top_k, n_experts, l.tile_rows, bounds, sorted_assign, sorted_token, inv_perm,
-                      ws, ws + l.off_tiles, ws + l.off_rows};
+                      ws, ws + kItemsAt};
 }
 
 int32_t launch_dispatch(const uint32_t* ids, int64_t n_tokens, int top_k, int n_experts, int32_t* bounds,

@@ -32,10 +32,10 @@ __device__ __forceinline__ WorkItem get_item(const GemvParams& p, int w, int n_r
   it.y = p.tiles == nullptr && p.m <= 8 ? 0 : w / n_rt;
   it.n0 = (w - it.y * n_rt) * RT;
   if (p.tiles != nullptr) {
-    const int2 v = *reinterpret_cast<const int2*>(p.tiles + 2 * it.y);
-    it.expert = v.x;
-    it.row0 = v.y;
-    it.nrows = p.item_rows[it.y];
+    const DecodeItem v = decode_item(p.tiles, it.y);
+    it.expert = v.expert;
+    it.row0 = v.row0;
+    it.nrows = min(p.tile_rows, v.rows);
   } else {
     it.expert = 0;
     it.row0 = 8 * it.y;

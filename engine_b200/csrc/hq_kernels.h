@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include "../../include/hanzoquant_b200.h"
+#include "hq_work_items.h"
 
 namespace hq {
 
@@ -37,8 +38,7 @@ struct GemvParams {
   int64_t y_stride;             // elements
   // expert-indexed mode: work items of <= tile_rows sorted rows of one expert
   int tile_rows;                // 4 or 8
-  const int32_t* tiles;         // [n_items][2] = (expert, first sorted row)
-  const int32_t* item_rows;     // [n_items]
+  const int32_t* tiles;         // work items (hq_work_items.h)
   const int32_t* tile_count;    // device word holding n_items
   const int32_t* expert_bounds; // [E+1]
   const int32_t* x_rows;        // sorted row -> activation row (nullptr = identity)
@@ -186,17 +186,7 @@ int32_t launch_mxfp8_quant_rows(const void* x, int x_dtype, int64_t x_stride, co
                                 cudaStream_t stream);
 
 // ---- dispatch tables (hq_dispatch.cu) -------------------------------------------
-// sorted rows of one expert in a work item of the decode kernels: 8, or 4 when a call has no more tokens than that (the
-// Q8_0 / Q4_K kernel then needs half the activation columns)
-constexpr int kDecodeShortTile = 4;
-struct DispatchLayout {
-  int tile_rows;         // rows of a work item
-  int64_t off_tiles;     // int32 words, [max_tiles][2]: expert, first sorted row
-  int64_t off_rows;      // [max_tiles]: rows of the item (a look at the expert's bounds would wait for the first word)
-  int64_t max_tiles;
-  int64_t total_words;
-};
-DispatchLayout dispatch_layout(int64_t n_tokens, int top_k, int n_experts);
+// (layout of the workspace and its work items: hq_work_items.h)
 int32_t launch_dispatch(const uint32_t* ids, int64_t n_tokens, int top_k, int n_experts, int32_t* bounds,
                         int32_t* sorted_assign, int32_t* sorted_token, int32_t* inv_perm, int32_t* ws,
                         cudaStream_t stream);

@@ -1,0 +1,49 @@
+// Work items of the expert-indexed decode kernels, and where the dispatch tables keep them in a call's workspace.  Plain
+// arithmetic on 32-bit words, the same on the host (tests/test_work_items.py) and in the kernels: a workspace may start at any
+// word, and a list can be read without the sizes it was built with (a projection that takes one row per slot may call itself
+// n_tokens * top_k tokens of one slot).
+#pragma once
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define HQ_ITEM_FN __host__ __device__ __forceinline__
+#else
+#define HQ_ITEM_FN inline
+#endif
+
+namespace hq {
+
+// Rows of a work item: 4 when every expert can have at most 4 rows (no token picks an expert twice), 8 otherwise.
+constexpr int kDecodeShortTile = 4;
+
+// workspace: 4 header words (0: items, 1: routed assignments), then the items
+constexpr int64_t kItemsAt = 4;
+constexpr int kItemWords = 3;
+
+struct DispatchLayout {
+  int tile_rows;         // rows of a work item
+  int64_t max_items;
+  int64_t total_words;
+};
+HQ_ITEM_FN constexpr DispatchLayout dispatch_layout(int64_t n_tokens, int top_k, int n_experts) {
+  const int rows = n_tokens <= kDecodeShortTile ? kDecodeShortTile : 8;
+  const int64_t items = (n_tokens * top_k + rows - 1) / rows + n_experts;
+  return DispatchLayout{rows, items, kItemsAt + kItemWords * items};
+}
+
+// (an item carries its rows: a look at the expert's bounds would wait for the first word)
+struct DecodeItem {
+  int32_t expert, row0, rows;      // row0: first sorted row
+};
+HQ_ITEM_FN DecodeItem decode_item(const int32_t* items, int64_t i) {
+  const int32_t* w = items + kItemWords * i;
+  return DecodeItem{w[0], w[1], w[2]};
+}
+HQ_ITEM_FN void put_decode_item(int32_t* items, int64_t i, int32_t expert, int32_t row0, int32_t rows) {
+  int32_t* w = items + kItemWords * i;
+  w[0] = expert;
+  w[1] = row0;
+  w[2] = rows;
+}
+
+}  // namespace hq

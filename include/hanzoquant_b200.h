@@ -239,7 +239,7 @@ int32_t hq_router_topk_grouped(const void* logits, int32_t logits_dtype, int64_t
  * Outputs: expert_bounds int32 [E+1]; sorted_assign int32 [T*k] (flat index);
  * sorted_token int32 [T*k] (token index); inv_perm int32 [T*k] (flat index ->
  * sorted position).  Also fills the tile lists for the expert GEMMs in the
- * workspace (see hq_moe_dispatch_workspace_bytes).
+ * workspace (see hq_moe_dispatch_workspace_bytes; any 4-byte alignment).
  * An id outside [0, n_experts) -- a padding slot such as 0xFFFFFFFF -- is skipped:
  * it gets no sorted row, expert_bounds[E] counts only the routed assignments (the
  * tail of sorted_assign / sorted_token beyond it is left unwritten), and its

@@ -1,0 +1,68 @@
+"""Work items of the expert-indexed decode kernels (engine_b200/csrc/hq_work_items.h, compiled for the host): the workspace of
+the dispatch tables is a run of 32-bit words that may start at any of them, and where an item lies does not depend on how a
+caller splits its assignments into tokens and slots.  Addresses are watched by the compiler's alignment sanitizer."""
+import os
+import re
+import subprocess
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+PROGRAM = r"""
+#include <stdio.h>
+#include <stdlib.h>
+#include <string.h>
+#include "hq_work_items.h"
+WIDE
+using namespace hq;
+int main() {
+  const int shapes[][3] = {{1, 8, 128}, {4, 8, 128}, {5, 8, 128}, {64, 8, 128}, {3, 64, 7}, {4096, 4, 512}};
+  for (auto& s : shapes) {
+    const DispatchLayout l = dispatch_layout(s[0], s[1], s[2]);
+    for (int shift = 0; shift < 4; ++shift) {                    // a workspace behind an odd number of words
+      int32_t* block = (int32_t*)aligned_alloc(16, (size_t)(l.total_words + 8) / 4 * 16 + 16);
+      int32_t* ws = block + shift;
+      for (int64_t i = 0; i < l.max_items; ++i) put_decode_item(ws + kItemsAt, i, 3 * (int)i, 5 * (int)i, 1 + (int)i % 8);
+      for (int64_t i = 0; i < l.max_items; ++i) {
+        const DecodeItem v = READ(ws + kItemsAt, i);
+        if (v.expert != 3 * i || v.row0 != 5 * i || v.rows != 1 + i % 8) return 2;
+      }
+      free(block);
+    }
+    // the last item ends where the workspace does
+    if (kItemsAt + kItemWords * l.max_items != l.total_words) return 3;
+    if (l.tile_rows != (s[0] <= 4 ? 4 : 8)) return 4;
+  }
+  return 0;
+}
+"""
+
+
+def run(tmp_path, wide, read):
+    src, exe = str(tmp_path / "items.cpp"), str(tmp_path / "items")
+    with open(src, "w") as f:
+        f.write(PROGRAM.replace("WIDE", wide).replace("READ", read))
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fsanitize=alignment", "-fno-sanitize-recover=all", "-I",
+                    os.path.join(ROOT, "engine_b200", "csrc"), src, "-o", exe], check=True)
+    return subprocess.run([exe], capture_output=True, text=True)
+
+
+def test_items_are_read_at_any_word(tmp_path):
+    res = run(tmp_path, "", "decode_item")
+    assert res.returncode == 0, res.stderr
+
+
+def test_a_wide_read_is_seen(tmp_path):
+    # the reader this rule excludes: two words of an item in one 8-byte load
+    wide = ("struct alignas(8) Pair { int32_t x, y; };\n"
+            "hq::DecodeItem wide(const int32_t* items, int64_t i) {\n"
+            "  const Pair v = *(const Pair*)(items + 3 * i);\n"
+            "  return hq::DecodeItem{v.x, v.y, items[3 * i + 2]};\n"
+            "}\n")
+    res = run(tmp_path, wide, "wide")
+    assert res.returncode != 0 and "misaligned" in res.stderr
+
+
+def test_the_kernels_read_items_so():
+    with open(os.path.join(ROOT, "engine_b200", "csrc", "hq_gemv_shared.cuh")) as f:
+        text = f.read()
+    assert "decode_item(p.tiles, " in text and re.search(r"p\.tiles *[\[+]|_cast<[^>]*>\(p\.tiles", text) is None
