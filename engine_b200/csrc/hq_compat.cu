@@ -22,10 +22,6 @@ void complain(const char* symbol, int32_t rc) {
 }
 
 // ---- scratch for the calls that need dispatch tables -----------------------------------------------
-constexpr int kCompatMaxAssign = 65536;
-constexpr int kCompatMaxExperts = 512;
-constexpr int64_t kCompatWsWords = 4 + 2 * ((int64_t)kCompatMaxAssign / 8 + kCompatMaxExperts);
-constexpr int64_t kCompatWords = (kCompatMaxExperts + 64) + 3 * (int64_t)kCompatMaxAssign + kCompatWsWords + 64;
 static __device__ __align__(256) int32_t g_compat_scratch[kCompatWords];
 
 struct Tables {
@@ -34,13 +30,11 @@ struct Tables {
   void* to_free;      // stream-ordered allocation to release after the launches, or nullptr
 };
 
-int64_t up64(int64_t words) { return (words + 63) / 64 * 64; }
-
 // Carves the tables out of the fixed array, or out of a stream-ordered allocation when the call is larger.
 int32_t get_tables(int64_t n_tokens, int top_k, int n_experts, cudaStream_t stream, Tables& t) {
   const int64_t assign = n_tokens * top_k;
   const int64_t ws_words = dispatch_layout(n_tokens, top_k, n_experts).total_words;
-  const int64_t need = up64(n_experts + 1) + 3 * up64(assign) + up64(ws_words);
+  const int64_t need = compat_words(assign, n_experts, ws_words);
   int32_t* base = nullptr;
   t.to_free = nullptr;
   if (assign <= kCompatMaxAssign && n_experts <= kCompatMaxExperts && need <= kCompatWords) {

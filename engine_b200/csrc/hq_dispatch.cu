@@ -330,7 +330,7 @@ int32_t launch_route_dispatch(const RouterCall& rc, int32_t* bounds, int32_t* so
 // first by the same call.
 constexpr int kNoAllocMaxAssignments = 65536;
 constexpr int kNoAllocMaxExperts = 512;
-constexpr int64_t kNoAllocWords = 4 + 3 * ((int64_t)kNoAllocMaxAssignments / 8 + kNoAllocMaxExperts);
+constexpr int64_t kNoAllocWords = dispatch_words_up_to(kNoAllocMaxAssignments, kNoAllocMaxExperts);
 static __device__ __align__(256) int32_t g_noalloc_scratch[kNoAllocWords];
 
 int32_t launch_dispatch_noalloc(const uint32_t* ids, int64_t n_tokens, int top_k, int n_experts, int32_t* bounds,

@@ -31,6 +31,21 @@ HQ_ITEM_FN constexpr DispatchLayout dispatch_layout(int64_t n_tokens, int top_k,
   return DispatchLayout{rows, items, kItemsAt + kItemWords * items};
 }
 
+// Largest workspace of up to `assignments` (more than 256, a multiple of 8) over `experts`, however they split into tokens and
+// slots (up to 64): what a fixed array has to hold.
+HQ_ITEM_FN constexpr int64_t dispatch_words_up_to(int64_t assignments, int experts) {
+  return dispatch_layout(assignments, 1, experts).total_words;
+}
+// The reference-named entry points keep all five tables in one fixed array, each from a multiple of 64 words on.
+constexpr int kCompatMaxAssign = 65536;
+constexpr int kCompatMaxExperts = 512;
+HQ_ITEM_FN constexpr int64_t up64(int64_t words) { return (words + 63) / 64 * 64; }
+HQ_ITEM_FN constexpr int64_t compat_words(int64_t assignments, int experts, int64_t ws_words) {
+  return up64(experts + 1) + 3 * up64(assignments) + up64(ws_words);
+}
+constexpr int64_t kCompatWords =
+    compat_words(kCompatMaxAssign, kCompatMaxExperts, dispatch_words_up_to(kCompatMaxAssign, kCompatMaxExperts));
+
 // (an item carries its rows: a look at the expert's bounds would wait for the first word)
 struct DecodeItem {
   int32_t expert, row0, rows;      // row0: first sorted row

@@ -66,3 +66,41 @@ def test_the_kernels_read_items_so():
     with open(os.path.join(ROOT, "engine_b200", "csrc", "hq_gemv_shared.cuh")) as f:
         text = f.read()
     assert "decode_item(p.tiles, " in text and re.search(r"p\.tiles *[\[+]|_cast<[^>]*>\(p\.tiles", text) is None
+
+
+FIXED = r"""
+#include <stdio.h>
+#include <initializer_list>
+#include "hq_work_items.h"
+using namespace hq;
+int main() {
+  // every call the header promises the fixed arrays for, at the sizes where its tables are largest
+  const int experts[] = {1, 7, 8, 128, 511, 512};
+  for (int e : experts)
+    for (int k = 1; k <= 64; ++k)
+      for (int64_t t : {(int64_t)1, (int64_t)4, (int64_t)5, (int64_t)(62968 / k), (int64_t)(kCompatMaxAssign / k)}) {
+        const int64_t ws = dispatch_layout(t, k, e).total_words;
+        if (compat_words(t * k, e, ws) > kCompatWords || ws > dispatch_words_up_to(65536, 512)) {
+          printf("%d experts, %lld x %d\n", e, (long long)t, k);
+          return 1;
+        }
+      }
+  return 0;
+}
+"""
+
+
+def test_fixed_arrays_hold_what_the_headers_promise(tmp_path):
+    src, exe = str(tmp_path / "fixed.cpp"), str(tmp_path / "fixed")
+    with open(src, "w") as f:
+        f.write(FIXED)
+    subprocess.run(["g++", "-std=c++17", "-I", os.path.join(ROOT, "engine_b200", "csrc"), src, "-o", exe], check=True)
+    res = subprocess.run([exe], capture_output=True, text=True)
+    assert res.returncode == 0, res.stdout
+    with open(os.path.join(ROOT, "include", "hanzoquant_compat.h")) as f:
+        assert "calls of up to 65536 assignments and 512 experts" in " ".join(f.read().replace("*", " ").split())
+    # the arrays are sized by these rules, not by numbers of their own
+    for name, size in (("hq_compat.cu", "g_compat_scratch[kCompatWords]"), ("hq_dispatch.cu", "g_noalloc_scratch[kNoAllocWords]")):
+        with open(os.path.join(ROOT, "engine_b200", "csrc", name)) as f:
+            text = f.read()
+        assert size in text and re.search(r"(Compat|NoAlloc)(Ws)?Words = [0-9(]", text) is None
