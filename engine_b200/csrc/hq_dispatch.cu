@@ -32,9 +32,6 @@ struct DispatchCall {
   int32_t *bounds, *sorted_assign, *sorted_token, *inv_perm, *header, *items;
 };
 
-// warps that own a run: as many as histogram rows fit
-static int dispatch_rows(int n_experts) { return n_experts <= 1024 ? 32 : 8; }
-
 static __device__ __forceinline__ uint32_t cluster_peer(const void* p, uint32_t rank) {
   uint32_t a;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
@@ -50,6 +47,7 @@ static __device__ __forceinline__ int32_t lds_cluster(uint32_t addr) {
 // steps of the block instead of six, 1 us instead of 4.3 for one token's tables.  ids_sm: the assignments' experts, filled up
 // to a multiple of four with 0xFFFFFFFF; keys_sm: as many words.
 constexpr int kDispatchSmall = 256;
+static_assert((2 * kDispatchSmall + 2 * 32) * 4 <= kDispatchStatic, "few_sm, warp_rows and warp_tiles");
 static __device__ __forceinline__ void dispatch_few(const DispatchCall& c, const uint32_t* ids_sm, uint32_t* keys_sm) {
   const int tid = threadIdx.x, E = c.n_experts, quads = (c.total + 3) >> 2;
   const uint4* ids4 = reinterpret_cast<const uint4*>(ids_sm);
@@ -272,17 +270,15 @@ __global__ void __launch_bounds__(kDispatchThreads) route_dispatch_kernel(const 
   else dispatch_block(c, rows, 0, 1, dsm);
 }
 
-static size_t dispatch_smem(int rows, int n_experts) { return (size_t)(rows + 5) * n_experts * 4; }
-
 template <typename K>
 static bool allow_smem(K kern, size_t bytes) {
   static std::atomic<size_t> have[64];
   int dev = 0;
-  if (bytes <= 48 * 1024) return true;
+  if (!dispatch_asks_for_smem((int64_t)bytes)) return true;
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
   if (dev < 64 && have[dev].load(std::memory_order_relaxed) >= bytes) return true;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 4096) != cudaSuccess) return false;
-  if (dev < 64) have[dev].store(227 * 1024 - 4096, std::memory_order_relaxed);
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDispatchDynamic) != cudaSuccess) return false;
+  if (dev < 64) have[dev].store((size_t)kDispatchDynamic, std::memory_order_relaxed);
   return true;
 }
 
@@ -298,7 +294,7 @@ int32_t launch_dispatch(const uint32_t* ids, int64_t n_tokens, int top_k, int n_
                         cudaStream_t stream) {
   const DispatchCall c = dispatch_call(ids, n_tokens, top_k, n_experts, bounds, sorted_assign, sorted_token, inv_perm, ws);
   const int rows = dispatch_rows(n_experts), n_ranks = c.total <= kDispatchOneBlock ? 1 : kDispatchCluster;
-  const size_t smem = dispatch_smem(rows, n_experts);
+  const size_t smem = (size_t)dispatch_smem(n_experts);
   if (!allow_smem(dispatch_kernel, smem)) return HQ_ERR_CUDA;
   return launch_pdl(dispatch_kernel, dim3((unsigned)n_ranks), kDispatchThreads, smem, stream, n_ranks, c, rows, n_ranks);
 }
@@ -308,7 +304,7 @@ int32_t launch_route_dispatch(const RouterCall& rc, int32_t* bounds, int32_t* so
   const DispatchCall c = dispatch_call(rc.ids, rc.n_rows, rc.a.top_k, rc.a.n_experts, bounds, sorted_assign, sorted_token,
                                        inv_perm, ws);
   const int rows = dispatch_rows(c.n_experts);
-  const size_t smem = dispatch_smem(rows, c.n_experts);
+  const size_t smem = (size_t)dispatch_smem(c.n_experts);
   auto run = [&](auto kern) {
     if (!allow_smem(kern, smem)) return (int32_t)HQ_ERR_CUDA;
     return launch_pdl(kern, dim3(1), kDispatchThreads, smem, stream, 1, rc, c, rows);

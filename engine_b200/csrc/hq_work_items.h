@@ -31,6 +31,15 @@ HQ_ITEM_FN constexpr DispatchLayout dispatch_layout(int64_t n_tokens, int top_k,
   return DispatchLayout{rows, items, kItemsAt + kItemWords * items};
 }
 
+// Shared memory of the kernels that build the tables: histogram rows and five arrays of one word per expert, sized by the launch,
+// beside at most kDispatchStatic bytes the kernel declares.  A launch gets 48 KiB of both together unless it asked for more, and
+// 227 KiB at most.
+constexpr int64_t kDispatchStatic = 4096;
+HQ_ITEM_FN constexpr int dispatch_rows(int n_experts) { return n_experts <= 1024 ? 32 : 8; }      // warps that own a run
+HQ_ITEM_FN constexpr int64_t dispatch_smem(int n_experts) { return (int64_t)(dispatch_rows(n_experts) + 5) * n_experts * 4; }
+constexpr int64_t kDispatchDynamic = 227 * 1024 - kDispatchStatic;
+HQ_ITEM_FN constexpr bool dispatch_asks_for_smem(int64_t dynamic) { return dynamic + kDispatchStatic > 48 * 1024; }
+
 // Largest workspace of up to `assignments` (more than 256, a multiple of 8) over `experts`, however they split into tokens and
 // slots (up to 64): what a fixed array has to hold.
 HQ_ITEM_FN constexpr int64_t dispatch_words_up_to(int64_t assignments, int experts) {

@@ -104,3 +104,20 @@ def test_fixed_arrays_hold_what_the_headers_promise(tmp_path):
         with open(os.path.join(ROOT, "engine_b200", "csrc", name)) as f:
             text = f.read()
         assert size in text and re.search(r"(Compat|NoAlloc)(Ws)?Words = [0-9(]", text) is None
+
+
+def test_tables_of_any_number_of_experts_get_their_shared_memory(tmp_path):
+    src, exe = str(tmp_path / "smem.cpp"), str(tmp_path / "smem")
+    with open(src, "w") as f:
+        f.write('#include <stdio.h>\n#include "hq_work_items.h"\n'
+                "int main() {\n"
+                "  for (int e = 1; e <= 4096; ++e)\n"
+                '    printf("%lld %d\\n", (long long)hq::dispatch_smem(e), (int)hq::dispatch_asks_for_smem(hq::dispatch_smem(e)));\n'
+                "}\n")
+    subprocess.run(["g++", "-std=c++17", "-I", os.path.join(ROOT, "engine_b200", "csrc"), src, "-o", exe], check=True)
+    lines = subprocess.run([exe], capture_output=True, text=True, check=True).stdout.split()
+    declared = (2 * 256 + 2 * 32) * 4                # what the kernels declare: ids and keys of few assignments, warp totals
+    for e in range(1, 4097):
+        dynamic, asks = int(lines[2 * e - 2]), int(lines[2 * e - 1])
+        assert dynamic >= 4 * 13 * e
+        assert dynamic + declared <= (227 if asks else 48) * 1024, e
