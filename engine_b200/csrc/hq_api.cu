@@ -446,9 +446,8 @@ int32_t hq_moe_gather_forward(const hq_weight* w, const hq_weight* w_up, const h
   p.x = x; p.x_dtype = x_dtype; p.x_stride = w->k;
   p.y = out; p.y_dtype = out_dtype;
   p.y_stride = (has_act && w_up == nullptr) ? w->n / 2 : w->n;
-  p.tiles = ws + kItemsAt;
+  p.tiles = ws;
   p.tile_rows = l.tile_rows;
-  p.tile_count = ws;
   p.expert_bounds = expert_bounds;
   p.x_rows = x_rows;
   p.y_rows = y_rows;

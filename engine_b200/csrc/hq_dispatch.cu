@@ -28,8 +28,8 @@ constexpr int64_t kDispatchOneBlock = 4096;
 
 struct DispatchCall {
   const uint32_t* ids;
-  int total, top_k, n_experts, tile_rows;
-  int32_t *bounds, *sorted_assign, *sorted_token, *inv_perm, *header, *items;
+  int total, top_k, n_experts, tile_rows, rows_at;
+  int32_t *bounds, *sorted_assign, *sorted_token, *inv_perm, *ws;
 };
 
 static __device__ __forceinline__ uint32_t cluster_peer(const void* p, uint32_t rank) {
@@ -88,7 +88,7 @@ static __device__ __forceinline__ void dispatch_few(const DispatchCall& c, const
         less += (v.x < (uint32_t)x ? 1 : 0) + (v.y < (uint32_t)x ? 1 : 0) + (v.z < (uint32_t)x ? 1 : 0) + (v.w < (uint32_t)x ? 1 : 0);
       }
       c.bounds[x] = less;
-      if (x == E) c.header[1] = less;
+      if (x == E) c.ws[1] = less;
     }
   }
   __syncthreads();
@@ -101,9 +101,10 @@ static __device__ __forceinline__ void dispatch_few(const DispatchCall& c, const
     before += (v.x < key ? 1 : 0) + (v.y < key ? 1 : 0) + (v.z < key ? 1 : 0) + (v.w < key ? 1 : 0);
   }
   if (tid == kDispatchSmall) {
-    c.header[0] = before;
+    c.ws[0] = before;
+    c.ws[kHeaderRowsAt] = c.rows_at;
   } else {
-    put_decode_item(c.items, before, (int32_t)e, pos, min(c.tile_rows, n - at));
+    put_decode_item(c.ws, c.rows_at, before, (int32_t)e, pos, min(c.tile_rows, n - at));
   }
 }
 
@@ -204,8 +205,9 @@ static __device__ __forceinline__ void dispatch_block(const DispatchCall& c, int
   }
   if (rank == 0 && tid == 0) {
     c.bounds[E] = r_all;
-    c.header[0] = t_all;
-    c.header[1] = r_all;
+    c.ws[0] = t_all;
+    c.ws[kHeaderRowsAt] = c.rows_at;
+    c.ws[1] = r_all;
   }
   __syncthreads();
   // stable scatter of this warp's run
@@ -233,7 +235,7 @@ static __device__ __forceinline__ void dispatch_block(const DispatchCall& c, int
   for (int e = rank * 32 + warp; e < E; e += 32 * n_ranks) {
     const int r = start[e], n = count[e];
     for (int i = lane; i * c.tile_rows < n; i += 32)
-      put_decode_item(c.items, tile0[e] + i, e, r + i * c.tile_rows, min(c.tile_rows, n - i * c.tile_rows));
+      put_decode_item(c.ws, c.rows_at, tile0[e] + i, e, r + i * c.tile_rows, min(c.tile_rows, n - i * c.tile_rows));
   }
   if (n_ranks > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -285,8 +287,8 @@ static bool allow_smem(K kern, size_t bytes) {
 static DispatchCall dispatch_call(const uint32_t* ids, int64_t n_tokens, int top_k, int n_experts, int32_t* bounds,
                                   int32_t* sorted_assign, int32_t* sorted_token, int32_t* inv_perm, int32_t* ws) {
   const DispatchLayout l = dispatch_layout(n_tokens, top_k, n_experts);
-  return DispatchCall{ids, (int)(n_tokens * top_k), top_k, n_experts, l.tile_rows, bounds, sorted_assign, sorted_token, inv_perm,
-                      ws, ws + kItemsAt};
+  return DispatchCall{ids, (int)(n_tokens * top_k), top_k, n_experts, l.tile_rows, (int)l.rows_at, bounds, sorted_assign,
+                      sorted_token, inv_perm, ws};
 }
 
 int32_t launch_dispatch(const uint32_t* ids, int64_t n_tokens, int top_k, int n_experts, int32_t* bounds,

@@ -247,7 +247,8 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   pdl_launch_dependents();
   if (p.tiles != nullptr) pdl_wait();      // the item list itself comes from the previous kernel
   const int n_rt = (p.n + RT - 1) / RT;
-  const int n_y = p.tiles != nullptr ? p.tile_count[0] : (p.m + 7) / 8;
+  const int n_y = p.tiles != nullptr ? p.tiles[0] : (p.m + 7) / 8;
+  const int rows_at = p.tiles != nullptr ? p.tiles[kHeaderRowsAt] : 0;
   const int total = n_y * n_rt;
   // Item walk: dense calls stride through the items; expert-indexed calls take a contiguous run each, so
   // consecutive items of a CTA share their activation rows (one expert tile) and are staged once.
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
     int s = 0, round = 0;
     for (int w = w_begin; w < w_end; w += w_step) {
-      const WorkItem wi = get_item<RT>(p, w, n_rt);
+      const WorkItem wi = get_item<RT>(p, w, n_rt, rows_at);
       if (wi.nrows <= 0) continue;
       const int rows_valid = min(RT, p.n - wi.n0);
       const int my_rows = max(0, min(RPP, rows_valid - pw * RPP));
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
     uint32_t spin = kSpinLimit;
     int item = 0;
     for (int w = w_begin; w < w_end; w += w_step) {
-      const WorkItem wi = get_item<RT>(p, w, n_rt);
+      const WorkItem wi = get_item<RT>(p, w, n_rt, rows_at);
       if (wi.nrows <= 0) continue;
       const int rb = item & 1;
       const float* rbuf = red + rb * (p.n_banks * kConsumerWarps * 4 * 32);
@@ -381,7 +382,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   bool pf_valid = false;
   int staged_y = -1;        // activation rows currently in shared memory (valid when n_super == 1)
   int staged_rows = 0;
-  WorkItem wi = get_item<RT>(p, w_begin, n_rt), nx;
+  WorkItem wi = get_item<RT>(p, w_begin, n_rt, rows_at), nx;
   if (wi.nrows > 0) {
     x_prefetch(pf, p, wi.row0, wi.nrows, 0, min(xk_sub, p.k), tid);
     pf_valid = true;
@@ -393,7 +394,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   int s = 0, item = 0, wrot = wk;
   uint32_t phase = 0;
   for (int w = w_begin; w < w_end; w += w_step, wi = nx) {
-    nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt);      // looked up an item ahead
+    nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt, rows_at);      // looked up an item ahead
     if (wi.nrows <= 0) continue;
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
     for (int sc = 0; sc < n_super; ++sc) {

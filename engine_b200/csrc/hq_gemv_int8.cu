@@ -593,7 +593,8 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
   if (p.pdl != kPdlFirst) pdl_launch_dependents();
   if (p.tiles != nullptr) pdl_wait();    // the item list itself comes from the previous kernel
   const int n_rt = (p.n + RT - 1) / RT;
-  const int n_y = p.tiles != nullptr ? p.tile_count[0] : (p.m + 7) / 8;
+  const int n_y = p.tiles != nullptr ? p.tiles[0] : (p.m + 7) / 8;
+  const int rows_at = p.tiles != nullptr ? p.tiles[kHeaderRowsAt] : 0;
   const int total = n_y * n_rt;
   // Split K: neighbouring CTAs take the K slices of one item, so each keeps only its slice of the activations
   // staged (once, for every item it meets) and the slices of an item finish at about the same time.
@@ -660,9 +661,9 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
     uint64_t policy;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
     int s = 0, round = 0;
-    WorkItem wi = get_item<RT>(p, w_begin, n_rt), nx;
+    WorkItem wi = get_item<RT>(p, w_begin, n_rt, rows_at), nx;
     for (int w = w_begin; w < w_end; w += w_step, wi = nx) {
-      nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt);      // fetched an item ahead
+      nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt, rows_at);      // fetched an item ahead
       if (wi.nrows <= 0) continue;
       const int rows_valid = min(RT, p.n - wi.n0);
       const int my_rows = max(0, min(RPP, rows_valid - pw * RPP));
@@ -703,9 +704,9 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
     const bool owner = NCS > 1 || t < (FMT == HQ_FMT_FP8_BLOCK ? 1 : 2);
     uint32_t spin = kQ8Spin;
     int item = 0;
-    WorkItem wi = get_item<RT>(p, w_begin, n_rt), nx;
+    WorkItem wi = get_item<RT>(p, w_begin, n_rt, rows_at), nx;
     for (int w = w_begin; w < w_end; w += w_step, wi = nx) {
-      nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt);
+      nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt, rows_at);
       if (wi.nrows <= 0) continue;
       const int rb = item & 1;
       const float* rbuf = red + rb * (p.n_banks * WK * 4 * 32) + vi * 32 + lane;
@@ -780,7 +781,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
   bool pf_valid = false;
   int staged_y = -1;        // activation rows currently staged (valid when n_super == 1)
   int staged_rows = 0;
-  WorkItem wi = get_item<RT>(p, w_begin, n_rt), nx;
+  WorkItem wi = get_item<RT>(p, w_begin, n_rt, rows_at), nx;
   if (wi.nrows > 0) {
     q8_x_prefetch(pf, p, wi.row0, wi.nrows, k_lo, min(xk_sub, k_hi - k_lo), tid);
     pf_valid = true;
@@ -792,7 +793,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
   int s = 0, item = 0;
   uint32_t phase = 0;
   for (int w = w_begin; w < w_end; w += w_step, wi = nx) {
-    nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt);      // fetched an item ahead
+    nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt, rows_at);      // fetched an item ahead
     if (wi.nrows <= 0) continue;
     float acc[2][NCS][4];
 #pragma unroll
@@ -933,7 +934,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
       for (int w = w_begin; w < w_end; w += w_step)
         for (int rt = 0; rt < RS; ++rt, ++idx) {
           if (idx % WK != warp) continue;
-          WorkItem wi = get_item<RT>(p, w, n_rt);
+          WorkItem wi = get_item<RT>(p, w, n_rt, rows_at);
           if (wi.nrows <= 0) continue;
           wi.n0 += kQ8RT * rt;
           const float* all = lay.partials + ((int64_t)w * S * RS + rt) * (nb * 128);

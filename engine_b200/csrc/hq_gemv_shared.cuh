@@ -27,12 +27,12 @@ struct WorkItem {
 };
 
 template <int RT>
-__device__ __forceinline__ WorkItem get_item(const GemvParams& p, int w, int n_rt) {
+__device__ __forceinline__ WorkItem get_item(const GemvParams& p, int w, int n_rt, int rows_at) {
   WorkItem it;
   it.y = p.tiles == nullptr && p.m <= 8 ? 0 : w / n_rt;
   it.n0 = (w - it.y * n_rt) * RT;
   if (p.tiles != nullptr) {
-    const DecodeItem v = decode_item(p.tiles, it.y);
+    const DecodeItem v = decode_item(p.tiles, rows_at, it.y);
     it.expert = v.expert;
     it.row0 = v.row0;
     it.nrows = min(p.tile_rows, v.rows);

@@ -38,8 +38,7 @@ struct GemvParams {
   int64_t y_stride;             // elements
   // expert-indexed mode: work items of <= tile_rows sorted rows of one expert
   int tile_rows;                // 4 or 8
-  const int32_t* tiles;         // work items (hq_work_items.h)
-  const int32_t* tile_count;    // device word holding n_items
+  const int32_t* tiles;         // the dispatch workspace with its work items (hq_work_items.h)
   const int32_t* expert_bounds; // [E+1]
   const int32_t* x_rows;        // sorted row -> activation row (nullptr = identity)
   const int32_t* y_rows;        // sorted row -> output row (nullptr = identity)

@@ -1,6 +1,6 @@
 // Work items of the expert-indexed decode kernels, and where the dispatch tables keep them in a call's workspace.  Plain
 // arithmetic on 32-bit words, the same on the host (tests/test_work_items.py) and in the kernels: a workspace may start at any
-// word, and a list can be read without the sizes it was built with (a projection that takes one row per slot may call itself
+// word, and the lists can be read without the sizes they were built with (a projection that takes one row per slot may call itself
 // n_tokens * top_k tokens of one slot).
 #pragma once
 #include <stdint.h>
@@ -16,19 +16,20 @@ namespace hq {
 // Rows of a work item: 4 when every expert can have at most 4 rows (no token picks an expert twice), 8 otherwise.
 constexpr int kDecodeShortTile = 4;
 
-// workspace: 4 header words (0: items, 1: routed assignments), then the items
+// workspace: 4 header words (items, routed assignments, word at which the items' rows start), two words per item (expert, first
+// sorted row), one word per item (its rows: a look at the expert's bounds would wait for the first word)
 constexpr int64_t kItemsAt = 4;
-constexpr int kItemWords = 3;
+constexpr int kHeaderRowsAt = 2;
 
 struct DispatchLayout {
   int tile_rows;         // rows of a work item
-  int64_t max_items;
+  int64_t rows_at, max_items;
   int64_t total_words;
 };
 HQ_ITEM_FN constexpr DispatchLayout dispatch_layout(int64_t n_tokens, int top_k, int n_experts) {
   const int rows = n_tokens <= kDecodeShortTile ? kDecodeShortTile : 8;
   const int64_t items = (n_tokens * top_k + rows - 1) / rows + n_experts;
-  return DispatchLayout{rows, items, kItemsAt + kItemWords * items};
+  return DispatchLayout{rows, kItemsAt + 2 * items, items, kItemsAt + 3 * items};
 }
 
 // Shared memory of the kernels that build the tables: histogram rows and five arrays of one word per expert, sized by the launch,
@@ -55,19 +56,19 @@ HQ_ITEM_FN constexpr int64_t compat_words(int64_t assignments, int experts, int6
 constexpr int64_t kCompatWords =
     compat_words(kCompatMaxAssign, kCompatMaxExperts, dispatch_words_up_to(kCompatMaxAssign, kCompatMaxExperts));
 
-// (an item carries its rows: a look at the expert's bounds would wait for the first word)
 struct DecodeItem {
   int32_t expert, row0, rows;      // row0: first sorted row
 };
-HQ_ITEM_FN DecodeItem decode_item(const int32_t* items, int64_t i) {
-  const int32_t* w = items + kItemWords * i;
-  return DecodeItem{w[0], w[1], w[2]};
+// ws: the workspace; rows_at: its header's word, or the layout's
+HQ_ITEM_FN DecodeItem decode_item(const int32_t* ws, int rows_at, int i) {
+  const int32_t* w = ws + kItemsAt + 2 * (int64_t)i;
+  return DecodeItem{w[0], w[1], ws[rows_at + (int64_t)i]};
 }
-HQ_ITEM_FN void put_decode_item(int32_t* items, int64_t i, int32_t expert, int32_t row0, int32_t rows) {
-  int32_t* w = items + kItemWords * i;
+HQ_ITEM_FN void put_decode_item(int32_t* ws, int rows_at, int i, int32_t expert, int32_t row0, int32_t rows) {
+  int32_t* w = ws + kItemsAt + 2 * (int64_t)i;
   w[0] = expert;
   w[1] = row0;
-  w[2] = rows;
+  ws[rows_at + (int64_t)i] = rows;
 }
 
 }  // namespace hq

@@ -21,15 +21,15 @@ int main() {
     for (int shift = 0; shift < 4; ++shift) {                    // a workspace behind an odd number of words
       int32_t* block = (int32_t*)aligned_alloc(16, (size_t)(l.total_words + 8) / 4 * 16 + 16);
       int32_t* ws = block + shift;
-      for (int64_t i = 0; i < l.max_items; ++i) put_decode_item(ws + kItemsAt, i, 3 * (int)i, 5 * (int)i, 1 + (int)i % 8);
+      for (int64_t i = 0; i < l.max_items; ++i) put_decode_item(ws, (int)l.rows_at, (int)i, 3 * (int)i, 5 * (int)i, 1 + (int)i % 8);
       for (int64_t i = 0; i < l.max_items; ++i) {
-        const DecodeItem v = READ(ws + kItemsAt, i);
+        const DecodeItem v = READ(ws, (int)l.rows_at, (int)i);
         if (v.expert != 3 * i || v.row0 != 5 * i || v.rows != 1 + i % 8) return 2;
       }
       free(block);
     }
     // the last item ends where the workspace does
-    if (kItemsAt + kItemWords * l.max_items != l.total_words) return 3;
+    if (l.rows_at + l.max_items != l.total_words) return 3;
     if (l.tile_rows != (s[0] <= 4 ? 4 : 8)) return 4;
   }
   return 0;
@@ -54,9 +54,9 @@ def test_items_are_read_at_any_word(tmp_path):
 def test_a_wide_read_is_seen(tmp_path):
     # the reader this rule excludes: two words of an item in one 8-byte load
     wide = ("struct alignas(8) Pair { int32_t x, y; };\n"
-            "hq::DecodeItem wide(const int32_t* items, int64_t i) {\n"
-            "  const Pair v = *(const Pair*)(items + 3 * i);\n"
-            "  return hq::DecodeItem{v.x, v.y, items[3 * i + 2]};\n"
+            "hq::DecodeItem wide(const int32_t* ws, int rows_at, int i) {\n"
+            "  const Pair v = *(const Pair*)(ws + 4 + 2 * i);\n"
+            "  return hq::DecodeItem{v.x, v.y, ws[rows_at + i]};\n"
             "}\n")
     res = run(tmp_path, wide, "wide")
     assert res.returncode != 0 and "misaligned" in res.stderr
@@ -65,7 +65,7 @@ def test_a_wide_read_is_seen(tmp_path):
 def test_the_kernels_read_items_so():
     with open(os.path.join(ROOT, "engine_b200", "csrc", "hq_gemv_shared.cuh")) as f:
         text = f.read()
-    assert "decode_item(p.tiles, " in text and re.search(r"p\.tiles *[\[+]|_cast<[^>]*>\(p\.tiles", text) is None
+    assert "decode_item(p.tiles, rows_at, " in text and re.search(r"p\.tiles *[\[+]|_cast<[^>]*>\(p\.tiles", text) is None
 
 
 FIXED = r"""
