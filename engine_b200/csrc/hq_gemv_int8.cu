@@ -66,7 +66,9 @@ struct I8Traits<HQ_FMT_Q4_K> {
 constexpr int kQ8MaxStages = 8;
 constexpr int kQ8SmemBudget = 227 * 1024 - 256;   // dynamic part; a few static words come on top
 constexpr int kQ8XGroups = 4;                    // 16-byte registers a thread prefetches activations into
-constexpr uint32_t kQ8Spin = 1u << 16;           // polls of a wait, each suspended for a while
+// Polls of a wait, each suspended for 20 us (warp_wait, warp_wait_uni): more than a second.  The copying warps start before the
+// kernel in front is complete, so what they wait for includes the rest of that one.
+constexpr uint32_t kQ8Spin = 1u << 16;
 constexpr int kQ8Magic = 0x4B400000;             // 1.5 * 2^23 as f32 bits: magic + n reads as 12582912.f + n
 template <>
 struct I8Traits<HQ_FMT_FP8_BLOCK> {
@@ -672,7 +674,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
         const uint32_t bytes = (uint32_t)T::row_bytes(kc_len);
         for (int bank = 0; bank < p.n_banks; ++bank) {
           if (round > 0) {
-            if (!mbar_wait_backoff(&empty[s], (round - 1) & 1, spin)) {
+            if (!warp_wait(&empty[s], (round - 1) & 1, spin)) {
               // give up waiting but keep the control flow intact: results are invalid and flagged
               if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 100 + s);
               spin = 1;
@@ -714,7 +716,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
       int64_t yrow = wi.row0 + col;
       if (mine && p.y_rows != nullptr && S == 1) yrow = p.y_rows[wi.row0 + col];
       bool failed = false;
-      if (!mbar_wait_backoff(&red_full[rb], (item >> 1) & 1, spin)) {
+      if (!warp_wait(&red_full[rb], (item >> 1) & 1, spin)) {
         if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 310 + rb);
         spin = 1;
         failed = true;                 // nothing is stored for an item whose partial sums never arrived

@@ -44,3 +44,20 @@ def test_copies_are_waited_for_by_the_warps_that_issue_them(name):
     for loop in re.findall(r"for \(int i = [^;]*(?:next|it) - pl\.n[rs]\)?;.*?warp_wait\(&([\w.]+)\[", text, re.S):
         drained.add(loop)
     assert rings and rings <= drained, (rings, drained)
+
+
+def short_waits(text):
+    """Waits by short polls in a file whose limit counts polls that are suspended for 20 us each: 64 times shorter than meant."""
+    limits = [1 << int(n) for n in re.findall(r"constexpr uint32_t k\w*Spin\w* = 1u << (\d+);", text)]
+    code = "\n".join(line.split("//")[0] for line in text.split("\n"))
+    return re.findall(r"\bmbar_(?:try_)?wait\w*\s*\(", code) if limits and min(limits) < 1 << 22 else []
+
+
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh")) and f != "hq_common.cuh"))
+def test_a_limit_of_long_polls_is_not_used_with_short_ones(name):
+    assert short_waits(open(os.path.join(CSRC, name)).read()) == []
+
+
+def test_a_short_wait_is_found():
+    assert short_waits("constexpr uint32_t kSpin = 1u << 16;\n  if (!mbar_wait_backoff(&empty[s], 0, spin)) {\n") != []
+    assert short_waits("constexpr uint32_t kSpin = 1u << 22;\n  if (!mbar_wait(&empty[s], 0, spin)) {\n") == []
