@@ -28,8 +28,10 @@
 // partial sums are exchanged through distributed shared memory (each CTA finishes a share of the tile's tokens) and
 // added in rank order, so the result does not depend on timing and no scratch is needed.
 //
-// Every wait is bounded; after a time-out the status word is set, nothing more is stored, the copy warps wait (bounded) for what
-// they have issued and the kernel reaches its normal exit.  No multicast, no peer memory.
+// Every wait is bounded; after a time-out the status word is set, the copy warps issue nothing more and wait (bounded) for what
+// they have issued, and the kernel reaches its normal exit.  The epilogue stores nothing behind a wait of its own or of the issuing
+// warp that ran out; an expanding warp hands over what it has, so with the status word set no output is to be used.  No
+// multicast, no peer memory.
 #pragma once
 #include <cuda.h>
 

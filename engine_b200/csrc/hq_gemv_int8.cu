@@ -623,6 +623,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
   uint64_t* empty = full + kQ8MaxStages;
   uint64_t* red_full = empty + kQ8MaxStages;   // [2] partial sums of an item are all written
   uint64_t* red_free = red_full + 2;           // [2] ... and have been consumed
+  volatile uint32_t* late = reinterpret_cast<uint32_t*>(red_free + 2);   // a copying or consumer warp's wait ran out: nothing more is stored
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
 
@@ -631,6 +632,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
   const bool producer = warp >= WK && warp < WK + kQ8Producers;
   if (producer) {
     if (tid == kQ8Consumers) {
+      *late = 0u;
       for (int s = 0; s < NSTAGE; ++s) {
         mbar_init(&full[s], kQ8Producers);
         mbar_init(&empty[s], WK);
@@ -675,8 +677,9 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
         for (int bank = 0; bank < p.n_banks; ++bank) {
           if (round > 0) {
             if (!warp_wait(&empty[s], (round - 1) & 1, spin)) {
-              // give up waiting but keep the control flow intact: results are invalid and flagged
+              // give up waiting but keep the control flow intact: what is copied over is never stored
               if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 100 + s);
+              *late = 1u;
               spin = 1;
             }
           }
@@ -721,6 +724,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
         spin = 1;
         failed = true;                 // nothing is stored for an item whose partial sums never arrived
       }
+      failed = failed || *late != 0u;
       WorkItem ti = wi;
 #pragma unroll 1
       for (int rt = 0; rt < RS; ++rt, ti.n0 += kQ8RT) {
@@ -790,7 +794,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
   }
 
   // (a wait that runs out makes `spin` 0: the waits left poll once, every warp still reaches every barrier, and it is reported
-  // at the end; the reducing warps keep what never arrived from being stored)
+  // at the end; `late` keeps the sums handed over from being stored)
   uint32_t spin = kQ8Spin;
   int s = 0, item = 0;
   uint32_t phase = 0;
@@ -910,6 +914,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
           rbuf[((b * WK + warp) * 4 + i) * 32 + lane] = sum;
         }
       }
+    warp_mark_late(smem_u32((const void*)late), spin);
     __syncwarp();
     warp_arrive(&red_full[rb]);
     ++item;
@@ -919,14 +924,17 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
 
   if (S > 1) {
     // ---- split K: whichever CTA of an item stream finishes last adds the slice sums of the stream's items, in
-    // slice order (so the result does not depend on who that is), and leaves the counter at zero ---------------
+    // slice order (so the result does not depend on who that is), and leaves the counter at zero.  A CTA that is late counts
+    // 256 times its arrival: the sums of its stream are not stored, whoever finishes last -----------------------
     __shared__ int last_flag;
     named_bar_sync(4, kQ8Consumers + 32 * kQ8Reducers);      // the reducing warps have written the CTA's slice sums
     if (tid == 0) {
       __threadfence();
-      const int old = atomicAdd(lay.counters + r0, 1);
-      last_flag = old == S - 1;
-      if (last_flag) lay.counters[r0] = 0;
+      const int mine = *late != 0u ? 257 : 1;
+      const int all = atomicAdd(lay.counters + r0, mine) + mine;
+      const bool last = (all & 255) == S;
+      last_flag = last && all == S;
+      if (last) lay.counters[r0] = 0;
     }
     named_bar_sync(1, kQ8Consumers);
     if (last_flag) {

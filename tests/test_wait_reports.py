@@ -34,7 +34,7 @@ def test_a_silent_wait_is_found():
     assert silent_waits("  for (;;)\n    if (!warp_wait(&full[i], 0, spin)) break;\n  }\n  next();\n  done();\n") == [2]
 
 
-@pytest.mark.parametrize("name", ["hq_dq_gemm.cuh", "hq_fp8_grouped.cu", "hq_mx_grouped.cu"])
+@pytest.mark.parametrize("name", ["hq_dq_gemm.cuh", "hq_fp8_grouped.cu", "hq_mx_grouped.cu", "hq_mx_rows.cu"])
 def test_copies_are_waited_for_by_the_warps_that_issue_them(name):
     # after a time-out nobody else waits for a stage any more: the rings box copies signal are drained before the CTA exits,
     # by warp_drain or by a loop over the last stages of the sequence
@@ -61,3 +61,27 @@ def test_a_limit_of_long_polls_is_not_used_with_short_ones(name):
 def test_a_short_wait_is_found():
     assert short_waits("constexpr uint32_t kSpin = 1u << 16;\n  if (!mbar_wait_backoff(&empty[s], 0, spin)) {\n") != []
     assert short_waits("constexpr uint32_t kSpin = 1u << 22;\n  if (!mbar_wait(&empty[s], 0, spin)) {\n") == []
+
+
+def unmarked(text):
+    """Waits of a role that hands its work on whether or not they ran out (`spin` becomes 0 or 1 and the loop goes on), in a kernel
+    that keeps a `late` word, without the word being set: (waits with a branch, waits by value whose role has no mark)."""
+    code = "\n".join(line.split("//")[0] for line in text.split("\n"))
+    branches = [b for b in re.findall(r"if \([^;{]*!warp_wait\([^{]*\{(.*?)\n\s*\}", code, re.S)
+                if "spin = 1" in b and "late = 1u" not in b and "failed = true" not in b]
+    roles = re.split(r"\n(?=[^\n]*={20,})", "\n".join(text.split("\n")))
+    by_value = [r[:60] for r in roles if "spin = warp_wait_uni(" in r and "warp_mark_late(" not in r]
+    return branches, by_value
+
+
+@pytest.mark.parametrize("name", ["hq_gemv.cu", "hq_gemv_int8.cu", "hq_mx_rows.cu", "hq_mx_grouped.cu"])
+def test_what_a_late_warp_hands_on_is_not_stored(name):
+    text = open(os.path.join(CSRC, name)).read()
+    assert unmarked(text) == ([], [])
+    assert len(re.findall(r"failed = failed \|\| \*(?:\(volatile uint32_t\*\))?late != 0u;", text)) == 1
+
+
+def test_a_missing_mark_is_found():
+    role = "// ===================== consumers\n  spin = warp_wait_uni(b, 0, spin) ? spin : 0u;\n  warp_arrive(&full);\n"
+    assert unmarked(role)[1] != []
+    assert unmarked("  if (!warp_wait(&empty[s], 0, spin)) {\n    report_status(s, 1, 2);\n    spin = 1;\n  }\n")[0] != []
