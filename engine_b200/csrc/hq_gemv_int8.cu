@@ -151,6 +151,14 @@ struct Q8XPrefetch {
   uint4 v[kQ8XGroups];
 };
 
+// Activations come from L2, not through L1 or the read-only path: a kPdlNext launch starts before it has waited for anything, and
+// what it reads was written by a kernel further up than the one whose completion releases it.  (Nothing is lost: a CTA reads a
+// row once, and the ring leaves L1 hardly any room.)
+__device__ __forceinline__ uint4 q8_load_x(const char* src) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src) : "memory");
+  return v;
+}
 __device__ __forceinline__ void q8_x_prefetch(Q8XPrefetch& pf, const GemvParams& p, int row0, int nrows, int k0,
                                               int k_len, int tid) {
   const bool wide = p.x_dtype == HQ_DT_F32;
@@ -166,10 +174,10 @@ __device__ __forceinline__ void q8_x_prefetch(Q8XPrefetch& pf, const GemvParams&
       const int64_t xr = p.x_rows ? (int64_t)p.x_rows[row0 + col] : (int64_t)(row0 + col);
       const char* src = (const char*)p.x + (xr * p.x_stride + k0 + kk) * (wide ? 4 : 2);
       if (wide) {
-        pf.v[(2 * i) % kQ8XGroups] = __ldg(reinterpret_cast<const uint4*>(src));
-        pf.v[(2 * i + 1) % kQ8XGroups] = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+        pf.v[(2 * i) % kQ8XGroups] = q8_load_x(src);
+        pf.v[(2 * i + 1) % kQ8XGroups] = q8_load_x(src + 16);
       } else {
-        pf.v[i] = __ldg(reinterpret_cast<const uint4*>(src));
+        pf.v[i] = q8_load_x(src);
       }
     }
   }

@@ -49,3 +49,41 @@ def test_a_run_of_projections_is_the_separate_calls(fmts, m):
         outs = hq.try_fused_quantized_qkv(x, *layers, out_dtype=torch.float32)
         for o, layer in zip(outs, layers):
             assert torch.equal(o, layer.forward_raw(x, torch.float32))
+
+
+@pytest.mark.parametrize("fmt", ["Q8_0", "Q4_K", "FP8"])
+@pytest.mark.parametrize("m", [1, 2])
+def test_a_run_reads_what_the_launch_before_it_wrote(fmt, m):
+    # one activation buffer, written anew in place before every run: by torch, then by a projection of this library, whose launch
+    # the run's first one follows programmatically; no synchronisation in between
+    import engine_b200 as hq
+    from engine_b200 import _lib as L
+    import ctypes as C
+    rng = T.rng_for(13, 21)
+    k = 2048
+    o, q, kk, v = [T.make_layer(fmt, T.make_weight(fmt, rng, n, k)[0], k, DEV) for n in (k, 2048, 256, 384)]
+    steps = 40
+    inputs = T.to_dev(rng.standard_normal((steps, m, k)).astype(np.float32), torch.float32, DEV)
+    want = []
+    for i in range(steps):
+        x = o.forward_raw(inputs[i], torch.float32)
+        torch.cuda.synchronize()
+        want.append([layer.forward_raw(x, torch.float32) for layer in (q, kk, v)])
+        torch.cuda.synchronize()
+    x = torch.empty((m, k), dtype=torch.float32, device=DEV)
+    w, stream = o._weight_struct(), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    got = []
+    for i in range(steps):
+        L.check(L.lib().hq_linear_forward(C.byref(w), C.c_void_p(inputs[i].data_ptr()), L.DT_F32, k, C.c_void_p(x.data_ptr()), L.DT_F32,
+                                          k, m, None, stream), "hq_linear_forward")
+        got.append(hq.try_fused_quantized_qkv(x, q, kk, v, out_dtype=torch.float32))
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        for s, t in zip(a, b):
+            assert torch.equal(s, t)
+    for i in range(steps):
+        x.copy_(inputs[i])
+        got[i] = hq.try_fused_quantized_qkv(x, q, kk, v, out_dtype=torch.float32)
+    for i in range(steps):
+        for s, layer in zip(got[i], (q, kk, v)):
+            assert torch.equal(s, layer.forward_raw(inputs[i], torch.float32))
