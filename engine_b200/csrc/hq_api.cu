@@ -448,7 +448,6 @@ int32_t hq_moe_gather_forward(const hq_weight* w, const hq_weight* w_up, const h
   p.y_stride = (has_act && w_up == nullptr) ? w->n / 2 : w->n;
   p.tiles = ws;
   p.tile_rows = l.tile_rows;
-  p.expert_bounds = expert_bounds;
   p.x_rows = x_rows;
   p.y_rows = y_rows;
   if (has_act) p.act = *act; else p.act.act = HQ_ACT_NONE;
@@ -914,7 +913,6 @@ void fill_mx_rows(MxRowsParams& g, const hq_weight* w, int terms, const uint8_t*
                   int y_dtype, int64_t y_stride, const int32_t* bounds, int32_t* status) {
   g.n = (int)w->n;
   g.k = (int)w->k;
-  g.m = (int)rows;
   g.n_experts = w->n_experts;
   g.w = w->data;
   g.w_scales = (const uint8_t*)w->scales;

@@ -39,7 +39,6 @@ struct GemvParams {
   // expert-indexed mode: work items of <= tile_rows sorted rows of one expert
   int tile_rows;                // 4 or 8
   const int32_t* tiles;         // the dispatch workspace with its work items (hq_work_items.h)
-  const int32_t* expert_bounds; // [E+1]
   const int32_t* x_rows;        // sorted row -> activation row (nullptr = identity)
   const int32_t* y_rows;        // sorted row -> output row (nullptr = identity)
   hq_act_args act;
@@ -129,7 +128,7 @@ int32_t launch_fp8_grouped(const Fp8GroupedParams& p, cudaStream_t stream);
 
 // ---- MXFP4 weights against few rows, three or four e5m2 terms per activation, on the block-scaled MMA (hq_mx_rows.cu) -----
 struct MxRowsParams {
-  int n, k, m;                  // m: dense rows (used when expert_bounds == nullptr)
+  int n, k;
   int n_experts;
   const void* w;                // packed e2m1 nibbles [E, N, K/2]
   const uint8_t* w_scales;      // e8m0 [E, N, K/32]
@@ -144,7 +143,6 @@ struct MxRowsParams {
   int64_t y_stride;
   hq_act_args act;
   const int32_t* expert_bounds; // [E+1]
-  const int32_t* y_rows;        // sorted row -> output row (nullptr = identity)
   int32_t* status;
 };
 int mx_terms(int x_dtype);       // 3 for 16-bit types, 4 for f32

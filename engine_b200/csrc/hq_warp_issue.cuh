@@ -141,6 +141,29 @@ __device__ __forceinline__ void warp_tma_2d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
+// K-major operand tile of 128-byte rows, 128-byte swizzle, 8-row groups 1024 bytes apart, descriptor version 1
+__device__ __forceinline__ uint64_t mx_smem_desc(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr >> 4) & 0x3FFFu);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+// block-scaled products, kind::mxf8f6f4: one MMA of K = 32
+__device__ __forceinline__ void warp_mx_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t sfa,
+                                            uint32_t sfb, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, e;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "setp.ne.b32 p, %6, 0;\n"
+      "@e tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], %1, %2, %3, [%4], [%5], p;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
+      : "memory");
+}
 // 128 k of block-scaled products, kind::mxf8f6f4: four MMAs of K = 32, 32 bytes along the swizzled rows of both operands and one
 // scale byte (instruction descriptor bits [4,6) of B, [29,31) of A) apart.  One election for the four: with one each, and their
 // operands made one by one, an MMA took 101 to 140 cycles to issue where the tensor core needs 44 (48 columns) to 96 (192).
