@@ -103,7 +103,7 @@ def test_values_that_are_not_finite_are_the_same_in_any_batch(dtype, limit):
     few = experts.forward_layer(x[:t], logits[:t], rcfg, out_dtype=torch.float32).cpu().numpy()
     many = experts.forward_layer(x, logits, rcfg, out_dtype=torch.float32)[:t].cpu().numpy()
     assert experts.gate_up.device_status()[0] == 0
-    assert np.isfinite(many).all() == limit
+    assert np.isfinite(many[[0, 6]]).all() and np.isfinite(many[1]).all() == limit
     for row in range(t):
         ok = np.isfinite(many[row])
         assert np.array_equal(np.isnan(few[row]), np.isnan(many[row])), row
