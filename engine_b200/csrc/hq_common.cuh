@@ -90,6 +90,18 @@ __device__ __forceinline__ void bulk_g2s_hint(void* dst_smem, const void* src_gm
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+inline int sm_count() {
+  static int cached[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 148;
+  if (cached[dev] == 0) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    cached[dev] = n;
+  }
+  return cached[dev];
+}
+
 // launch of a kernel that calls pdl_wait() before it touches memory, in clusters of `cluster` blocks
 template <typename... K, typename... A>
 inline int32_t launch_pdl(void (*kern)(K...), dim3 grid, int threads, size_t smem, cudaStream_t stream, int cluster,

@@ -300,9 +300,9 @@ int32_t launch_fp8_quant_rows(const void* x, int x_dtype, int64_t x_stride, cons
                               const int32_t* n_valid, int64_t n_rows, int64_t k, uint8_t* codes, float* scales,
                               cudaStream_t stream) {
   if (n_rows == 0) return HQ_OK;
-  // four loads a warp where that leaves half of the chip's 148 x 64 warps or more something to do.  One load against four, bf16:
+  // four loads a warp where that leaves half of the chip's warps (64 an SM) or more something to do.  One load against four, bf16:
   // 512 x 7,168 (14,336 loads) 4.9 us against 5.8, 1,024 x 7,168 (28,672) 8.9 against 8.2, 4,096 x 7,168 30.8 against 24.8
-  const bool wide = n_rows * (k / 256) >= 2 * 148 * 64;
+  const bool wide = n_rows * (k / 256) >= 2 * (int64_t)sm_count() * 64;
 #define HQ_FQ(T) \
   return wide ? launch_fq<T, 4>(x, x_stride, row_map, n_valid, n_rows, k, codes, scales, stream) \
               : launch_fq<T, 1>(x, x_stride, row_map, n_valid, n_rows, k, codes, scales, stream)

@@ -128,17 +128,6 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-inline int sm_count() {
-  static int cached[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 148;
-  if (cached[dev] == 0) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    cached[dev] = n;
-  }
-  return cached[dev];
-}
 
 // the Q6_K / Q5_K / Q4_0 / Q5_0 decode kernel on warp MMAs (hq_gemv_ggml_mma.cu)
 int32_t launch_gemv_ggml_mma(const GemvParams& p, int n_y_max, cudaStream_t stream);
