@@ -266,12 +266,10 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   uint64_t* empty = full + kMaxStages;
   uint64_t* red_full = empty + kMaxStages;   // [2] partial sums of an item are all written
   uint64_t* red_free = red_full + 2;     // [2] ... and have been consumed
-  volatile uint32_t* late = reinterpret_cast<uint32_t*>(red_free + 2);   // a copying or consumer warp's wait ran out: nothing more is stored
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
-    *late = 0u;
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(&full[s], kProducerWarps);
       mbar_init(&empty[s], kConsumerWarps);
@@ -309,10 +307,9 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
         for (int bank = 0; bank < p.n_banks; ++bank) {
           if (round > 0) {
             if (!warp_wait(&empty[s], (round - 1) & 1, spin)) {
-              // give up waiting but keep the control flow intact: what is copied over is never stored
+              // nothing more is copied (the stage may still be in use): the consumers' waits run out
               if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 100 + s);
-              *late = 1u;
-              spin = 1;
+              return;
             }
           }
           const uint8_t* wsrc = reinterpret_cast<const uint8_t*>(bank == 0 ? p.w : p.w_up) +
@@ -340,19 +337,18 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
     // ================= reducing warp: adds the K-split partial sums in warp order and writes ==========
     pdl_wait();
     uint32_t spin = kSpinLimit;
+    bool failed = false;
     int item = 0;
     for (int w = w_begin; w < w_end; w += w_step) {
       const WorkItem wi = get_item<RT>(p, w, n_rt, rows_at);
       if (wi.nrows <= 0) continue;
       const int rb = item & 1;
       const float* rbuf = red + rb * (p.n_banks * kConsumerWarps * 4 * 32);
-      bool failed = false;
       if (!warp_wait(&red_full[rb], (item >> 1) & 1, spin)) {
         if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 310 + rb);
         spin = 1;
-        failed = true;                 // nothing is stored for an item whose partial sums never arrived
+        failed = true;                 // nothing is stored from an item on whose partial sums never arrived
       }
-      failed = failed || *late != 0u;
       float v[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
       for (int b = 0; b < 2; ++b)
@@ -393,7 +389,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
   }
 
   // (a wait that runs out makes `spin` 0: the waits left poll once, every warp still reaches every barrier, and it is reported
-  // at the end; `late` keeps the sums handed over from being stored)
+  // at the end; a warp that was late hands over nothing more, so the reducing warp's wait runs out and nothing is stored)
   uint32_t spin = kSpinLimit;
   int s = 0, item = 0, wrot = wk;
   uint32_t phase = 0;
@@ -502,9 +498,8 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_kernel(const GemvParams 
 #pragma unroll
         for (int i = 0; i < 4; ++i) rbuf[((b * kConsumerWarps + warp) * 4 + i) * 32 + lane] = acc[b][i];
       }
-    warp_mark_late(smem_u32((const void*)late), spin);
     __syncwarp();
-    if (lane == 0) mbar_arrive(&red_full[rb]);
+    if (lane == 0 && spin != 0u) mbar_arrive(&red_full[rb]);
     ++item;
   }
   if (spin == 0u && lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 200);

@@ -151,16 +151,22 @@ struct Q8XPrefetch {
   uint4 v[kQ8XGroups];
 };
 
-// Activations come from L2, not through L1 or the read-only path: a kPdlNext launch starts before it has waited for anything, and
-// what it reads was written by a kernel further up than the one whose completion releases it.  (Nothing is lost: a CTA reads a
-// row once, and the ring leaves L1 hardly any room.)
-__device__ __forceinline__ uint4 q8_load_x(const char* src) {
-  uint4 v;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src) : "memory");
-  return v;
-}
-__device__ __forceinline__ void q8_x_prefetch(Q8XPrefetch& pf, const GemvParams& p, int row0, int nrows, int k0,
-                                              int k_len, int tid) {
+// A kPdlNext launch reads activations from L2 and not through the read-only path: it starts before it has waited for anything, and
+// what it reads was written by a kernel further up than the one whose completion releases it.  (Such loads for every launch cost
+// the 64-token Q4_K layer 1 %.)
+struct Q8LoadL2 {
+  __device__ __forceinline__ uint4 operator()(const char* src) const {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src) : "memory");
+    return v;
+  }
+};
+struct Q8LoadReadOnly {
+  __device__ __forceinline__ uint4 operator()(const char* src) const { return __ldg(reinterpret_cast<const uint4*>(src)); }
+};
+template <typename LOAD>
+__device__ __forceinline__ void q8_x_fetch(Q8XPrefetch& pf, const GemvParams& p, int row0, int nrows, int k0, int k_len, int tid,
+                                           LOAD load) {
   const bool wide = p.x_dtype == HQ_DT_F32;
   const int ipr = k_len >> 3;            // items per activation row in this epoch
   const int nitems = nrows * ipr;
@@ -174,13 +180,17 @@ __device__ __forceinline__ void q8_x_prefetch(Q8XPrefetch& pf, const GemvParams&
       const int64_t xr = p.x_rows ? (int64_t)p.x_rows[row0 + col] : (int64_t)(row0 + col);
       const char* src = (const char*)p.x + (xr * p.x_stride + k0 + kk) * (wide ? 4 : 2);
       if (wide) {
-        pf.v[(2 * i) % kQ8XGroups] = q8_load_x(src);
-        pf.v[(2 * i + 1) % kQ8XGroups] = q8_load_x(src + 16);
+        pf.v[(2 * i) % kQ8XGroups] = load(src);
+        pf.v[(2 * i + 1) % kQ8XGroups] = load(src + 16);
       } else {
-        pf.v[i] = q8_load_x(src);
+        pf.v[i] = load(src);
       }
     }
   }
+}
+__device__ __forceinline__ void q8_x_prefetch(Q8XPrefetch& pf, const GemvParams& p, int row0, int nrows, int k0, int k_len, int tid) {
+  if (p.pdl == kPdlNext) q8_x_fetch(pf, p, row0, nrows, k0, k_len, tid, Q8LoadL2{});
+  else q8_x_fetch(pf, p, row0, nrows, k0, k_len, tid, Q8LoadReadOnly{});
 }
 
 // k_len is a multiple of 256, so a warp never straddles two activation rows and is valid or idle as a whole.
@@ -631,7 +641,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
   uint64_t* empty = full + kQ8MaxStages;
   uint64_t* red_full = empty + kQ8MaxStages;   // [2] partial sums of an item are all written
   uint64_t* red_free = red_full + 2;           // [2] ... and have been consumed
-  volatile uint32_t* late = reinterpret_cast<uint32_t*>(red_free + 2);   // a copying or consumer warp's wait ran out: nothing more is stored
+  volatile uint32_t* late = reinterpret_cast<uint32_t*>(red_free + 2);   // split K: the reducing warps stored not all of their sums
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
 
@@ -673,22 +683,23 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
     uint64_t policy;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
     int s = 0, round = 0;
+    bool stop = false;
     WorkItem wi = get_item<RT>(p, w_begin, n_rt, rows_at), nx;
-    for (int w = w_begin; w < w_end; w += w_step, wi = nx) {
+    for (int w = w_begin; w < w_end && !stop; w += w_step, wi = nx) {
       nx = get_item<RT>(p, min(w + w_step, total - 1), n_rt, rows_at);      // fetched an item ahead
       if (wi.nrows <= 0) continue;
       const int rows_valid = min(RT, p.n - wi.n0);
       const int my_rows = max(0, min(RPP, rows_valid - pw * RPP));
-      for (int chunk = 0; chunk < nchunk; ++chunk) {
+      for (int chunk = 0; chunk < nchunk && !stop; ++chunk) {
         const int kc_len = min(KC, k_hi - (k_lo + chunk * KC));
         const uint32_t bytes = (uint32_t)T::row_bytes(kc_len);
         for (int bank = 0; bank < p.n_banks; ++bank) {
           if (round > 0) {
             if (!warp_wait(&empty[s], (round - 1) & 1, spin)) {
-              // give up waiting but keep the control flow intact: what is copied over is never stored
+              // nothing more is copied (the stage may still be in use): the consumers' waits run out
               if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 100 + s);
-              *late = 1u;
-              spin = 1;
+              stop = true;
+              break;
             }
           }
           const uint8_t* wsrc = reinterpret_cast<const uint8_t*>(bank == 0 ? p.w : p.w_up) +
@@ -716,6 +727,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
     const int row = g + 8 * (vi >> 1), col = 2 * t + (vi & 1);
     const bool owner = NCS > 1 || t < (FMT == HQ_FMT_FP8_BLOCK ? 1 : 2);
     uint32_t spin = kQ8Spin;
+    bool failed = false;
     int item = 0;
     WorkItem wi = get_item<RT>(p, w_begin, n_rt, rows_at), nx;
     for (int w = w_begin; w < w_end; w += w_step, wi = nx) {
@@ -726,13 +738,12 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
       const bool mine = owner && col < wi.nrows;
       int64_t yrow = wi.row0 + col;
       if (mine && p.y_rows != nullptr && S == 1) yrow = p.y_rows[wi.row0 + col];
-      bool failed = false;
       if (!warp_wait(&red_full[rb], (item >> 1) & 1, spin)) {
         if (lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 310 + rb);
         spin = 1;
-        failed = true;                 // nothing is stored for an item whose partial sums never arrived
+        failed = true;                 // nothing is stored from an item on whose partial sums never arrived
+        *late = 1u;
       }
-      failed = failed || *late != 0u;
       WorkItem ti = wi;
 #pragma unroll 1
       for (int rt = 0; rt < RS; ++rt, ti.n0 += kQ8RT) {
@@ -802,7 +813,7 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
   }
 
   // (a wait that runs out makes `spin` 0: the waits left poll once, every warp still reaches every barrier, and it is reported
-  // at the end; `late` keeps the sums handed over from being stored)
+  // at the end; a warp that was late hands over nothing more, so the reducing warps' waits run out and nothing is stored)
   uint32_t spin = kQ8Spin;
   int s = 0, item = 0;
   uint32_t phase = 0;
@@ -922,9 +933,8 @@ __global__ void __launch_bounds__(kQ8Threads, 1) gemv_int8_kernel(const GemvPara
           rbuf[((b * WK + warp) * 4 + i) * 32 + lane] = sum;
         }
       }
-    warp_mark_late(smem_u32((const void*)late), spin);
     __syncwarp();
-    warp_arrive(&red_full[rb]);
+    warp_arrive_live(&red_full[rb], spin);
     ++item;
   }
   if (spin == 0u && lane == 0) report_status(p.status, HQ_DEV_WAIT_TIMEOUT, 200);

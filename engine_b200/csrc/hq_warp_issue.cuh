@@ -108,6 +108,19 @@ __device__ __forceinline__ void warp_arrive_at(uint32_t bar) {
       : "memory");
 }
 __device__ __forceinline__ void warp_arrive(uint64_t* bar) { warp_arrive_at(smem_u32(bar)); }
+// The same by a warp that keeps its waits' outcome in `spin` (warp_wait_uni): once one has run out it arrives no more, so whoever
+// would take what it hands on runs out too, and stores nothing.  (A word of shared memory that the storing warps looked at per
+// item cost the 64-token Q4_K layer 1 %.)
+__device__ __forceinline__ void warp_arrive_live(uint64_t* bar, uint32_t spin) {
+  asm volatile(
+      "{\n"
+      ".reg .pred e, q;\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "setp.ne.and.u32 q, %1, 0, e;\n"
+      "@q mbarrier.arrive.shared::cta.b64 _, [%0];\n"
+      "}\n" ::"r"(smem_u32(bar)), "r"(spin)
+      : "memory");
+}
 __device__ __forceinline__ void warp_arrive_expect(uint64_t* bar, uint32_t bytes) {
   asm volatile(
       "{\n"
