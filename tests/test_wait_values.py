@@ -1,4 +1,4 @@
-"""Waits that leave no branch behind (warp_wait_uni) return the polls that were left; a caller keeps the value in `spin`, where 0
+"""Waits that leave no branch behind (warp_wait_uni) return 1, or 0 when they ran out; a caller keeps that in `spin`, where 0
 says that a wait ran out, and reports that behind its loop.  Read from the source, as the waits with a branch are."""
 import os
 import re
