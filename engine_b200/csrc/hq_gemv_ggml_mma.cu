@@ -419,8 +419,7 @@ __global__ void __launch_bounds__(kGmThreads, 3) gemv_ggml_mma_kernel(const Gemv
   pdl_launch_dependents();
   const int n_rt = (p.n + kGmRows - 1) / kGmRows;
   const int n_y = p.tiles != nullptr ? p.tiles[0] : (p.m + 7) / 8;
-  // (not kept: at 80 registers one more costs a dense block of Q4_K_M 1.4 %)
-  auto rows_of = [&]() { return p.tiles != nullptr ? p.tiles[kHeaderRowsAt] : 0; };
+  const int rows_at = p.tiles != nullptr ? p.tiles[kHeaderRowsAt] : 0;
   const int total = n_y * n_rt;
   const int spans = p.k / 256;
   const int64_t row_bytes = (int64_t)spans * F::SPAN;
@@ -431,12 +430,12 @@ __global__ void __launch_bounds__(kGmThreads, 3) gemv_ggml_mma_kernel(const Gemv
   // One commit group per step, empty once the walk is over (or for a warp without spans), so that the group count
   // stays in step with the waits.
   auto next_item = [&](int w) {
-    while (w < total && get_item<kGmRows>(p, w, n_rt, rows_of()).nrows <= 0) w += (int)gridDim.x;
+    while (w < total && get_item<kGmRows>(p, w, n_rt, rows_at).nrows <= 0) w += (int)gridDim.x;
     return w;
   };
   int iw = warp < spans ? next_item((int)blockIdx.x) : total;
   int ispan = warp, ibank = 0, islot = 0;
-  WorkItem iwi = iw < total ? get_item<kGmRows>(p, iw, n_rt, rows_of()) : WorkItem{};
+  WorkItem iwi = iw < total ? get_item<kGmRows>(p, iw, n_rt, rows_at) : WorkItem{};
   auto issue = [&]() {
     if (iw < total) {
       const int r = lane >> 1;
@@ -457,7 +456,7 @@ __global__ void __launch_bounds__(kGmThreads, 3) gemv_ggml_mma_kernel(const Gemv
         if (ispan >= spans) {
           ispan = warp;
           iw = next_item(iw + (int)gridDim.x);
-          if (iw < total) iwi = get_item<kGmRows>(p, iw, n_rt, rows_of());
+          if (iw < total) iwi = get_item<kGmRows>(p, iw, n_rt, rows_at);
         }
       }
     }
@@ -470,7 +469,7 @@ __global__ void __launch_bounds__(kGmThreads, 3) gemv_ggml_mma_kernel(const Gemv
   int cslot = 0, item = 0;
   bool clamped = false;
   for (int w = blockIdx.x; w < total; w += gridDim.x) {
-    const WorkItem wi = get_item<kGmRows>(p, w, n_rt, rows_of());
+    const WorkItem wi = get_item<kGmRows>(p, w, n_rt, rows_at);
     if (wi.nrows <= 0) continue;                                 // the same for every thread of the CTA
     float acc[BANKS][4];
 #pragma unroll

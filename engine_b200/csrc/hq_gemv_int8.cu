@@ -151,22 +151,17 @@ struct Q8XPrefetch {
   uint4 v[kQ8XGroups];
 };
 
-// A kPdlNext launch reads activations from L2 and not through the read-only path: it starts before it has waited for anything, and
-// what it reads was written by a kernel further up than the one whose completion releases it.  (Such loads for every launch cost
-// the 64-token Q4_K layer 1 %.)
-struct Q8LoadL2 {
-  __device__ __forceinline__ uint4 operator()(const char* src) const {
-    uint4 v;
-    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src) : "memory");
-    return v;
-  }
-};
-struct Q8LoadReadOnly {
-  __device__ __forceinline__ uint4 operator()(const char* src) const { return __ldg(reinterpret_cast<const uint4*>(src)); }
-};
-template <typename LOAD>
-__device__ __forceinline__ void q8_x_fetch(Q8XPrefetch& pf, const GemvParams& p, int row0, int nrows, int k0, int k_len, int tid,
-                                           LOAD load) {
+// Activations come from L2, not through the read-only path: a kPdlNext launch starts before it has waited for anything, and what it
+// reads was written by a kernel further up than the one whose completion releases it.  (Volatile keeps the loads behind
+// pdl_wait; no memory clobber, or every row number waits for the values before it.  4,096 x 4,096 Q4_K at one row 6.04 us, 6.08
+// through the read-only path; the 64-token Q4_K layer 154.5 : 152.4 with all that keeps late sums from being stored.)
+__device__ __forceinline__ uint4 q8_load_x(const char* src) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src));
+  return v;
+}
+__device__ __forceinline__ void q8_x_prefetch(Q8XPrefetch& pf, const GemvParams& p, int row0, int nrows, int k0,
+                                              int k_len, int tid) {
   const bool wide = p.x_dtype == HQ_DT_F32;
   const int ipr = k_len >> 3;            // items per activation row in this epoch
   const int nitems = nrows * ipr;
@@ -180,17 +175,13 @@ __device__ __forceinline__ void q8_x_fetch(Q8XPrefetch& pf, const GemvParams& p,
       const int64_t xr = p.x_rows ? (int64_t)p.x_rows[row0 + col] : (int64_t)(row0 + col);
       const char* src = (const char*)p.x + (xr * p.x_stride + k0 + kk) * (wide ? 4 : 2);
       if (wide) {
-        pf.v[(2 * i) % kQ8XGroups] = load(src);
-        pf.v[(2 * i + 1) % kQ8XGroups] = load(src + 16);
+        pf.v[(2 * i) % kQ8XGroups] = q8_load_x(src);
+        pf.v[(2 * i + 1) % kQ8XGroups] = q8_load_x(src + 16);
       } else {
-        pf.v[i] = load(src);
+        pf.v[i] = q8_load_x(src);
       }
     }
   }
-}
-__device__ __forceinline__ void q8_x_prefetch(Q8XPrefetch& pf, const GemvParams& p, int row0, int nrows, int k0, int k_len, int tid) {
-  if (p.pdl == kPdlNext) q8_x_fetch(pf, p, row0, nrows, k0, k_len, tid, Q8LoadL2{});
-  else q8_x_fetch(pf, p, row0, nrows, k0, k_len, tid, Q8LoadReadOnly{});
 }
 
 // k_len is a multiple of 256, so a warp never straddles two activation rows and is valid or idle as a whole.

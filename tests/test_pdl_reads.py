@@ -10,6 +10,5 @@ def test_a_run_of_projections_reads_its_activations_from_l2():
     with open(os.path.join(ROOT, "engine_b200", "csrc", "hq_gemv_int8.cu")) as f:
         text = f.read()
     body = re.search(r"void q8_x_prefetch\(.*?\n}\n", text, re.S).group(0)
-    assert "if (p.pdl == kPdlNext) q8_x_fetch(pf, p, row0, nrows, k0, k_len, tid, Q8LoadL2{});" in body
-    assert "__ldg" not in re.search(r"void q8_x_fetch\(.*?\n}\n", text, re.S).group(0)
-    assert "ld.relaxed.gpu.global" in re.search(r"struct Q8LoadL2 .*?\n};\n", text, re.S).group(0)
+    assert "q8_load_x(" in body and "__ldg" not in body
+    assert "asm volatile(\"ld.relaxed.gpu.global" in re.search(r"uint4 q8_load_x\(.*?\n}\n", text, re.S).group(0)
