@@ -18,8 +18,8 @@ def test_tables_around_the_line(t, k, e):
     tables_match(t, k, e)
 
 
-# the tables' histogram of 319 .. 332 experts fits 48 KiB of shared memory, but not beside what the kernel declares
-@pytest.mark.parametrize("e", [318, 319, 320, 332, 333])
+# the tables' histogram of 318 .. 332 experts fits 48 KiB of shared memory, but not beside what the kernel declares
+@pytest.mark.parametrize("e", [317, 318, 320, 332, 333])
 @pytest.mark.parametrize("t", [4, 64])
 def test_tables_around_48_kib(t, e):
     tables_match(t, 8, e)
